@@ -115,9 +115,12 @@ int nbg_batch_destroy(nbg_batch *bt);
  * with pointwise product, 2 reverse pass, 3 unpack, 4 carry, 5 carries through
  * runs of all-ones limbs, 6 the last pass with one CTA per prime, 7 the last
  * pass of products with a kept operand spectrum, 8 and 9 the forward and
- * reverse column passes with tiles staged by TMA), jobs, and the
- * algorithmic FP64 instruction count and compulsory bytes of the reference
- * schedule for that launch.  Any output pointer may be NULL. */
+ * reverse column passes with tiles staged by TMA; products through 30-bit
+ * primes, see nbg_set_tuning: 10 forward column passes, 11 blocks, 12 reverse
+ * column passes, 13 unpack), jobs, and the
+ * algorithmic FP64 instruction count (zero for kinds 10 to 13) and compulsory
+ * bytes of the reference schedule for that launch.  Any output pointer may be
+ * NULL. */
 int nbg_batch_stats(const nbg_batch *bt, int32_t *kinds, int64_t *njobs, double *alg_ops, double *alg_bytes,
                     int32_t cap);
 /* Runs the batch's launches one by one (not as a graph) on `stream` with a
@@ -286,7 +289,11 @@ int nbg_plan_layout(int64_t N, int32_t sqr, int64_t *stages, int32_t *nst, int64
  * "overrides": a list of
  * {"N", "sqr", "pass_ends": [last stage of each pass], "tile_target", "cmax"}
  * giving an explicit pass split per transform class).  Changing them drops
- * cached plans. */
+ * cached plans.  The knobs describe the FP64 passes.  While they are the ones
+ * the library started with or loaded from a tuning file, products within its
+ * range run through transforms over 30-bit primes instead, which have no knobs;
+ * with other knobs every product runs the FP64 passes they describe.  The
+ * results are the same integers. */
 int nbg_set_tuning(const char *json);
 /* Current tuning as a JSON object into buf (NUL-terminated). */
 int nbg_get_tuning(char *buf, int64_t cap);

@@ -426,9 +426,22 @@ int host_batch(const nbg_desc* descs, int64_t count) {
 // Reads the operands' top limbs on the device (magnitude_bits) for
 // descriptors that leave bits_a / bits_b at 0.
 int fill_bits_dev(std::vector<ProdIn>& in, cudaStream_t st) {
+    // word products are sized by limb counts: only a one-limb operand needs its
+    // bits read (a zero there is refused)
+    auto unread = [](int64_t bits, int64_t limbs, bool word) { return bits <= 0 && !(word && limbs > 1); };
     std::vector<int64_t> need;
-    for (size_t k = 0; k < in.size(); k++)
-        if (in[k].bits_a <= 0 || (!in[k].sqr && in[k].bits_b <= 0)) need.push_back((int64_t)k);
+    for (size_t k = 0; k < in.size(); k++) {
+        ProdIn& q = in[k];
+        WordShape ws;
+        const bool word = word_product(g_eng, q, &ws);
+        if (unread(q.bits_a, q.m, word) || (!q.sqr && unread(q.bits_b, q.n, word))) {
+            need.push_back((int64_t)k);
+        } else {
+            if (q.bits_a <= 0) q.bits_a = 64 * q.m;
+            if (q.sqr) q.bits_b = q.bits_a;
+            else if (q.bits_b <= 0) q.bits_b = 64 * q.n;
+        }
+    }
     if (need.empty()) return NBG_OK;
     Engine& E = g_eng;
     std::vector<DProd> tmp(need.size());
@@ -528,7 +541,7 @@ int load_tuning_file(const char* path) {
     if (ob == std::string::npos) return fail(NBG_EINVAL, "tuning file %s malformed", path);
     int rc = g_eng.tun.from_json(js.c_str() + ob);
     if (rc) return rc;
-    g_eng.drop_plans();
+    g_eng.tuning_changed(true);
     return NBG_OK;
 }
 
@@ -845,14 +858,12 @@ int nbg_batch_profile(nbg_batch* bt, void* stream, float* ms, int32_t cap) {
     const auto& ls = bt->bb.launches;
     std::vector<cudaEvent_t> ev(ls.size() + 1);
     for (auto& e : ev) CUDA_TRY(cudaEventCreate(&e));
-    const DProd* prods = (const DProd*)(bt->dmem + bt->bb.off_prods);
-    const Job* jobs = (const Job*)(bt->dmem + bt->bb.off_joblist);
     CUDA_TRY(expand_jobs(bt->bb, bt->dmem, st));
     int rc = NBG_OK;
     CUDA_TRY(cudaEventRecord(ev[0], st));
     for (size_t i = 0; i < ls.size(); i++) {
         const Launch& L = ls[i];
-        cudaError_t e = launch_jobs(L.kind, prods, g_eng.d_plans, job_list(jobs + L.off), L.n, L.smem, 0, st, L.odd);
+        cudaError_t e = launch_one(g_eng, bt->bb, L, bt->dmem, st);
         if (e != cudaSuccess) { rc = fail(NBG_ECUDA, "profile launch: %s", cudaGetErrorString(e)); break; }
         g_launches++;
         CUDA_TRY(cudaEventRecord(ev[i + 1], st));
@@ -1010,7 +1021,7 @@ int nbg_set_tuning(const char* json) {
     std::lock_guard<std::recursive_mutex> lk(g_eng.mu);
     int rc = g_eng.tun.from_json(json);
     if (rc) return rc;
-    g_eng.drop_plans();
+    g_eng.tuning_changed(false);
     return NBG_OK;
 }
 

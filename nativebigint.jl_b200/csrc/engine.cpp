@@ -347,6 +347,7 @@ int Engine::init(int device) {
     for (auto& row : hb_ev)
         for (cudaEvent_t& e : row) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CUDA_TRY(kernels_init((double)PR[0], (double)PR[1]));
+    CUDA_TRY(word_init());
     CUDA_TRY(cudaMalloc(&d_plans, sizeof(DPlan) * (size_t)plan_cap));
     CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device));
     smem_optin = kernels_smem_optin();
@@ -656,6 +657,47 @@ void Engine::trim_plans() {
     for (auto& kv : plans) cudaFree(kv.second.dtab);
     plans.clear();
     plan_used = 0;
+    for (WordTab& w : wtab) {
+        cudaFree(w.fwd);
+        cudaFree(w.inv);
+        w = WordTab();
+    }
+}
+
+void Engine::tuning_changed(bool loaded) {
+    drop_plans();
+    const std::string js = tun.to_json();
+    if (loaded) base_tuning = js;
+    word_ok = tun.queue == 0 && js == base_tuning;
+}
+
+// Tables for heap sizes up to 2^L.  One size serves every length up to
+// odd * 2^17 points; longer ones get the largest (old tables stay for live graphs).
+int Engine::word_table(int odd, int L, const WordTab** out) {
+    WordTab& w = wtab[odd];
+    if (w.L < L) {
+        const int want = L <= 15 ? 15 : WORD_MAX_LOG2 - 2;
+        const size_t bytes = word_table_bytes(odd, want);
+        WordTab n;
+        n.L = want;
+        if (cudaMalloc(&n.fwd, bytes) != cudaSuccess || cudaMalloc(&n.inv, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFree(n.fwd);
+            return fail(NBG_ENOMEM, "constant tables of %zu bytes unavailable", 2 * bytes);
+        }
+        cudaError_t e = word_build_tables(odd, want, n.fwd, n.inv, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) {
+            cudaFree(n.fwd);
+            cudaFree(n.inv);
+            return fail(NBG_ECUDA, "constant tables: %s", cudaGetErrorString(e));
+        }
+        if (w.fwd) graveyard.push_back((double*)w.fwd);
+        if (w.inv) graveyard.push_back((double*)w.inv);
+        w = n;
+    }
+    *out = &w;
+    return NBG_OK;
 }
 
 int Engine::ensure_stage(int i, size_t bytes) {
@@ -735,6 +777,18 @@ static int encode_pass_map(void* out, double* base, int64_t N, int64_t nbuf, con
 
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// Operand limbs that can be nonzero: the caller's magnitude bits, rounded up.
+static inline int64_t eff_limbs(int64_t limbs, int64_t bits) {
+    return bits < 1 ? limbs : std::max<int64_t>(1, std::min(limbs, (bits + 63) / 64));
+}
+
+bool word_product(const Engine& E, const ProdIn& q, WordShape* s) {
+    if (!E.word_ok || q.fp64 || q.keep_b) return false;
+    const int64_t la = eff_limbs(q.m, q.bits_a), lb = q.sqr ? la : eff_limbs(q.n, q.bits_b);
+    if (std::min(la, lb) > WORD_MIN_OPERAND_MAX) return false;
+    return word_shape(la + lb - 1, *s);
+}
+
 int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     bb = BatchBuild();
     if (count <= 0) return fail(NBG_EINVAL, "empty batch");
@@ -743,6 +797,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     int pmax = 1;
     int bmin = 64;
     size_t work = 0, aggw = 0;
+    std::vector<int32_t> words;  // products of the word engine
     std::vector<size_t> xa_off((size_t)count), xb_off((size_t)count), agg_off((size_t)count);
     for (int64_t k = 0; k < count; k++) {
         const ProdIn& q = in[k];
@@ -753,6 +808,40 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         // case to handle, as NBig * does before reaching the engine.
         if (q.bits_a < 1 || q.bits_a > 64 * q.m || (!q.sqr && (q.bits_b < 1 || q.bits_b > 64 * q.n)))
             return fail(NBG_EINVAL, "product %lld: magnitude bits out of range (zero operand?)", (long long)k);
+        P.a = q.a;
+        P.b = q.sqr ? q.a : q.b;
+        P.r = q.r;
+        P.m = q.m;
+        P.n = q.sqr ? q.m : q.n;
+        P.rn = P.m + P.n;
+        WordShape ws;
+        if (word_product(E, q, &ws)) {
+            const WordTab* wt = nullptr;
+            int rc = E.word_table(ws.odd, ws.lj + ws.lm - 2, &wt);
+            if (rc) return rc;
+            P.sqr = q.sqr;
+            P.nca = eff_limbs(P.m, q.bits_a);
+            P.ncb = q.sqr ? P.nca : eff_limbs(P.n, q.bits_b);
+            P.nconv = P.nca + P.ncb - 1;
+            P.ntl = (P.rn + UNPACK_TL - 1) / UNPACK_TL;
+            P.wN = ws.N;
+            P.wodd = ws.odd;
+            P.wlj = ws.lj;
+            P.wlm = ws.lm;
+            P.wL = wt->L;
+            P.wtf = wt->fwd;
+            P.wti = wt->inv;
+            word_scales(ws, P.wsc);
+            agg_off[(size_t)k] = aggw;
+            aggw += (size_t)P.ntl;
+            xa_off[(size_t)k] = bb.word_words;
+            bb.word_words += align_up((size_t)WPR * (size_t)ws.N, 64);
+            xb_off[(size_t)k] = q.sqr ? SIZE_MAX : bb.word_words;
+            if (!q.sqr) bb.word_words += align_up((size_t)WPR * (size_t)ws.N, 64);
+            bb.plan_of.push_back(nullptr);
+            words.push_back((int32_t)k);
+            continue;
+        }
         int bch;
         int64_t N;
         int rc = ntt_params(q.bits_a, q.sqr ? q.bits_a : q.bits_b, &bch, &N);
@@ -760,12 +849,6 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         PlanRec* pr;
         rc = E.get_plan(N, q.sqr, &pr);
         if (rc) return rc;
-        P.a = q.a;
-        P.b = q.sqr ? q.a : q.b;
-        P.r = q.r;
-        P.m = q.m;
-        P.n = q.sqr ? q.m : q.n;
-        P.rn = P.m + P.n;
         P.bch = bch;
         P.sqr = q.sqr;
         P.nca = (q.bits_a + bch - 1) / bch;
@@ -787,6 +870,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     }
     bb.agg_words = aggw;
     bb.agg_off = agg_off;
+    if (!words.empty()) pmax = std::max(pmax, 2);  // their column, block and column-back steps
 
     // Jobs of one pipeline step, grouped by kernel and shared-memory size: a
     // launch reserves its largest job's shared memory for every CTA, so a
@@ -834,8 +918,10 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     // length (longest first, so the tail of each launch is short), then tile,
     // then operand, then product.  CTAs that run together read the same
     // twiddle slice, which comes from DRAM once and from L2 for the rest.
-    std::vector<int32_t> byclass((size_t)count);
-    for (int64_t k = 0; k < count; k++) byclass[(size_t)k] = (int32_t)k;
+    std::vector<int32_t> byclass;
+    byclass.reserve((size_t)count);
+    for (int64_t k = 0; k < count; k++)
+        if (bb.plan_of[(size_t)k]) byclass.push_back((int32_t)k);
     std::stable_sort(byclass.begin(), byclass.end(), [&](int32_t x, int32_t y) {
         const int64_t nx = bb.plan_of[(size_t)x]->d.N, ny = bb.plan_of[(size_t)y]->d.N;
         if (nx != ny) return nx > ny;
@@ -850,7 +936,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     // gives each prime of a tile its own CTA: twice the CTAs, half the
     // critical path each (small batches are latency-bound).
     int64_t pwr_tiles = 0;
-    for (int64_t k = 0; k < count; k++) {
+    for (int32_t k : byclass) {
         const DPlan& pl = bb.plan_of[(size_t)k]->d;
         pwr_tiles += pl.pass[pl.npass - 1].ntiles;
     }
@@ -959,21 +1045,28 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     bb.work_doubles = work;
     bb.xa_off = xa_off;
     bb.xb_off = xb_off;
-    const size_t unp_smem = unpack_smem_bytes(bmin);
     // unpack: product k owns tiles [agg_off[k], agg_off[k] + ntl); carry: one CTA per product
-    Group& gu = group_of(2 * pmax - 1, JK_UNPACK, unp_smem);
-    gu.mode = JM_TILES;
-    gu.njobs = (int64_t)aggw;
+    double carry_bytes = 0, unp_ops = 0, unp_bytes = 0;
+    int64_t fp_tiles = 0;
     bool any_carry = false;
-    double carry_bytes = 0;
     for (int64_t k = 0; k < count; k++) {
         const DProd& P = bb.prods[(size_t)k];
-        gu.ops += 28.0 * (double)P.nconv;
-        gu.bytes += 16.0 * (double)P.nconv + 8.0 * (double)P.rn;
+        if (!P.wN) {
+            unp_ops += 28.0 * (double)P.nconv;
+            unp_bytes += 16.0 * (double)P.nconv + 8.0 * (double)P.rn;
+            fp_tiles += P.ntl;
+        }
         if (P.ntl > 1) {
             any_carry = true;
             carry_bytes += 4.0 * (double)P.ntl;
         }
+    }
+    if (fp_tiles) {
+        Group& gu = group_of(2 * pmax - 1, JK_UNPACK, unpack_smem_bytes(bmin));
+        gu.mode = JM_TILES;
+        gu.njobs = fp_tiles;
+        gu.ops = unp_ops;
+        gu.bytes = unp_bytes;
     }
     if (any_carry) {
         Group& gc = group_of(2 * pmax, JK_CARRY, 0);
@@ -984,6 +1077,39 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         gf.mode = JM_TILES;
         gf.njobs = (int64_t)aggw;
     }
+    // word products: one launch per step and kernel variant, the products of a
+    // shape together (their tables are shared), longest first
+    struct WGroup {
+        std::vector<WSeg> segs;
+        std::vector<int32_t> plist;
+        int64_t nctas = 0;
+        double bytes = 0;
+    };
+    std::map<std::tuple<int, int, int>, WGroup> wgroups;  // step, kind, variant
+    std::stable_sort(words.begin(), words.end(), [&](int32_t x, int32_t y) {
+        const DProd &a = bb.prods[(size_t)x], &b = bb.prods[(size_t)y];
+        return a.wN != b.wN ? a.wN > b.wN : a.sqr < b.sqr;
+    });
+    for (int32_t k : words) {
+        const DProd& P = bb.prods[(size_t)k];
+        const WordShape ws{P.wN, P.wodd, P.wlj, P.wlm};
+        const double res = 4.0 * WPR * P.wN, nop = P.sqr ? 1 : 2;
+        auto put = [&](int step, int kind, int variant, double bytes) {
+            WGroup& g = wgroups[std::make_tuple(step, kind, variant)];
+            const int64_t cpp = word_ctas(kind, ws, P.sqr, P.rn);
+            if (g.segs.empty() || g.segs.back().cpp != cpp)
+                g.segs.push_back(WSeg{(int32_t)g.nctas, (int32_t)g.plist.size(), (int32_t)cpp, 0});
+            g.plist.push_back(k);
+            g.nctas += cpp;
+            g.bytes += bytes;
+        };
+        put(pmax - 2, JK_WCOL_FWD, (P.wodd << 8) | P.wlj, 8.0 * (double)(P.nca + (P.sqr ? 0 : P.ncb)) + nop * res);
+        put(pmax - 1, JK_WBLOCK, P.wlm, (nop + 1) * res);
+        put(pmax, JK_WCOL_REV, (P.wodd << 8) | P.wlj, 2 * res);
+        put(2 * pmax - 1, JK_WUNPACK, 0, res + 8.0 * (double)P.rn);
+    }
+    for (auto& kv : wgroups)
+        if (kv.second.nctas > 0x7fffffff) return fail(NBG_EINVAL, "batch too large");
     // job table: [segments | product list] per launch, then the unpack tile starts
     size_t tb = 0;
     for (auto& kv : groups) {
@@ -1006,12 +1132,30 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         }
         bb.launches.push_back(L);
     }
+    bb.nexpand = (int)bb.launches.size();
+    for (auto& kv : wgroups) {
+        const WGroup& g = kv.second;
+        Launch L{std::get<1>(kv.first), 0, g.nctas, 0};
+        L.odd = false;
+        L.step = std::get<0>(kv.first);
+        L.variant = std::get<2>(kv.first);
+        L.alg_bytes = g.bytes;
+        L.mode = JM_WORD;
+        L.nseg = (int)g.segs.size();
+        L.seg_off = tb;
+        tb = align_up(tb + sizeof(WSeg) * g.segs.size(), 16);
+        L.plist_off = tb;
+        tb = align_up(tb + sizeof(int32_t) * g.plist.size(), 16);
+        bb.launches.push_back(L);
+    }
     bb.tstart_off = tb;
+    tb = align_up(tb + sizeof(int64_t) * ((size_t)count + 1), 128);
+    bb.tstart_fp_off = tb;
     tb = align_up(tb + sizeof(int64_t) * ((size_t)count + 1), 128);
     bb.tmap_off = tb;  // 128-byte tensor maps, written by bind_batch
     tb = align_up(tb + 128 * (size_t)bb.ntmaps, 16);
     bb.expand_off = tb;
-    tb = align_up(tb + sizeof(ExpandEntry) * bb.launches.size(), 16);
+    tb = align_up(tb + sizeof(ExpandEntry) * (size_t)bb.nexpand, 16);
     bb.table.assign(tb, 0);
     {
         size_t li = 0;
@@ -1022,10 +1166,26 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
             memcpy(bb.table.data() + L.seg_off, g.segs.data(), sizeof(JobSeg) * g.segs.size());
             memcpy(bb.table.data() + L.plist_off, g.plist.data(), sizeof(int32_t) * g.plist.size());
         }
+        for (auto& kv : wgroups) {
+            const WGroup& g = kv.second;
+            const Launch& L = bb.launches[li++];
+            memcpy(bb.table.data() + L.seg_off, g.segs.data(), sizeof(WSeg) * g.segs.size());
+            memcpy(bb.table.data() + L.plist_off, g.plist.data(), sizeof(int32_t) * g.plist.size());
+        }
         int64_t* ts = (int64_t*)(bb.table.data() + bb.tstart_off);
-        for (int64_t k = 0; k < count; k++) ts[k] = (int64_t)agg_off[(size_t)k];
+        int64_t* tf = (int64_t*)(bb.table.data() + bb.tstart_fp_off);
+        int64_t fp = 0;
+        for (int64_t k = 0; k < count; k++) {
+            ts[k] = (int64_t)agg_off[(size_t)k];
+            tf[k] = fp;
+            if (!bb.prods[(size_t)k].wN) fp += bb.prods[(size_t)k].ntl;
+        }
         ts[count] = (int64_t)aggw;
+        tf[count] = fp;
     }
+    // the explicit launches come first in the table; the run order is by step
+    std::stable_sort(bb.launches.begin(), bb.launches.end(),
+                     [](const Launch& x, const Launch& y) { return x.step < y.step; });
 
     // device layout: [prods | jobs | work | agg]
     bb.off_prods = 0;
@@ -1033,7 +1193,8 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     bb.head_bytes = bb.off_jobs + bb.table.size();
     bb.off_joblist = align_up(bb.head_bytes, 256);
     bb.off_work = align_up(bb.off_joblist + sizeof(Job) * (size_t)bb.total_jobs, 256);
-    bb.off_agg = align_up(bb.off_work + sizeof(double) * work, 256);
+    bb.off_word = align_up(bb.off_work + sizeof(double) * work, 256);
+    bb.off_agg = align_up(bb.off_word + sizeof(uint32_t) * bb.word_words, 256);
     bb.dev_bytes = align_up(bb.off_agg + sizeof(uint32_t) * aggw, 256);
     return NBG_OK;
 }
@@ -1058,6 +1219,13 @@ int bind_batch(BatchBuild& bb, char* dbase) {
     }
     for (size_t k = 0; k < bb.prods.size(); k++) {
         DProd& P = bb.prods[k];
+        P.agg = agg + bb.agg_off[k];
+        if (P.wN) {
+            uint32_t* ww = (uint32_t*)(dbase + bb.off_word);
+            P.wa = ww + bb.xa_off[k];
+            P.wb = bb.xb_off[k] == SIZE_MAX ? nullptr : ww + bb.xb_off[k];
+            continue;
+        }
         const int64_t N = bb.plan_of[k]->d.N;
         P.xa[0] = work + bb.xa_off[k];
         P.xa[1] = P.xa[0] + N;
@@ -1067,15 +1235,16 @@ int bind_batch(BatchBuild& bb, char* dbase) {
         } else {
             P.xb[0] = P.xb[1] = nullptr;
         }
-        P.agg = agg + bb.agg_off[k];
         const BatchBuild::ClassRec& cr = bb.classes[(size_t)bb.class_of[k]];
         P.tmap = cr.map0 < 0 ? nullptr : dbase + bb.off_jobs + bb.tmap_off + 128 * (size_t)cr.map0;
     }
     ExpandEntry* ex = (ExpandEntry*)(bb.table.data() + bb.expand_off);
-    for (size_t i = 0; i < bb.launches.size(); i++) {
-        ex[i].src = launch_src(bb, bb.launches[i], dbase);
-        ex[i].begin = bb.launches[i].off;
-        ex[i].n = bb.launches[i].n;
+    for (const Launch& L : bb.launches) {  // in step order, as the job offsets are
+        if (L.mode == JM_WORD) continue;
+        ex->src = launch_src(bb, L, dbase);
+        ex->begin = L.off;
+        ex->n = L.n;
+        ex++;
     }
     return NBG_OK;
 }
@@ -1093,7 +1262,7 @@ JobSrc launch_src(const BatchBuild& bb, const Launch& L, const char* dbase) {
     s.segs = (const JobSeg*)(t + L.seg_off);
     s.nseg = L.nseg;
     s.plist = (const int32_t*)(t + L.plist_off);
-    s.tstart = (const int64_t*)(t + bb.tstart_off);
+    s.tstart = (const int64_t*)(t + (L.kind == JK_UNPACK ? bb.tstart_fp_off : bb.tstart_off));
     s.nprod = (int64_t)bb.prods.size();
     return s;
 }
@@ -1112,19 +1281,28 @@ int upload_batch(Engine& E, BatchBuild& bb, char* dbase, cudaStream_t st) {
 }
 
 cudaError_t expand_jobs(const BatchBuild& bb, char* dbase, cudaStream_t st) {
-    return launch_expand((const ExpandEntry*)(dbase + bb.off_jobs + bb.expand_off), (int)bb.launches.size(),
+    return launch_expand((const ExpandEntry*)(dbase + bb.off_jobs + bb.expand_off), bb.nexpand,
                          (Job*)(dbase + bb.off_joblist), bb.total_jobs, st);
 }
 
-int run_launches(Engine& E, const BatchBuild& bb, char* dbase, cudaStream_t st, bool expand) {
+cudaError_t launch_one(Engine& E, const BatchBuild& bb, const Launch& L, char* dbase, cudaStream_t st) {
     const DProd* prods = (const DProd*)(dbase + bb.off_prods);
+    if (L.mode == JM_WORD) {
+        const char* t = dbase + bb.off_jobs;
+        return launch_word(L.kind, L.variant, prods, (const WSeg*)(t + L.seg_off), L.nseg,
+                           (const int32_t*)(t + L.plist_off), L.n, st);
+    }
     const Job* jobs = (const Job*)(dbase + bb.off_joblist);
-    if (expand) {
+    return launch_jobs(L.kind, prods, E.d_plans, job_list(jobs + L.off), L.n, L.smem, 0, st, L.odd);
+}
+
+int run_launches(Engine& E, const BatchBuild& bb, char* dbase, cudaStream_t st, bool expand) {
+    if (expand && bb.total_jobs) {
         CUDA_TRY(expand_jobs(bb, dbase, st));
         g_launches++;
     }
     for (const Launch& L : bb.launches) {
-        cudaError_t e = launch_jobs(L.kind, prods, E.d_plans, job_list(jobs + L.off), L.n, L.smem, 0, st, L.odd);
+        cudaError_t e = launch_one(E, bb, L, dbase, st);
         if (e != cudaSuccess) return fail(NBG_ECUDA, "launch (kind %d, %lld jobs): %s", L.kind, (long long)L.n,
                                           cudaGetErrorString(e));
         g_launches++;
@@ -1134,10 +1312,10 @@ int run_launches(Engine& E, const BatchBuild& bb, char* dbase, cudaStream_t st, 
 
 int run_launches_branched(Engine& E, const BatchBuild& bb, char* dbase, cudaStream_t st, cudaStream_t* side,
                           int nside) {
-    const DProd* prods = (const DProd*)(dbase + bb.off_prods);
-    const Job* jobs = (const Job*)(dbase + bb.off_joblist);
-    CUDA_TRY(expand_jobs(bb, dbase, st));
-    g_launches++;
+    if (bb.total_jobs) {
+        CUDA_TRY(expand_jobs(bb, dbase, st));
+        g_launches++;
+    }
     size_t i = 0;
     while (i < bb.launches.size()) {
         size_t j = i;
@@ -1156,7 +1334,7 @@ int run_launches_branched(Engine& E, const BatchBuild& bb, char* dbase, cudaStre
                 s = side[(k - i - 1) % (size_t)nside];
                 CUDA_TRY(cudaStreamWaitEvent(s, fork, 0));
             }
-            cudaError_t e = launch_jobs(L.kind, prods, E.d_plans, job_list(jobs + L.off), L.n, L.smem, 0, s, L.odd);
+            cudaError_t e = launch_one(E, bb, L, dbase, s);
             if (e != cudaSuccess)
                 return fail(NBG_ECUDA, "launch (kind %d, %lld jobs): %s", L.kind, (long long)L.n, cudaGetErrorString(e));
             g_launches++;

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "types.h"
+#include "word.h"
 
 namespace nbg {
 
@@ -59,6 +60,13 @@ struct PlanRec {
     int slot = -1;
 };
 
+// Constant tables of the word products of one `odd` (word.h).
+struct WordTab {
+    void* fwd = nullptr;
+    void* inv = nullptr;
+    int L = 0;
+};
+
 struct Engine {
     bool ready = false;
     int dev = -1;
@@ -71,6 +79,12 @@ struct Engine {
     cudaEvent_t hb_ev[3][4] = {};    // host-buffer batches: per slot, operands in / computed / results out
     std::recursive_mutex mu;
     Tuning tun;
+    // the tuning the engine started with or loaded from a file: while `tun`
+    // equals it, products within the word engine's range run there; a caller
+    // that sets other pass knobs gets the FP64 passes they describe
+    std::string base_tuning = Tuning().to_json();
+    bool word_ok = true;
+    WordTab wtab[8];  // by odd
     std::map<int64_t, PlanRec> plans;
     std::vector<double*> graveyard;
     DPlan* d_plans = nullptr;
@@ -93,6 +107,8 @@ struct Engine {
     int build_plan(int64_t N, PlanRec& pr, int for_sqr);
     int get_plan(int64_t N, int for_sqr, PlanRec** out);
     void drop_plans();
+    void tuning_changed(bool loaded);  // after `tun` was set (loaded: it is the new base)
+    int word_table(int odd, int L, const WordTab** out);
     void trim_plans();  // frees every plan's tables: no batch may exist or be running
     int ensure_pool(size_t bytes);
     int ensure_stage(int i, size_t bytes);
@@ -109,7 +125,11 @@ struct ProdIn {
     int sqr;
     // one-pass products only: keep operand b's spectrum in workspace (PF_BSAVE)
     int keep_b = 0;
+    int fp64 = 0;  // 1: never a word product
 };
+
+// Whether the product runs on the word engine (shape in *s), from its sizes alone.
+bool word_product(const Engine& E, const ProdIn& q, WordShape* s);
 
 struct Launch {
     int kind;
@@ -120,6 +140,7 @@ struct Launch {
     int mode = JM_LIST;
     int nseg = 0;
     size_t seg_off = 0, plist_off = 0;
+    int variant = 0;       // word launches (JM_WORD): kernel variant; n counts CTAs
     int step = 0;          // pipeline step: launches of one step are independent
     bool odd = true;       // some pass of the launch holds a radix-3/5/7 stage
     double alg_ops = 0;    // FP64 instructions of the reference schedule done by this launch
@@ -131,12 +152,15 @@ struct BatchBuild {
     std::vector<PlanRec*> plan_of;
     std::vector<char> table;  // job table: per launch segments and product lists, then tile starts
     size_t tstart_off = 0;    // per-product first unpack tile (count + 1 int64), in the table
+    size_t tstart_fp_off = 0; // the same with no tiles for word products (the FP64 unpack's list)
+    int nexpand = 0;          // launches with explicit jobs
     size_t expand_off = 0;    // ExpandEntry per launch, in the table (written by bind_batch)
     int64_t total_jobs = 0;   // explicit jobs, written on the device by the expansion kernel
     size_t off_joblist = 0;   // region offset of that job list
     size_t head_bytes = 0;    // [0, head_bytes): descriptors and table, the host-written head
     std::vector<Launch> launches;
-    std::vector<size_t> xa_off, xb_off, agg_off;
+    std::vector<size_t> xa_off, xb_off, agg_off;  // word products: word offsets into the word workspace
+    size_t word_words = 0, off_word = 0;
     // product classes (one plan, one kept-spectrum flag): contiguous transform
     // buffers, and the tensor maps of their TMA column passes
     struct ClassRec {
@@ -168,6 +192,8 @@ void stage_batch(const BatchBuild& bb, char* host);
 cudaError_t expand_jobs(const BatchBuild& bb, char* dbase, cudaStream_t st);
 // The job source of launch L of a batch whose region starts at dbase.
 JobSrc launch_src(const BatchBuild& bb, const Launch& L, const char* dbase);
+// One launch of a batch (its explicit jobs already expanded).
+cudaError_t launch_one(Engine& E, const BatchBuild& bb, const Launch& L, char* dbase, cudaStream_t st);
 // expand = false reuses the job list a previous run wrote (same region).
 int run_launches(Engine& E, const BatchBuild& bb, char* dbase, cudaStream_t st, bool expand = true);
 // Work-queue execution of a batch: one persistent launch (k_queue) walks the

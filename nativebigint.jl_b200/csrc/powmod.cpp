@@ -298,6 +298,7 @@ static int powmod_run(Engine& E, const nbg_powmod_desc* d, int64_t count, int64_
         uint64_t* q2 = d_q2 + c * q2_stride;
         const int64_t l = lmu[(size_t)c];
         in1[(size_t)c] = ProdIn{sl + (int64_t)S.acc() * k, sl + (int64_t)S.one() * k, T, k, k, 64 * k, 64 * k, 0};
+        in1[(size_t)c].fp64 = 1;
         // mu and m are the same on every step: as operand b their transforms
         // are kept from the first run (one-pass products) and reused
         in2[(size_t)c] = ProdIn{T + (k - 1), d_mu + c * lmu_max, q2, k + 1, l, 64 * (k + 1), bits_mu[(size_t)c], 0};

@@ -81,6 +81,14 @@ struct DProd {
     double* xb[2];       // per-prime buffers of operand b (multi-pass products only)
     uint32_t* agg;       // per limb-tile carry aggregates (bit0 generate, bit1 propagate)
     int64_t ntl;         // number of limb tiles
+    // word products (word.h; `wN` nonzero): residues of operand a (and the
+    // result) and b as five arrays of wN words, constant tables, shape
+    uint32_t* wa;
+    uint32_t* wb;
+    const void* wtf;     // forward and inverse constants, [prime][block][2^wL]
+    const void* wti;
+    int32_t wN, wodd, wlj, wlm, wL;
+    uint32_t wsc[5];     // unpack scale per prime
 };
 
 // Work item of one launch.  kind-specific meaning of `sub`:
@@ -137,6 +145,7 @@ enum JobMode : int32_t {
     JM_SEGS = 1,     // segs[nseg] over plist
     JM_TILES = 2,    // product k owns jobs [tstart[k], tstart[k+1]): tile = ji - tstart[k]
     JM_PERPROD = 3,  // job ji is product ji, tile 0
+    JM_WORD = 4,     // a word launch: CTAs find their product in WSeg segments
 };
 struct JobSrc {
     const Job* list;
@@ -205,6 +214,10 @@ enum JobKind : int32_t {
     JK_PWR_KEEP = 7, // JK_PWR for products with a kept operand spectrum (PF_BSAVE / PF_BSPEC)
     JK_FWD_TMA = 8,  // JK_FWD with tiles staged by TMA (DProd.tmap; at least 16 columns per tile)
     JK_REV_TMA = 9,  // JK_REV with tiles staged by TMA
+    JK_WCOL_FWD = 10,// word products (word.h): limbs to residues and the first levels
+    JK_WBLOCK = 11,  // word products: blocks of the remaining levels, leaf products, and back
+    JK_WCOL_REV = 12,// word products: the first levels backwards
+    JK_WUNPACK = 13, // word products: coefficients and carried limbs
 };
 
 constexpr int UNPACK_TL = 1024;  // output limbs per unpack tile

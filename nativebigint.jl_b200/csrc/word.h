@@ -1,0 +1,60 @@
+// word.h — products through transforms over five 30-bit primes ("word"
+// products): every 64-bit limb is one coefficient, so packing is a reduction
+// and the results are the carried sums of the convolution's coefficients.
+//
+// A transform of length N = odd * 2^k (odd in {1, 3, 5, 7}) works modulo
+// X^N - 1: one radix-`odd` step splits it into X^(2^k) - e(j/odd) (e(t) a fixed
+// primitive root's t-th turn), then each X^L - e(t) splits into
+// X^(L/2) - e(t/2) and X^(L/2) + e(t/2).  Node n of level l under block j
+// (level 0 is the block itself) has t = (j/odd + bitrev_l(n)) / 2^l; its
+// butterfly constant e(t/2) is entry 2^l + n of block j's table, so a subtree's
+// constants are contiguous per level and every size shares one table.  The
+// splitting stops two levels early: the leaves are polynomials modulo
+// X^4 - e(t), multiplied directly, which needs a quarter of the table.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "types.h"
+
+namespace nbg {
+
+constexpr int WPR = 5;  // primes
+// p = 1 mod 105 * 2^18, so e(t) exists for t = i / (odd * 2^18); their product
+// exceeds 2^149: any min(m, n) <= 2^21 limbs convolve without wrapping.
+constexpr uint32_t WPRIMES[WPR] = {1073479681u, 1018429441u, 908328961u, 880803841u, 825753601u};
+constexpr int WORD_MAX_LOG2 = 20;               // k <= 20 (leaves at level k - 2 <= 18)
+constexpr int64_t WORD_MIN_OPERAND_MAX = int64_t(1) << 21;
+
+// Shape of a word product's transform: N = R * M, R = odd * 2^lj rows.  Column
+// passes work on the R rows of one column in registers; blocks of M = 2^lm
+// consecutive values (each one subtree) are transformed in shared memory.
+struct WordShape {
+    int32_t N = 0, odd = 0, lj = 0, lm = 0;
+};
+// The smallest supported length >= nconv; false when there is none.
+bool word_shape(int64_t nconv, WordShape& s);
+
+// One launch's CTAs: products of one shape are consecutive, `cpp` CTAs each.
+struct WSeg {
+    int32_t begin;  // first CTA
+    int32_t first;  // into the launch's product list
+    int32_t cpp;    // CTAs per product
+    int32_t pad_;
+};
+
+// variant of a word launch: (odd << 8) | lj for column passes, lm for blocks
+cudaError_t word_init();  // constant memory of the current device
+cudaError_t launch_word(int kind, int variant, const DProd* prods, const WSeg* segs, int nseg, const int32_t* plist,
+                        int64_t nctas, cudaStream_t st);
+// CTAs one product needs in a word launch.
+int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t rn);
+
+// Tables of one `odd` for heap sizes up to 2^L: per prime and block, fwd then inverse.
+size_t word_table_bytes(int odd, int L);
+cudaError_t word_build_tables(int odd, int L, void* fwd, void* inv, cudaStream_t st);
+// Per-product scale constants of the unpack (the inverse transform's 1/(odd * 2^(k-2)) and the pointwise 2^-32).
+void word_scales(const WordShape& s, uint32_t out[WPR]);
+
+}  // namespace nbg

@@ -1,0 +1,774 @@
+// word_kernels.cu — kernels of the word products (word.h): products through
+// transforms modulo five 30-bit primes, one coefficient per 64-bit limb.
+//
+//   k_wcol_fwd  limbs -> residues, the radix-`odd` step and the first lj levels
+//               of one column's R rows, in registers
+//   k_wblock    per block of M values: the other levels of a and b, the leaf
+//               products, the levels back
+//   k_wcol_rev  the first lj levels and the radix-`odd` step backwards
+//   k_wunpack   five residues -> coefficient (mixed radix), carried limb sums
+#include <cuda_runtime.h>
+
+#include <atomic>
+#include <type_traits>
+
+#include "word.cuh"
+#include "word.h"
+
+namespace nbg {
+
+using wd::Tw;
+
+struct WConst {
+    uint32_t p[WPR], pinv[WPR];
+    Tw c32[WPR], one[WPR];       // 2^32 mod p, 1
+    Tw r3[WPR];                  // e(1/3)
+    Tw r5[WPR][5];               // -1/4, (c1-c2)/2, f1, f2 of e(1/5) (see dft5); [4] unused
+    uint32_t c7[WPR][3], f7[WPR][3];  // cosine and sine halves of e(j/7) in 2^32 form
+    uint32_t gar[WPR][WPR];      // mixed radix: gar[i][j] = -W_j / W_i mod p_i in 2^32 form (j < i)
+};
+__constant__ WConst c_w;
+
+// ---------------------------------------------------------------------------
+// host constants
+
+static uint64_t pw(uint64_t a, uint64_t e, uint64_t p) {
+    uint64_t r = 1;
+    for (a %= p; e; e >>= 1, a = a * a % p)
+        if (e & 1) r = r * a % p;
+    return r;
+}
+static uint64_t inv(uint64_t a, uint64_t p) { return pw(a, p - 2, p); }
+// a primitive root: p - 1 = 105 * 2^18 * c, its prime factors are 2, 3, 5, 7 and c's
+static uint64_t prim_root(uint64_t p) {
+    for (uint64_t g = 2;; g++) {
+        bool ok = true;
+        uint64_t n = p - 1;
+        for (uint64_t f = 2; ok && f * f <= n; f++)
+            if (n % f == 0) {
+                ok = pw(g, (p - 1) / f, p) != 1;
+                while (n % f == 0) n /= f;
+            }
+        if (ok && n > 1) ok = pw(g, (p - 1) / n, p) != 1;
+        if (ok) return g;
+    }
+}
+static uint64_t root_of(int i) {
+    static const uint64_t g[WPR] = {prim_root(WPRIMES[0]), prim_root(WPRIMES[1]), prim_root(WPRIMES[2]),
+                                    prim_root(WPRIMES[3]), prim_root(WPRIMES[4])};
+    return g[i];
+}
+static Tw mk(uint64_t w, uint64_t p) { return Tw{(uint32_t)w, (uint32_t)((w << 32) / p)}; }
+static uint32_t mont(uint64_t w, uint64_t p) { return (uint32_t)(((w % p) << 32) % p); }
+
+cudaError_t word_init() {
+    WConst h{};
+    for (int i = 0; i < WPR; i++) {
+        const uint64_t p = WPRIMES[i], g = root_of(i);
+        h.p[i] = (uint32_t)p;
+        uint32_t x = 1;
+        for (int k = 0; k < 5; k++) x *= 2 - (uint32_t)p * x;  // Newton: p^-1 mod 2^32
+        h.pinv[i] = x;
+        h.c32[i] = mk((uint64_t(1) << 32) % p, p);
+        h.one[i] = mk(1, p);
+        h.r3[i] = mk(pw(g, (p - 1) / 3, p), p);
+        const uint64_t h2 = inv(2, p), w5 = pw(g, (p - 1) / 5, p), w7 = pw(g, (p - 1) / 7, p);
+        auto half = [&](uint64_t w, int a, int b, bool minus) {  // (w^a +- w^b) / 2
+            const uint64_t x1 = pw(w, a, p), x2 = pw(w, b, p);
+            return (x1 + (minus ? p - x2 : x2)) % p * h2 % p;
+        };
+        const uint64_t c1 = half(w5, 1, 4, false), c2 = half(w5, 2, 3, false);
+        h.r5[i][0] = mk((p - inv(4, p)) % p, p);
+        h.r5[i][1] = mk((c1 + p - c2) % p * h2 % p, p);
+        h.r5[i][2] = mk(half(w5, 1, 4, true), p);
+        h.r5[i][3] = mk(half(w5, 2, 3, true), p);
+        for (int k = 0; k < 3; k++) {
+            h.c7[i][k] = mont(half(w7, k + 1, 6 - k, false), p);
+            h.f7[i][k] = mont(half(w7, k + 1, 6 - k, true), p);
+        }
+        uint64_t Wi = 1;
+        for (int t = 0; t < i; t++) Wi = Wi * (WPRIMES[t] % p) % p;
+        const uint64_t iw = inv(Wi, p);
+        uint64_t Wj = 1;
+        for (int j = 0; j < i; j++) {
+            h.gar[i][j] = mont((p - Wj * iw % p) % p, p);
+            Wj = Wj * (WPRIMES[j] % p) % p;
+        }
+        (void)0;
+    }
+    return cudaMemcpyToSymbol(c_w, &h, sizeof h);
+}
+
+void word_scales(const WordShape& s, uint32_t out[WPR]) {
+    for (int i = 0; i < WPR; i++) {
+        const uint64_t p = WPRIMES[i];
+        const int lev = s.lj + s.lm - 2;
+        const uint64_t t = (uint64_t)s.odd % p * pw(2, (uint64_t)lev, p) % p;
+        uint64_t Wi = 1;
+        for (int j = 0; j < i; j++) Wi = Wi * (WPRIMES[j] % p) % p;
+        // 2^32 (pointwise) * 2^32 (unpack's reduction) / (odd * 2^levels * W_i)
+        const uint64_t r = (uint64_t(1) << 32) % p;
+        out[i] = (uint32_t)(r * r % p * inv(t * Wi % p, p) % p);
+    }
+}
+
+bool word_shape(int64_t nconv, WordShape& s) {
+    int64_t best = INT64_MAX;
+    for (int odd : {1, 3, 5, 7}) {
+        for (int k = 6; k <= WORD_MAX_LOG2; k++) {
+            const int64_t N = (int64_t)odd << k;
+            if (N < nconv || N >= best) continue;
+            // block of at most 4096 with 2 <= R <= 32 rows
+            for (int lm : {12, 10, 8, 6}) {
+                const int lj = k - lm;
+                if (lj < 0) continue;
+                const int64_t R = (int64_t)odd << lj;
+                if (R < 2 || R > 32) continue;
+                best = N;
+                s.N = (int32_t)N;
+                s.odd = odd;
+                s.lj = lj;
+                s.lm = lm;
+                break;
+            }
+        }
+    }
+    return best != INT64_MAX;
+}
+
+// ---------------------------------------------------------------------------
+// tables
+
+size_t word_table_bytes(int odd, int L) { return sizeof(Tw) * ((size_t)WPR * odd << L); }
+
+__device__ uint32_t pw_dev(uint32_t a, uint32_t e, uint32_t p) {
+    uint64_t r = 1, b = a;
+    for (; e; e >>= 1, b = b * b % p)
+        if (e & 1) r = r * b % p;
+    return (uint32_t)r;
+}
+
+struct WRoots {
+    uint32_t g[WPR];
+};
+// entry h = 2^l + n of (prime i, block j): e((j + odd * bitrev_l(n)) / (odd * 2^(l+1))) and its inverse
+__global__ void k_wtable(Tw* __restrict__ fwd, Tw* __restrict__ bwd, int odd, int L, WRoots g) {
+    const int64_t total = (int64_t)WPR * odd << L;
+    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < total; x += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t h = (uint32_t)(x & ((int64_t(1) << L) - 1));
+        const int ij = (int)(x >> L), i = ij / odd, j = ij - i * odd;
+        const uint32_t p = c_w.p[i];
+        uint32_t e = 0;
+        if (h) {
+            const int l = 31 - __clz(h);
+            const uint32_t n = h - (1u << l);
+            const uint32_t brv = l ? __brev(n) >> (32 - l) : 0;
+            e = (p - 1) / ((uint32_t)odd << (l + 1)) * ((uint32_t)j + (uint32_t)odd * brv);
+        }
+        const uint32_t w = pw_dev(g.g[i], e, p), v = e ? pw_dev(g.g[i], p - 1 - e, p) : 1u;
+        fwd[x] = Tw{w, (uint32_t)(((uint64_t)w << 32) / p)};
+        bwd[x] = Tw{v, (uint32_t)(((uint64_t)v << 32) / p)};
+    }
+}
+
+cudaError_t word_build_tables(int odd, int L, void* fwd, void* bwd, cudaStream_t st) {
+    WRoots g;
+    for (int i = 0; i < WPR; i++) g.g[i] = (uint32_t)root_of(i);
+    k_wtable<<<148 * 8, 256, 0, st>>>((Tw*)fwd, (Tw*)bwd, odd, L, g);
+    return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// radix-odd steps: in and out in [0, 2p) unless said otherwise
+
+// y_j = sum x_i e(ij/3): with w + w^2 = -1 one product suffices
+__device__ __forceinline__ void dft3(uint32_t* x, int st, int i, uint32_t p) {
+    const uint32_t p2 = 2 * p;
+    uint32_t &a = x[0], &b = x[st], &c = x[2 * st];
+    const uint32_t t = wd::mulw(b - c + p2, c_w.r3[i], p);
+    const uint32_t y0 = wd::sub_if(wd::sub_if(a + b, p2) + c, p2);
+    const uint32_t y1 = wd::sub_if(wd::sub_if(a - c + p2, p2) + t, p2);
+    const uint32_t u = wd::sub_if(a - b + p2, p2);
+    const uint32_t y2 = wd::sub_if(u - t + p2, p2);
+    a = y0;
+    b = y1;
+    c = y2;
+}
+// cosine halves c1, c2 = -1/4 +- d: two products for the even part, four for the odd
+__device__ __forceinline__ void dft5(uint32_t* x, int st, int i, uint32_t p) {
+    const uint32_t p2 = 2 * p;
+    const Tw q = c_w.r5[i][0], d = c_w.r5[i][1], f1 = c_w.r5[i][2], f2 = c_w.r5[i][3];
+    const uint32_t x0 = x[0], x1 = x[st], x2 = x[2 * st], x3 = x[3 * st], x4 = x[4 * st];
+    const uint32_t s1 = wd::sub_if(x1 + x4, p2), s2 = wd::sub_if(x2 + x3, p2);
+    const uint32_t d1 = x1 - x4 + p2, d2 = x2 - x3 + p2;
+    const uint32_t s = wd::sub_if(s1 + s2, p2);
+    const uint32_t b0 = wd::sub_if(x0 + wd::mulw(s, q, p), p2);
+    const uint32_t e = wd::mulw(s1 - s2 + p2, d, p);
+    const uint32_t C1 = wd::sub_if(b0 + e, p2), C2 = wd::sub_if(b0 - e + p2, p2);
+    const uint32_t S1 = wd::sub_if(wd::mulw(d1, f1, p) + wd::mulw(d2, f2, p), p2);
+    const uint32_t S2 = wd::sub_if(wd::mulw(d1, f2, p) - wd::mulw(d2, f1, p) + p2, p2);
+    x[0] = wd::sub_if(x0 + s, p2);
+    x[st] = wd::sub_if(C1 + S1, p2);
+    x[4 * st] = wd::sub_if(C1 - S1 + p2, p2);
+    x[2 * st] = wd::sub_if(C2 + S2, p2);
+    x[3 * st] = wd::sub_if(C2 - S2 + p2, p2);
+}
+// even and odd parts as sums of three wide products and one reduction each
+__device__ __forceinline__ void dft7(uint32_t* x, int st, int i, uint32_t p) {
+    const uint32_t p2 = 2 * p, pinv = c_w.pinv[i];
+    const uint32_t x0 = x[0];
+    uint32_t s[3], d[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        s[k] = wd::sub_if(x[(k + 1) * st] + x[(6 - k) * st], p2);
+        d[k] = wd::sub_if(x[(k + 1) * st] - x[(6 - k) * st] + p2, p2);
+    }
+    x[0] = wd::sub_if(wd::sub_if(wd::sub_if(x0 + s[0], p2) + s[1], p2) + s[2], p2);
+#pragma unroll
+    for (int j = 1; j <= 3; j++) {
+        uint64_t ce = 0, so = 0;
+#pragma unroll
+        for (int k = 1; k <= 3; k++) {
+            const int t = j * k % 7, a = t <= 3 ? t : 7 - t;  // cos(t) = cos(7 - t), sin(t) = -sin(7 - t)
+            ce += wd::mulx(s[k - 1], c_w.c7[i][a - 1]);
+            so += wd::mulx(t <= 3 ? d[k - 1] : p2 - d[k - 1], c_w.f7[i][a - 1]);
+        }
+        // each sum < 3 * 2p * p, reduced below 1.5p + p
+        const uint32_t C = wd::sub_if(x0 + wd::sub_if(wd::redc(ce, p, pinv), p2), p2);
+        const uint32_t S = wd::sub_if(wd::redc(so, p, pinv), p2);
+        x[j * st] = wd::sub_if(C + S, p2);
+        x[(7 - j) * st] = wd::sub_if(C - S + p2, p2);
+    }
+}
+
+template <int ODD, int LJ>
+__device__ __forceinline__ void dft_odd(uint32_t* x, int i, uint32_t p) {
+#pragma unroll
+    for (int r = 0; r < (1 << LJ); r++) {
+        if (ODD == 3) dft3(x + r, 1 << LJ, i, p);
+        if (ODD == 5) dft5(x + r, 1 << LJ, i, p);
+        if (ODD == 7) dft7(x + r, 1 << LJ, i, p);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// job lookup: segment of this CTA, its product and the CTA's index inside it
+
+__device__ __forceinline__ const DProd& wjob(const DProd* __restrict__ prods, const WSeg* __restrict__ segs, int nseg,
+                                             const int32_t* __restrict__ plist, int& local) {
+    int lo = 0, hi = nseg - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (segs[mid].begin <= (int)blockIdx.x) lo = mid;
+        else hi = mid - 1;
+    }
+    const WSeg g = segs[lo];
+    const int q = ((int)blockIdx.x - g.begin) / g.cpp;
+    local = (int)blockIdx.x - g.begin - q * g.cpp;
+    return prods[plist[g.first + q]];
+}
+
+constexpr int WT = 256;  // threads per CTA
+
+// ---------------------------------------------------------------------------
+// column passes: one thread holds the R rows of one column of one prime
+
+template <int ODD, int LJ>
+__global__ void __launch_bounds__(WT) k_wcol_fwd(const DProd* __restrict__ prods, const WSeg* __restrict__ segs,
+                                                 int nseg, const int32_t* __restrict__ plist) {
+    constexpr int R = ODD << LJ;
+    int local;
+    const DProd& P = wjob(prods, segs, nseg, plist, local);
+    const int lm = P.wlm;
+    const int id = local * WT + (int)threadIdx.x;
+    const int c = id & ((1 << lm) - 1);
+    int pi = id >> lm;  // operand-major: a's primes, then b's
+    const bool isb = pi >= WPR;
+    if (isb) pi -= WPR;
+    if (pi >= WPR || (isb && P.sqr)) return;
+    const uint64_t* __restrict__ src = isb ? P.b : P.a;
+    const int n = (int)(isb ? P.ncb : P.nca);
+    uint32_t* __restrict__ dst = (isb ? P.wb : P.wa) + (size_t)pi * (size_t)P.wN;
+    const uint32_t p = c_w.p[pi], p2 = 2 * p;
+    const Tw c32 = c_w.c32[pi], one = c_w.one[pi];
+    uint32_t x[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int i = c + (r << lm);
+        const uint64_t v = i < n ? __ldg(src + i) : 0ull;
+        const uint32_t y = wd::mulw((uint32_t)(v >> 32), c32, p) + wd::mulw((uint32_t)v, one, p);
+        x[r] = ODD > 1 ? wd::sub_if(y, p2) : y;
+    }
+    dft_odd<ODD, LJ>(x, pi, p);
+    const Tw* tab = (const Tw*)P.wtf + (((size_t)pi * ODD) << P.wL);
+#pragma unroll
+    for (int j = 0; j < ODD; j++) wd::tree_fwd<LJ, 1>(x + (j << LJ), tab + ((size_t)j << P.wL), 1u, p);
+#pragma unroll
+    for (int r = 0; r < R; r++) dst[c + (r << lm)] = x[r];
+}
+
+template <int ODD, int LJ>
+__global__ void __launch_bounds__(WT) k_wcol_rev(const DProd* __restrict__ prods, const WSeg* __restrict__ segs,
+                                                 int nseg, const int32_t* __restrict__ plist) {
+    constexpr int R = ODD << LJ;
+    int local;
+    const DProd& P = wjob(prods, segs, nseg, plist, local);
+    const int lm = P.wlm;
+    const int id = local * WT + (int)threadIdx.x;
+    const int c = id & ((1 << lm) - 1);
+    const int pi = id >> lm;
+    if (pi >= WPR) return;
+    uint32_t* __restrict__ dst = P.wa + (size_t)pi * (size_t)P.wN;
+    const uint32_t p = c_w.p[pi];
+    uint32_t x[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) x[r] = dst[c + (r << lm)];
+    const Tw* tab = (const Tw*)P.wti + (((size_t)pi * ODD) << P.wL);
+#pragma unroll
+    for (int j = 0; j < ODD; j++) wd::tree_rev<LJ, 1>(x + (j << LJ), tab + ((size_t)j << P.wL), 1u, p);
+    dft_odd<ODD, LJ>(x, pi, p);
+    // the inverse step is the forward one with output i at -i mod odd
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int i = r >> LJ, ri = (ODD - i) % ODD;
+        dst[c + (((ri << LJ) + (r & ((1 << LJ) - 1))) << lm)] = x[r];
+    }
+}
+
+// ---------------------------------------------------------------------------
+// blocks: M = 2^LM consecutive values on M/16 threads, 16 values per thread.
+// A round runs J levels on sub-blocks of 2^LL values; a thread takes 2^(4-J)
+// groups of 2^J values at stride S = 2^(LL-J).  The last round always runs two
+// levels on 16 consecutive values, leaving the thread four whole leaves.
+// Shared memory is padded by one word in 16: free of bank conflicts for the
+// strides 1, 4 and 16, at most two-way for the larger ones.
+
+__device__ __forceinline__ int wpad(int i) { return i + (i >> 4); }
+
+template <int LM, int LL, int J>
+__device__ __forceinline__ int wpos(int t, int q, int e) {
+    constexpr int S = 1 << (LL - J), T = 1 << (LM - 4);
+    const int gi = t + q * T;
+    return ((gi >> (LL - J)) << LL) + (gi & (S - 1)) + e * S;
+}
+template <int LM, int LL, int J>
+__device__ __forceinline__ void wround_fwd(uint32_t* x, int t, const Tw* __restrict__ tab, uint32_t h0, uint32_t p) {
+    constexpr int T = 1 << (LM - 4);
+#pragma unroll
+    for (int q = 0; q < (1 << (4 - J)); q++)
+        wd::tree_fwd<J, 1>(x + (q << J), tab, (h0 << (LM - LL)) + (uint32_t)((t + q * T) >> (LL - J)), p);
+}
+template <int LM, int LL, int J>
+__device__ __forceinline__ void wround_rev(uint32_t* x, int t, const Tw* __restrict__ tab, uint32_t h0, uint32_t p) {
+    constexpr int T = 1 << (LM - 4);
+#pragma unroll
+    for (int q = 0; q < (1 << (4 - J)); q++)
+        wd::tree_rev<J, 1>(x + (q << J), tab, (h0 << (LM - LL)) + (uint32_t)((t + q * T) >> (LL - J)), p);
+}
+template <int LM, int LL, int J>
+__device__ __forceinline__ void wput(uint32_t* s, const uint32_t* x, int t) {
+#pragma unroll
+    for (int k = 0; k < 16; k++) s[wpad(wpos<LM, LL, J>(t, k >> J, k & ((1 << J) - 1)))] = x[k];
+}
+template <int LM, int LL, int J>
+__device__ __forceinline__ void wget(const uint32_t* s, uint32_t* x, int t) {
+#pragma unroll
+    for (int k = 0; k < 16; k++) x[k] = s[wpad(wpos<LM, LL, J>(t, k >> J, k & ((1 << J) - 1)))];
+}
+
+// level splits of a block: J1, J2 (0: none), then the two leaf levels
+template <int LM>
+struct WSplit;
+template <>
+struct WSplit<12> { static constexpr int J1 = 4, J2 = 4; };
+template <>
+struct WSplit<10> { static constexpr int J1 = 3, J2 = 3; };
+template <>
+struct WSplit<8> { static constexpr int J1 = 4, J2 = 0; };
+template <>
+struct WSplit<6> { static constexpr int J1 = 2, J2 = 0; };
+
+// The block of `src` down to its leaves: x[0..16) = values 16t .. 16t+15 in [0, 4p).
+template <int LM>
+__device__ __forceinline__ void wblock_down(uint32_t* x, uint32_t* s, const uint32_t* __restrict__ src, int t,
+                                            const Tw* __restrict__ tab, uint32_t h0, uint32_t p, bool live) {
+    constexpr int J1 = WSplit<LM>::J1, J2 = WSplit<LM>::J2;
+    if (live) {
+#pragma unroll
+        for (int k = 0; k < 16; k++) x[k] = src[wpos<LM, LM, J1>(t, k >> J1, k & ((1 << J1) - 1))];
+        wround_fwd<LM, LM, J1>(x, t, tab, h0, p);
+        wput<LM, LM, J1>(s, x, t);
+    }
+    __syncthreads();
+    if constexpr (J2 > 0) {
+        if (live) {
+            wget<LM, LM - J1, J2>(s, x, t);
+            wround_fwd<LM, LM - J1, J2>(x, t, tab, h0, p);
+            wput<LM, LM - J1, J2>(s, x, t);
+        }
+        __syncthreads();
+    }
+    if (live) {
+#pragma unroll
+        for (int k = 0; k < 16; k++) x[k] = s[17 * t + k];
+        const uint32_t idx = (h0 << (LM - 4)) + (uint32_t)t, p2 = 2 * p;
+        Tw w1[1], w2[2];
+        wd::load_tw<0>(tab, idx, w1);
+        wd::load_tw<1>(tab, idx, w2);
+#pragma unroll
+        for (int e = 0; e < 8; e++) wd::bf_fwd(x[e], x[e + 8], w1[0], p, p2);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            wd::bf_fwd(x[e], x[e + 4], w2[0], p, p2);
+            wd::bf_fwd(x[e + 8], x[e + 12], w2[1], p, p2);
+        }
+    }
+}
+
+// c = a * b mod X^4 - rho (rho in 2^32 form), a in [0, p), b in [0, 2p); the
+// result carries a factor 2^-32 and lies in [0, 2p).  Sums of at most four
+// products of 2p^2 and one of 2.5p * p stay below 2^64.
+__device__ __forceinline__ void wleaf(uint32_t* a, const uint32_t* b, uint32_t rho, uint32_t p, uint32_t pinv) {
+    uint32_t h[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        uint64_t s = 0;
+#pragma unroll
+        for (int i = k + 1; i < 4; i++) s += wd::mulx(a[i], b[k + 4 - i]);
+        h[k] = wd::redc(s, p, pinv);
+    }
+    uint32_t c[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        uint64_t s = k < 3 ? wd::mulx(h[k], rho) : 0;
+#pragma unroll
+        for (int i = 0; i <= k; i++) s += wd::mulx(a[i], b[k - i]);
+        c[k] = wd::sub_if(wd::redc(s, p, pinv), 2 * p);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) a[k] = c[k];
+}
+
+template <int LM>
+__global__ void __launch_bounds__(WT, 3) k_wblock(const DProd* __restrict__ prods, const WSeg* __restrict__ segs,
+                                                  int nseg, const int32_t* __restrict__ plist) {
+    constexpr int T = 1 << (LM - 4), PER = WT / T;  // threads per block, blocks per CTA
+    constexpr int SM = (1 << LM) + (1 << (LM - 4));
+    constexpr int J1 = WSplit<LM>::J1, J2 = WSplit<LM>::J2;
+    __shared__ uint32_t sm[2][PER][SM];
+    int local;
+    const DProd& P = wjob(prods, segs, nseg, plist, local);
+    const int g = (int)threadIdx.x / T, t = (int)threadIdx.x & (T - 1);
+    const int R = P.wodd << P.wlj;
+    const int blk = local * PER + g;  // prime-major, then block
+    const bool live = blk < WPR * R;
+    const int pi = live ? blk / R : 0, row = live ? blk - pi * R : 0;
+    const int j = row >> P.wlj;
+    const uint32_t h0 = (1u << P.wlj) + (uint32_t)(row & ((1 << P.wlj) - 1));
+    const uint32_t p = c_w.p[pi], pinv = c_w.pinv[pi], p2 = 2 * p;
+    const size_t toff = ((size_t)pi * P.wodd + j) << P.wL;
+    const Tw* tf = (const Tw*)P.wtf + toff;
+    uint32_t* xa = P.wa + (size_t)pi * (size_t)P.wN + ((size_t)row << LM);
+    uint32_t a[16];
+    wblock_down<LM>(a, sm[0][g], xa, t, tf, h0, p, live);
+    if (!P.sqr) {
+        uint32_t b[16];
+        wblock_down<LM>(b, sm[1][g], P.wb + (size_t)pi * (size_t)P.wN + ((size_t)row << LM), t, tf, h0, p, live);
+        if (live) {
+            Tw w2[2];
+            wd::load_tw<1>(tf, (h0 << (LM - 4)) + (uint32_t)t, w2);
+            const uint32_t r0 = 0u - w2[0].q * p, r1 = 0u - w2[1].q * p;  // w * 2^32 mod p
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                a[k] = wd::sub_if(wd::sub_if(a[k], p2), p);
+                b[k] = wd::sub_if(b[k], p2);
+            }
+            wleaf(a, b, r0, p, pinv);
+            wleaf(a + 4, b + 4, p - r0, p, pinv);
+            wleaf(a + 8, b + 8, r1, p, pinv);
+            wleaf(a + 12, b + 12, p - r1, p, pinv);
+        }
+    } else if (live) {
+        Tw w2[2];
+        wd::load_tw<1>(tf, (h0 << (LM - 4)) + (uint32_t)t, w2);
+        const uint32_t r0 = 0u - w2[0].q * p, r1 = 0u - w2[1].q * p;
+#pragma unroll
+        for (int k = 0; k < 16; k++) a[k] = wd::sub_if(wd::sub_if(a[k], p2), p);
+#pragma unroll
+        for (int l = 0; l < 4; l++) {
+            uint32_t b[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) b[k] = a[4 * l + k];
+            const uint32_t rr = l < 2 ? r0 : r1;
+            wleaf(a + 4 * l, b, (l & 1) ? p - rr : rr, p, pinv);
+        }
+    }
+    // back up (shared buffer 1: its last readers passed a barrier, or none used it)
+    const Tw* ti = (const Tw*)P.wti + toff;
+    uint32_t* s = sm[1][g];
+    if (live) {
+        const uint32_t idx = (h0 << (LM - 4)) + (uint32_t)t;
+        Tw w1[1], w2[2];
+        wd::load_tw<0>(ti, idx, w1);
+        wd::load_tw<1>(ti, idx, w2);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            wd::bf_rev(a[e], a[e + 4], w2[0], p, p2);
+            wd::bf_rev(a[e + 8], a[e + 12], w2[1], p, p2);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e++) wd::bf_rev(a[e], a[e + 8], w1[0], p, p2);
+        // each thread rewrites the 16 words only it read last
+#pragma unroll
+        for (int k = 0; k < 16; k++) s[17 * t + k] = a[k];
+    }
+    __syncthreads();
+    if constexpr (J2 > 0) {
+        if (live) {
+            wget<LM, LM - J1, J2>(s, a, t);
+            wround_rev<LM, LM - J1, J2>(a, t, ti, h0, p);
+            wput<LM, LM - J1, J2>(s, a, t);
+        }
+        __syncthreads();
+    }
+    if (live) {
+        wget<LM, LM, J1>(s, a, t);
+        wround_rev<LM, LM, J1>(a, t, ti, h0, p);
+#pragma unroll
+        for (int k = 0; k < 16; k++) xa[wpos<LM, LM, J1>(t, k >> J1, k & ((1 << J1) - 1))] = a[k];
+    }
+}
+
+// ---------------------------------------------------------------------------
+// unpack: coefficients and carried limbs, tiles of UNPACK_TL limbs
+
+// The coefficient whose residues (any representatives below 4p, scaled) are r:
+// mixed-radix digits y_i, each one sum of wide products and one reduction,
+// then sum y_i W_i by Horner's rule.
+__device__ __forceinline__ void wcoef(const uint32_t* r, const uint32_t* sc, uint32_t* v) {
+    uint32_t y[WPR];
+#pragma unroll
+    for (int i = 0; i < WPR; i++) {
+        const uint32_t p = c_w.p[i];
+        uint64_t s = wd::mulx(r[i], sc[i]);  // < 4p^2; the others < 1.3p^2 each
+#pragma unroll
+        for (int j = 0; j < i; j++) s += wd::mulx(y[j], c_w.gar[i][j]);
+        y[i] = wd::sub_if(wd::sub_if(wd::redc(s, p, c_w.pinv[i]), 2 * p), p);
+    }
+    v[0] = y[WPR - 1];
+#pragma unroll
+    for (int i = WPR - 2; i >= 0; i--) {
+        uint64_t cy = y[i];
+        const uint32_t p = c_w.p[i];
+#pragma unroll
+        for (int k = 0; k < WPR - 1 - i; k++) {
+            cy += wd::mulx(v[k], p);
+            v[k] = (uint32_t)cy;
+            cy >>= 32;
+        }
+        v[WPR - 1 - i] = (uint32_t)cy;
+    }
+}
+
+__device__ __forceinline__ uint32_t gp_join(uint32_t lower, uint32_t upper) {
+    // bit 0 generate, bit 1 propagate; lower limbs, then upper
+    return ((upper & 1u) | ((upper >> 1) & lower & 1u)) | (upper & lower & 2u);
+}
+
+__global__ void __launch_bounds__(WT) k_wunpack(const DProd* __restrict__ prods, const WSeg* __restrict__ segs, int nseg,
+                                                const int32_t* __restrict__ plist) {
+    __shared__ uint64_t s_mid[WT + 1];           // mid word of the last coefficient of thread t - 1
+    __shared__ uint32_t s_hi[WT + 1][2];         // high words of its last two coefficients
+    __shared__ uint32_t s_c[WT + 1];             // carry out of its last limb sum
+    __shared__ uint64_t h_lo, h_mid2;            // halo: limb sum w0 - 1
+    __shared__ uint32_t h_hi3;
+    __shared__ uint32_t wagg[WT / 32];
+    int tile;
+    const DProd& P = wjob(prods, segs, nseg, plist, tile);
+    const int t = (int)threadIdx.x;
+    const int N = P.wN;
+    const uint32_t* __restrict__ x = P.wa;
+    const int64_t w0 = (int64_t)tile * UNPACK_TL, w1 = min(w0 + (int64_t)UNPACK_TL, P.rn);
+    uint32_t sc[WPR];
+#pragma unroll
+    for (int i = 0; i < WPR; i++) sc[i] = P.wsc[i];
+    // the three coefficients before the tile
+    if (t < 3) {
+        const int64_t i = w0 - 1 - t;
+        uint32_t v[WPR] = {0, 0, 0, 0, 0};
+        if (i >= 0 && i < N) {
+            uint32_t r[WPR];
+#pragma unroll
+            for (int k = 0; k < WPR; k++) r[k] = x[(size_t)k * N + i];
+            wcoef(r, sc, v);
+        }
+        const uint64_t lo = v[0] | (uint64_t)v[1] << 32, mid = v[2] | (uint64_t)v[3] << 32;
+        if (t == 0) {
+            h_lo = lo;
+            s_mid[0] = mid;
+            s_hi[0][1] = v[4];
+        } else if (t == 1) {
+            h_mid2 = mid;
+            s_hi[0][0] = v[4];
+        } else {
+            h_hi3 = v[4];
+        }
+    }
+    const int64_t wt = w0 + 4 * t;
+    uint64_t lo[4], mid[4];
+    uint32_t hi[4];
+    if (wt < N) {  // N is a multiple of 4: all four or none
+        uint32_t r[4][WPR];
+#pragma unroll
+        for (int k = 0; k < WPR; k++) {
+            const uint4 q = *reinterpret_cast<const uint4*>(x + (size_t)k * N + wt);
+            r[0][k] = q.x;
+            r[1][k] = q.y;
+            r[2][k] = q.z;
+            r[3][k] = q.w;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            uint32_t v[WPR];
+            wcoef(r[q], sc, v);
+            lo[q] = v[0] | (uint64_t)v[1] << 32;
+            mid[q] = v[2] | (uint64_t)v[3] << 32;
+            hi[q] = v[4];
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; q++) lo[q] = mid[q] = 0, hi[q] = 0;
+    }
+    s_mid[t + 1] = mid[3];
+    s_hi[t + 1][0] = hi[2];
+    s_hi[t + 1][1] = hi[3];
+    __syncthreads();
+    // limb sums lo_i + mid_(i-1) + hi_(i-2) and their carries (0..2)
+    uint64_t own[4];
+    uint32_t cy[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint64_t m1 = q ? mid[q - 1] : s_mid[t];
+        const uint32_t h2 = q > 1 ? hi[q - 2] : s_hi[t][q];
+        uint64_t s = lo[q] + m1;
+        uint32_t c = s < m1;
+        s += h2;
+        c += s < h2;
+        own[q] = s;
+        cy[q] = c;
+    }
+    s_c[t + 1] = cy[3];
+    if (t == 0) {
+        uint64_t s = h_lo + h_mid2;
+        uint32_t c = s < h_mid2;
+        s += h_hi3;
+        c += s < h_hi3;
+        s_c[0] = c;
+    }
+    __syncthreads();
+    uint32_t gen = 0, prop = 1;
+    {
+        uint32_t k = s_c[t];  // carry of the sum below
+        uint32_t g = 0;       // carry generated by adding it
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint64_t s = own[q] + k + g;  // at most one of the wraps happens: k + g <= 3
+            g = s < (uint64_t)(k + g);
+            own[q] = s;
+            k = cy[q];
+            prop &= (wt + q < w1 && s == ~0ULL) ? 1u : 0u;
+        }
+        gen = g;
+    }
+    const uint32_t agg = gen | (prop << 1);
+    const int lane = t & 31, wid = t >> 5;
+    uint32_t incl = agg;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl = gp_join(o, incl);
+    }
+    if (lane == 31) wagg[wid] = incl;
+    __syncthreads();
+    uint32_t wpre = 2u;
+    for (int k = 0; k < wid; k++) wpre = gp_join(wpre, wagg[k]);
+    uint32_t excl = __shfl_up_sync(0xffffffffu, incl, 1);
+    if (lane == 0) excl = 2u;
+    uint64_t cin = gp_join(wpre, excl) & 1u;  // tile carry-in taken as 0; k_carry adds it
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        own[q] += cin;
+        cin = cin && own[q] == 0;
+    }
+    if (wt + 3 < w1) {
+        ulonglong2* dst = reinterpret_cast<ulonglong2*>(P.r + wt);
+        if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+            dst[0] = make_ulonglong2(own[0], own[1]);
+            dst[1] = make_ulonglong2(own[2], own[3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; q++) P.r[wt + q] = own[q];
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (wt + q < w1) P.r[wt + q] = own[q];
+    }
+    if (t == WT - 1) {
+        uint32_t tot = 2u;
+        for (int k = 0; k < WT / 32; k++) tot = gp_join(tot, wagg[k]);
+        P.agg[tile] = tot;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// launches
+
+int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t rn) {
+    const int64_t M = int64_t(1) << s.lm, R = (int64_t)s.odd << s.lj;
+    switch (kind) {
+        case JK_WCOL_FWD: return ((sqr ? 1 : 2) * WPR * M + WT - 1) / WT;
+        case JK_WCOL_REV: return (WPR * M + WT - 1) / WT;
+        case JK_WBLOCK: return (WPR * R * (M / 16) + WT - 1) / WT;
+        default: return (rn + UNPACK_TL - 1) / UNPACK_TL;
+    }
+}
+
+template <int ODD, int LJ>
+static void col_launch(int kind, const DProd* prods, const WSeg* segs, int nseg, const int32_t* plist, unsigned grid,
+                       cudaStream_t st) {
+    if (kind == JK_WCOL_FWD) k_wcol_fwd<ODD, LJ><<<grid, WT, 0, st>>>(prods, segs, nseg, plist);
+    else k_wcol_rev<ODD, LJ><<<grid, WT, 0, st>>>(prods, segs, nseg, plist);
+}
+
+cudaError_t launch_word(int kind, int variant, const DProd* prods, const WSeg* segs, int nseg, const int32_t* plist,
+                        int64_t nctas, cudaStream_t st) {
+    if (nctas <= 0) return cudaSuccess;
+    if (nctas > 0x7fffffff) return cudaErrorInvalidValue;
+    const unsigned grid = (unsigned)nctas;
+    if (kind == JK_WUNPACK) {
+        k_wunpack<<<grid, WT, 0, st>>>(prods, segs, nseg, plist);
+    } else if (kind == JK_WBLOCK) {
+        switch (variant) {
+            case 12: k_wblock<12><<<grid, WT, 0, st>>>(prods, segs, nseg, plist); break;
+            case 10: k_wblock<10><<<grid, WT, 0, st>>>(prods, segs, nseg, plist); break;
+            case 8: k_wblock<8><<<grid, WT, 0, st>>>(prods, segs, nseg, plist); break;
+            case 6: k_wblock<6><<<grid, WT, 0, st>>>(prods, segs, nseg, plist); break;
+            default: return cudaErrorInvalidValue;
+        }
+    } else {
+        switch (variant) {
+#define NBG_COL(O, J) \
+    case (O << 8) | J: col_launch<O, J>(kind, prods, segs, nseg, plist, grid, st); break;
+            NBG_COL(1, 1) NBG_COL(1, 2) NBG_COL(1, 3) NBG_COL(1, 4) NBG_COL(1, 5)
+            NBG_COL(3, 0) NBG_COL(3, 1) NBG_COL(3, 2) NBG_COL(3, 3)
+            NBG_COL(5, 0) NBG_COL(5, 1) NBG_COL(5, 2)
+            NBG_COL(7, 0) NBG_COL(7, 1) NBG_COL(7, 2)
+#undef NBG_COL
+            default: return cudaErrorInvalidValue;
+        }
+    }
+    return cudaGetLastError();
+}
+
+}  // namespace nbg

@@ -1,0 +1,86 @@
+"""Products through the five-prime word transforms (one 64-bit limb per
+coefficient): every transform shape at its exact length and one below, values
+whose coefficients and carries are extreme, and mixed batches, all equal to
+GMP's product and to the FP64 passes' (integers: no tolerance)."""
+import json
+
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import adversarial, rand_limbs
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+# (odd multiplier, log2 of the rest): each column-pass and block variant, the
+# smallest and largest lengths of the range
+SHAPES = [(1, 7), (1, 8), (1, 9), (1, 10), (1, 11), (1, 12), (1, 13), (1, 14), (1, 15), (1, 16), (1, 17),
+          (3, 6), (3, 7), (3, 9), (3, 10), (3, 12), (3, 13), (3, 14), (3, 15),
+          (5, 6), (5, 7), (5, 8), (5, 12), (5, 13), (5, 14),
+          (7, 6), (7, 7), (7, 10), (7, 12), (7, 13), (7, 14)]
+
+
+def _want(a, b):
+    return O.gmp_sqr(a) if b is None else O.gmp_mul(a, b)
+
+
+def _kinds(nbgpu, a, b):
+    da, db = torch.from_numpy(a).cuda(), None if b is None else torch.from_numpy(b).cuda()
+    r = torch.zeros(a.size + (a.size if b is None else b.size), dtype=torch.uint64, device="cuda")
+    bits = [64 * x.size for x in (a, a if b is None else b)]
+    bt = nbgpu.Batch(nbgpu.make_descs([(r, da, db, a.size, r.numel() - a.size, *bits)]))
+    kinds = {s["kind"] for s in bt.stats()}
+    bt.close()
+    return kinds
+
+
+@pytest.mark.parametrize("odd,k", SHAPES)
+def test_word_shapes(gpu_lib, odd, k):
+    N = odd << k
+    rng = np.random.default_rng(N)
+    for n1 in (N + 1, N):  # m + n - 1 = N and N - 1 coefficients
+        n = n1 * 2 // 5
+        a, b = rand_limbs(rng, n1 - n), rand_limbs(rng, n)
+        assert np.array_equal(gpu_lib.mul(a, b), _want(a, b))
+        # the largest coefficients and a carry through every limb
+        ones = np.full(n1 - n, 2**64 - 1, dtype=np.uint64)
+        assert np.array_equal(gpu_lib.mul(ones, ones[:n].copy()), _want(ones, ones[:n].copy()))
+    s = rand_limbs(rng, (N + 1) // 2)
+    assert np.array_equal(gpu_lib.sqr(s), _want(s, None))
+
+
+def test_word_kernels_run_and_edge_operands(gpu_lib):
+    rng = np.random.default_rng(77)
+    a, b = rand_limbs(rng, 3000), rand_limbs(rng, 2500)
+    assert "k_wunpack" in _kinds(gpu_lib, a, b) and "k_wunpack" in _kinds(gpu_lib, a, None)
+    for m, n in ((1, 1), (2, 1), (700, 1), (513, 512), (65536, 65537), (130000, 3)):
+        x, y = adversarial(rng, m), adversarial(rng, n)
+        assert np.array_equal(gpu_lib.mul(x, y), _want(x, y))
+    z = np.zeros(4096, dtype=np.uint64)  # zero limbs above the magnitude
+    z[:3] = rand_limbs(rng, 3)
+    assert np.array_equal(gpu_lib.mul(z, a), _want(z, a))
+    # odd limb offsets on both sides (8-byte aligned buffers)
+    buf, out = rand_limbs(rng, 9001), np.zeros(9003, dtype=np.uint64)
+    gpu_lib.mul_(out, 1, buf, 3, 5000, buf, 5003, 3998)
+    assert np.array_equal(out[1:8999], _want(buf[3:5003].copy(), buf[5003:9001].copy()))
+
+
+def test_word_batch_equals_fp64_passes(gpu_lib):
+    rng = np.random.default_rng(78)
+    pairs = [(adversarial(rng, int(m)), None if k % 5 == 0 else adversarial(rng, max(1, int(m * f))))
+             for k, (m, f) in enumerate(zip(np.exp(rng.uniform(0, np.log(150000), 120)), rng.uniform(0.01, 1, 120)))]
+    got = gpu_lib.mul_batch(pairs)
+    old = gpu_lib.get_tuning()
+    try:
+        t = json.loads(old)
+        t["cmax"] = 64  # pass knobs other than the loaded ones: the FP64 passes
+        gpu_lib.set_tuning(json.dumps(t))
+        assert "k_wunpack" not in _kinds(gpu_lib, *pairs[1])
+        ref = gpu_lib.mul_batch(pairs)
+    finally:
+        gpu_lib.set_tuning(old)
+    for (a, b), g, r in zip(pairs, got, ref):
+        assert np.array_equal(g, r)
+        assert np.array_equal(g, _want(a, b))
