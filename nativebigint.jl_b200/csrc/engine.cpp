@@ -782,6 +782,13 @@ static inline int64_t eff_limbs(int64_t limbs, int64_t bits) {
     return bits < 1 ? limbs : std::max<int64_t>(1, std::min(limbs, (bits + 63) / 64));
 }
 
+size_t fp64_work_bytes(const ProdIn& q) {
+    int b;
+    int64_t N;
+    if (ntt_params(q.bits_a, q.sqr ? q.bits_a : q.bits_b, &b, &N) != NBG_OK) return SIZE_MAX;
+    return sizeof(double) * 2 * (size_t)N * (q.sqr ? 1 : 2);
+}
+
 bool word_product(const Engine& E, const ProdIn& q, WordShape* s) {
     if (!E.word_ok || q.fp64 || q.keep_b) return false;
     const int64_t la = eff_limbs(q.m, q.bits_a), lb = q.sqr ? la : eff_limbs(q.n, q.bits_b);
@@ -827,6 +834,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
             P.wN = ws.N;
             P.wodd = ws.odd;
             P.wlj = ws.lj;
+            P.wj2 = ws.j2;
             P.wlm = ws.lm;
             P.wL = wt->L;
             P.wtf = wt->fwd;
@@ -870,7 +878,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     }
     bb.agg_words = aggw;
     bb.agg_off = agg_off;
-    if (!words.empty()) pmax = std::max(pmax, 2);  // their column, block and column-back steps
+    for (int32_t k : words) pmax = std::max(pmax, bb.prods[(size_t)k].wj2 ? 3 : 2);  // column passes before and after the blocks
 
     // Jobs of one pipeline step, grouped by kernel and shared-memory size: a
     // launch reserves its largest job's shared memory for every CTA, so a
@@ -1092,7 +1100,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     });
     for (int32_t k : words) {
         const DProd& P = bb.prods[(size_t)k];
-        const WordShape ws{P.wN, P.wodd, P.wlj, P.wlm};
+        const WordShape ws{P.wN, P.wodd, P.wlj, P.wj2, P.wlm};
         const double res = 4.0 * WPR * P.wN, nop = P.sqr ? 1 : 2;
         auto put = [&](int step, int kind, int variant, double bytes) {
             WGroup& g = wgroups[std::make_tuple(step, kind, variant)];
@@ -1103,9 +1111,14 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
             g.nctas += cpp;
             g.bytes += bytes;
         };
-        put(pmax - 2, JK_WCOL_FWD, (P.wodd << 8) | P.wlj, 8.0 * (double)(P.nca + (P.sqr ? 0 : P.ncb)) + nop * res);
+        const int col = (P.wodd << 8) | (P.wlj - P.wj2);
+        // the block step is pmax - 1; a middle pass takes the steps next to it
+        const int far = P.wj2 ? 2 : 1;
+        put(pmax - 1 - far, JK_WCOL_FWD, col, 8.0 * (double)(P.nca + (P.sqr ? 0 : P.ncb)) + nop * res);
+        if (P.wj2) put(pmax - 2, JK_WMID_FWD, P.wj2, 2 * nop * res);
         put(pmax - 1, JK_WBLOCK, P.wlm, (nop + 1) * res);
-        put(pmax, JK_WCOL_REV, (P.wodd << 8) | P.wlj, 2 * res);
+        if (P.wj2) put(pmax, JK_WMID_REV, P.wj2, 2 * res);
+        put(pmax - 1 + far, JK_WCOL_REV, col, 2 * res);
         put(2 * pmax - 1, JK_WUNPACK, 0, res + 8.0 * (double)P.rn);
     }
     for (auto& kv : wgroups)

@@ -130,6 +130,8 @@ struct ProdIn {
 
 // Whether the product runs on the word engine (shape in *s), from its sizes alone.
 bool word_product(const Engine& E, const ProdIn& q, WordShape* s);
+// Transform buffers of the product on the multi-pass FP64 engine (SIZE_MAX: no such transform).
+size_t fp64_work_bytes(const ProdIn& q);
 
 struct Launch {
     int kind;

@@ -194,8 +194,21 @@ bool nbg_server::launch_batch(std::unique_lock<std::mutex>& lk) {
     int refuse = 0;
     {
         std::lock_guard<std::recursive_mutex> elk(E.mu);
+        // Admission is by the FP64 engine's workspace, the larger one: the
+        // budget admits the same requests whichever engine runs them.  An
+        // oversized request is refused when it reaches the front.
+        for (size_t k = 0; k < in.size(); k++) {
+            if (in[k].bits_a < 1 || (!in[k].sqr && in[k].bits_b < 1)) continue;
+            size_t need = fp64_work_bytes(in[k]);
+            if (need < ((size_t)1 << 20) || need == SIZE_MAX) continue;  // one pass, or refused by build_batch
+            if (host[k]) need += 8 * (size_t)(in[k].sqr ? 3 * in[k].m : 2 * (in[k].m + in[k].n));
+            if (need <= arena.size()) continue;
+            if (k) in.resize(k);
+            else refuse = fail(NBG_ENOMEM, "request needs %zu bytes, over the server's HBM budget", need);
+            break;
+        }
         // shrink the batch until it fits in the free arena
-        for (;;) {
+        while (!refuse) {
             int rc = build_batch(E, in.data(), (int64_t)in.size(), f.bb);
             if (rc) {  // a request the engine refuses (size): fail it alone
                 if (in.size() == 1) {

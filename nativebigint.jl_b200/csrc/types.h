@@ -87,7 +87,7 @@ struct DProd {
     uint32_t* wb;
     const void* wtf;     // forward and inverse constants, [prime][block][2^wL]
     const void* wti;
-    int32_t wN, wodd, wlj, wlm, wL;
+    int32_t wN, wodd, wlj, wj2, wlm, wL;
     uint32_t wsc[5];     // unpack scale per prime
 };
 
@@ -218,6 +218,8 @@ enum JobKind : int32_t {
     JK_WBLOCK = 11,  // word products: blocks of the remaining levels, leaf products, and back
     JK_WCOL_REV = 12,// word products: the first levels backwards
     JK_WUNPACK = 13, // word products: coefficients and carried limbs
+    JK_WMID_FWD = 14,// word products: a middle column pass
+    JK_WMID_REV = 15,// word products: a middle column pass backwards
 };
 
 constexpr int UNPACK_TL = 1024;  // output limbs per unpack tile

@@ -27,11 +27,13 @@ constexpr uint32_t WPRIMES[WPR] = {1073479681u, 1018429441u, 908328961u, 8808038
 constexpr int WORD_MAX_LOG2 = 20;               // k <= 20 (leaves at level k - 2 <= 18)
 constexpr int64_t WORD_MIN_OPERAND_MAX = int64_t(1) << 21;
 
-// Shape of a word product's transform: N = R * M, R = odd * 2^lj rows.  Column
-// passes work on the R rows of one column in registers; blocks of M = 2^lm
-// consecutive values (each one subtree) are transformed in shared memory.
+// Shape of a word product's transform: N = odd * 2^lj * M.  Blocks of M = 2^lm
+// consecutive values (each one subtree) are transformed in shared memory;
+// column passes above them work on the rows of one column in registers: one
+// pass of odd * 2^lj rows, or, past 32 rows, a first one of odd * 2^(lj - j2)
+// and a middle one of 2^j2.
 struct WordShape {
-    int32_t N = 0, odd = 0, lj = 0, lm = 0;
+    int32_t N = 0, odd = 0, lj = 0, j2 = 0, lm = 0;
 };
 // The smallest supported length >= nconv; false when there is none.
 bool word_shape(int64_t nconv, WordShape& s);
@@ -44,7 +46,7 @@ struct WSeg {
     int32_t pad_;
 };
 
-// variant of a word launch: (odd << 8) | lj for column passes, lm for blocks
+// variant of a word launch: (odd << 8) | (lj - j2) for column passes, j2 for middle ones, lm for blocks
 cudaError_t word_init();  // constant memory of the current device
 cudaError_t launch_word(int kind, int variant, const DProd* prods, const WSeg* segs, int nseg, const int32_t* plist,
                         int64_t nctas, cudaStream_t st);

@@ -3,13 +3,15 @@
 //
 //   k_wcol_fwd  limbs -> residues, the radix-`odd` step and the first lj levels
 //               of one column's R rows, in registers
+//   k_wmid      long transforms: the levels between the first column pass and
+//               the blocks, in registers
 //   k_wblock    per block of M values: the other levels of a and b, the leaf
 //               products, the levels back
 //   k_wcol_rev  the first lj levels and the radix-`odd` step backwards
 //   k_wunpack   five residues -> coefficient (mixed radix), carried limb sums
 #include <cuda_runtime.h>
 
-#include <atomic>
+#include <algorithm>
 #include <type_traits>
 
 #include "word.cuh"
@@ -112,23 +114,34 @@ void word_scales(const WordShape& s, uint32_t out[WPR]) {
     }
 }
 
+// The split of the rows above the blocks: one column pass up to 32 rows (its
+// values fit a thread's registers), else the two passes whose larger row count
+// is least.
+static bool row_split(int odd, int lj, int& j2) {
+    j2 = 0;
+    const int64_t R = (int64_t)odd << lj;
+    if (R <= 32) return R >= 2;
+    int64_t best = INT64_MAX;
+    for (int j = 2; j <= 5 && j <= lj; j++) {
+        const int64_t r1 = (int64_t)odd << (lj - j), r2 = int64_t(1) << j;
+        if (r1 < 2 || r1 > 32 || std::max(r1, r2) >= best) continue;
+        best = std::max(r1, r2);
+        j2 = j;
+    }
+    return best != INT64_MAX;
+}
+
 bool word_shape(int64_t nconv, WordShape& s) {
     int64_t best = INT64_MAX;
     for (int odd : {1, 3, 5, 7}) {
         for (int k = 6; k <= WORD_MAX_LOG2; k++) {
             const int64_t N = (int64_t)odd << k;
             if (N < nconv || N >= best) continue;
-            // block of at most 4096 with 2 <= R <= 32 rows
             for (int lm : {12, 10, 8, 6}) {
-                const int lj = k - lm;
-                if (lj < 0) continue;
-                const int64_t R = (int64_t)odd << lj;
-                if (R < 2 || R > 32) continue;
+                int j2;
+                if (k < lm || !row_split(odd, k - lm, j2)) continue;
                 best = N;
-                s.N = (int32_t)N;
-                s.odd = odd;
-                s.lj = lj;
-                s.lm = lm;
+                s = WordShape{(int32_t)N, odd, k - lm, j2, lm};
                 break;
             }
         }
@@ -279,7 +292,7 @@ __global__ void __launch_bounds__(WT) k_wcol_fwd(const DProd* __restrict__ prods
     constexpr int R = ODD << LJ;
     int local;
     const DProd& P = wjob(prods, segs, nseg, plist, local);
-    const int lm = P.wlm;
+    const int lm = P.wlm + P.wj2;  // log2 of the column count
     const int id = local * WT + (int)threadIdx.x;
     const int c = id & ((1 << lm) - 1);
     int pi = id >> lm;  // operand-major: a's primes, then b's
@@ -313,7 +326,7 @@ __global__ void __launch_bounds__(WT) k_wcol_rev(const DProd* __restrict__ prods
     constexpr int R = ODD << LJ;
     int local;
     const DProd& P = wjob(prods, segs, nseg, plist, local);
-    const int lm = P.wlm;
+    const int lm = P.wlm + P.wj2;  // log2 of the column count
     const int id = local * WT + (int)threadIdx.x;
     const int c = id & ((1 << lm) - 1);
     const int pi = id >> lm;
@@ -333,6 +346,35 @@ __global__ void __launch_bounds__(WT) k_wcol_rev(const DProd* __restrict__ prods
         const int i = r >> LJ, ri = (ODD - i) % ODD;
         dst[c + (((ri << LJ) + (r & ((1 << LJ) - 1))) << lm)] = x[r];
     }
+}
+
+// Middle passes: the 2^J rows (2^lm apart) of one column of a segment, the
+// subtree of the segment's node.  In place; all columns of a segment share
+// their constants.
+template <int J, bool FWD>
+__global__ void __launch_bounds__(WT) k_wmid(const DProd* __restrict__ prods, const WSeg* __restrict__ segs, int nseg,
+                                             const int32_t* __restrict__ plist) {
+    int local;
+    const DProd& P = wjob(prods, segs, nseg, plist, local);
+    const int lm = P.wlm, j1 = P.wlj - J, R1 = P.wodd << j1;
+    const int id = local * WT + (int)threadIdx.x;
+    const int c = id & ((1 << lm) - 1);
+    int op = (id >> lm) / R1;  // operand-major, then prime
+    const int seg = (id >> lm) - op * R1;
+    const bool isb = op >= WPR;
+    const int pi = isb ? op - WPR : op;
+    if (pi >= WPR || (isb && (!FWD || P.sqr))) return;
+    uint32_t* __restrict__ x0 = (isb ? P.wb : P.wa) + (size_t)pi * (size_t)P.wN + ((size_t)seg << (lm + J)) + c;
+    const uint32_t p = c_w.p[pi];
+    const Tw* tab = (const Tw*)(FWD ? P.wtf : P.wti) + (((size_t)pi * P.wodd + (seg >> j1)) << P.wL);
+    const uint32_t node = (1u << j1) + (uint32_t)(seg & ((1 << j1) - 1));
+    uint32_t x[1 << J];
+#pragma unroll
+    for (int r = 0; r < (1 << J); r++) x[r] = x0[(size_t)r << lm];
+    if (FWD) wd::tree_fwd<J, 1>(x, tab, node, p);
+    else wd::tree_rev<J, 1>(x, tab, node, p);
+#pragma unroll
+    for (int r = 0; r < (1 << J); r++) x0[(size_t)r << lm] = x[r];
 }
 
 // ---------------------------------------------------------------------------
@@ -726,9 +768,12 @@ __global__ void __launch_bounds__(WT) k_wunpack(const DProd* __restrict__ prods,
 
 int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t rn) {
     const int64_t M = int64_t(1) << s.lm, R = (int64_t)s.odd << s.lj;
+    const int64_t cols = M << s.j2, mcols = (int64_t)s.N >> s.j2;
     switch (kind) {
-        case JK_WCOL_FWD: return ((sqr ? 1 : 2) * WPR * M + WT - 1) / WT;
-        case JK_WCOL_REV: return (WPR * M + WT - 1) / WT;
+        case JK_WCOL_FWD: return ((sqr ? 1 : 2) * WPR * cols + WT - 1) / WT;
+        case JK_WCOL_REV: return (WPR * cols + WT - 1) / WT;
+        case JK_WMID_FWD: return ((sqr ? 1 : 2) * WPR * mcols + WT - 1) / WT;
+        case JK_WMID_REV: return (WPR * mcols + WT - 1) / WT;
         case JK_WBLOCK: return (WPR * R * (M / 16) + WT - 1) / WT;
         default: return (rn + UNPACK_TL - 1) / UNPACK_TL;
     }
@@ -754,6 +799,18 @@ cudaError_t launch_word(int kind, int variant, const DProd* prods, const WSeg* s
             case 10: k_wblock<10><<<grid, WT, 0, st>>>(prods, segs, nseg, plist); break;
             case 8: k_wblock<8><<<grid, WT, 0, st>>>(prods, segs, nseg, plist); break;
             case 6: k_wblock<6><<<grid, WT, 0, st>>>(prods, segs, nseg, plist); break;
+            default: return cudaErrorInvalidValue;
+        }
+    } else if (kind == JK_WMID_FWD || kind == JK_WMID_REV) {
+        const bool f = kind == JK_WMID_FWD;
+        switch (variant) {
+#define NBG_MID(J)                                                               \
+    case J:                                                                      \
+        if (f) k_wmid<J, true><<<grid, WT, 0, st>>>(prods, segs, nseg, plist);   \
+        else k_wmid<J, false><<<grid, WT, 0, st>>>(prods, segs, nseg, plist);    \
+        break;
+            NBG_MID(2) NBG_MID(3) NBG_MID(4) NBG_MID(5)
+#undef NBG_MID
             default: return cudaErrorInvalidValue;
         }
     } else {

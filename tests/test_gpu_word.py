@@ -19,7 +19,10 @@ torch = pytest.importorskip("torch")
 SHAPES = [(1, 7), (1, 8), (1, 9), (1, 10), (1, 11), (1, 12), (1, 13), (1, 14), (1, 15), (1, 16), (1, 17),
           (3, 6), (3, 7), (3, 9), (3, 10), (3, 12), (3, 13), (3, 14), (3, 15),
           (5, 6), (5, 7), (5, 8), (5, 12), (5, 13), (5, 14),
-          (7, 6), (7, 7), (7, 10), (7, 12), (7, 13), (7, 14)]
+          (7, 6), (7, 7), (7, 10), (7, 12), (7, 13), (7, 14),
+          # two column passes
+          (1, 18), (1, 19), (1, 20), (3, 16), (3, 17), (3, 18), (3, 20), (5, 15), (5, 16), (5, 17), (5, 19),
+          (7, 15), (7, 16), (7, 18), (7, 19)]
 
 
 def _want(a, b):
