@@ -455,7 +455,7 @@ int fill_bits_dev(std::vector<ProdIn>& in, cudaStream_t st) {
     }
     const size_t pb = align_up(sizeof(DProd) * tmp.size(), 256);
     const size_t bb = sizeof(int64_t) * 2 * tmp.size();
-    int rc = E.ensure_pool(pb + bb);
+    int rc = E.ensure_pool(pb + bb, st);
     if (rc) return rc;
     char* d = (char*)E.pool;
     CUDA_TRY(cudaMemcpyAsync(d, tmp.data(), sizeof(DProd) * tmp.size(), cudaMemcpyHostToDevice, st));
@@ -484,16 +484,25 @@ int dev_batch(const nbg_desc* descs, int64_t count, cudaStream_t st) {
     if (rc) return rc;
     rc = fill_bits_dev(in, st);
     if (rc) return rc;
+    WordShape ws;
+    if (count == 1 && in[0].bits_a > 0 && in[0].bits_a <= 64 * in[0].m && in[0].bits_b > 0 &&
+        in[0].bits_b <= 64 * in[0].n && word_product(E, in[0], &ws)) {
+        cudaStreamCaptureStatus cap;
+        CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+        if (cap != cudaStreamCaptureStatusNone) return fail(NBG_ECUDA, "products cannot be captured into a CUDA graph");
+        return run_word_one(E, in[0], ws, st);
+    }
     BatchBuild bb;
     rc = build_batch(E, in.data(), count, bb);
     if (rc) return rc;
-    // the pool is reused by the next call: order it after earlier work on E.stream
-    rc = E.ensure_pool(bb.dev_bytes);
+    rc = E.ensure_pool(bb.dev_bytes, st);
     if (rc) return rc;
     char* dbase = (char*)E.pool;
     rc = upload_batch(E, bb, dbase, st);
     if (rc) return rc;
-    rc = run_launches(E, bb, dbase, st);
+    // one step's launches are small here (a fresh batch is seldom large), so
+    // they run side by side
+    rc = run_launches_branched(E, bb, dbase, st, E.side, 4);
     if (rc) return rc;
     // descriptors/jobs live in pageable host memory copied asynchronously;
     // keep them valid until the copies ran.
@@ -597,7 +606,7 @@ int transform_passes(double* x, int64_t N, int prime, bool fwd, cudaStream_t st)
     }
     const size_t jo = 256;
     const size_t so = align_up(jo + sizeof(Job) * jobs.size(), 256);
-    rc = E.ensure_pool(so + sizeof(double) * (size_t)N);
+    rc = E.ensure_pool(so + sizeof(double) * (size_t)N, st);
     if (rc) return rc;
     char* d = (char*)E.pool;
     P.xa[prime] = x;
@@ -961,7 +970,7 @@ int nbg_unpack_dev(uint64_t* r, int64_t rn, const double* x1, const double* x2, 
     for (int64_t t = 0; t < P.ntl; t++) jobs.push_back(Job{0, 0, t});
     jobs.push_back(Job{0, 0, 0});
     const size_t jo = 256, ao = align_up(jo + sizeof(Job) * jobs.size(), 256);
-    rc = E.ensure_pool(ao + sizeof(uint32_t) * (size_t)P.ntl);
+    rc = E.ensure_pool(ao + sizeof(uint32_t) * (size_t)P.ntl, st);
     if (rc) return rc;
     char* d = (char*)E.pool;
     P.agg = (uint32_t*)(d + ao);

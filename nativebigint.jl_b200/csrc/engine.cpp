@@ -714,20 +714,30 @@ int Engine::ensure_stage(int i, size_t bytes) {
     return NBG_OK;
 }
 
-int Engine::ensure_pool(size_t bytes) {
-    if (bytes <= pool_bytes) return NBG_OK;
-    if (pool) {
-        cudaStreamSynchronize(stream);
-        cudaFree(pool);
-        pool = nullptr;
-        pool_bytes = 0;
+int Engine::ensure_pool(size_t bytes, cudaStream_t st) {
+    if (bytes > pool_bytes) {
+        if (pool) {
+            if (pool_used) cudaEventSynchronize(pool_ev);
+            cudaStreamSynchronize(stream);
+            cudaFree(pool);
+            pool = nullptr;
+            pool_bytes = 0;
+        }
+        size_t want = std::max(bytes, (size_t)64 << 20);
+        if (cudaMalloc(&pool, want) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(NBG_ENOMEM, "device workspace of %zu bytes unavailable", want);
+        }
+        pool_bytes = want;
     }
-    size_t want = std::max(bytes, (size_t)64 << 20);
-    if (cudaMalloc(&pool, want) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(NBG_ENOMEM, "device workspace of %zu bytes unavailable", want);
-    }
-    pool_bytes = want;
+    if (pool_used) CUDA_TRY(cudaStreamWaitEvent(st, pool_ev, 0));
+    return NBG_OK;
+}
+
+int Engine::pool_release(cudaStream_t st) {
+    if (!pool_ev) CUDA_TRY(cudaEventCreateWithFlags(&pool_ev, cudaEventDisableTiming));
+    CUDA_TRY(cudaEventRecord(pool_ev, st));
+    pool_used = true;
     return NBG_OK;
 }
 
@@ -796,6 +806,69 @@ bool word_product(const Engine& E, const ProdIn& q, WordShape* s) {
     return word_shape(la + lb - 1, *s);
 }
 
+int word_setup(Engine& E, const ProdIn& q, const WordShape& s, DProd& P) {
+    const WordTab* wt = nullptr;
+    int rc = E.word_table(s.odd, s.lj + s.lm - 2, &wt);
+    if (rc) return rc;
+    memset(&P, 0, sizeof P);
+    P.a = q.a;
+    P.b = q.sqr ? q.a : q.b;
+    P.r = q.r;
+    P.m = q.m;
+    P.n = q.sqr ? q.m : q.n;
+    P.rn = P.m + P.n;
+    P.sqr = q.sqr;
+    P.nca = eff_limbs(P.m, q.bits_a);
+    P.ncb = q.sqr ? P.nca : eff_limbs(P.n, q.bits_b);
+    P.nconv = P.nca + P.ncb - 1;
+    P.ntl = s.small ? 0 : (P.rn + UNPACK_TL - 1) / UNPACK_TL;
+    P.wN = s.N;
+    P.wodd = s.odd;
+    P.wlj = s.lj;
+    P.wj2 = s.j2;
+    P.wlm = s.lm;
+    P.wL = wt->L;
+    P.wtf = wt->fwd;
+    P.wti = wt->inv;
+    word_scales(s, P.wsc);
+    return NBG_OK;
+}
+
+// Launches of one word product in order: kind and variant.
+static std::vector<std::pair<int, int>> word_steps(const WordShape& s) {
+    if (s.small) return {{JK_WSMALL, (s.odd << 8) | s.lm}};
+    const int col = (s.odd << 8) | (s.lj - s.j2);
+    std::vector<std::pair<int, int>> v{{JK_WCOL_FWD, col}};
+    if (s.j2) v.push_back({JK_WMID_FWD, s.j2});
+    v.push_back({JK_WBLOCK, s.lm});
+    if (s.j2) v.push_back({JK_WMID_REV, s.j2});
+    v.push_back({JK_WCOL_REV, col});
+    v.push_back({JK_WUNPACK, 0});
+    return v;
+}
+
+int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, cudaStream_t st) {
+    DProd P;
+    int rc = word_setup(E, q, s, P);
+    if (rc) return rc;
+    if (!s.small) {
+        const size_t op = align_up(sizeof(uint32_t) * (size_t)WPR * (size_t)s.N, 256);
+        const size_t res = op * (q.sqr ? 1 : 2);
+        if ((rc = E.ensure_pool(res + sizeof(uint32_t) * (size_t)P.ntl, st))) return rc;
+        char* d = (char*)E.pool;
+        P.wa = (uint32_t*)d;
+        P.wb = q.sqr ? nullptr : (uint32_t*)(d + op);
+        P.agg = (uint32_t*)(d + res);
+    }
+    auto steps = word_steps(s);
+    if (P.ntl > 1) steps.push_back({JK_WCARRY, 0});
+    for (const auto& kv : steps) {
+        CUDA_TRY(launch_word_one(kv.first, kv.second, P, word_ctas(kv.first, s, P.sqr, P.rn), st));
+        g_launches++;
+    }
+    return s.small ? NBG_OK : E.pool_release(st);
+}
+
 int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     bb = BatchBuild();
     if (count <= 0) return fail(NBG_EINVAL, "empty batch");
@@ -804,7 +877,11 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     int pmax = 1;
     int bmin = 64;
     size_t work = 0, aggw = 0;
-    std::vector<int32_t> words;  // products of the word engine
+    struct WordProd {
+        int32_t k;
+        WordShape s;
+    };
+    std::vector<WordProd> words;  // products of the word engine
     std::vector<size_t> xa_off((size_t)count), xb_off((size_t)count), agg_off((size_t)count);
     for (int64_t k = 0; k < count; k++) {
         const ProdIn& q = in[k];
@@ -815,41 +892,27 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         // case to handle, as NBig * does before reaching the engine.
         if (q.bits_a < 1 || q.bits_a > 64 * q.m || (!q.sqr && (q.bits_b < 1 || q.bits_b > 64 * q.n)))
             return fail(NBG_EINVAL, "product %lld: magnitude bits out of range (zero operand?)", (long long)k);
+        WordShape ws;
+        if (word_product(E, q, &ws)) {
+            int rc = word_setup(E, q, ws, P);
+            if (rc) return rc;
+            agg_off[(size_t)k] = aggw;
+            aggw += (size_t)P.ntl;
+            const size_t op = ws.small ? 0 : align_up((size_t)WPR * (size_t)ws.N, 64);
+            xa_off[(size_t)k] = bb.word_words;
+            xb_off[(size_t)k] = q.sqr ? SIZE_MAX : bb.word_words + op;
+            bb.word_words += op * (q.sqr ? 1 : 2);
+            bb.plan_of.push_back(nullptr);
+            words.push_back(WordProd{(int32_t)k, ws});
+            if (!ws.small) pmax = std::max(pmax, ws.j2 ? 3 : 2);  // column passes before and after the blocks
+            continue;
+        }
         P.a = q.a;
         P.b = q.sqr ? q.a : q.b;
         P.r = q.r;
         P.m = q.m;
         P.n = q.sqr ? q.m : q.n;
         P.rn = P.m + P.n;
-        WordShape ws;
-        if (word_product(E, q, &ws)) {
-            const WordTab* wt = nullptr;
-            int rc = E.word_table(ws.odd, ws.lj + ws.lm - 2, &wt);
-            if (rc) return rc;
-            P.sqr = q.sqr;
-            P.nca = eff_limbs(P.m, q.bits_a);
-            P.ncb = q.sqr ? P.nca : eff_limbs(P.n, q.bits_b);
-            P.nconv = P.nca + P.ncb - 1;
-            P.ntl = (P.rn + UNPACK_TL - 1) / UNPACK_TL;
-            P.wN = ws.N;
-            P.wodd = ws.odd;
-            P.wlj = ws.lj;
-            P.wj2 = ws.j2;
-            P.wlm = ws.lm;
-            P.wL = wt->L;
-            P.wtf = wt->fwd;
-            P.wti = wt->inv;
-            word_scales(ws, P.wsc);
-            agg_off[(size_t)k] = aggw;
-            aggw += (size_t)P.ntl;
-            xa_off[(size_t)k] = bb.word_words;
-            bb.word_words += align_up((size_t)WPR * (size_t)ws.N, 64);
-            xb_off[(size_t)k] = q.sqr ? SIZE_MAX : bb.word_words;
-            if (!q.sqr) bb.word_words += align_up((size_t)WPR * (size_t)ws.N, 64);
-            bb.plan_of.push_back(nullptr);
-            words.push_back((int32_t)k);
-            continue;
-        }
         int bch;
         int64_t N;
         int rc = ntt_params(q.bits_a, q.sqr ? q.bits_a : q.bits_b, &bch, &N);
@@ -878,7 +941,6 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     }
     bb.agg_words = aggw;
     bb.agg_off = agg_off;
-    for (int32_t k : words) pmax = std::max(pmax, bb.prods[(size_t)k].wj2 ? 3 : 2);  // column passes before and after the blocks
 
     // Jobs of one pipeline step, grouped by kernel and shared-memory size: a
     // launch reserves its largest job's shared memory for every CTA, so a
@@ -1076,7 +1138,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         gu.ops = unp_ops;
         gu.bytes = unp_bytes;
     }
-    if (any_carry) {
+    if (any_carry && tun.queue) {  // the work queue's carry jobs
         Group& gc = group_of(2 * pmax, JK_CARRY, 0);
         gc.mode = JM_PERPROD;
         gc.njobs = count;
@@ -1094,33 +1156,40 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         double bytes = 0;
     };
     std::map<std::tuple<int, int, int>, WGroup> wgroups;  // step, kind, variant
-    std::stable_sort(words.begin(), words.end(), [&](int32_t x, int32_t y) {
-        const DProd &a = bb.prods[(size_t)x], &b = bb.prods[(size_t)y];
-        return a.wN != b.wN ? a.wN > b.wN : a.sqr < b.sqr;
-    });
-    for (int32_t k : words) {
+    auto put = [&](int step, int kind, int variant, int32_t k, const WordShape& ws, double bytes) {
+        WGroup& g = wgroups[std::make_tuple(step, kind, variant)];
         const DProd& P = bb.prods[(size_t)k];
-        const WordShape ws{P.wN, P.wodd, P.wlj, P.wj2, P.wlm};
+        const int64_t cpp = word_ctas(kind, ws, P.sqr, P.rn);
+        if (g.segs.empty() || g.segs.back().cpp != cpp)
+            g.segs.push_back(WSeg{(int32_t)g.nctas, (int32_t)g.plist.size(), (int32_t)cpp, 0});
+        g.plist.push_back(k);
+        g.nctas += cpp;
+        g.bytes += bytes;
+    };
+    std::stable_sort(words.begin(), words.end(), [&](const WordProd& x, const WordProd& y) {
+        return x.s.N != y.s.N ? x.s.N > y.s.N : bb.prods[(size_t)x.k].sqr < bb.prods[(size_t)y.k].sqr;
+    });
+    for (const WordProd& w : words) {
+        const DProd& P = bb.prods[(size_t)w.k];
         const double res = 4.0 * WPR * P.wN, nop = P.sqr ? 1 : 2;
-        auto put = [&](int step, int kind, int variant, double bytes) {
-            WGroup& g = wgroups[std::make_tuple(step, kind, variant)];
-            const int64_t cpp = word_ctas(kind, ws, P.sqr, P.rn);
-            if (g.segs.empty() || g.segs.back().cpp != cpp)
-                g.segs.push_back(WSeg{(int32_t)g.nctas, (int32_t)g.plist.size(), (int32_t)cpp, 0});
-            g.plist.push_back(k);
-            g.nctas += cpp;
-            g.bytes += bytes;
-        };
-        const int col = (P.wodd << 8) | (P.wlj - P.wj2);
-        // the block step is pmax - 1; a middle pass takes the steps next to it
-        const int far = P.wj2 ? 2 : 1;
-        put(pmax - 1 - far, JK_WCOL_FWD, col, 8.0 * (double)(P.nca + (P.sqr ? 0 : P.ncb)) + nop * res);
-        if (P.wj2) put(pmax - 2, JK_WMID_FWD, P.wj2, 2 * nop * res);
-        put(pmax - 1, JK_WBLOCK, P.wlm, (nop + 1) * res);
-        if (P.wj2) put(pmax, JK_WMID_REV, P.wj2, 2 * res);
-        put(pmax - 1 + far, JK_WCOL_REV, col, 2 * res);
-        put(2 * pmax - 1, JK_WUNPACK, 0, res + 8.0 * (double)P.rn);
+        const double in_b = 8.0 * (double)(P.nca + (P.sqr ? 0 : P.ncb)), out_b = 8.0 * (double)P.rn;
+        for (const auto& kv : word_steps(w.s)) {
+            // the block step is pmax - 1, a middle column pass takes the steps next to it
+            const int far = w.s.j2 ? 2 : 1;
+            switch (kv.first) {
+                case JK_WCOL_FWD: put(pmax - 1 - far, kv.first, kv.second, w.k, w.s, in_b + nop * res); break;
+                case JK_WMID_FWD: put(pmax - 2, kv.first, kv.second, w.k, w.s, 2 * nop * res); break;
+                case JK_WBLOCK: put(pmax - 1, kv.first, kv.second, w.k, w.s, (nop + 1) * res); break;
+                case JK_WMID_REV: put(pmax, kv.first, kv.second, w.k, w.s, 2 * res); break;
+                case JK_WCOL_REV: put(pmax - 1 + far, kv.first, kv.second, w.k, w.s, 2 * res); break;
+                case JK_WSMALL: put(pmax - 1, kv.first, kv.second, w.k, w.s, in_b + out_b); break;
+                default: put(2 * pmax - 1, kv.first, kv.second, w.k, w.s, res + out_b); break;
+            }
+        }
     }
+    for (int64_t k = 0; k < count && !tun.queue; k++)
+        if (bb.prods[(size_t)k].ntl > 1)
+            put(2 * pmax, JK_WCARRY, 0, (int32_t)k, WordShape(), 4.0 * (double)bb.prods[(size_t)k].ntl);
     for (auto& kv : wgroups)
         if (kv.second.nctas > 0x7fffffff) return fail(NBG_EINVAL, "batch too large");
     // job table: [segments | product list] per launch, then the unpack tile starts

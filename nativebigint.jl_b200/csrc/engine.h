@@ -110,7 +110,12 @@ struct Engine {
     void tuning_changed(bool loaded);  // after `tun` was set (loaded: it is the new base)
     int word_table(int odd, int L, const WordTab** out);
     void trim_plans();  // frees every plan's tables: no batch may exist or be running
-    int ensure_pool(size_t bytes);
+    // The shared workspace, at least `bytes`, for work on `st`: ordered after the
+    // last call that left work using it in flight (pool_release).
+    int ensure_pool(size_t bytes, cudaStream_t st);
+    int pool_release(cudaStream_t st);
+    cudaEvent_t pool_ev = nullptr;
+    bool pool_used = false;  // pool_ev recorded
     int ensure_stage(int i, size_t bytes);
 };
 extern Engine g_eng;
@@ -130,6 +135,11 @@ struct ProdIn {
 
 // Whether the product runs on the word engine (shape in *s), from its sizes alone.
 bool word_product(const Engine& E, const ProdIn& q, WordShape* s);
+// Fills P for a word product (device pointers as in q; workspace pointers left null).
+int word_setup(Engine& E, const ProdIn& q, const WordShape& s, DProd& P);
+// One word product on `st` with its descriptor passed by value: no copies and
+// no host wait; the shared workspace holds its transforms.
+int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, cudaStream_t st);
 // Transform buffers of the product on the multi-pass FP64 engine (SIZE_MAX: no such transform).
 size_t fp64_work_bytes(const ProdIn& q);
 

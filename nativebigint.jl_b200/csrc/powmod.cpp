@@ -298,13 +298,17 @@ static int powmod_run(Engine& E, const nbg_powmod_desc* d, int64_t count, int64_
         uint64_t* q2 = d_q2 + c * q2_stride;
         const int64_t l = lmu[(size_t)c];
         in1[(size_t)c] = ProdIn{sl + (int64_t)S.acc() * k, sl + (int64_t)S.one() * k, T, k, k, 64 * k, 64 * k, 0};
-        in1[(size_t)c].fp64 = 1;
         // mu and m are the same on every step: as operand b their transforms
         // are kept from the first run (one-pass products) and reused
         in2[(size_t)c] = ProdIn{T + (k - 1), d_mu + c * lmu_max, q2, k + 1, l, 64 * (k + 1), bits_mu[(size_t)c], 0};
         in3[(size_t)c] = ProdIn{q2 + (k + 1), d_mod + c * k, d_r2 + c * C.r2_stride, l, k, 64 * l, bits_m[(size_t)c], 0};
-        in2[(size_t)c].keep_b = one_pass(E, 64 * (k + 1), bits_mu[(size_t)c]);
-        in3[(size_t)c].keep_b = one_pass(E, 64 * l, bits_m[(size_t)c]);
+        // (products that fit one CTA of the word engine are faster still)
+        WordShape ws;
+        if (!(word_product(E, in2[(size_t)c], &ws) && ws.small)) {
+            in1[(size_t)c].fp64 = one_pass(E, 64 * k, 64 * k);
+            in2[(size_t)c].keep_b = one_pass(E, 64 * (k + 1), bits_mu[(size_t)c]);
+            in3[(size_t)c].keep_b = one_pass(E, 64 * l, bits_m[(size_t)c]);
+        }
     }
     BatchBuild bb[3];
     char* reg[3];

@@ -220,6 +220,8 @@ enum JobKind : int32_t {
     JK_WUNPACK = 13, // word products: coefficients and carried limbs
     JK_WMID_FWD = 14,// word products: a middle column pass
     JK_WMID_REV = 15,// word products: a middle column pass backwards
+    JK_WSMALL = 16,  // word products: a whole small product per CTA
+    JK_WCARRY = 17,  // carries between unpack tiles (any product)
 };
 
 constexpr int UNPACK_TL = 1024;  // output limbs per unpack tile

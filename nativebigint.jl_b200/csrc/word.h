@@ -34,6 +34,7 @@ constexpr int64_t WORD_MIN_OPERAND_MAX = int64_t(1) << 21;
 // and a middle one of 2^j2.
 struct WordShape {
     int32_t N = 0, odd = 0, lj = 0, j2 = 0, lm = 0;
+    bool small = false;  // one CTA per product (at most 3072 values; lj = 0, no column pass)
 };
 // The smallest supported length >= nconv; false when there is none.
 bool word_shape(int64_t nconv, WordShape& s);
@@ -46,10 +47,13 @@ struct WSeg {
     int32_t pad_;
 };
 
-// variant of a word launch: (odd << 8) | (lj - j2) for column passes, j2 for middle ones, lm for blocks
+// variant of a word launch: (odd << 8) | (lj - j2) for column passes, j2 for middle ones, lm for
+// blocks, (odd << 8) | lm for one-CTA products
 cudaError_t word_init();  // constant memory of the current device
 cudaError_t launch_word(int kind, int variant, const DProd* prods, const WSeg* segs, int nseg, const int32_t* plist,
                         int64_t nctas, cudaStream_t st);
+// The same for one product passed by value (no device tables).
+cudaError_t launch_word_one(int kind, int variant, const DProd& P, int64_t nctas, cudaStream_t st);
 // CTAs one product needs in a word launch.
 int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t rn);
 

@@ -9,10 +9,13 @@
 //               products, the levels back
 //   k_wcol_rev  the first lj levels and the radix-`odd` step backwards
 //   k_wunpack   five residues -> coefficient (mixed radix), carried limb sums
+//   k_wcarry    carries between unpack tiles
+//   k_wsmall    a whole product of at most 3072 coefficients in one CTA
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <type_traits>
+#include <vector>
 
 #include "word.cuh"
 #include "word.h"
@@ -63,6 +66,8 @@ static uint64_t root_of(int i) {
 static Tw mk(uint64_t w, uint64_t p) { return Tw{(uint32_t)w, (uint32_t)((w << 32) / p)}; }
 static uint32_t mont(uint64_t w, uint64_t p) { return (uint32_t)(((w % p) << 32) % p); }
 
+static cudaError_t small_attributes();
+
 cudaError_t word_init() {
     WConst h{};
     for (int i = 0; i < WPR; i++) {
@@ -96,22 +101,30 @@ cudaError_t word_init() {
             h.gar[i][j] = mont((p - Wj * iw % p) % p, p);
             Wj = Wj * (WPRIMES[j] % p) % p;
         }
-        (void)0;
     }
-    return cudaMemcpyToSymbol(c_w, &h, sizeof h);
+    cudaError_t e = small_attributes();
+    return e == cudaSuccess ? cudaMemcpyToSymbol(c_w, &h, sizeof h) : e;
 }
 
 void word_scales(const WordShape& s, uint32_t out[WPR]) {
-    for (int i = 0; i < WPR; i++) {
-        const uint64_t p = WPRIMES[i];
-        const int lev = s.lj + s.lm - 2;
-        const uint64_t t = (uint64_t)s.odd % p * pw(2, (uint64_t)lev, p) % p;
-        uint64_t Wi = 1;
-        for (int j = 0; j < i; j++) Wi = Wi * (WPRIMES[j] % p) % p;
-        // 2^32 (pointwise) * 2^32 (unpack's reduction) / (odd * 2^levels * W_i)
-        const uint64_t r = (uint64_t(1) << 32) % p;
-        out[i] = (uint32_t)(r * r % p * inv(t * Wi % p, p) % p);
-    }
+    // 2^32 (pointwise) * 2^32 (unpack's reduction) / (odd * 2^levels * W_i)
+    static const struct Table {
+        uint32_t v[8][WORD_MAX_LOG2][WPR];
+        Table() {
+            uint64_t W[WPR];
+            for (int i = 0; i < WPR; i++) {
+                W[i] = 1;
+                for (int j = 0; j < i; j++) W[i] = W[i] * (WPRIMES[j] % WPRIMES[i]) % WPRIMES[i];
+            }
+            for (int odd = 1; odd < 8; odd += 2)
+                for (int lev = 0; lev < WORD_MAX_LOG2; lev++)
+                    for (int i = 0; i < WPR; i++) {
+                        const uint64_t p = WPRIMES[i], r = (uint64_t(1) << 32) % p;
+                        v[odd][lev][i] = (uint32_t)(r * r % p * inv(odd * pw(2, (uint64_t)lev, p) % p * W[i] % p, p) % p);
+                    }
+        }
+    } t;
+    for (int i = 0; i < WPR; i++) out[i] = t.v[s.odd][s.lj + s.lm - 2][i];
 }
 
 // The split of the rows above the blocks: one column pass up to 32 rows (its
@@ -131,22 +144,37 @@ static bool row_split(int odd, int lj, int& j2) {
     return best != INT64_MAX;
 }
 
-bool word_shape(int64_t nconv, WordShape& s) {
-    int64_t best = INT64_MAX;
-    for (int odd : {1, 3, 5, 7}) {
-        for (int k = 6; k <= WORD_MAX_LOG2; k++) {
-            const int64_t N = (int64_t)odd << k;
-            if (N < nconv || N >= best) continue;
-            for (int lm : {12, 10, 8, 6}) {
-                int j2;
-                if (k < lm || !row_split(odd, k - lm, j2)) continue;
-                best = N;
-                s = WordShape{(int32_t)N, odd, k - lm, j2, lm};
-                break;
+// Every supported shape, shortest first.
+static const std::vector<WordShape>& shape_list() {
+    static const std::vector<WordShape> list = [] {
+        std::vector<WordShape> v;
+        for (int odd : {1, 3, 5, 7})
+            for (int k = 6; k <= WORD_MAX_LOG2; k++) {
+                const int64_t N = (int64_t)odd << k;
+                if (k <= 11 && WPR * N <= 16 * 1024) {
+                    v.push_back(WordShape{(int32_t)N, odd, 0, 0, k, true});
+                    continue;
+                }
+                for (int lm : {12, 10, 8, 6}) {
+                    int j2;
+                    if (k < lm || !row_split(odd, k - lm, j2)) continue;
+                    v.push_back(WordShape{(int32_t)N, odd, k - lm, j2, lm, false});
+                    break;
+                }
             }
-        }
-    }
-    return best != INT64_MAX;
+        std::sort(v.begin(), v.end(), [](const WordShape& x, const WordShape& y) { return x.N < y.N; });
+        return v;
+    }();
+    return list;
+}
+
+bool word_shape(int64_t nconv, WordShape& s) {
+    const std::vector<WordShape>& v = shape_list();
+    const auto it = std::lower_bound(v.begin(), v.end(), nconv,
+                                     [](const WordShape& x, int64_t n) { return x.N < n; });
+    if (it == v.end()) return false;
+    s = *it;
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -267,9 +295,20 @@ __device__ __forceinline__ void dft_odd(uint32_t* x, int i, uint32_t p) {
 // ---------------------------------------------------------------------------
 // job lookup: segment of this CTA, its product and the CTA's index inside it
 
-__device__ __forceinline__ const DProd& wjob(const DProd* __restrict__ prods, const WSeg* __restrict__ segs, int nseg,
-                                             const int32_t* __restrict__ plist, int& local) {
-    int lo = 0, hi = nseg - 1;
+// A launch's products: a batch's tables, or (nseg = 0) one product by value.
+struct WArgs {
+    const DProd* prods;
+    const WSeg* segs;
+    const int32_t* plist;
+    int32_t nseg;
+    DProd one;
+};
+
+__device__ __forceinline__ const DProd& wjob(const WArgs& A, int& local) {
+    local = (int)blockIdx.x;
+    if (A.nseg == 0) return A.one;
+    const WSeg* __restrict__ segs = A.segs;
+    int lo = 0, hi = A.nseg - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (segs[mid].begin <= (int)blockIdx.x) lo = mid;
@@ -278,7 +317,7 @@ __device__ __forceinline__ const DProd& wjob(const DProd* __restrict__ prods, co
     const WSeg g = segs[lo];
     const int q = ((int)blockIdx.x - g.begin) / g.cpp;
     local = (int)blockIdx.x - g.begin - q * g.cpp;
-    return prods[plist[g.first + q]];
+    return A.prods[A.plist[g.first + q]];
 }
 
 constexpr int WT = 256;  // threads per CTA
@@ -286,12 +325,18 @@ constexpr int WT = 256;  // threads per CTA
 // ---------------------------------------------------------------------------
 // column passes: one thread holds the R rows of one column of one prime
 
+// A limb modulo p, in [0, 4p) (RED: [0, 2p)).
+template <bool RED>
+__device__ __forceinline__ uint32_t wpack(uint64_t v, int pi, uint32_t p) {
+    const uint32_t y = wd::mulw((uint32_t)(v >> 32), c_w.c32[pi], p) + wd::mulw((uint32_t)v, c_w.one[pi], p);
+    return RED ? wd::sub_if(y, 2 * p) : y;
+}
+
 template <int ODD, int LJ>
-__global__ void __launch_bounds__(WT) k_wcol_fwd(const DProd* __restrict__ prods, const WSeg* __restrict__ segs,
-                                                 int nseg, const int32_t* __restrict__ plist) {
+__global__ void __launch_bounds__(WT) k_wcol_fwd(const __grid_constant__ WArgs A) {
     constexpr int R = ODD << LJ;
     int local;
-    const DProd& P = wjob(prods, segs, nseg, plist, local);
+    const DProd& P = wjob(A, local);
     const int lm = P.wlm + P.wj2;  // log2 of the column count
     const int id = local * WT + (int)threadIdx.x;
     const int c = id & ((1 << lm) - 1);
@@ -302,15 +347,12 @@ __global__ void __launch_bounds__(WT) k_wcol_fwd(const DProd* __restrict__ prods
     const uint64_t* __restrict__ src = isb ? P.b : P.a;
     const int n = (int)(isb ? P.ncb : P.nca);
     uint32_t* __restrict__ dst = (isb ? P.wb : P.wa) + (size_t)pi * (size_t)P.wN;
-    const uint32_t p = c_w.p[pi], p2 = 2 * p;
-    const Tw c32 = c_w.c32[pi], one = c_w.one[pi];
+    const uint32_t p = c_w.p[pi];
     uint32_t x[R];
 #pragma unroll
     for (int r = 0; r < R; r++) {
         const int i = c + (r << lm);
-        const uint64_t v = i < n ? __ldg(src + i) : 0ull;
-        const uint32_t y = wd::mulw((uint32_t)(v >> 32), c32, p) + wd::mulw((uint32_t)v, one, p);
-        x[r] = ODD > 1 ? wd::sub_if(y, p2) : y;
+        x[r] = wpack<(ODD > 1)>(i < n ? __ldg(src + i) : 0ull, pi, p);
     }
     dft_odd<ODD, LJ>(x, pi, p);
     const Tw* tab = (const Tw*)P.wtf + (((size_t)pi * ODD) << P.wL);
@@ -321,11 +363,10 @@ __global__ void __launch_bounds__(WT) k_wcol_fwd(const DProd* __restrict__ prods
 }
 
 template <int ODD, int LJ>
-__global__ void __launch_bounds__(WT) k_wcol_rev(const DProd* __restrict__ prods, const WSeg* __restrict__ segs,
-                                                 int nseg, const int32_t* __restrict__ plist) {
+__global__ void __launch_bounds__(WT) k_wcol_rev(const __grid_constant__ WArgs A) {
     constexpr int R = ODD << LJ;
     int local;
-    const DProd& P = wjob(prods, segs, nseg, plist, local);
+    const DProd& P = wjob(A, local);
     const int lm = P.wlm + P.wj2;  // log2 of the column count
     const int id = local * WT + (int)threadIdx.x;
     const int c = id & ((1 << lm) - 1);
@@ -352,10 +393,9 @@ __global__ void __launch_bounds__(WT) k_wcol_rev(const DProd* __restrict__ prods
 // subtree of the segment's node.  In place; all columns of a segment share
 // their constants.
 template <int J, bool FWD>
-__global__ void __launch_bounds__(WT) k_wmid(const DProd* __restrict__ prods, const WSeg* __restrict__ segs, int nseg,
-                                             const int32_t* __restrict__ plist) {
+__global__ void __launch_bounds__(WT) k_wmid(const __grid_constant__ WArgs A) {
     int local;
-    const DProd& P = wjob(prods, segs, nseg, plist, local);
+    const DProd& P = wjob(A, local);
     const int lm = P.wlm, j1 = P.wlj - J, R1 = P.wodd << j1;
     const int id = local * WT + (int)threadIdx.x;
     const int c = id & ((1 << lm) - 1);
@@ -424,20 +464,25 @@ struct WSplit;
 template <>
 struct WSplit<12> { static constexpr int J1 = 4, J2 = 4; };
 template <>
+struct WSplit<11> { static constexpr int J1 = 4, J2 = 3; };
+template <>
 struct WSplit<10> { static constexpr int J1 = 3, J2 = 3; };
+template <>
+struct WSplit<9> { static constexpr int J1 = 3, J2 = 2; };
 template <>
 struct WSplit<8> { static constexpr int J1 = 4, J2 = 0; };
 template <>
+struct WSplit<7> { static constexpr int J1 = 3, J2 = 0; };
+template <>
 struct WSplit<6> { static constexpr int J1 = 2, J2 = 0; };
 
-// The block of `src` down to its leaves: x[0..16) = values 16t .. 16t+15 in [0, 4p).
+// A block down to its leaves, from the first round's values in x: x[0..16) =
+// values 16t .. 16t+15 in [0, 4p).
 template <int LM>
-__device__ __forceinline__ void wblock_down(uint32_t* x, uint32_t* s, const uint32_t* __restrict__ src, int t,
-                                            const Tw* __restrict__ tab, uint32_t h0, uint32_t p, bool live) {
+__device__ __forceinline__ void wblock_down(uint32_t* x, uint32_t* s, int t, const Tw* __restrict__ tab, uint32_t h0,
+                                            uint32_t p, bool live) {
     constexpr int J1 = WSplit<LM>::J1, J2 = WSplit<LM>::J2;
     if (live) {
-#pragma unroll
-        for (int k = 0; k < 16; k++) x[k] = src[wpos<LM, LM, J1>(t, k >> J1, k & ((1 << J1) - 1))];
         wround_fwd<LM, LM, J1>(x, t, tab, h0, p);
         wput<LM, LM, J1>(s, x, t);
     }
@@ -467,6 +512,44 @@ __device__ __forceinline__ void wblock_down(uint32_t* x, uint32_t* s, const uint
     }
 }
 
+// The way back: a[0..16) = leaf values 16t .. 16t+15 in [0, 2p), out: the
+// first round's values.  Safe right after wblock_down on the same `s`: each
+// thread first writes the 16 words that only it read last.
+template <int LM>
+__device__ __forceinline__ void wblock_up(uint32_t* a, uint32_t* s, int t, const Tw* __restrict__ ti, uint32_t h0,
+                                          uint32_t p, bool live) {
+    constexpr int J1 = WSplit<LM>::J1, J2 = WSplit<LM>::J2;
+    const uint32_t p2 = 2 * p;
+    if (live) {
+        const uint32_t idx = (h0 << (LM - 4)) + (uint32_t)t;
+        Tw w1[1], w2[2];
+        wd::load_tw<0>(ti, idx, w1);
+        wd::load_tw<1>(ti, idx, w2);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            wd::bf_rev(a[e], a[e + 4], w2[0], p, p2);
+            wd::bf_rev(a[e + 8], a[e + 12], w2[1], p, p2);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e++) wd::bf_rev(a[e], a[e + 8], w1[0], p, p2);
+#pragma unroll
+        for (int k = 0; k < 16; k++) s[17 * t + k] = a[k];
+    }
+    __syncthreads();
+    if constexpr (J2 > 0) {
+        if (live) {
+            wget<LM, LM - J1, J2>(s, a, t);
+            wround_rev<LM, LM - J1, J2>(a, t, ti, h0, p);
+            wput<LM, LM - J1, J2>(s, a, t);
+        }
+        __syncthreads();
+    }
+    if (live) {
+        wget<LM, LM, J1>(s, a, t);
+        wround_rev<LM, LM, J1>(a, t, ti, h0, p);
+    }
+}
+
 // c = a * b mod X^4 - rho (rho in 2^32 form), a in [0, p), b in [0, 2p); the
 // result carries a factor 2^-32 and lies in [0, 2p).  Sums of at most four
 // products of 2p^2 and one of 2.5p * p stay below 2^64.
@@ -491,15 +574,33 @@ __device__ __forceinline__ void wleaf(uint32_t* a, const uint32_t* b, uint32_t r
     for (int k = 0; k < 4; k++) a[k] = c[k];
 }
 
+// The 16 consecutive leaf values a *= b (or a *= a), all in [0, 4p) before, [0, 2p) after.
 template <int LM>
-__global__ void __launch_bounds__(WT, 3) k_wblock(const DProd* __restrict__ prods, const WSeg* __restrict__ segs,
-                                                  int nseg, const int32_t* __restrict__ plist) {
+__device__ __forceinline__ void wpoint(uint32_t* a, uint32_t* b, bool sqr, int t, const Tw* __restrict__ tf, uint32_t h0,
+                                       uint32_t p, uint32_t pinv) {
+    const uint32_t p2 = 2 * p;
+    Tw w2[2];
+    wd::load_tw<1>(tf, (h0 << (LM - 4)) + (uint32_t)t, w2);
+    const uint32_t r0 = 0u - w2[0].q * p, r1 = 0u - w2[1].q * p;  // w * 2^32 mod p
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        a[k] = wd::sub_if(wd::sub_if(a[k], p2), p);
+        b[k] = sqr ? a[k] : wd::sub_if(b[k], p2);
+    }
+    wleaf(a, b, r0, p, pinv);
+    wleaf(a + 4, b + 4, p - r0, p, pinv);
+    wleaf(a + 8, b + 8, r1, p, pinv);
+    wleaf(a + 12, b + 12, p - r1, p, pinv);
+}
+
+template <int LM>
+__global__ void __launch_bounds__(WT, 3) k_wblock(const __grid_constant__ WArgs A) {
     constexpr int T = 1 << (LM - 4), PER = WT / T;  // threads per block, blocks per CTA
     constexpr int SM = (1 << LM) + (1 << (LM - 4));
-    constexpr int J1 = WSplit<LM>::J1, J2 = WSplit<LM>::J2;
+    constexpr int J1 = WSplit<LM>::J1;
     __shared__ uint32_t sm[2][PER][SM];
     int local;
-    const DProd& P = wjob(prods, segs, nseg, plist, local);
+    const DProd& P = wjob(A, local);
     const int g = (int)threadIdx.x / T, t = (int)threadIdx.x & (T - 1);
     const int R = P.wodd << P.wlj;
     const int blk = local * PER + g;  // prime-major, then block
@@ -507,75 +608,27 @@ __global__ void __launch_bounds__(WT, 3) k_wblock(const DProd* __restrict__ prod
     const int pi = live ? blk / R : 0, row = live ? blk - pi * R : 0;
     const int j = row >> P.wlj;
     const uint32_t h0 = (1u << P.wlj) + (uint32_t)(row & ((1 << P.wlj) - 1));
-    const uint32_t p = c_w.p[pi], pinv = c_w.pinv[pi], p2 = 2 * p;
-    const size_t toff = ((size_t)pi * P.wodd + j) << P.wL;
+    const uint32_t p = c_w.p[pi], pinv = c_w.pinv[pi];
+    const size_t toff = ((size_t)pi * P.wodd + j) << P.wL, xoff = (size_t)pi * (size_t)P.wN + ((size_t)row << LM);
     const Tw* tf = (const Tw*)P.wtf + toff;
-    uint32_t* xa = P.wa + (size_t)pi * (size_t)P.wN + ((size_t)row << LM);
-    uint32_t a[16];
-    wblock_down<LM>(a, sm[0][g], xa, t, tf, h0, p, live);
+    uint32_t* xa = P.wa + xoff;
+    uint32_t a[16], b[16];
+    auto load = [&](uint32_t* x, const uint32_t* src) {
+        if (!live) return;
+#pragma unroll
+        for (int k = 0; k < 16; k++) x[k] = src[wpos<LM, LM, J1>(t, k >> J1, k & ((1 << J1) - 1))];
+    };
+    load(a, xa);
+    wblock_down<LM>(a, sm[0][g], t, tf, h0, p, live);
     if (!P.sqr) {
-        uint32_t b[16];
-        wblock_down<LM>(b, sm[1][g], P.wb + (size_t)pi * (size_t)P.wN + ((size_t)row << LM), t, tf, h0, p, live);
-        if (live) {
-            Tw w2[2];
-            wd::load_tw<1>(tf, (h0 << (LM - 4)) + (uint32_t)t, w2);
-            const uint32_t r0 = 0u - w2[0].q * p, r1 = 0u - w2[1].q * p;  // w * 2^32 mod p
-#pragma unroll
-            for (int k = 0; k < 16; k++) {
-                a[k] = wd::sub_if(wd::sub_if(a[k], p2), p);
-                b[k] = wd::sub_if(b[k], p2);
-            }
-            wleaf(a, b, r0, p, pinv);
-            wleaf(a + 4, b + 4, p - r0, p, pinv);
-            wleaf(a + 8, b + 8, r1, p, pinv);
-            wleaf(a + 12, b + 12, p - r1, p, pinv);
-        }
+        load(b, P.wb + xoff);
+        wblock_down<LM>(b, sm[1][g], t, tf, h0, p, live);
+        if (live) wpoint<LM>(a, b, false, t, tf, h0, p, pinv);
     } else if (live) {
-        Tw w2[2];
-        wd::load_tw<1>(tf, (h0 << (LM - 4)) + (uint32_t)t, w2);
-        const uint32_t r0 = 0u - w2[0].q * p, r1 = 0u - w2[1].q * p;
-#pragma unroll
-        for (int k = 0; k < 16; k++) a[k] = wd::sub_if(wd::sub_if(a[k], p2), p);
-#pragma unroll
-        for (int l = 0; l < 4; l++) {
-            uint32_t b[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) b[k] = a[4 * l + k];
-            const uint32_t rr = l < 2 ? r0 : r1;
-            wleaf(a + 4 * l, b, (l & 1) ? p - rr : rr, p, pinv);
-        }
+        wpoint<LM>(a, b, true, t, tf, h0, p, pinv);
     }
-    // back up (shared buffer 1: its last readers passed a barrier, or none used it)
-    const Tw* ti = (const Tw*)P.wti + toff;
-    uint32_t* s = sm[1][g];
+    wblock_up<LM>(a, sm[1][g], t, (const Tw*)P.wti + toff, h0, p, live);
     if (live) {
-        const uint32_t idx = (h0 << (LM - 4)) + (uint32_t)t;
-        Tw w1[1], w2[2];
-        wd::load_tw<0>(ti, idx, w1);
-        wd::load_tw<1>(ti, idx, w2);
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            wd::bf_rev(a[e], a[e + 4], w2[0], p, p2);
-            wd::bf_rev(a[e + 8], a[e + 12], w2[1], p, p2);
-        }
-#pragma unroll
-        for (int e = 0; e < 8; e++) wd::bf_rev(a[e], a[e + 8], w1[0], p, p2);
-        // each thread rewrites the 16 words only it read last
-#pragma unroll
-        for (int k = 0; k < 16; k++) s[17 * t + k] = a[k];
-    }
-    __syncthreads();
-    if constexpr (J2 > 0) {
-        if (live) {
-            wget<LM, LM - J1, J2>(s, a, t);
-            wround_rev<LM, LM - J1, J2>(a, t, ti, h0, p);
-            wput<LM, LM - J1, J2>(s, a, t);
-        }
-        __syncthreads();
-    }
-    if (live) {
-        wget<LM, LM, J1>(s, a, t);
-        wround_rev<LM, LM, J1>(a, t, ti, h0, p);
 #pragma unroll
         for (int k = 0; k < 16; k++) xa[wpos<LM, LM, J1>(t, k >> J1, k & ((1 << J1) - 1))] = a[k];
     }
@@ -617,16 +670,117 @@ __device__ __forceinline__ uint32_t gp_join(uint32_t lower, uint32_t upper) {
     return ((upper & 1u) | ((upper >> 1) & lower & 1u)) | (upper & lower & 2u);
 }
 
-__global__ void __launch_bounds__(WT) k_wunpack(const DProd* __restrict__ prods, const WSeg* __restrict__ segs, int nseg,
-                                                const int32_t* __restrict__ plist) {
-    __shared__ uint64_t s_mid[WT + 1];           // mid word of the last coefficient of thread t - 1
-    __shared__ uint32_t s_hi[WT + 1][2];         // high words of its last two coefficients
-    __shared__ uint32_t s_c[WT + 1];             // carry out of its last limb sum
-    __shared__ uint64_t h_lo, h_mid2;            // halo: limb sum w0 - 1
+// Limb sums of up to 4 * NT limbs, four per thread, from their coefficients'
+// words lo + mid 2^64 + hi 2^128.  s_mid/s_hi entry 0 and s_c[0]: what reaches
+// the first limb from below (s_c[0] may be written until the first barrier).
+// own: the limbs with every carry inside the run; returns this thread's
+// inclusive (generate, propagate) state of the run in the last thread.
+template <int NT>
+struct LimbShared {
+    uint64_t mid[NT + 1];
+    uint32_t hi[NT + 1][2];
+    uint32_t c[NT + 1];
+    uint32_t wagg[32];
+};
+template <int NT>
+__device__ __forceinline__ uint32_t limb_sums(LimbShared<NT>& S, int t, int nt, const uint64_t* lo, const uint64_t* mid,
+                                              const uint32_t* hi, int nlimbs, uint64_t* own) {
+    const bool in = t < nt;
+    if (in) {
+        S.mid[t + 1] = mid[3];
+        S.hi[t + 1][0] = hi[2];
+        S.hi[t + 1][1] = hi[3];
+    }
+    __syncthreads();
+    // limb sums lo_i + mid_(i-1) + hi_(i-2) and their carries (0..2)
+    uint32_t cy[4] = {0, 0, 0, 0};
+    if (in) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint64_t m1 = q ? mid[q - 1] : S.mid[t];
+            const uint32_t h2 = q > 1 ? hi[q - 2] : S.hi[t][q];
+            uint64_t s = lo[q] + m1;
+            uint32_t c = s < m1;
+            s += h2;
+            c += s < h2;
+            own[q] = s;
+            cy[q] = c;
+        }
+        S.c[t + 1] = cy[3];
+    }
+    __syncthreads();
+    uint32_t agg = 0;
+    if (in) {
+        uint32_t k = S.c[t], g = 0, prop = 1;  // carry of the sum below; carry of adding it
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint64_t s = own[q] + k + g;  // k + g <= 3
+            g = s < (uint64_t)(k + g);
+            own[q] = s;
+            k = cy[q];
+            prop &= (4 * t + q < nlimbs && s == ~0ULL) ? 1u : 0u;
+        }
+        agg = g | (prop << 1);
+    }
+    // carry-lookahead over the threads, then over the warps
+    const int lane = t & 31, wid = t >> 5;
+    uint32_t incl = agg;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl = gp_join(o, incl);
+    }
+    if (lane == 31) S.wagg[wid] = incl;
+    __syncthreads();
+    uint32_t wpre = lane < (int)(blockDim.x >> 5) ? S.wagg[lane] : 2u;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xffffffffu, wpre, off);
+        if (lane >= off) wpre = gp_join(o, wpre);
+    }
+    wpre = wid ? __shfl_sync(0xffffffffu, wpre, wid ? wid - 1 : 0) : 2u;
+    uint32_t excl = __shfl_up_sync(0xffffffffu, incl, 1);
+    if (lane == 0) excl = 2u;
+    uint64_t cin = gp_join(wpre, excl) & 1u;  // carry into the run taken as 0
+    if (in) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            own[q] += cin;
+            cin = cin && own[q] == 0;
+        }
+    }
+    return gp_join(wpre, incl);
+}
+
+__device__ __forceinline__ void store_limbs(uint64_t* __restrict__ r, int64_t wt, int64_t w1, const uint64_t* own) {
+    if (wt + 3 < w1) {
+        ulonglong2* dst = reinterpret_cast<ulonglong2*>(r + wt);
+        if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+            dst[0] = make_ulonglong2(own[0], own[1]);
+            dst[1] = make_ulonglong2(own[2], own[3]);
+            return;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if (wt + q < w1) r[wt + q] = own[q];
+}
+
+__device__ __forceinline__ void coef_words(const uint32_t* r, const uint32_t* sc, uint64_t& lo, uint64_t& mid,
+                                           uint32_t& hi) {
+    uint32_t v[WPR];
+    wcoef(r, sc, v);
+    lo = v[0] | (uint64_t)v[1] << 32;
+    mid = v[2] | (uint64_t)v[3] << 32;
+    hi = v[4];
+}
+
+__global__ void __launch_bounds__(WT) k_wunpack(const __grid_constant__ WArgs A) {
+    __shared__ LimbShared<WT> S;
+    __shared__ uint64_t h_lo, h_mid2;  // the limb sum below the tile
     __shared__ uint32_t h_hi3;
-    __shared__ uint32_t wagg[WT / 32];
     int tile;
-    const DProd& P = wjob(prods, segs, nseg, plist, tile);
+    const DProd& P = wjob(A, tile);
     const int t = (int)threadIdx.x;
     const int N = P.wN;
     const uint32_t* __restrict__ x = P.wa;
@@ -637,28 +791,36 @@ __global__ void __launch_bounds__(WT) k_wunpack(const DProd* __restrict__ prods,
     // the three coefficients before the tile
     if (t < 3) {
         const int64_t i = w0 - 1 - t;
-        uint32_t v[WPR] = {0, 0, 0, 0, 0};
+        uint64_t lo = 0, mid = 0;
+        uint32_t hi = 0;
         if (i >= 0 && i < N) {
             uint32_t r[WPR];
 #pragma unroll
             for (int k = 0; k < WPR; k++) r[k] = x[(size_t)k * N + i];
-            wcoef(r, sc, v);
+            coef_words(r, sc, lo, mid, hi);
         }
-        const uint64_t lo = v[0] | (uint64_t)v[1] << 32, mid = v[2] | (uint64_t)v[3] << 32;
         if (t == 0) {
             h_lo = lo;
-            s_mid[0] = mid;
-            s_hi[0][1] = v[4];
+            S.mid[0] = mid;
+            S.hi[0][1] = hi;
         } else if (t == 1) {
             h_mid2 = mid;
-            s_hi[0][0] = v[4];
+            S.hi[0][0] = hi;
         } else {
-            h_hi3 = v[4];
+            h_hi3 = hi;
+        }
+        __syncwarp(7u);
+        if (t == 0) {
+            uint64_t s = h_lo + h_mid2;
+            uint32_t c = s < h_mid2;
+            s += h_hi3;
+            c += s < h_hi3;
+            S.c[0] = c;
         }
     }
     const int64_t wt = w0 + 4 * t;
-    uint64_t lo[4], mid[4];
-    uint32_t hi[4];
+    uint64_t lo[4] = {0, 0, 0, 0}, mid[4] = {0, 0, 0, 0}, own[4];
+    uint32_t hi[4] = {0, 0, 0, 0};
     if (wt < N) {  // N is a multiple of 4: all four or none
         uint32_t r[4][WPR];
 #pragma unroll
@@ -670,97 +832,170 @@ __global__ void __launch_bounds__(WT) k_wunpack(const DProd* __restrict__ prods,
             r[3][k] = q.w;
         }
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            uint32_t v[WPR];
-            wcoef(r[q], sc, v);
-            lo[q] = v[0] | (uint64_t)v[1] << 32;
-            mid[q] = v[2] | (uint64_t)v[3] << 32;
-            hi[q] = v[4];
+        for (int q = 0; q < 4; q++) coef_words(r[q], sc, lo[q], mid[q], hi[q]);
+    }
+    const uint32_t tot = limb_sums<WT>(S, t, WT, lo, mid, hi, (int)(w1 - w0), own);
+    store_limbs(P.r, wt, w1, own);
+    if (t == WT - 1) P.agg[tile] = tot;
+}
+
+// Carries between a product's unpack tiles: one warp per 32 tiles.  The carry
+// into its first tile comes from the last lower tile that does not propagate
+// (almost always the one before); a tile's carry stops at its first limb
+// unless that limb is all ones, and then the warp walks the run.  Only r is
+// written, each tile by one warp.
+__global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) {
+    int local;
+    const DProd& P = wjob(A, local);
+    const int lane = (int)threadIdx.x & 31;
+    const int64_t k0 = ((int64_t)local * (WT / 32) + (threadIdx.x >> 5)) * 32, nt = P.ntl;
+    if (k0 >= nt) return;
+    uint32_t cin = 0;
+    for (int64_t k = k0 - 32; k >= 0; k -= 32) {
+        const uint32_t a = P.agg[k + lane];
+        const unsigned stop = __ballot_sync(0xffffffffu, !(a & 2u));
+        if (stop) {
+            cin = __shfl_sync(0xffffffffu, a, 31 - __clz(stop)) & 1u;
+            break;
         }
-    } else {
-#pragma unroll
-        for (int q = 0; q < 4; q++) lo[q] = mid[q] = 0, hi[q] = 0;
     }
-    s_mid[t + 1] = mid[3];
-    s_hi[t + 1][0] = hi[2];
-    s_hi[t + 1][1] = hi[3];
-    __syncthreads();
-    // limb sums lo_i + mid_(i-1) + hi_(i-2) and their carries (0..2)
-    uint64_t own[4];
-    uint32_t cy[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const uint64_t m1 = q ? mid[q - 1] : s_mid[t];
-        const uint32_t h2 = q > 1 ? hi[q - 2] : s_hi[t][q];
-        uint64_t s = lo[q] + m1;
-        uint32_t c = s < m1;
-        s += h2;
-        c += s < h2;
-        own[q] = s;
-        cy[q] = c;
-    }
-    s_c[t + 1] = cy[3];
-    if (t == 0) {
-        uint64_t s = h_lo + h_mid2;
-        uint32_t c = s < h_mid2;
-        s += h_hi3;
-        c += s < h_hi3;
-        s_c[0] = c;
-    }
-    __syncthreads();
-    uint32_t gen = 0, prop = 1;
-    {
-        uint32_t k = s_c[t];  // carry of the sum below
-        uint32_t g = 0;       // carry generated by adding it
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const uint64_t s = own[q] + k + g;  // at most one of the wraps happens: k + g <= 3
-            g = s < (uint64_t)(k + g);
-            own[q] = s;
-            k = cy[q];
-            prop &= (wt + q < w1 && s == ~0ULL) ? 1u : 0u;
-        }
-        gen = g;
-    }
-    const uint32_t agg = gen | (prop << 1);
-    const int lane = t & 31, wid = t >> 5;
-    uint32_t incl = agg;
+    const int64_t k = k0 + lane;
+    uint32_t incl = k < nt ? P.agg[k] : 0u;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
         const uint32_t o = __shfl_up_sync(0xffffffffu, incl, off);
         if (lane >= off) incl = gp_join(o, incl);
     }
-    if (lane == 31) wagg[wid] = incl;
-    __syncthreads();
-    uint32_t wpre = 2u;
-    for (int k = 0; k < wid; k++) wpre = gp_join(wpre, wagg[k]);
     uint32_t excl = __shfl_up_sync(0xffffffffu, incl, 1);
     if (lane == 0) excl = 2u;
-    uint64_t cin = gp_join(wpre, excl) & 1u;  // tile carry-in taken as 0; k_carry adds it
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        own[q] += cin;
-        cin = cin && own[q] == 0;
+    bool walk = false;
+    if (k < nt && (gp_join(cin, excl) & 1u)) {
+        uint64_t* w = P.r + k * UNPACK_TL;
+        if (*w != ~0ULL) *w += 1;
+        else walk = true;
     }
-    if (wt + 3 < w1) {
-        ulonglong2* dst = reinterpret_cast<ulonglong2*>(P.r + wt);
-        if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-            dst[0] = make_ulonglong2(own[0], own[1]);
-            dst[1] = make_ulonglong2(own[2], own[3]);
-        } else {
-#pragma unroll
-            for (int q = 0; q < 4; q++) P.r[wt + q] = own[q];
+    for (unsigned m = __ballot_sync(0xffffffffu, walk); m; m &= m - 1) {
+        const int64_t b0 = (k0 + __ffs(m) - 1) * UNPACK_TL, b1 = min(b0 + (int64_t)UNPACK_TL, P.rn);
+        for (int64_t w = b0; w < b1; w += 32) {
+            const int64_t wl = w + lane;
+            const uint64_t v = wl < b1 ? P.r[wl] : 0ULL;  // past the tile: stops the run
+            const unsigned stop = __ballot_sync(0xffffffffu, v != ~0ULL);
+            const int e = stop ? __ffs(stop) - 1 : 32;
+            if (lane < e) P.r[wl] = 0;
+            else if (lane == e && wl < b1) P.r[wl] = v + 1;
+            if (stop) break;
         }
-    } else {
+    }
+}
+
+// ---------------------------------------------------------------------------
+// small products: one CTA does all of it, N/16 threads per prime; the
+// transforms, the residues and the limbs stay on chip
+
+template <int ODD, int LM>
+struct WSmall {
+    static constexpr int N = ODD << LM, M = 1 << LM, T = M / 16, TP = N / 16;
+    static constexpr int NT = (WPR * TP + 31) / 32 * 32, SM = M + M / 16;
+    static constexpr int LT = N / 4 + 1;  // threads with limbs: r may have N + 1
+    static constexpr size_t bytes = (sizeof(LimbShared<LT>) + 15) / 16 * 16 + sizeof(uint32_t) * WPR * ODD * SM;
+};
+
+template <int ODD, int LM>
+__global__ void __launch_bounds__(WSmall<ODD, LM>::NT, WSmall<ODD, LM>::NT > 384 ? 1 : 768 / WSmall<ODD, LM>::NT)
+    k_wsmall(const __grid_constant__ WArgs A) {
+    using W = WSmall<ODD, LM>;
+    constexpr int J1 = WSplit<LM>::J1, N = W::N, M = W::M, SM = W::SM, TP = W::TP;
+    static_assert(W::LT <= W::NT && W::NT <= 1024, "limb threads");
+    extern __shared__ __align__(16) unsigned char dyn[];
+    LimbShared<W::LT>& S = *reinterpret_cast<LimbShared<W::LT>*>(dyn);
+    uint32_t* sm = reinterpret_cast<uint32_t*>(dyn + (sizeof(LimbShared<W::LT>) + 15) / 16 * 16);
+    int local;
+    const DProd& P = wjob(A, local);
+    const int tid = (int)threadIdx.x;
+    const bool live = tid < WPR * TP;
+    const int pi = live ? tid / TP : 0, u = live ? tid - pi * TP : 0;
+    const int j = u / W::T, t = u & (W::T - 1);
+    const uint32_t p = c_w.p[pi], pinv = c_w.pinv[pi];
+    const size_t toff = ((size_t)pi * ODD + j) << P.wL;
+    const Tw *tf = (const Tw*)P.wtf + toff, *ti = (const Tw*)P.wti + toff;
+    uint32_t* const sp = sm + pi * ODD * SM;  // this prime's blocks
+    uint32_t* const s = sp + j * SM;
+    uint32_t a[16], b[16];
+    auto down = [&](uint32_t* x, const uint64_t* __restrict__ src, int n) {
+        if (ODD == 1) {
+            if (live) {
 #pragma unroll
-        for (int q = 0; q < 4; q++)
-            if (wt + q < w1) P.r[wt + q] = own[q];
+                for (int k = 0; k < 16; k++) {
+                    const int i = wpos<LM, LM, J1>(t, k >> J1, k & ((1 << J1) - 1));
+                    x[k] = wpack<false>(i < n ? __ldg(src + i) : 0ull, pi, p);
+                }
+            }
+        } else {
+            if (live) {
+                for (int c = u; c < M; c += TP) {
+                    uint32_t v[ODD];
+#pragma unroll
+                    for (int r = 0; r < ODD; r++) {
+                        const int i = c + (r << LM);
+                        v[r] = wpack<true>(i < n ? __ldg(src + i) : 0ull, pi, p);
+                    }
+                    dft_odd<ODD, 0>(v, pi, p);
+#pragma unroll
+                    for (int r = 0; r < ODD; r++) sp[r * SM + wpad(c)] = v[r];
+                }
+            }
+            __syncthreads();
+            if (live) wget<LM, LM, J1>(s, x, t);
+        }
+        wblock_down<LM>(x, s, t, tf, 1u, p, live);
+    };
+    down(a, P.a, (int)P.nca);
+    if (!P.sqr) {
+        __syncthreads();  // a's last reads of the shared blocks
+        down(b, P.b, (int)P.ncb);
     }
-    if (t == WT - 1) {
-        uint32_t tot = 2u;
-        for (int k = 0; k < WT / 32; k++) tot = gp_join(tot, wagg[k]);
-        P.agg[tile] = tot;
+    if (live) wpoint<LM>(a, b, P.sqr, t, tf, 1u, p, pinv);
+    wblock_up<LM>(a, s, t, ti, 1u, p, live);
+    if (live) wput<LM, LM, J1>(s, a, t);
+    __syncthreads();
+    if (ODD > 1) {
+        if (live) {
+            for (int c = u; c < M; c += TP) {
+                uint32_t v[ODD];
+#pragma unroll
+                for (int r = 0; r < ODD; r++) v[r] = sp[r * SM + wpad(c)];
+                dft_odd<ODD, 0>(v, pi, p);
+#pragma unroll
+                for (int r = 0; r < ODD; r++) sp[((ODD - r) % ODD) * SM + wpad(c)] = v[r];
+            }
+        }
+        __syncthreads();
     }
+    // coefficients and limbs: thread tid < LT has four
+    uint64_t lo[4] = {0, 0, 0, 0}, mid[4] = {0, 0, 0, 0}, own[4];
+    uint32_t hi[4] = {0, 0, 0, 0};
+    if (tid == 0) {
+        S.mid[0] = 0;
+        S.hi[0][0] = S.hi[0][1] = 0;
+        S.c[0] = 0;
+    }
+    if (4 * tid < N) {
+        uint32_t sc[WPR];
+#pragma unroll
+        for (int k = 0; k < WPR; k++) sc[k] = P.wsc[k];
+        const uint32_t* q0 = sm + ((4 * tid) >> LM) * SM + wpad((4 * tid) & (M - 1));  // four within one padded run
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            uint32_t r[WPR];
+#pragma unroll
+            for (int k = 0; k < WPR; k++) r[k] = q0[k * ODD * SM + q];
+            coef_words(r, sc, lo[q], mid[q], hi[q]);
+        }
+    }
+    const int rn = (int)P.rn, top = min(rn, 4 * W::LT);
+    limb_sums<W::LT>(S, tid, W::LT, lo, mid, hi, top, own);
+    if (tid < W::LT) store_limbs(P.r, 4 * tid, top, own);
+    for (int i = top + tid; i < rn; i += W::NT) P.r[i] = 0;  // limbs above the operands' magnitudes
 }
 
 // ---------------------------------------------------------------------------
@@ -769,63 +1004,121 @@ __global__ void __launch_bounds__(WT) k_wunpack(const DProd* __restrict__ prods,
 int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t rn) {
     const int64_t M = int64_t(1) << s.lm, R = (int64_t)s.odd << s.lj;
     const int64_t cols = M << s.j2, mcols = (int64_t)s.N >> s.j2;
+    const int64_t tiles = (rn + UNPACK_TL - 1) / UNPACK_TL;
     switch (kind) {
         case JK_WCOL_FWD: return ((sqr ? 1 : 2) * WPR * cols + WT - 1) / WT;
         case JK_WCOL_REV: return (WPR * cols + WT - 1) / WT;
         case JK_WMID_FWD: return ((sqr ? 1 : 2) * WPR * mcols + WT - 1) / WT;
         case JK_WMID_REV: return (WPR * mcols + WT - 1) / WT;
         case JK_WBLOCK: return (WPR * R * (M / 16) + WT - 1) / WT;
-        default: return (rn + UNPACK_TL - 1) / UNPACK_TL;
+        case JK_WSMALL: return 1;
+        case JK_WCARRY: return (tiles + WT - 1) / WT;  // 8 warps of 32 tiles
+        default: return tiles;
     }
 }
 
+using WKernel = void (*)(const WArgs);
+struct WLaunch {
+    WKernel fn;
+    int threads;
+    size_t smem;
+};
+
+template <int ODD, int LM>
+static WLaunch small_kernel() {
+    return WLaunch{k_wsmall<ODD, LM>, WSmall<ODD, LM>::NT, WSmall<ODD, LM>::bytes};
+}
 template <int ODD, int LJ>
-static void col_launch(int kind, const DProd* prods, const WSeg* segs, int nseg, const int32_t* plist, unsigned grid,
-                       cudaStream_t st) {
-    if (kind == JK_WCOL_FWD) k_wcol_fwd<ODD, LJ><<<grid, WT, 0, st>>>(prods, segs, nseg, plist);
-    else k_wcol_rev<ODD, LJ><<<grid, WT, 0, st>>>(prods, segs, nseg, plist);
+static WLaunch col_kernel(int kind) {
+    return WLaunch{kind == JK_WCOL_FWD ? k_wcol_fwd<ODD, LJ> : k_wcol_rev<ODD, LJ>, WT, 0};
+}
+template <int J>
+static WLaunch mid_kernel(int kind) {
+    return WLaunch{kind == JK_WMID_FWD ? k_wmid<J, true> : k_wmid<J, false>, WT, 0};
+}
+
+static WLaunch word_kernel(int kind, int variant) {
+    switch (kind) {
+        case JK_WUNPACK: return WLaunch{k_wunpack, WT, 0};
+        case JK_WCARRY: return WLaunch{k_wcarry, WT, 0};
+        case JK_WBLOCK:
+            switch (variant) {
+                case 12: return WLaunch{k_wblock<12>, WT, 0};
+                case 10: return WLaunch{k_wblock<10>, WT, 0};
+                case 8: return WLaunch{k_wblock<8>, WT, 0};
+                case 6: return WLaunch{k_wblock<6>, WT, 0};
+            }
+            break;
+        case JK_WMID_FWD:
+        case JK_WMID_REV:
+            switch (variant) {
+                case 2: return mid_kernel<2>(kind);
+                case 3: return mid_kernel<3>(kind);
+                case 4: return mid_kernel<4>(kind);
+                case 5: return mid_kernel<5>(kind);
+            }
+            break;
+        case JK_WCOL_FWD:
+        case JK_WCOL_REV:
+            switch (variant) {
+#define NBG_COL(O, J) \
+    case (O << 8) | J: return col_kernel<O, J>(kind);
+                NBG_COL(1, 1) NBG_COL(1, 2) NBG_COL(1, 3) NBG_COL(1, 4) NBG_COL(1, 5)
+                NBG_COL(3, 0) NBG_COL(3, 1) NBG_COL(3, 2) NBG_COL(3, 3)
+                NBG_COL(5, 0) NBG_COL(5, 1) NBG_COL(5, 2)
+                NBG_COL(7, 0) NBG_COL(7, 1) NBG_COL(7, 2)
+#undef NBG_COL
+            }
+            break;
+        case JK_WSMALL:
+            switch (variant) {
+#define NBG_SMALL(O, M) \
+    case (O << 8) | M: return small_kernel<O, M>();
+#define NBG_SMALLS                                                                                          \
+    NBG_SMALL(1, 6) NBG_SMALL(1, 7) NBG_SMALL(1, 8) NBG_SMALL(1, 9) NBG_SMALL(1, 10) NBG_SMALL(1, 11)       \
+    NBG_SMALL(3, 6) NBG_SMALL(3, 7) NBG_SMALL(3, 8) NBG_SMALL(3, 9) NBG_SMALL(3, 10) NBG_SMALL(5, 6)        \
+    NBG_SMALL(5, 7) NBG_SMALL(5, 8) NBG_SMALL(5, 9) NBG_SMALL(7, 6) NBG_SMALL(7, 7) NBG_SMALL(7, 8)
+                NBG_SMALLS
+#undef NBG_SMALL
+            }
+            break;
+    }
+    return WLaunch{nullptr, 0, 0};
+}
+
+static cudaError_t small_attributes() {
+    cudaError_t e = cudaSuccess;
+#define NBG_SMALL(O, M)                                                                                     \
+    if (e == cudaSuccess)                                                                                   \
+        e = cudaFuncSetAttribute(k_wsmall<O, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,               \
+                                 (int)WSmall<O, M>::bytes);
+    NBG_SMALLS
+#undef NBG_SMALL
+    return e;
+}
+
+static cudaError_t launch(int kind, int variant, const WArgs& a, int64_t nctas, cudaStream_t st) {
+    if (nctas <= 0) return cudaSuccess;
+    const WLaunch k = word_kernel(kind, variant);
+    if (!k.fn || nctas > 0x7fffffff) return cudaErrorInvalidValue;
+    k.fn<<<(unsigned)nctas, k.threads, k.smem, st>>>(a);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_word(int kind, int variant, const DProd* prods, const WSeg* segs, int nseg, const int32_t* plist,
                         int64_t nctas, cudaStream_t st) {
-    if (nctas <= 0) return cudaSuccess;
-    if (nctas > 0x7fffffff) return cudaErrorInvalidValue;
-    const unsigned grid = (unsigned)nctas;
-    if (kind == JK_WUNPACK) {
-        k_wunpack<<<grid, WT, 0, st>>>(prods, segs, nseg, plist);
-    } else if (kind == JK_WBLOCK) {
-        switch (variant) {
-            case 12: k_wblock<12><<<grid, WT, 0, st>>>(prods, segs, nseg, plist); break;
-            case 10: k_wblock<10><<<grid, WT, 0, st>>>(prods, segs, nseg, plist); break;
-            case 8: k_wblock<8><<<grid, WT, 0, st>>>(prods, segs, nseg, plist); break;
-            case 6: k_wblock<6><<<grid, WT, 0, st>>>(prods, segs, nseg, plist); break;
-            default: return cudaErrorInvalidValue;
-        }
-    } else if (kind == JK_WMID_FWD || kind == JK_WMID_REV) {
-        const bool f = kind == JK_WMID_FWD;
-        switch (variant) {
-#define NBG_MID(J)                                                               \
-    case J:                                                                      \
-        if (f) k_wmid<J, true><<<grid, WT, 0, st>>>(prods, segs, nseg, plist);   \
-        else k_wmid<J, false><<<grid, WT, 0, st>>>(prods, segs, nseg, plist);    \
-        break;
-            NBG_MID(2) NBG_MID(3) NBG_MID(4) NBG_MID(5)
-#undef NBG_MID
-            default: return cudaErrorInvalidValue;
-        }
-    } else {
-        switch (variant) {
-#define NBG_COL(O, J) \
-    case (O << 8) | J: col_launch<O, J>(kind, prods, segs, nseg, plist, grid, st); break;
-            NBG_COL(1, 1) NBG_COL(1, 2) NBG_COL(1, 3) NBG_COL(1, 4) NBG_COL(1, 5)
-            NBG_COL(3, 0) NBG_COL(3, 1) NBG_COL(3, 2) NBG_COL(3, 3)
-            NBG_COL(5, 0) NBG_COL(5, 1) NBG_COL(5, 2)
-            NBG_COL(7, 0) NBG_COL(7, 1) NBG_COL(7, 2)
-#undef NBG_COL
-            default: return cudaErrorInvalidValue;
-        }
-    }
-    return cudaGetLastError();
+    WArgs a{};
+    a.prods = prods;
+    a.segs = segs;
+    a.plist = plist;
+    a.nseg = nseg;
+    return launch(kind, variant, a, nctas, st);
+}
+
+cudaError_t launch_word_one(int kind, int variant, const DProd& P, int64_t nctas, cudaStream_t st) {
+    WArgs a{};
+    a.one = P;
+    return launch(kind, variant, a, nctas, st);
 }
 
 }  // namespace nbg

@@ -16,7 +16,7 @@ torch = pytest.importorskip("torch")
 
 # (odd multiplier, log2 of the rest): each column-pass and block variant, the
 # smallest and largest lengths of the range
-SHAPES = [(1, 7), (1, 8), (1, 9), (1, 10), (1, 11), (1, 12), (1, 13), (1, 14), (1, 15), (1, 16), (1, 17),
+SHAPES = [(1, 6), (3, 8), (5, 9), (7, 8), (1, 7), (1, 8), (1, 9), (1, 10), (1, 11), (1, 12), (1, 13), (1, 14), (1, 15), (1, 16), (1, 17),
           (3, 6), (3, 7), (3, 9), (3, 10), (3, 12), (3, 13), (3, 14), (3, 15),
           (5, 6), (5, 7), (5, 8), (5, 12), (5, 13), (5, 14),
           (7, 6), (7, 7), (7, 10), (7, 12), (7, 13), (7, 14),
@@ -57,6 +57,7 @@ def test_word_shapes(gpu_lib, odd, k):
 def test_word_kernels_run_and_edge_operands(gpu_lib):
     rng = np.random.default_rng(77)
     a, b = rand_limbs(rng, 3000), rand_limbs(rng, 2500)
+    assert "k_wsmall" in _kinds(gpu_lib, a[:200].copy(), b[:100].copy())
     assert "k_wunpack" in _kinds(gpu_lib, a, b) and "k_wunpack" in _kinds(gpu_lib, a, None)
     for m, n in ((1, 1), (2, 1), (700, 1), (513, 512), (65536, 65537), (130000, 3)):
         x, y = adversarial(rng, m), adversarial(rng, n)
