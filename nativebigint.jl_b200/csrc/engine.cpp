@@ -837,7 +837,7 @@ int word_setup(Engine& E, const ProdIn& q, const WordShape& s, DProd& P) {
 // Launches of one word product in order: kind and variant.
 static std::vector<std::pair<int, int>> word_steps(const WordShape& s) {
     if (s.small) return {{JK_WSMALL, (s.odd << 8) | s.lm}};
-    const int col = (s.odd << 8) | (s.lj - s.j2);
+    const int col = (s.lm + s.j2 == 12 ? 1 << 16 : 0) | (s.odd << 8) | (s.lj - s.j2);
     std::vector<std::pair<int, int>> v{{JK_WCOL_FWD, col}};
     if (s.j2) v.push_back({JK_WMID_FWD, s.j2});
     v.push_back({JK_WBLOCK, s.lm});

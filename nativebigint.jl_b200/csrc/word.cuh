@@ -60,8 +60,9 @@ __device__ __forceinline__ void load_tw(const Tw* __restrict__ tab, uint32_t i, 
 }
 
 // J levels on 2^J values x[0], x[ST], x[2 ST], ...: the subtree under node
-// `idx` (heap order) of a forward table.
-template <int J, int ST>
+// `idx` (heap order) of a forward table.  NV vectors, VS apart, share the constants; the first T0 levels
+// are the caller's.
+template <int J, int ST, int NV = 1, int VS = 0, int T0 = 0>
 __device__ __forceinline__ void tree_fwd(uint32_t* x, const Tw* __restrict__ tab, uint32_t idx, uint32_t p) {
     const uint32_t p2 = 2 * p;
     auto level = [&](auto tc) {
@@ -72,9 +73,12 @@ __device__ __forceinline__ void tree_fwd(uint32_t* x, const Tw* __restrict__ tab
 #pragma unroll
         for (int i = 0; i < (1 << t); i++)
 #pragma unroll
-            for (int e = 0; e < h; e++) bf_fwd(x[(2 * h * i + e) * ST], x[(2 * h * i + e + h) * ST], w[i], p, p2);
+            for (int e = 0; e < h; e++)
+#pragma unroll
+                for (int v = 0; v < NV; v++)
+                    bf_fwd(x[v * VS + (2 * h * i + e) * ST], x[v * VS + (2 * h * i + e + h) * ST], w[i], p, p2);
     };
-    if constexpr (J > 0) level(std::integral_constant<int, 0>{});
+    if constexpr (J > 0 && T0 < 1) level(std::integral_constant<int, 0>{});
     if constexpr (J > 1) level(std::integral_constant<int, 1>{});
     if constexpr (J > 2) level(std::integral_constant<int, 2>{});
     if constexpr (J > 3) level(std::integral_constant<int, 3>{});

@@ -47,7 +47,7 @@ struct WSeg {
     int32_t pad_;
 };
 
-// variant of a word launch: (odd << 8) | (lj - j2) for column passes, j2 for middle ones, lm for
+// variant of a word launch: (odd << 8) | (lj - j2) for column passes (bit 16: of 4096 columns), j2 for middle ones, lm for
 // blocks, (odd << 8) | lm for one-CTA products
 cudaError_t word_init();  // constant memory of the current device
 cudaError_t launch_word(int kind, int variant, const DProd* prods, const WSeg* segs, int nseg, const int32_t* plist,

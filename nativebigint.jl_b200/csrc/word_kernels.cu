@@ -30,6 +30,7 @@ struct WConst {
     Tw r3[WPR];                  // e(1/3)
     Tw r5[WPR][5];               // -1/4, (c1-c2)/2, f1, f2 of e(1/5) (see dft5); [4] unused
     uint32_t c7[WPR][3], f7[WPR][3];  // cosine and sine halves of e(j/7) in 2^32 form
+    uint32_t wt[WPR][WPR];       // words of W_i = p_0 ... p_(i-1) (i words)
     uint32_t gar[WPR][WPR];      // mixed radix: gar[i][j] = -W_j / W_i mod p_i in 2^32 form (j < i)
 };
 __constant__ WConst c_w;
@@ -101,6 +102,16 @@ cudaError_t word_init() {
             h.gar[i][j] = mont((p - Wj * iw % p) % p, p);
             Wj = Wj * (WPRIMES[j] % p) % p;
         }
+        uint32_t w[WPR] = {1};
+        for (int t = 0; t < i; t++) {
+            uint64_t cy = 0;
+            for (int k = 0; k < WPR; k++) {
+                cy += (uint64_t)w[k] * WPRIMES[t];
+                w[k] = (uint32_t)cy;
+                cy >>= 32;
+            }
+        }
+        for (int k = 0; k < WPR; k++) h.wt[i][k] = w[k];
     }
     cudaError_t e = small_attributes();
     return e == cudaSuccess ? cudaMemcpyToSymbol(c_w, &h, sizeof h) : e;
@@ -332,51 +343,73 @@ __device__ __forceinline__ uint32_t wpack(uint64_t v, int pi, uint32_t p) {
     return RED ? wd::sub_if(y, 2 * p) : y;
 }
 
-template <int ODD, int LJ>
-__global__ void __launch_bounds__(WT) k_wcol_fwd(const __grid_constant__ WArgs A) {
+// LM: log2 of the column count when the blocks are 4096 values (row strides are
+// then immediate offsets), 0: read from the product.  Rows past the operand are
+// not packed, and when they are its upper half (odd = 1, a half-length operand,
+// which one of two always is) the first level is a copy.
+template <int ODD, int LJ, int LM>
+__global__ void __launch_bounds__(WT, 4) k_wcol_fwd(const __grid_constant__ WArgs A) {
     constexpr int R = ODD << LJ;
     int local;
     const DProd& P = wjob(A, local);
-    const int lm = P.wlm + P.wj2;  // log2 of the column count
+    const int lm = LM ? LM : P.wlm + P.wj2;
     const int id = local * WT + (int)threadIdx.x;
     const int c = id & ((1 << lm) - 1);
     int pi = id >> lm;  // operand-major: a's primes, then b's
     const bool isb = pi >= WPR;
     if (isb) pi -= WPR;
     if (pi >= WPR || (isb && P.sqr)) return;
-    const uint64_t* __restrict__ src = isb ? P.b : P.a;
     const int n = (int)(isb ? P.ncb : P.nca);
-    uint32_t* __restrict__ dst = (isb ? P.wb : P.wa) + (size_t)pi * (size_t)P.wN;
+    const int rows = (n + (1 << lm) - 1) >> lm;
+    const uint64_t* __restrict__ src = (isb ? P.b : P.a) + c;
+    uint32_t* __restrict__ dst = (isb ? P.wb : P.wa) + (size_t)pi * (size_t)P.wN + c;
     const uint32_t p = c_w.p[pi];
-    uint32_t x[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        const int i = c + (r << lm);
-        x[r] = wpack<(ODD > 1)>(i < n ? __ldg(src + i) : 0ull, pi, p);
-    }
-    dft_odd<ODD, LJ>(x, pi, p);
     const Tw* tab = (const Tw*)P.wtf + (((size_t)pi * ODD) << P.wL);
+    uint32_t x[R];
+    auto rowsin = [&](auto r0c, auto r1c) {
+        constexpr int r0 = decltype(r0c)::value, r1 = decltype(r1c)::value;
+        uint64_t v[r1 - r0];
 #pragma unroll
-    for (int j = 0; j < ODD; j++) wd::tree_fwd<LJ, 1>(x + (j << LJ), tab + ((size_t)j << P.wL), 1u, p);
+        for (int r = r0; r < r1; r++) v[r - r0] = c + (r << lm) < n ? __ldg(src + ((size_t)r << lm)) : 0ull;
 #pragma unroll
-    for (int r = 0; r < R; r++) dst[c + (r << lm)] = x[r];
+        for (int r = r0; r < r1; r++) x[r] = r < rows ? wpack<(ODD > 1)>(v[r - r0], pi, p) : 0u;
+    };
+    constexpr int H = R / 2;
+    if (ODD == 1 && LJ > 0 && rows <= H) {
+        rowsin(std::integral_constant<int, 0>{}, std::integral_constant<int, H>{});
+#pragma unroll
+        for (int r = 0; r < H; r++) x[r + H] = x[r];
+        wd::tree_fwd<LJ, 1, 1, 0, 1>(x, tab, 1u, p);
+    } else {
+        if (R > 16) {  // at most half of the limbs in registers at once
+            rowsin(std::integral_constant<int, 0>{}, std::integral_constant<int, H>{});
+            rowsin(std::integral_constant<int, H>{}, std::integral_constant<int, R>{});
+        } else {
+            rowsin(std::integral_constant<int, 0>{}, std::integral_constant<int, R>{});
+        }
+        dft_odd<ODD, LJ>(x, pi, p);
+#pragma unroll
+        for (int j = 0; j < ODD; j++) wd::tree_fwd<LJ, 1>(x + (j << LJ), tab + ((size_t)j << P.wL), 1u, p);
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) dst[(size_t)r << lm] = x[r];
 }
 
-template <int ODD, int LJ>
-__global__ void __launch_bounds__(WT) k_wcol_rev(const __grid_constant__ WArgs A) {
+template <int ODD, int LJ, int LM>
+__global__ void __launch_bounds__(WT, LM ? 4 : 3) k_wcol_rev(const __grid_constant__ WArgs A) {
     constexpr int R = ODD << LJ;
     int local;
     const DProd& P = wjob(A, local);
-    const int lm = P.wlm + P.wj2;  // log2 of the column count
+    const int lm = LM ? LM : P.wlm + P.wj2;
     const int id = local * WT + (int)threadIdx.x;
     const int c = id & ((1 << lm) - 1);
     const int pi = id >> lm;
     if (pi >= WPR) return;
-    uint32_t* __restrict__ dst = P.wa + (size_t)pi * (size_t)P.wN;
+    uint32_t* __restrict__ dst = P.wa + (size_t)pi * (size_t)P.wN + c;
     const uint32_t p = c_w.p[pi];
     uint32_t x[R];
 #pragma unroll
-    for (int r = 0; r < R; r++) x[r] = dst[c + (r << lm)];
+    for (int r = 0; r < R; r++) x[r] = dst[(size_t)r << lm];
     const Tw* tab = (const Tw*)P.wti + (((size_t)pi * ODD) << P.wL);
 #pragma unroll
     for (int j = 0; j < ODD; j++) wd::tree_rev<LJ, 1>(x + (j << LJ), tab + ((size_t)j << P.wL), 1u, p);
@@ -385,18 +418,19 @@ __global__ void __launch_bounds__(WT) k_wcol_rev(const __grid_constant__ WArgs A
 #pragma unroll
     for (int r = 0; r < R; r++) {
         const int i = r >> LJ, ri = (ODD - i) % ODD;
-        dst[c + (((ri << LJ) + (r & ((1 << LJ) - 1))) << lm)] = x[r];
+        dst[(size_t)((ri << LJ) + (r & ((1 << LJ) - 1))) << lm] = x[r];
     }
 }
 
 // Middle passes: the 2^J rows (2^lm apart) of one column of a segment, the
-// subtree of the segment's node.  In place; all columns of a segment share
+// subtree of the segment's node, above blocks of 4096.  In place; all columns of a segment share
 // their constants.
 template <int J, bool FWD>
 __global__ void __launch_bounds__(WT) k_wmid(const __grid_constant__ WArgs A) {
     int local;
     const DProd& P = wjob(A, local);
-    const int lm = P.wlm, j1 = P.wlj - J, R1 = P.wodd << j1;
+    constexpr int lm = 12;  // more than 32 rows only stand above 4096-value blocks
+    const int j1 = P.wlj - J, R1 = P.wodd << j1;
     const int id = local * WT + (int)threadIdx.x;
     const int c = id & ((1 << lm) - 1);
     int op = (id >> lm) / R1;  // operand-major, then prime
@@ -422,23 +456,30 @@ __global__ void __launch_bounds__(WT) k_wmid(const __grid_constant__ WArgs A) {
 // A round runs J levels on sub-blocks of 2^LL values; a thread takes 2^(4-J)
 // groups of 2^J values at stride S = 2^(LL-J).  The last round always runs two
 // levels on 16 consecutive values, leaving the thread four whole leaves.
-// Shared memory is padded by one word in 16: free of bank conflicts for the
-// strides 1, 4 and 16, at most two-way for the larger ones.
+// Shared memory is padded by four words in 16 and 16 in 256: the last round's
+// 16 words per thread move as four 16-byte accesses, and every stride (16 at
+// least before that round) is free of bank conflicts or two-way.  A group's
+// values lie at compile-time offsets from its first one: its index has zeros
+// in the bits that e * S occupies, so the padding of the sum is the sum of the
+// paddings.
 
-__device__ __forceinline__ int wpad(int i) { return i + (i >> 4); }
+__host__ __device__ constexpr int wpad(int i) { return i + ((i >> 4) << 2) + ((i >> 8) << 4); }
+__host__ __device__ constexpr int wwords(int m) { return m + m / 4 + m / 16; }  // padded words of m >= 64 values
 
+// index of the first value of thread t's q-th group
 template <int LM, int LL, int J>
-__device__ __forceinline__ int wpos(int t, int q, int e) {
+__device__ __forceinline__ int wpos(int t, int q) {
     constexpr int S = 1 << (LL - J), T = 1 << (LM - 4);
+    static_assert(S >= 16, "strides below the padding period");
     const int gi = t + q * T;
-    return ((gi >> (LL - J)) << LL) + (gi & (S - 1)) + e * S;
+    return ((gi >> (LL - J)) << LL) + (gi & (S - 1));
 }
-template <int LM, int LL, int J>
+template <int LM, int LL, int J, int NV>
 __device__ __forceinline__ void wround_fwd(uint32_t* x, int t, const Tw* __restrict__ tab, uint32_t h0, uint32_t p) {
     constexpr int T = 1 << (LM - 4);
 #pragma unroll
     for (int q = 0; q < (1 << (4 - J)); q++)
-        wd::tree_fwd<J, 1>(x + (q << J), tab, (h0 << (LM - LL)) + (uint32_t)((t + q * T) >> (LL - J)), p);
+        wd::tree_fwd<J, 1, NV, 16>(x + (q << J), tab, (h0 << (LM - LL)) + (uint32_t)((t + q * T) >> (LL - J)), p);
 }
 template <int LM, int LL, int J>
 __device__ __forceinline__ void wround_rev(uint32_t* x, int t, const Tw* __restrict__ tab, uint32_t h0, uint32_t p) {
@@ -450,12 +491,36 @@ __device__ __forceinline__ void wround_rev(uint32_t* x, int t, const Tw* __restr
 template <int LM, int LL, int J>
 __device__ __forceinline__ void wput(uint32_t* s, const uint32_t* x, int t) {
 #pragma unroll
-    for (int k = 0; k < 16; k++) s[wpad(wpos<LM, LL, J>(t, k >> J, k & ((1 << J) - 1)))] = x[k];
+    for (int q = 0; q < (1 << (4 - J)); q++) {
+        uint32_t* d = s + wpad(wpos<LM, LL, J>(t, q));
+#pragma unroll
+        for (int e = 0; e < (1 << J); e++) d[wpad(e << (LL - J))] = x[(q << J) + e];
+    }
 }
 template <int LM, int LL, int J>
 __device__ __forceinline__ void wget(const uint32_t* s, uint32_t* x, int t) {
 #pragma unroll
-    for (int k = 0; k < 16; k++) x[k] = s[wpad(wpos<LM, LL, J>(t, k >> J, k & ((1 << J) - 1)))];
+    for (int q = 0; q < (1 << (4 - J)); q++) {
+        const uint32_t* d = s + wpad(wpos<LM, LL, J>(t, q));
+#pragma unroll
+        for (int e = 0; e < (1 << J); e++) x[(q << J) + e] = d[wpad(e << (LL - J))];
+    }
+}
+// the 16 consecutive values 16t .. 16t+15
+__device__ __forceinline__ uint4* wrow(uint32_t* s, int t) { return reinterpret_cast<uint4*>(s + wpad(16 * t)); }
+__device__ __forceinline__ void wput16(uint32_t* s, const uint32_t* x, int t) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) wrow(s, t)[k] = make_uint4(x[4 * k], x[4 * k + 1], x[4 * k + 2], x[4 * k + 3]);
+}
+__device__ __forceinline__ void wget16(uint32_t* s, uint32_t* x, int t) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint4 v = wrow(s, t)[k];
+        x[4 * k] = v.x;
+        x[4 * k + 1] = v.y;
+        x[4 * k + 2] = v.z;
+        x[4 * k + 3] = v.w;
+    }
 }
 
 // level splits of a block: J1, J2 (0: none), then the two leaf levels
@@ -476,39 +541,36 @@ struct WSplit<7> { static constexpr int J1 = 3, J2 = 0; };
 template <>
 struct WSplit<6> { static constexpr int J1 = 2, J2 = 0; };
 
-// A block down to its leaves, from the first round's values in x: x[0..16) =
-// values 16t .. 16t+15 in [0, 4p).
-template <int LM>
+// NV blocks (the operands' values at x[16 v ..], their shared memory SM words
+// apart) down to their leaves, from the first round's values: x[16 v + k] =
+// value 16t + k in [0, 4p).  The operands of a product go down together: they
+// share every constant load and barrier and double the independent butterflies.
+template <int LM, int NV, int SM>
 __device__ __forceinline__ void wblock_down(uint32_t* x, uint32_t* s, int t, const Tw* __restrict__ tab, uint32_t h0,
                                             uint32_t p, bool live) {
     constexpr int J1 = WSplit<LM>::J1, J2 = WSplit<LM>::J2;
     if (live) {
-        wround_fwd<LM, LM, J1>(x, t, tab, h0, p);
-        wput<LM, LM, J1>(s, x, t);
+        wround_fwd<LM, LM, J1, NV>(x, t, tab, h0, p);
+#pragma unroll
+        for (int v = 0; v < NV; v++) wput<LM, LM, J1>(s + v * SM, x + 16 * v, t);
     }
     __syncthreads();
     if constexpr (J2 > 0) {
         if (live) {
-            wget<LM, LM - J1, J2>(s, x, t);
-            wround_fwd<LM, LM - J1, J2>(x, t, tab, h0, p);
-            wput<LM, LM - J1, J2>(s, x, t);
+#pragma unroll
+            for (int v = 0; v < NV; v++) wget<LM, LM - J1, J2>(s + v * SM, x + 16 * v, t);
+            wround_fwd<LM, LM - J1, J2, NV>(x, t, tab, h0, p);
+#pragma unroll
+            for (int v = 0; v < NV; v++) wput<LM, LM - J1, J2>(s + v * SM, x + 16 * v, t);
         }
         __syncthreads();
     }
     if (live) {
 #pragma unroll
-        for (int k = 0; k < 16; k++) x[k] = s[17 * t + k];
-        const uint32_t idx = (h0 << (LM - 4)) + (uint32_t)t, p2 = 2 * p;
-        Tw w1[1], w2[2];
-        wd::load_tw<0>(tab, idx, w1);
-        wd::load_tw<1>(tab, idx, w2);
+        for (int v = 0; v < NV; v++) wget16(s + v * SM, x + 16 * v, t);
+        const uint32_t idx = (h0 << (LM - 4)) + (uint32_t)t;
 #pragma unroll
-        for (int e = 0; e < 8; e++) wd::bf_fwd(x[e], x[e + 8], w1[0], p, p2);
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            wd::bf_fwd(x[e], x[e + 4], w2[0], p, p2);
-            wd::bf_fwd(x[e + 8], x[e + 12], w2[1], p, p2);
-        }
+        for (int q = 0; q < 4; q++) wd::tree_fwd<2, 4, NV, 16>(x + q, tab, idx, p);
     }
 }
 
@@ -532,8 +594,7 @@ __device__ __forceinline__ void wblock_up(uint32_t* a, uint32_t* s, int t, const
         }
 #pragma unroll
         for (int e = 0; e < 8; e++) wd::bf_rev(a[e], a[e + 8], w1[0], p, p2);
-#pragma unroll
-        for (int k = 0; k < 16; k++) s[17 * t + k] = a[k];
+        wput16(s, a, t);
     }
     __syncthreads();
     if constexpr (J2 > 0) {
@@ -596,9 +657,9 @@ __device__ __forceinline__ void wpoint(uint32_t* a, uint32_t* b, bool sqr, int t
 template <int LM>
 __global__ void __launch_bounds__(WT, 3) k_wblock(const __grid_constant__ WArgs A) {
     constexpr int T = 1 << (LM - 4), PER = WT / T;  // threads per block, blocks per CTA
-    constexpr int SM = (1 << LM) + (1 << (LM - 4));
+    constexpr int SM = wwords(1 << LM);
     constexpr int J1 = WSplit<LM>::J1;
-    __shared__ uint32_t sm[2][PER][SM];
+    __shared__ __align__(16) uint32_t sm[PER][2][SM];
     int local;
     const DProd& P = wjob(A, local);
     const int g = (int)threadIdx.x / T, t = (int)threadIdx.x & (T - 1);
@@ -612,57 +673,59 @@ __global__ void __launch_bounds__(WT, 3) k_wblock(const __grid_constant__ WArgs 
     const size_t toff = ((size_t)pi * P.wodd + j) << P.wL, xoff = (size_t)pi * (size_t)P.wN + ((size_t)row << LM);
     const Tw* tf = (const Tw*)P.wtf + toff;
     uint32_t* xa = P.wa + xoff;
-    uint32_t a[16], b[16];
-    auto load = [&](uint32_t* x, const uint32_t* src) {
-        if (!live) return;
+    uint32_t x[32];  // a's 16 values, then b's
+    auto load = [&](uint32_t* v, const uint32_t* src) {
 #pragma unroll
-        for (int k = 0; k < 16; k++) x[k] = src[wpos<LM, LM, J1>(t, k >> J1, k & ((1 << J1) - 1))];
+        for (int k = 0; k < 16; k++)
+            v[k] = src[wpos<LM, LM, J1>(t, k >> J1) + ((k & ((1 << J1) - 1)) << (LM - J1))];
     };
-    load(a, xa);
-    wblock_down<LM>(a, sm[0][g], t, tf, h0, p, live);
+    uint32_t* const a = x;
+    if (live) load(x, xa);
     if (!P.sqr) {
-        load(b, P.wb + xoff);
-        wblock_down<LM>(b, sm[1][g], t, tf, h0, p, live);
-        if (live) wpoint<LM>(a, b, false, t, tf, h0, p, pinv);
-    } else if (live) {
-        wpoint<LM>(a, b, true, t, tf, h0, p, pinv);
+        if (live) load(x + 16, P.wb + xoff);
+        wblock_down<LM, 2, SM>(x, sm[g][0], t, tf, h0, p, live);
+    } else {
+        wblock_down<LM, 1, SM>(x, sm[g][0], t, tf, h0, p, live);
     }
-    wblock_up<LM>(a, sm[1][g], t, (const Tw*)P.wti + toff, h0, p, live);
+    if (live) wpoint<LM>(x, x + 16, P.sqr, t, tf, h0, p, pinv);
+    wblock_up<LM>(x, sm[g][0], t, (const Tw*)P.wti + toff, h0, p, live);
     if (live) {
 #pragma unroll
-        for (int k = 0; k < 16; k++) xa[wpos<LM, LM, J1>(t, k >> J1, k & ((1 << J1) - 1))] = a[k];
+        for (int k = 0; k < 16; k++)
+            xa[wpos<LM, LM, J1>(t, k >> J1) + ((k & ((1 << J1) - 1)) << (LM - J1))] = a[k];
     }
 }
 
 // ---------------------------------------------------------------------------
 // unpack: coefficients and carried limbs, tiles of UNPACK_TL limbs
 
-// The coefficient whose residues (any representatives below 4p, scaled) are r:
-// mixed-radix digits y_i, each one sum of wide products and one reduction,
-// then sum y_i W_i by Horner's rule.
+// The coefficient whose residues (representatives below 2p, scaled) are r:
+// mixed-radix digits y_i, each one sum of wide products and one reduction, then
+// sum y_i W_i by columns of 32 bits (at most four products below 2^62 each).
 __device__ __forceinline__ void wcoef(const uint32_t* r, const uint32_t* sc, uint32_t* v) {
     uint32_t y[WPR];
 #pragma unroll
     for (int i = 0; i < WPR; i++) {
         const uint32_t p = c_w.p[i];
-        uint64_t s = wd::mulx(r[i], sc[i]);  // < 4p^2; the others < 1.3p^2 each
+        uint64_t s = wd::mulx(r[i], sc[i]);  // < 2p^2; the others < 1.3p^2 each
 #pragma unroll
         for (int j = 0; j < i; j++) s += wd::mulx(y[j], c_w.gar[i][j]);
-        y[i] = wd::sub_if(wd::sub_if(wd::redc(s, p, c_w.pinv[i]), 2 * p), p);
+        // below 1.5p, 1.85p, 2.2p, 2.5p, 2.8p: one or two subtractions
+        y[i] = wd::sub_if(wd::redc(s, p, c_w.pinv[i]), p);
+        if (i > 1) y[i] = wd::sub_if(y[i], p);
     }
-    v[0] = y[WPR - 1];
+    uint64_t s = y[0];
 #pragma unroll
-    for (int i = WPR - 2; i >= 0; i--) {
-        uint64_t cy = y[i];
-        const uint32_t p = c_w.p[i];
+    for (int k = 0; k < WPR - 1; k++) {
+        uint64_t col = wd::mulx(y[k + 1], c_w.wt[k + 1][k]);
 #pragma unroll
-        for (int k = 0; k < WPR - 1 - i; k++) {
-            cy += wd::mulx(v[k], p);
-            v[k] = (uint32_t)cy;
-            cy >>= 32;
-        }
-        v[WPR - 1 - i] = (uint32_t)cy;
+        for (int i = k + 2; i < WPR; i++) col += wd::mulx(y[i], c_w.wt[i][k]);
+        // col < (4 - k) * 2^62 and s < 2^33: no overflow
+        s += col;
+        v[k] = (uint32_t)s;
+        s >>= 32;
     }
+    v[WPR - 1] = (uint32_t)s;
 }
 
 __device__ __forceinline__ uint32_t gp_join(uint32_t lower, uint32_t upper) {
@@ -775,6 +838,22 @@ __device__ __forceinline__ void coef_words(const uint32_t* r, const uint32_t* sc
     hi = v[4];
 }
 
+// Four consecutive coefficients; prime k's residues are x[k * stride].
+__device__ __forceinline__ void coef4(const uint4* __restrict__ x, int stride, const uint32_t* sc, uint64_t* lo,
+                                      uint64_t* mid, uint32_t* hi) {
+    uint32_t r[4][WPR];
+#pragma unroll
+    for (int k = 0; k < WPR; k++) {
+        const uint4 q = x[(size_t)k * stride];
+        r[0][k] = q.x;
+        r[1][k] = q.y;
+        r[2][k] = q.z;
+        r[3][k] = q.w;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) coef_words(r[q], sc, lo[q], mid[q], hi[q]);
+}
+
 __global__ void __launch_bounds__(WT) k_wunpack(const __grid_constant__ WArgs A) {
     __shared__ LimbShared<WT> S;
     __shared__ uint64_t h_lo, h_mid2;  // the limb sum below the tile
@@ -822,17 +901,7 @@ __global__ void __launch_bounds__(WT) k_wunpack(const __grid_constant__ WArgs A)
     uint64_t lo[4] = {0, 0, 0, 0}, mid[4] = {0, 0, 0, 0}, own[4];
     uint32_t hi[4] = {0, 0, 0, 0};
     if (wt < N) {  // N is a multiple of 4: all four or none
-        uint32_t r[4][WPR];
-#pragma unroll
-        for (int k = 0; k < WPR; k++) {
-            const uint4 q = *reinterpret_cast<const uint4*>(x + (size_t)k * N + wt);
-            r[0][k] = q.x;
-            r[1][k] = q.y;
-            r[2][k] = q.z;
-            r[3][k] = q.w;
-        }
-#pragma unroll
-        for (int q = 0; q < 4; q++) coef_words(r[q], sc, lo[q], mid[q], hi[q]);
+        coef4(reinterpret_cast<const uint4*>(x + wt), N / 4, sc, lo, mid, hi);
     }
     const uint32_t tot = limb_sums<WT>(S, t, WT, lo, mid, hi, (int)(w1 - w0), own);
     store_limbs(P.r, wt, w1, own);
@@ -895,13 +964,14 @@ __global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) 
 template <int ODD, int LM>
 struct WSmall {
     static constexpr int N = ODD << LM, M = 1 << LM, T = M / 16, TP = N / 16;
-    static constexpr int NT = (WPR * TP + 31) / 32 * 32, SM = M + M / 16;
+    static constexpr int NT = (WPR * TP + 31) / 32 * 32, SM = wwords(M);
     static constexpr int LT = N / 4 + 1;  // threads with limbs: r may have N + 1
-    static constexpr size_t bytes = (sizeof(LimbShared<LT>) + 15) / 16 * 16 + sizeof(uint32_t) * WPR * ODD * SM;
+    static constexpr int OPW = WPR * ODD * SM;  // words of one operand's blocks
+    static constexpr size_t bytes = (sizeof(LimbShared<LT>) + 15) / 16 * 16 + sizeof(uint32_t) * 2 * OPW;
 };
 
 template <int ODD, int LM>
-__global__ void __launch_bounds__(WSmall<ODD, LM>::NT, WSmall<ODD, LM>::NT > 384 ? 1 : 768 / WSmall<ODD, LM>::NT)
+__global__ void __launch_bounds__(WSmall<ODD, LM>::NT, WSmall<ODD, LM>::NT > 320 ? 1 : 640 / WSmall<ODD, LM>::NT)
     k_wsmall(const __grid_constant__ WArgs A) {
     using W = WSmall<ODD, LM>;
     constexpr int J1 = WSplit<LM>::J1, N = W::N, M = W::M, SM = W::SM, TP = W::TP;
@@ -920,41 +990,48 @@ __global__ void __launch_bounds__(WSmall<ODD, LM>::NT, WSmall<ODD, LM>::NT > 384
     const Tw *tf = (const Tw*)P.wtf + toff, *ti = (const Tw*)P.wti + toff;
     uint32_t* const sp = sm + pi * ODD * SM;  // this prime's blocks
     uint32_t* const s = sp + j * SM;
-    uint32_t a[16], b[16];
-    auto down = [&](uint32_t* x, const uint64_t* __restrict__ src, int n) {
+    uint32_t x[32];  // a's 16 values, then b's
+    uint32_t* const a = x;
+    auto load = [&](uint32_t* v, uint32_t* spv, const uint64_t* __restrict__ src, int n) {
+        if (!live) return;
         if (ODD == 1) {
-            if (live) {
 #pragma unroll
-                for (int k = 0; k < 16; k++) {
-                    const int i = wpos<LM, LM, J1>(t, k >> J1, k & ((1 << J1) - 1));
-                    x[k] = wpack<false>(i < n ? __ldg(src + i) : 0ull, pi, p);
-                }
+            for (int k = 0; k < 16; k++) {
+                const int i = wpos<LM, LM, J1>(t, k >> J1) + ((k & ((1 << J1) - 1)) << (LM - J1));
+                v[k] = wpack<false>(i < n ? __ldg(src + i) : 0ull, pi, p);
             }
         } else {
-            if (live) {
-                for (int c = u; c < M; c += TP) {
-                    uint32_t v[ODD];
+            for (int c = u; c < M; c += TP) {
+                uint32_t y[ODD];
 #pragma unroll
-                    for (int r = 0; r < ODD; r++) {
-                        const int i = c + (r << LM);
-                        v[r] = wpack<true>(i < n ? __ldg(src + i) : 0ull, pi, p);
-                    }
-                    dft_odd<ODD, 0>(v, pi, p);
-#pragma unroll
-                    for (int r = 0; r < ODD; r++) sp[r * SM + wpad(c)] = v[r];
+                for (int r = 0; r < ODD; r++) {
+                    const int i = c + (r << LM);
+                    y[r] = wpack<true>(i < n ? __ldg(src + i) : 0ull, pi, p);
                 }
+                dft_odd<ODD, 0>(y, pi, p);
+#pragma unroll
+                for (int r = 0; r < ODD; r++) spv[r * SM + wpad(c)] = y[r];
             }
-            __syncthreads();
-            if (live) wget<LM, LM, J1>(s, x, t);
         }
-        wblock_down<LM>(x, s, t, tf, 1u, p, live);
     };
-    down(a, P.a, (int)P.nca);
-    if (!P.sqr) {
-        __syncthreads();  // a's last reads of the shared blocks
-        down(b, P.b, (int)P.ncb);
+    // the constants of every later round, on their way while the limbs load: a
+    // round then waits for the L1 instead of the L2
+    constexpr int LINES = (1 << (LM - 2)) / 16;  // 128-byte lines per block and direction
+    for (int i = tid; i < 2 * WPR * ODD * LINES; i += W::NT) {
+        const int ln = i % LINES, blk = i / LINES % (WPR * ODD);
+        const Tw* tb = (const Tw*)(i / (LINES * WPR * ODD) ? P.wti : P.wtf) + ((size_t)blk << P.wL) + 16 * ln;
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(tb));
     }
-    if (live) wpoint<LM>(a, b, P.sqr, t, tf, 1u, p, pinv);
+    load(x, sp, P.a, (int)P.nca);
+    if (!P.sqr) load(x + 16, sp + W::OPW, P.b, (int)P.ncb);
+    if (ODD > 1) {
+        __syncthreads();
+        if (live) wget<LM, LM, J1>(s, x, t);
+        if (live && !P.sqr) wget<LM, LM, J1>(s + W::OPW, x + 16, t);
+    }
+    if (!P.sqr) wblock_down<LM, 2, W::OPW>(x, s, t, tf, 1u, p, live);
+    else wblock_down<LM, 1, W::OPW>(x, s, t, tf, 1u, p, live);
+    if (live) wpoint<LM>(x, x + 16, P.sqr, t, tf, 1u, p, pinv);
     wblock_up<LM>(a, s, t, ti, 1u, p, live);
     if (live) wput<LM, LM, J1>(s, a, t);
     __syncthreads();
@@ -983,14 +1060,8 @@ __global__ void __launch_bounds__(WSmall<ODD, LM>::NT, WSmall<ODD, LM>::NT > 384
         uint32_t sc[WPR];
 #pragma unroll
         for (int k = 0; k < WPR; k++) sc[k] = P.wsc[k];
-        const uint32_t* q0 = sm + ((4 * tid) >> LM) * SM + wpad((4 * tid) & (M - 1));  // four within one padded run
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            uint32_t r[WPR];
-#pragma unroll
-            for (int k = 0; k < WPR; k++) r[k] = q0[k * ODD * SM + q];
-            coef_words(r, sc, lo[q], mid[q], hi[q]);
-        }
+        const uint32_t* q0 = sm + ((4 * tid) >> LM) * SM + wpad((4 * tid) & (M - 1));  // four in one padded run
+        coef4(reinterpret_cast<const uint4*>(q0), ODD * SM / 4, sc, lo, mid, hi);
     }
     const int rn = (int)P.rn, top = min(rn, 4 * W::LT);
     limb_sums<W::LT>(S, tid, W::LT, lo, mid, hi, top, own);
@@ -1029,8 +1100,9 @@ static WLaunch small_kernel() {
     return WLaunch{k_wsmall<ODD, LM>, WSmall<ODD, LM>::NT, WSmall<ODD, LM>::bytes};
 }
 template <int ODD, int LJ>
-static WLaunch col_kernel(int kind) {
-    return WLaunch{kind == JK_WCOL_FWD ? k_wcol_fwd<ODD, LJ> : k_wcol_rev<ODD, LJ>, WT, 0};
+static WLaunch col_kernel(int kind, bool lm12) {
+    if (kind == JK_WCOL_FWD) return WLaunch{lm12 ? k_wcol_fwd<ODD, LJ, 12> : k_wcol_fwd<ODD, LJ, 0>, WT, 0};
+    return WLaunch{lm12 ? k_wcol_rev<ODD, LJ, 12> : k_wcol_rev<ODD, LJ, 0>, WT, 0};
 }
 template <int J>
 static WLaunch mid_kernel(int kind) {
@@ -1060,9 +1132,9 @@ static WLaunch word_kernel(int kind, int variant) {
             break;
         case JK_WCOL_FWD:
         case JK_WCOL_REV:
-            switch (variant) {
+            switch (variant & 0xffff) {
 #define NBG_COL(O, J) \
-    case (O << 8) | J: return col_kernel<O, J>(kind);
+    case (O << 8) | J: return col_kernel<O, J>(kind, variant >> 16);
                 NBG_COL(1, 1) NBG_COL(1, 2) NBG_COL(1, 3) NBG_COL(1, 4) NBG_COL(1, 5)
                 NBG_COL(3, 0) NBG_COL(3, 1) NBG_COL(3, 2) NBG_COL(3, 3)
                 NBG_COL(5, 0) NBG_COL(5, 1) NBG_COL(5, 2)
