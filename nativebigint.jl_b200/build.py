@@ -11,6 +11,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -25,7 +26,7 @@ NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-Xcompile
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-fno-fast-math", "-Wall", "-Wextra",
              "-Wno-unused-parameter", f"-I{CUDA}/include"]
 
-CU_SOURCES = ["kernels.cu", "word_kernels.cu", "noalloc.cu", "powmod_kernels.cu", "linalg.cu"]
+CU_SOURCES = ["kernels.cu", "word_kernels.cu", "powmod_chain.cu", "noalloc.cu", "powmod_kernels.cu", "linalg.cu"]
 CXX_SOURCES = ["engine.cpp", "api.cpp", "serve.cpp", "powmod.cpp"]
 
 
@@ -50,21 +51,23 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> str:
     os.makedirs(LIB, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     headers.append(os.path.join(HERE, "..", "include", "nbgpu.h"))
-    objs = []
+    objs, cmds = [], []
     for src in CU_SOURCES:
         s = os.path.join(CSRC, src)
         o = os.path.join(BUILD, src + ".o")
         if _stale(o, [s] + headers) or ptxas_info:
             extra = ["-Xptxas", "-v"] if ptxas_info else []
-            _run([NVCC] + NVCC_FLAGS + extra + ["-c", s, "-o", o])
+            cmds.append([NVCC] + NVCC_FLAGS + extra + ["-c", s, "-o", o])
         objs.append(o)
     cxx = shutil.which("g++") or "g++"
     for src in CXX_SOURCES:
         s = os.path.join(CSRC, src)
         o = os.path.join(BUILD, src + ".o")
         if _stale(o, [s] + headers):
-            _run([cxx] + CXX_FLAGS + ["-c", s, "-o", o])
+            cmds.append([cxx] + CXX_FLAGS + ["-c", s, "-o", o])
         objs.append(o)
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as ex:  # the compilers run in their own processes
+        list(ex.map(_run, cmds))
     out = os.path.join(LIB, "libnbgpu.so")
     if _stale(out, objs):
         _run([NVCC] + ARCH + ["-shared", "-o", out] + objs + ["-cudart", "static", "-lpthread", "-ldl", "-lrt"])

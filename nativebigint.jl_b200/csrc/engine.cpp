@@ -29,6 +29,7 @@
 #include "engine.h"
 #include "consts.h"
 #include "kernels.h"
+#include "powmod_kernels.h"
 
 namespace nbg {
 
@@ -348,6 +349,7 @@ int Engine::init(int device) {
         for (cudaEvent_t& e : row) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CUDA_TRY(kernels_init((double)PR[0], (double)PR[1]));
     CUDA_TRY(word_init());
+    CUDA_TRY(pm_chain_init());
     CUDA_TRY(cudaMalloc(&d_plans, sizeof(DPlan) * (size_t)plan_cap));
     CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device));
     smem_optin = kernels_smem_optin();

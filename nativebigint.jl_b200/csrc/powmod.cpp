@@ -16,7 +16,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
+#include <thread>
 #include <vector>
 
 #include "../../include/nbgpu.h"
@@ -199,6 +201,27 @@ static bool one_pass(Engine& E, int64_t bits_a, int64_t bits_b) {
 
 // Steps replayed per graph launch.
 constexpr int64_t PM_GRAPH_STEPS = 64;
+// Steps per launch of whole chains.
+constexpr int64_t PM_CHAIN_STEPS = 4096;
+
+// f(c) for every chain, on a few host threads when the k^2 work of each is
+// worth it (64 moduli of 256 limbs: 5.1 ms on one thread).
+template <class F>
+static void for_each_chain(int64_t count, int64_t k, F f) {
+    const unsigned hc = std::thread::hardware_concurrency();
+    const int64_t n = std::min<int64_t>({count, (int64_t)std::min(hc ? hc : 1u, 16u), count * k * k / 100000 + 1});
+    std::atomic<int64_t> next{0};
+    auto work = [&] {
+        for (int64_t c; (c = next++) < count;) f(c);
+    };
+    std::vector<std::thread> th;
+    try {
+        for (int64_t i = 1; i < n; i++) th.emplace_back(work);
+    } catch (...) {  // no more threads: the ones there are and this one do the rest
+    }
+    work();
+    for (std::thread& t : th) t.join();
+}
 
 // The chains of d[0..count) (device pointers), modulus size k; hm/he are host
 // copies of each chain's modulus and exponent.  Runs on the engine stream and
@@ -226,17 +249,26 @@ static int powmod_run(Engine& E, const nbg_powmod_desc* d, int64_t count, int64_
         for (size_t i = 0; i < o.size(); i++) hops[(size_t)(c * max_steps * 3) + i] = remap(o[i]);
         hn[(size_t)c] = (int64_t)(o.size() / 3);
     }
-    // μ per chain (host long division, once per modulus)
+    // μ per chain (host long division, once per modulus; the moduli are independent)
     const int64_t lmu_max = k + 2;
     std::vector<uint64_t> hmu((size_t)(count * lmu_max), 0);
     std::vector<int64_t> lmu((size_t)count), bits_mu((size_t)count), bits_m((size_t)count);
+    for_each_chain(count, k, [&](int64_t c) {
+        lmu[(size_t)c] = nbg_barrett_mu(hm[(size_t)c].data(), k, hmu.data() + c * lmu_max);
+    });
+    bool chainable = true;  // every μ has k + 1 limbs (k + 2 only for m = β^(k-1))
     for (int64_t c = 0; c < count; c++) {
-        const int64_t l = nbg_barrett_mu(hm[(size_t)c].data(), k, hmu.data() + c * lmu_max);
-        if (l < 0) return fail(NBG_EINVAL, "chain %lld: modulus top limb is zero", (long long)c);
-        lmu[(size_t)c] = l;
-        bits_mu[(size_t)c] = magnitude_bits(hmu.data() + c * lmu_max, l);
+        if (lmu[(size_t)c] < 0) return fail(NBG_EINVAL, "chain %lld: modulus top limb is zero", (long long)c);
+        bits_mu[(size_t)c] = magnitude_bits(hmu.data() + c * lmu_max, lmu[(size_t)c]);
         bits_m[(size_t)c] = magnitude_bits(hm[(size_t)c].data(), k);
+        chainable = chainable && lmu[(size_t)c] == k + 1;
     }
+    // whole chains in one CTA each where the products fit one (word engine)
+    WordShape cs;
+    const WordTab* ctab = nullptr;
+    chainable = chainable && E.word_ok && pm_chain_shape(k, cs);
+    int rc = 0;
+    if (chainable && (rc = E.word_table(cs.odd, cs.lm - 2, &ctab))) return rc;
     // device state
     PmMem mem;
     PmChains C{};
@@ -256,11 +288,11 @@ static int powmod_run(Engine& E, const nbg_powmod_desc* d, int64_t count, int64_
     int4* d_cur = nullptr;
     const uint64_t** d_bases = nullptr;
     uint64_t** d_outs = nullptr;
-    int rc = 0;
+    const size_t pc = chainable ? 0 : (size_t)count;  // chains run as product batches
     if ((rc = mem.get(&d_ops, hops.size())) || (rc = mem.get(&d_n, (size_t)count)) || (rc = mem.get(&d_ctr, 1)) ||
         (rc = mem.get(&d_lb, (size_t)count)) || (rc = mem.get(&d_slots, (size_t)(count * C.nslot * k))) ||
-        (rc = mem.get(&d_prod, (size_t)(count * C.prod_stride))) || (rc = mem.get(&d_q2, (size_t)(count * q2_stride))) ||
-        (rc = mem.get(&d_r2, (size_t)(count * C.r2_stride))) || (rc = mem.get(&d_mod, (size_t)(count * k))) ||
+        (rc = mem.get(&d_prod, (size_t)(count * C.prod_stride))) || (rc = mem.get(&d_q2, pc * (size_t)q2_stride)) ||
+        (rc = mem.get(&d_r2, pc * (size_t)C.r2_stride)) || (rc = mem.get(&d_mod, (size_t)(count * k))) ||
         (rc = mem.get(&d_mu, (size_t)(count * lmu_max))) || (rc = mem.get(&d_cur, (size_t)count)) ||
         (rc = mem.get(&d_bases, (size_t)count)) || (rc = mem.get(&d_outs, (size_t)count)))
         return rc;
@@ -290,6 +322,19 @@ static int powmod_run(Engine& E, const nbg_powmod_desc* d, int64_t count, int64_
     C.prod = d_prod;
     C.r2 = d_r2;
     C.mod = d_mod;
+    if (chainable) {
+        WScale sc;
+        word_scales(cs, sc.v);
+        PM_TRY(pm_launch_init(C, d_bases, d_lb, st));
+        // a few thousand steps per launch: no launch runs for seconds
+        int64_t nl = 0;
+        for (int64_t s = 0; s < max_steps; s += PM_CHAIN_STEPS, nl++)
+            PM_TRY(pm_launch_chain(C, d_mu, ctab->fwd, ctab->inv, ctab->L, sc, s, std::min(s + PM_CHAIN_STEPS, max_steps), st));
+        PM_TRY(pm_launch_output(C, d_outs, st));
+        PM_TRY(cudaStreamSynchronize(st));
+        g_launches += nl + 2;
+        return NBG_OK;
+    }
     // the three product batches: T = x*y, q2 = q1*mu, r2 = m*q3 (q1, q3 windows of T, q2)
     std::vector<ProdIn> in1((size_t)count), in2((size_t)count), in3((size_t)count);
     for (int64_t c = 0; c < count; c++) {

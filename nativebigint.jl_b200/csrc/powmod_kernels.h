@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "types.h"
+#include "word.h"
 
 namespace nbg {
 
@@ -35,5 +36,15 @@ cudaError_t pm_launch_finish(const PmChains& C, cudaStream_t st);
 cudaError_t pm_launch_advance(int64_t* ctr, cudaStream_t st);
 cudaError_t pm_launch_init(const PmChains& C, const uint64_t* const* bases, const int64_t* lbs, cudaStream_t st);
 cudaError_t pm_launch_output(const PmChains& C, uint64_t* const* outs, cudaStream_t st);
+
+// Whole chains, one CTA each (powmod_chain.cu): moduli of up to 768 limbs.
+struct WScale {
+    uint32_t v[WPR];  // word_scales of the chain's transform
+};
+bool pm_chain_shape(int64_t k, WordShape& s);  // the transform the chains of k-limb moduli use
+cudaError_t pm_chain_init();                   // constants and kernel settings of the current device
+// Steps [s0, s1) of every chain; mu: [count][k + 2], k + 1 limbs each.  C.prods, prod, r2, cur are not used.
+cudaError_t pm_launch_chain(const PmChains& C, const uint64_t* mu, const void* wtf, const void* wti, int wL,
+                            const WScale& sc, int64_t s0, int64_t s1, cudaStream_t st);
 
 }  // namespace nbg

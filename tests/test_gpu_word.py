@@ -88,3 +88,34 @@ def test_word_batch_equals_fp64_passes(gpu_lib):
     for (a, b), g, r in zip(pairs, got, ref):
         assert np.array_equal(g, r)
         assert np.array_equal(g, _want(a, b))
+
+
+@pytest.mark.parametrize("k", [1, 31, 32, 33, 64, 65, 96, 97, 128, 192, 256, 257, 384, 512, 513, 768, 769])
+def test_power_chains_at_transform_edges(gpu_lib, k):
+    # moduli at and around half of each one-CTA length (2k + 1 coefficients:
+    # the last one wraps when 2k is the length), extreme limbs, the largest
+    # base; 769 limbs: the product batches
+    rng = np.random.default_rng(4000 + k)
+
+    def num(x):
+        return int.from_bytes(np.ascontiguousarray(x).tobytes(), "little")
+
+    mods, bases, exps = [], [], []
+    for style in range(4):
+        m = rand_limbs(rng, k)
+        if style == 1:
+            m[:] = 2**64 - 1
+        if style == 2:
+            m[:] = 0
+            m[-1] = 1 << 13
+            m[0] |= np.uint64(3)
+        m[0] |= np.uint64(2)
+        b = rand_limbs(rng, k) if style != 3 else np.full(k, 2**64 - 1, dtype=np.uint64)
+        if style == 1:
+            b = m.copy()
+            b[0] -= np.uint64(1)
+        mods.append(m)
+        bases.append(b)
+        exps.append(rand_limbs(rng, 1))
+    for r, b, e, m in zip(gpu_lib.powermod_batch(bases, exps, mods), bases, exps, mods):
+        assert num(r) == pow(num(b), num(e), num(m))
