@@ -659,11 +659,12 @@ void Engine::trim_plans() {
     for (auto& kv : plans) cudaFree(kv.second.dtab);
     plans.clear();
     plan_used = 0;
-    for (WordTab& w : wtab) {
-        cudaFree(w.fwd);
-        cudaFree(w.inv);
-        w = WordTab();
-    }
+    for (auto& set : wtab)
+        for (WordTab& w : set) {
+            cudaFree(w.fwd);
+            cudaFree(w.inv);
+            w = WordTab();
+        }
 }
 
 void Engine::tuning_changed(bool loaded) {
@@ -673,13 +674,14 @@ void Engine::tuning_changed(bool loaded) {
     word_ok = tun.queue == 0 && js == base_tuning;
 }
 
-// Tables for heap sizes up to 2^L.  One size serves every length up to
-// odd * 2^17 points; longer ones get the largest (old tables stay for live graphs).
-int Engine::word_table(int odd, int L, const WordTab** out) {
-    WordTab& w = wtab[odd];
+// Tables for heap sizes up to 2^L.  In set 0 one size serves every length up to
+// odd * 2^17 points and longer ones get the largest; the six-prime sets, whose
+// tables reach hundreds of MB, get what they need (old tables stay for live graphs).
+int Engine::word_table(int set, int odd, int L, const WordTab** out) {
+    WordTab& w = wtab[set][odd];
     if (w.L < L) {
-        const int want = L <= 15 ? 15 : WORD_MAX_LOG2 - 2;
-        const size_t bytes = word_table_bytes(odd, want);
+        const int want = set ? L : L <= 15 ? 15 : WORD_MAX_LOG2 - 2;
+        const size_t bytes = word_table_bytes(set, odd, want);
         WordTab n;
         n.L = want;
         if (cudaMalloc(&n.fwd, bytes) != cudaSuccess || cudaMalloc(&n.inv, bytes) != cudaSuccess) {
@@ -687,7 +689,7 @@ int Engine::word_table(int odd, int L, const WordTab** out) {
             cudaFree(n.fwd);
             return fail(NBG_ENOMEM, "constant tables of %zu bytes unavailable", 2 * bytes);
         }
-        cudaError_t e = word_build_tables(odd, want, n.fwd, n.inv, stream);
+        cudaError_t e = word_build_tables(set, odd, want, n.fwd, n.inv, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) {
             cudaFree(n.fwd);
@@ -804,13 +806,12 @@ size_t fp64_work_bytes(const ProdIn& q) {
 bool word_product(const Engine& E, const ProdIn& q, WordShape* s) {
     if (!E.word_ok || q.fp64 || q.keep_b) return false;
     const int64_t la = eff_limbs(q.m, q.bits_a), lb = q.sqr ? la : eff_limbs(q.n, q.bits_b);
-    if (std::min(la, lb) > WORD_MIN_OPERAND_MAX) return false;
-    return word_shape(la + lb - 1, *s);
+    return word_shape(la + lb - 1, *s) && (s->set || std::min(la, lb) <= WORD_MIN_OPERAND_MAX);
 }
 
 int word_setup(Engine& E, const ProdIn& q, const WordShape& s, DProd& P) {
     const WordTab* wt = nullptr;
-    int rc = E.word_table(s.odd, s.lj + s.lm - 2, &wt);
+    int rc = E.word_table(s.set, s.odd, s.lj + s.lm - 2, &wt);
     if (rc) return rc;
     memset(&P, 0, sizeof P);
     P.a = q.a;
@@ -839,13 +840,14 @@ int word_setup(Engine& E, const ProdIn& q, const WordShape& s, DProd& P) {
 // Launches of one word product in order: kind and variant.
 static std::vector<std::pair<int, int>> word_steps(const WordShape& s) {
     if (s.small) return {{JK_WSMALL, (s.odd << 8) | s.lm}};
-    const int col = (s.lm + s.j2 == 12 ? 1 << 16 : 0) | (s.odd << 8) | (s.lj - s.j2);
+    const int set = s.set << 20;
+    const int col = set | (s.lm + s.j2 == 12 ? 1 << 16 : 0) | (s.odd << 8) | (s.lj - s.j2);
     std::vector<std::pair<int, int>> v{{JK_WCOL_FWD, col}};
-    if (s.j2) v.push_back({JK_WMID_FWD, s.j2});
-    v.push_back({JK_WBLOCK, s.lm});
-    if (s.j2) v.push_back({JK_WMID_REV, s.j2});
+    if (s.j2) v.push_back({JK_WMID_FWD, set | s.j2});
+    v.push_back({JK_WBLOCK, set | s.lm});
+    if (s.j2) v.push_back({JK_WMID_REV, set | s.j2});
     v.push_back({JK_WCOL_REV, col});
-    v.push_back({JK_WUNPACK, 0});
+    v.push_back({JK_WUNPACK, set});
     return v;
 }
 
@@ -854,7 +856,7 @@ int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, cudaStream_t st
     int rc = word_setup(E, q, s, P);
     if (rc) return rc;
     if (!s.small) {
-        const size_t op = align_up(sizeof(uint32_t) * (size_t)WPR * (size_t)s.N, 256);
+        const size_t op = align_up(sizeof(uint32_t) * (size_t)word_np(s.set) * (size_t)s.N, 256);
         const size_t res = op * (q.sqr ? 1 : 2);
         if ((rc = E.ensure_pool(res + sizeof(uint32_t) * (size_t)P.ntl, st))) return rc;
         char* d = (char*)E.pool;
@@ -900,7 +902,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
             if (rc) return rc;
             agg_off[(size_t)k] = aggw;
             aggw += (size_t)P.ntl;
-            const size_t op = ws.small ? 0 : align_up((size_t)WPR * (size_t)ws.N, 64);
+            const size_t op = ws.small ? 0 : align_up((size_t)word_np(ws.set) * (size_t)ws.N, 64);
             xa_off[(size_t)k] = bb.word_words;
             xb_off[(size_t)k] = q.sqr ? SIZE_MAX : bb.word_words + op;
             bb.word_words += op * (q.sqr ? 1 : 2);
@@ -1173,7 +1175,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     });
     for (const WordProd& w : words) {
         const DProd& P = bb.prods[(size_t)w.k];
-        const double res = 4.0 * WPR * P.wN, nop = P.sqr ? 1 : 2;
+        const double res = 4.0 * word_np(w.s.set) * P.wN, nop = P.sqr ? 1 : 2;
         const double in_b = 8.0 * (double)(P.nca + (P.sqr ? 0 : P.ncb)), out_b = 8.0 * (double)P.rn;
         for (const auto& kv : word_steps(w.s)) {
             // the block step is pmax - 1, a middle column pass takes the steps next to it

@@ -84,7 +84,7 @@ struct Engine {
     // that sets other pass knobs gets the FP64 passes they describe
     std::string base_tuning = Tuning().to_json();
     bool word_ok = true;
-    WordTab wtab[8];  // by odd
+    WordTab wtab[WSETS][8];  // by prime set and odd
     std::map<int64_t, PlanRec> plans;
     std::vector<double*> graveyard;
     DPlan* d_plans = nullptr;
@@ -108,7 +108,7 @@ struct Engine {
     int get_plan(int64_t N, int for_sqr, PlanRec** out);
     void drop_plans();
     void tuning_changed(bool loaded);  // after `tun` was set (loaded: it is the new base)
-    int word_table(int odd, int L, const WordTab** out);
+    int word_table(int set, int odd, int L, const WordTab** out);
     void trim_plans();  // frees every plan's tables: no batch may exist or be running
     // The shared workspace, at least `bytes`, for work on `st`: ordered after the
     // last call that left work using it in flight (pool_release).

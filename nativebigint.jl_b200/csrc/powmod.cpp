@@ -268,7 +268,7 @@ static int powmod_run(Engine& E, const nbg_powmod_desc* d, int64_t count, int64_
     const WordTab* ctab = nullptr;
     chainable = chainable && E.word_ok && pm_chain_shape(k, cs);
     int rc = 0;
-    if (chainable && (rc = E.word_table(cs.odd, cs.lm - 2, &ctab))) return rc;
+    if (chainable && (rc = E.word_table(0, cs.odd, cs.lm - 2, &ctab))) return rc;
     // device state
     PmMem mem;
     PmChains C{};

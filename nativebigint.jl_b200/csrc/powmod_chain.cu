@@ -218,14 +218,14 @@ static const ChainKernel* chain_for(int64_t k) {
 bool pm_chain_shape(int64_t k, WordShape& s) {
     const ChainKernel* c = chain_for(k);
     if (!c) return false;
-    s = WordShape{c->odd << c->lm, c->odd, 0, 0, c->lm, true};
+    s = WordShape{c->odd << c->lm, c->odd, 0, 0, c->lm, true, 0};
     return true;
 }
 
 cudaError_t pm_chain_init() {
-    WConst h;
+    WConst h[WSETS];
     word_fill_const(h);
-    cudaError_t e = cudaMemcpyToSymbol(c_w, &h, sizeof h);
+    cudaError_t e = cudaMemcpyToSymbol(c_w, h, sizeof h);
     for (const ChainKernel& c : CHAINS)
         if (e == cudaSuccess) e = cudaFuncSetAttribute(c.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
     return e;

@@ -82,13 +82,13 @@ struct DProd {
     uint32_t* agg;       // per limb-tile carry aggregates (bit0 generate, bit1 propagate)
     int64_t ntl;         // number of limb tiles
     // word products (word.h; `wN` nonzero): residues of operand a (and the
-    // result) and b as five arrays of wN words, constant tables, shape
+    // result) and b as one array of wN words per prime, constant tables, shape
     uint32_t* wa;
     uint32_t* wb;
     const void* wtf;     // forward and inverse constants, [prime][block][2^wL]
     const void* wti;
     int32_t wN, wodd, wlj, wj2, wlm, wL;
-    uint32_t wsc[5];     // unpack scale per prime
+    uint32_t wsc[6];     // unpack scale per prime
 };
 
 // Work item of one launch.  kind-specific meaning of `sub`:

@@ -1,4 +1,4 @@
-// word.h — products through transforms over five 30-bit primes ("word"
+// word.h — products through transforms over five (or six) 30-bit primes ("word"
 // products): every 64-bit limb is one coefficient, so packing is a reduction
 // and the results are the carried sums of the convolution's coefficients.
 //
@@ -20,21 +20,31 @@
 
 namespace nbg {
 
-constexpr int WPR = 5;  // primes
-// p = 1 mod 105 * 2^18, so e(t) exists for t = i / (odd * 2^18); their product
-// exceeds 2^149: any min(m, n) <= 2^21 limbs convolve without wrapping.
-constexpr uint32_t WPRIMES[WPR] = {1073479681u, 1018429441u, 908328961u, 880803841u, 825753601u};
-constexpr int WORD_MAX_LOG2 = 20;               // k <= 20 (leaves at level k - 2 <= 18)
-constexpr int64_t WORD_MIN_OPERAND_MAX = int64_t(1) << 21;
+// Prime sets.  Set 0 (p = 1 mod 105 * 2^18, product above 2^149) serves
+// lengths odd * 2^k with k <= 20 and any min(m, n) <= 2^21 limbs.  Above 3.6M
+// points the coefficients need a sixth prime and the roots more twos: set 1
+// (p = 1 mod 3 * 2^22) for 3 * 2^k, set 2 (p = 1 mod 2^23) for 2^k, k <= 25;
+// their products exceed 2^176.
+constexpr int WPR = 5;      // primes of set 0
+constexpr int WPR_MAX = 6;
+constexpr int WSETS = 3;
+constexpr int word_np(int set) { return set ? 6 : WPR; }
+constexpr uint32_t WPRIMES[WSETS][WPR_MAX] = {
+    {1073479681u, 1018429441u, 908328961u, 880803841u, 825753601u, 0},
+    {943718401u, 918552577u, 880803841u, 754974721u, 666894337u, 415236097u},
+    {998244353u, 897581057u, 880803841u, 754974721u, 645922817u, 595591169u}};
+constexpr int WORD_MAX_LOG2 = 20;               // set 0: k <= 20 (leaves at level k - 2 <= 18)
+constexpr int64_t WORD_MIN_OPERAND_MAX = int64_t(1) << 21;  // set 0
 
 // Shape of a word product's transform: N = odd * 2^lj * M.  Blocks of M = 2^lm
 // consecutive values (each one subtree) are transformed in shared memory;
 // column passes above them work on the rows of one column in registers: one
 // pass of odd * 2^lj rows, or, past 32 rows, a first one of odd * 2^(lj - j2)
-// and a middle one of 2^j2.
+// and a middle one of 2^j2 (from 64 rows on with a turn through shared memory).
 struct WordShape {
     int32_t N = 0, odd = 0, lj = 0, j2 = 0, lm = 0;
     bool small = false;  // one CTA per product (at most 3072 values; lj = 0, no column pass)
+    int32_t set = 0;     // prime set
 };
 // The smallest supported length >= nconv; false when there is none.
 bool word_shape(int64_t nconv, WordShape& s);
@@ -47,7 +57,7 @@ struct WSeg {
     int32_t pad_;
 };
 
-// variant of a word launch: (odd << 8) | (lj - j2) for column passes (bit 16: of 4096 columns), j2 for middle ones, lm for
+// variant of a word launch: bits 20 on the prime set, then (odd << 8) | (lj - j2) for column passes (bit 16: of 4096 columns), j2 for middle ones, lm for
 // blocks, (odd << 8) | lm for one-CTA products
 cudaError_t word_init();  // constant memory of the current device
 cudaError_t launch_word(int kind, int variant, const DProd* prods, const WSeg* segs, int nseg, const int32_t* plist,
@@ -58,9 +68,9 @@ cudaError_t launch_word_one(int kind, int variant, const DProd& P, int64_t nctas
 int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t rn);
 
 // Tables of one `odd` for heap sizes up to 2^L: per prime and block, fwd then inverse.
-size_t word_table_bytes(int odd, int L);
-cudaError_t word_build_tables(int odd, int L, void* fwd, void* inv, cudaStream_t st);
+size_t word_table_bytes(int set, int odd, int L);
+cudaError_t word_build_tables(int set, int odd, int L, void* fwd, void* inv, cudaStream_t st);
 // Per-product scale constants of the unpack (the inverse transform's 1/(odd * 2^(k-2)) and the pointwise 2^-32).
-void word_scales(const WordShape& s, uint32_t out[WPR]);
+void word_scales(const WordShape& s, uint32_t* out);
 
 }  // namespace nbg

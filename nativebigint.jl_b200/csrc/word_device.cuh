@@ -14,26 +14,27 @@ namespace nbg {
 using wd::Tw;
 
 struct WConst {
-    uint32_t p[WPR], pinv[WPR];
-    Tw c32[WPR], one[WPR];       // 2^32 mod p, 1
-    Tw r3[WPR];                  // e(1/3)
-    Tw r5[WPR][5];               // -1/4, (c1-c2)/2, f1, f2 of e(1/5) (see dft5); [4] unused
-    uint32_t c7[WPR][3], f7[WPR][3];  // cosine and sine halves of e(j/7) in 2^32 form
-    uint32_t wt[WPR][WPR];       // words of W_i = p_0 ... p_(i-1) (i words)
-    uint32_t gar[WPR][WPR];      // mixed radix: gar[i][j] = -W_j / W_i mod p_i in 2^32 form (j < i)
+    uint32_t p[WPR_MAX], pinv[WPR_MAX];
+    Tw c32[WPR_MAX], one[WPR_MAX];       // 2^32 mod p, 1
+    Tw r3[WPR_MAX];                  // e(1/3)
+    Tw r5[WPR_MAX][5];               // -1/4, (c1-c2)/2, f1, f2 of e(1/5) (see dft5); [4] unused
+    uint32_t c7[WPR_MAX][3], f7[WPR_MAX][3];  // cosine and sine halves of e(j/7) in 2^32 form
+    uint32_t wt[WPR_MAX][WPR_MAX];       // words of W_i = p_0 ... p_(i-1) (i words)
+    uint32_t gar[WPR_MAX][WPR_MAX];      // mixed radix: gar[i][j] = -W_j / W_i mod p_i in 2^32 form (j < i)
 };
-static __constant__ WConst c_w;
+static __constant__ WConst c_w[WSETS];
 // Fills the constants (host); every file that includes this copies them to its c_w.
-void word_fill_const(WConst& h);
+void word_fill_const(WConst h[WSETS]);
 
 // ---------------------------------------------------------------------------
 // radix-odd steps: in and out in [0, 2p) unless said otherwise
 
 // y_j = sum x_i e(ij/3): with w + w^2 = -1 one product suffices
+template <int SET>
 __device__ __forceinline__ void dft3(uint32_t* x, int st, int i, uint32_t p) {
     const uint32_t p2 = 2 * p;
     uint32_t &a = x[0], &b = x[st], &c = x[2 * st];
-    const uint32_t t = wd::mulw(b - c + p2, c_w.r3[i], p);
+    const uint32_t t = wd::mulw(b - c + p2, c_w[SET].r3[i], p);
     const uint32_t y0 = wd::sub_if(wd::sub_if(a + b, p2) + c, p2);
     const uint32_t y1 = wd::sub_if(wd::sub_if(a - c + p2, p2) + t, p2);
     const uint32_t u = wd::sub_if(a - b + p2, p2);
@@ -43,9 +44,10 @@ __device__ __forceinline__ void dft3(uint32_t* x, int st, int i, uint32_t p) {
     c = y2;
 }
 // cosine halves c1, c2 = -1/4 +- d: two products for the even part, four for the odd
+template <int SET>
 __device__ __forceinline__ void dft5(uint32_t* x, int st, int i, uint32_t p) {
     const uint32_t p2 = 2 * p;
-    const Tw q = c_w.r5[i][0], d = c_w.r5[i][1], f1 = c_w.r5[i][2], f2 = c_w.r5[i][3];
+    const Tw q = c_w[SET].r5[i][0], d = c_w[SET].r5[i][1], f1 = c_w[SET].r5[i][2], f2 = c_w[SET].r5[i][3];
     const uint32_t x0 = x[0], x1 = x[st], x2 = x[2 * st], x3 = x[3 * st], x4 = x[4 * st];
     const uint32_t s1 = wd::sub_if(x1 + x4, p2), s2 = wd::sub_if(x2 + x3, p2);
     const uint32_t d1 = x1 - x4 + p2, d2 = x2 - x3 + p2;
@@ -62,8 +64,9 @@ __device__ __forceinline__ void dft5(uint32_t* x, int st, int i, uint32_t p) {
     x[3 * st] = wd::sub_if(C2 - S2 + p2, p2);
 }
 // even and odd parts as sums of three wide products and one reduction each
+template <int SET>
 __device__ __forceinline__ void dft7(uint32_t* x, int st, int i, uint32_t p) {
-    const uint32_t p2 = 2 * p, pinv = c_w.pinv[i];
+    const uint32_t p2 = 2 * p, pinv = c_w[SET].pinv[i];
     const uint32_t x0 = x[0];
     uint32_t s[3], d[3];
 #pragma unroll
@@ -78,8 +81,8 @@ __device__ __forceinline__ void dft7(uint32_t* x, int st, int i, uint32_t p) {
 #pragma unroll
         for (int k = 1; k <= 3; k++) {
             const int t = j * k % 7, a = t <= 3 ? t : 7 - t;  // cos(t) = cos(7 - t), sin(t) = -sin(7 - t)
-            ce += wd::mulx(s[k - 1], c_w.c7[i][a - 1]);
-            so += wd::mulx(t <= 3 ? d[k - 1] : p2 - d[k - 1], c_w.f7[i][a - 1]);
+            ce += wd::mulx(s[k - 1], c_w[SET].c7[i][a - 1]);
+            so += wd::mulx(t <= 3 ? d[k - 1] : p2 - d[k - 1], c_w[SET].f7[i][a - 1]);
         }
         // each sum < 3 * 2p * p, reduced below 1.5p + p
         const uint32_t C = wd::sub_if(x0 + wd::sub_if(wd::redc(ce, p, pinv), p2), p2);
@@ -89,13 +92,13 @@ __device__ __forceinline__ void dft7(uint32_t* x, int st, int i, uint32_t p) {
     }
 }
 
-template <int ODD, int LJ>
+template <int ODD, int LJ, int SET = 0>
 __device__ __forceinline__ void dft_odd(uint32_t* x, int i, uint32_t p) {
 #pragma unroll
     for (int r = 0; r < (1 << LJ); r++) {
-        if (ODD == 3) dft3(x + r, 1 << LJ, i, p);
-        if (ODD == 5) dft5(x + r, 1 << LJ, i, p);
-        if (ODD == 7) dft7(x + r, 1 << LJ, i, p);
+        if (ODD == 3) dft3<SET>(x + r, 1 << LJ, i, p);
+        if (ODD == 5) dft5<SET>(x + r, 1 << LJ, i, p);
+        if (ODD == 7) dft7<SET>(x + r, 1 << LJ, i, p);
     }
 }
 
@@ -103,9 +106,9 @@ __device__ __forceinline__ void dft_odd(uint32_t* x, int i, uint32_t p) {
 // packing
 
 // A limb modulo p, in [0, 4p) (RED: [0, 2p)).
-template <bool RED>
+template <bool RED, int SET = 0>
 __device__ __forceinline__ uint32_t wpack(uint64_t v, int pi, uint32_t p) {
-    const uint32_t y = wd::mulw((uint32_t)(v >> 32), c_w.c32[pi], p) + wd::mulw((uint32_t)v, c_w.one[pi], p);
+    const uint32_t y = wd::mulw((uint32_t)(v >> 32), c_w[SET].c32[pi], p) + wd::mulw((uint32_t)v, c_w[SET].one[pi], p);
     return RED ? wd::sub_if(y, 2 * p) : y;
 }
 
@@ -315,33 +318,36 @@ __device__ __forceinline__ void wpoint(uint32_t* a, uint32_t* b, bool sqr, int t
 // ---------------------------------------------------------------------------
 // unpack: coefficients and carried limbs, tiles of UNPACK_TL limbs
 
-// The coefficient whose residues (representatives below 2p, scaled) are r:
-// mixed-radix digits y_i, each one sum of wide products and one reduction, then
-// sum y_i W_i by columns of 32 bits (at most four products below 2^62 each).
+// The coefficient (below 2^160) whose residues (representatives below 2p,
+// scaled) are r: mixed-radix digits y_i, each one sum of wide products and one
+// reduction, then sum y_i W_i by columns of 32 bits.
+constexpr int WCOEF = 5;  // 32-bit words of a coefficient
+template <int SET>
 __device__ __forceinline__ void wcoef(const uint32_t* r, const uint32_t* sc, uint32_t* v) {
-    uint32_t y[WPR];
+    constexpr int NP = word_np(SET);
+    uint32_t y[NP];
 #pragma unroll
-    for (int i = 0; i < WPR; i++) {
-        const uint32_t p = c_w.p[i];
-        uint64_t s = wd::mulx(r[i], sc[i]);  // < 2p^2; the others < 1.3p^2 each
+    for (int i = 0; i < NP; i++) {
+        const uint32_t p = c_w[SET].p[i];
+        uint64_t s = wd::mulx(r[i], sc[i]);  // < 2p^2; the others < p_j p, p_j < 2.3p
 #pragma unroll
-        for (int j = 0; j < i; j++) s += wd::mulx(y[j], c_w.gar[i][j]);
-        // below 1.5p, 1.85p, 2.2p, 2.5p, 2.8p: one or two subtractions
-        y[i] = wd::sub_if(wd::redc(s, p, c_w.pinv[i]), p);
+        for (int j = 0; j < i; j++) s += wd::mulx(y[j], c_w[SET].gar[i][j]);
+        // below 1.5p, 1.9p, then 3p: one or two subtractions
+        y[i] = wd::sub_if(wd::redc(s, p, c_w[SET].pinv[i]), p);
         if (i > 1) y[i] = wd::sub_if(y[i], p);
     }
     uint64_t s = y[0];
 #pragma unroll
-    for (int k = 0; k < WPR - 1; k++) {
-        uint64_t col = wd::mulx(y[k + 1], c_w.wt[k + 1][k]);
+    for (int k = 0; k < WCOEF; k++) {
+        // at most four full products (below 2^62 each) per column: the sixth
+        // digit is below 2^8, as the coefficient is below 2^153
+        uint64_t col = k + 1 < NP ? wd::mulx(y[k + 1], c_w[SET].wt[k + 1][k]) : 0;
 #pragma unroll
-        for (int i = k + 2; i < WPR; i++) col += wd::mulx(y[i], c_w.wt[i][k]);
-        // col < (4 - k) * 2^62 and s < 2^33: no overflow
-        s += col;
+        for (int i = k + 2; i < NP; i++) col += wd::mulx(y[i], c_w[SET].wt[i][k]);
+        s += col;  // s < 2^33 before
         v[k] = (uint32_t)s;
         s >>= 32;
     }
-    v[WPR - 1] = (uint32_t)s;
 }
 
 __device__ __forceinline__ uint32_t gp_join(uint32_t lower, uint32_t upper) {
@@ -451,21 +457,24 @@ __device__ __forceinline__ void store_limbs(uint64_t* __restrict__ r, int64_t wt
         if (wt + q < w1) r[wt + q] = own[q];
 }
 
+template <int SET>
 __device__ __forceinline__ void coef_words(const uint32_t* r, const uint32_t* sc, uint64_t& lo, uint64_t& mid,
                                            uint32_t& hi) {
-    uint32_t v[WPR];
-    wcoef(r, sc, v);
+    uint32_t v[WCOEF];
+    wcoef<SET>(r, sc, v);
     lo = v[0] | (uint64_t)v[1] << 32;
     mid = v[2] | (uint64_t)v[3] << 32;
     hi = v[4];
 }
 
 // Four consecutive coefficients; prime k's residues are x[k * stride].
+template <int SET>
 __device__ __forceinline__ void coef4(const uint4* __restrict__ x, int stride, const uint32_t* sc, uint64_t* lo,
                                       uint64_t* mid, uint32_t* hi) {
-    uint32_t r[4][WPR];
+    constexpr int NP = word_np(SET);
+    uint32_t r[4][NP];
 #pragma unroll
-    for (int k = 0; k < WPR; k++) {
+    for (int k = 0; k < NP; k++) {
         const uint4 q = x[(size_t)k * stride];
         r[0][k] = q.x;
         r[1][k] = q.y;
@@ -473,7 +482,7 @@ __device__ __forceinline__ void coef4(const uint4* __restrict__ x, int stride, c
         r[3][k] = q.w;
     }
 #pragma unroll
-    for (int q = 0; q < 4; q++) coef_words(r[q], sc, lo[q], mid[q], hi[q]);
+    for (int q = 0; q < 4; q++) coef_words<SET>(r[q], sc, lo[q], mid[q], hi[q]);
 }
 
 // ---------------------------------------------------------------------------
@@ -506,8 +515,8 @@ struct SmallThread {
         u = live ? tid - pi * W::TP : 0;
         j = u / W::T;
         t = u & (W::T - 1);
-        p = c_w.p[pi];
-        pinv = c_w.pinv[pi];
+        p = c_w[0].p[pi];
+        pinv = c_w[0].pinv[pi];
         const size_t toff = ((size_t)pi * ODD + j) << wL;
         tf = (const Tw*)wtf + toff;
         ti = (const Tw*)wti + toff;
@@ -588,7 +597,7 @@ struct SmallThread {
 #pragma unroll
         for (int k = 0; k < WPR; k++) sc[k] = wsc[k];
         const uint32_t* q0 = sm + ((4 * tid) >> LM) * W::SM + wpad((4 * tid) & (W::M - 1));  // four in one padded run
-        coef4(reinterpret_cast<const uint4*>(q0), ODD * W::SM / 4, sc, lo, mid, hi);
+        coef4<0>(reinterpret_cast<const uint4*>(q0), ODD * W::SM / 4, sc, lo, mid, hi);
     }
 };
 

@@ -31,7 +31,7 @@ static uint64_t pw(uint64_t a, uint64_t e, uint64_t p) {
     return r;
 }
 static uint64_t inv(uint64_t a, uint64_t p) { return pw(a, p - 2, p); }
-// a primitive root: p - 1 = 105 * 2^18 * c, its prime factors are 2, 3, 5, 7 and c's
+// the least primitive root of p (trial division of p - 1)
 static uint64_t prim_root(uint64_t p) {
     for (uint64_t g = 2;; g++) {
         bool ok = true;
@@ -45,27 +45,34 @@ static uint64_t prim_root(uint64_t p) {
         if (ok) return g;
     }
 }
-static uint64_t root_of(int i) {
-    static const uint64_t g[WPR] = {prim_root(WPRIMES[0]), prim_root(WPRIMES[1]), prim_root(WPRIMES[2]),
-                                    prim_root(WPRIMES[3]), prim_root(WPRIMES[4])};
-    return g[i];
+static uint64_t root_of(int set, int i) {
+    static const struct Table {
+        uint64_t g[WSETS][WPR_MAX];
+        Table() {
+            for (int t = 0; t < WSETS; t++)
+                for (int k = 0; k < word_np(t); k++) g[t][k] = prim_root(WPRIMES[t][k]);
+        }
+    } t;
+    return t.g[set][i];
 }
 static Tw mk(uint64_t w, uint64_t p) { return Tw{(uint32_t)w, (uint32_t)((w << 32) / p)}; }
 static uint32_t mont(uint64_t w, uint64_t p) { return (uint32_t)(((w % p) << 32) % p); }
 
 static cudaError_t small_attributes();
 
-void word_fill_const(WConst& h) {
+static void fill_set(int set, WConst& h) {
     h = WConst{};
-    for (int i = 0; i < WPR; i++) {
-        const uint64_t p = WPRIMES[i], g = root_of(i);
+    const uint32_t* P = WPRIMES[set];
+    for (int i = 0; i < word_np(set); i++) {
+        const uint64_t p = P[i], g = root_of(set, i);
         h.p[i] = (uint32_t)p;
         uint32_t x = 1;
         for (int k = 0; k < 5; k++) x *= 2 - (uint32_t)p * x;  // Newton: p^-1 mod 2^32
         h.pinv[i] = x;
         h.c32[i] = mk((uint64_t(1) << 32) % p, p);
         h.one[i] = mk(1, p);
-        h.r3[i] = mk(pw(g, (p - 1) / 3, p), p);
+        if ((p - 1) % 3 == 0) h.r3[i] = mk(pw(g, (p - 1) / 3, p), p);
+        if (set == 0) {
         const uint64_t h2 = inv(2, p), w5 = pw(g, (p - 1) / 5, p), w7 = pw(g, (p - 1) / 7, p);
         auto half = [&](uint64_t w, int a, int b, bool minus) {  // (w^a +- w^b) / 2
             const uint64_t x1 = pw(w, a, p), x2 = pw(w, b, p);
@@ -80,53 +87,57 @@ void word_fill_const(WConst& h) {
             h.c7[i][k] = mont(half(w7, k + 1, 6 - k, false), p);
             h.f7[i][k] = mont(half(w7, k + 1, 6 - k, true), p);
         }
+        }
         uint64_t Wi = 1;
-        for (int t = 0; t < i; t++) Wi = Wi * (WPRIMES[t] % p) % p;
+        for (int t = 0; t < i; t++) Wi = Wi * (P[t] % p) % p;
         const uint64_t iw = inv(Wi, p);
         uint64_t Wj = 1;
         for (int j = 0; j < i; j++) {
             h.gar[i][j] = mont((p - Wj * iw % p) % p, p);
-            Wj = Wj * (WPRIMES[j] % p) % p;
+            Wj = Wj * (P[j] % p) % p;
         }
-        uint32_t w[WPR] = {1};
+        uint32_t w[WPR_MAX] = {1};
         for (int t = 0; t < i; t++) {
             uint64_t cy = 0;
-            for (int k = 0; k < WPR; k++) {
-                cy += (uint64_t)w[k] * WPRIMES[t];
+            for (int k = 0; k < WPR_MAX; k++) {
+                cy += (uint64_t)w[k] * P[t];
                 w[k] = (uint32_t)cy;
                 cy >>= 32;
             }
         }
-        for (int k = 0; k < WPR; k++) h.wt[i][k] = w[k];
+        for (int k = 0; k < WPR_MAX; k++) h.wt[i][k] = w[k];
     }
 }
 
-cudaError_t word_init() {
-    WConst h;
-    word_fill_const(h);
-    cudaError_t e = small_attributes();
-    return e == cudaSuccess ? cudaMemcpyToSymbol(c_w, &h, sizeof h) : e;
+void word_fill_const(WConst h[WSETS]) {
+    for (int t = 0; t < WSETS; t++) fill_set(t, h[t]);
 }
 
-void word_scales(const WordShape& s, uint32_t out[WPR]) {
+cudaError_t word_init() {
+    WConst h[WSETS];
+    word_fill_const(h);
+    cudaError_t e = small_attributes();
+    return e == cudaSuccess ? cudaMemcpyToSymbol(c_w, h, sizeof h) : e;
+}
+
+void word_scales(const WordShape& s, uint32_t* out) {
     // 2^32 (pointwise) * 2^32 (unpack's reduction) / (odd * 2^levels * W_i)
+    constexpr int LEV = 26;
     static const struct Table {
-        uint32_t v[8][WORD_MAX_LOG2][WPR];
+        uint32_t v[WSETS][8][LEV][WPR_MAX];
         Table() {
-            uint64_t W[WPR];
-            for (int i = 0; i < WPR; i++) {
-                W[i] = 1;
-                for (int j = 0; j < i; j++) W[i] = W[i] * (WPRIMES[j] % WPRIMES[i]) % WPRIMES[i];
-            }
-            for (int odd = 1; odd < 8; odd += 2)
-                for (int lev = 0; lev < WORD_MAX_LOG2; lev++)
-                    for (int i = 0; i < WPR; i++) {
-                        const uint64_t p = WPRIMES[i], r = (uint64_t(1) << 32) % p;
-                        v[odd][lev][i] = (uint32_t)(r * r % p * inv(odd * pw(2, (uint64_t)lev, p) % p * W[i] % p, p) % p);
-                    }
+            for (int set = 0; set < WSETS; set++)
+                for (int i = 0; i < word_np(set); i++) {
+                    const uint64_t p = WPRIMES[set][i], r = (uint64_t(1) << 32) % p;
+                    uint64_t W = 1;
+                    for (int j = 0; j < i; j++) W = W * (WPRIMES[set][j] % p) % p;
+                    for (int odd = 1; odd < 8; odd += 2)
+                        for (int lev = 0; lev < LEV; lev++)
+                            v[set][odd][lev][i] = (uint32_t)(r * r % p * inv(odd * pw(2, (uint64_t)lev, p) % p * W % p, p) % p);
+                }
         }
     } t;
-    for (int i = 0; i < WPR; i++) out[i] = t.v[s.odd][s.lj + s.lm - 2][i];
+    for (int i = 0; i < word_np(s.set); i++) out[i] = t.v[s.set][s.odd][s.lj + s.lm - 2][i];
 }
 
 // The split of the rows above the blocks: one column pass up to 32 rows (its
@@ -154,16 +165,19 @@ static const std::vector<WordShape>& shape_list() {
             for (int k = 6; k <= WORD_MAX_LOG2; k++) {
                 const int64_t N = (int64_t)odd << k;
                 if (k <= 11 && WPR * N <= 16 * 1024) {
-                    v.push_back(WordShape{(int32_t)N, odd, 0, 0, k, true});
+                    v.push_back(WordShape{(int32_t)N, odd, 0, 0, k, true, 0});
                     continue;
                 }
                 for (int lm : {12, 10, 8}) {
                     int j2;
                     if (k < lm || !row_split(odd, k - lm, j2)) continue;
-                    v.push_back(WordShape{(int32_t)N, odd, k - lm, j2, lm, false});
+                    v.push_back(WordShape{(int32_t)N, odd, k - lm, j2, lm, false, 0});
                     break;
                 }
             }
+        // six primes: 32 (24) first rows, then a middle pass of up to 256
+        for (int k = 22; k <= 25; k++) v.push_back(WordShape{1 << k, 1, k - 12, k - 17, 12, false, 2});
+        for (int k = 21; k <= 23; k++) v.push_back(WordShape{3 << k, 3, k - 12, k - 15, 12, false, 1});
         std::sort(v.begin(), v.end(), [](const WordShape& x, const WordShape& y) { return x.N < y.N; });
         return v;
     }();
@@ -182,7 +196,7 @@ bool word_shape(int64_t nconv, WordShape& s) {
 // ---------------------------------------------------------------------------
 // tables
 
-size_t word_table_bytes(int odd, int L) { return sizeof(Tw) * ((size_t)WPR * odd << L); }
+size_t word_table_bytes(int set, int odd, int L) { return sizeof(Tw) * ((size_t)word_np(set) * odd << L); }
 
 __device__ uint32_t pw_dev(uint32_t a, uint32_t e, uint32_t p) {
     uint64_t r = 1, b = a;
@@ -192,15 +206,26 @@ __device__ uint32_t pw_dev(uint32_t a, uint32_t e, uint32_t p) {
 }
 
 struct WRoots {
-    uint32_t g[WPR];
+    uint32_t g[WPR_MAX];
 };
+constexpr int PWB = 15;  // powers g^e through g^(e mod 2^15) and g^(2^15 (e / 2^15))
+// pwt[i][0][x] = g_i^x, pwt[i][1][x] = g_i^(2^15 x), x < 2^15
+__global__ void k_wpowers(uint32_t* __restrict__ pwt, int set, int np, WRoots g) {
+    const int total = np << (PWB + 1);
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < total; x += gridDim.x * blockDim.x) {
+        const int i = x >> (PWB + 1);
+        const uint32_t e = (uint32_t)x & ((1u << PWB) - 1);
+        pwt[x] = pw_dev(g.g[i], (x >> PWB) & 1 ? e << PWB : e, c_w[set].p[i]);
+    }
+}
 // entry h = 2^l + n of (prime i, block j): e((j + odd * bitrev_l(n)) / (odd * 2^(l+1))) and its inverse
-__global__ void k_wtable(Tw* __restrict__ fwd, Tw* __restrict__ bwd, int odd, int L, WRoots g) {
-    const int64_t total = (int64_t)WPR * odd << L;
+__global__ void k_wtable(Tw* __restrict__ fwd, Tw* __restrict__ bwd, const uint32_t* __restrict__ pwt, int set, int np,
+                         int odd, int L) {
+    const int64_t total = (int64_t)np * odd << L;
     for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < total; x += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t h = (uint32_t)(x & ((int64_t(1) << L) - 1));
         const int ij = (int)(x >> L), i = ij / odd, j = ij - i * odd;
-        const uint32_t p = c_w.p[i];
+        const uint32_t p = c_w[set].p[i];
         uint32_t e = 0;
         if (h) {
             const int l = 31 - __clz(h);
@@ -208,17 +233,27 @@ __global__ void k_wtable(Tw* __restrict__ fwd, Tw* __restrict__ bwd, int odd, in
             const uint32_t brv = l ? __brev(n) >> (32 - l) : 0;
             e = (p - 1) / ((uint32_t)odd << (l + 1)) * ((uint32_t)j + (uint32_t)odd * brv);
         }
-        const uint32_t w = pw_dev(g.g[i], e, p), v = e ? pw_dev(g.g[i], p - 1 - e, p) : 1u;
+        const uint32_t* t = pwt + ((size_t)i << (PWB + 1));
+        auto power = [&](uint32_t q) {
+            return (uint32_t)((uint64_t)t[q & ((1u << PWB) - 1)] * t[(1u << PWB) + (q >> PWB)] % p);
+        };
+        const uint32_t w = power(e), v = e ? power(p - 1 - e) : 1u;
         fwd[x] = Tw{w, (uint32_t)(((uint64_t)w << 32) / p)};
         bwd[x] = Tw{v, (uint32_t)(((uint64_t)v << 32) / p)};
     }
 }
 
-cudaError_t word_build_tables(int odd, int L, void* fwd, void* bwd, cudaStream_t st) {
-    WRoots g;
-    for (int i = 0; i < WPR; i++) g.g[i] = (uint32_t)root_of(i);
-    k_wtable<<<148 * 8, 256, 0, st>>>((Tw*)fwd, (Tw*)bwd, odd, L, g);
-    return cudaGetLastError();
+cudaError_t word_build_tables(int set, int odd, int L, void* fwd, void* bwd, cudaStream_t st) {
+    WRoots g{};
+    for (int i = 0; i < word_np(set); i++) g.g[i] = (uint32_t)root_of(set, i);
+    uint32_t* pwt = nullptr;
+    cudaError_t e = cudaMallocAsync((void**)&pwt, sizeof(uint32_t) * ((size_t)word_np(set) << (PWB + 1)), st);
+    if (e != cudaSuccess) return e;
+    k_wpowers<<<148 * 4, 256, 0, st>>>(pwt, set, word_np(set), g);
+    k_wtable<<<148 * 8, 256, 0, st>>>((Tw*)fwd, (Tw*)bwd, pwt, set, word_np(set), odd, L);
+    e = cudaGetLastError();
+    const cudaError_t f = cudaFreeAsync(pwt, st);
+    return e != cudaSuccess ? e : f;
 }
 
 // ---------------------------------------------------------------------------
@@ -258,23 +293,23 @@ constexpr int WT = 256;  // threads per CTA
 // then immediate offsets), 0: read from the product.  Rows past the operand are
 // not packed, and when they are its upper half (odd = 1, a half-length operand,
 // which one of two always is) the first level is a copy.
-template <int ODD, int LJ, int LM>
+template <int ODD, int LJ, int LM, int SET>
 __global__ void __launch_bounds__(WT, 4) k_wcol_fwd(const __grid_constant__ WArgs A) {
-    constexpr int R = ODD << LJ;
+    constexpr int R = ODD << LJ, NP = word_np(SET);
     int local;
     const DProd& P = wjob(A, local);
     const int lm = LM ? LM : P.wlm + P.wj2;
     const int id = local * WT + (int)threadIdx.x;
     const int c = id & ((1 << lm) - 1);
     int pi = id >> lm;  // operand-major: a's primes, then b's
-    const bool isb = pi >= WPR;
-    if (isb) pi -= WPR;
-    if (pi >= WPR || (isb && P.sqr)) return;
+    const bool isb = pi >= NP;
+    if (isb) pi -= NP;
+    if (pi >= NP || (isb && P.sqr)) return;
     const int n = (int)(isb ? P.ncb : P.nca);
     const int rows = (n + (1 << lm) - 1) >> lm;
     const uint64_t* __restrict__ src = (isb ? P.b : P.a) + c;
     uint32_t* __restrict__ dst = (isb ? P.wb : P.wa) + (size_t)pi * (size_t)P.wN + c;
-    const uint32_t p = c_w.p[pi];
+    const uint32_t p = c_w[SET].p[pi];
     const Tw* tab = (const Tw*)P.wtf + (((size_t)pi * ODD) << P.wL);
     uint32_t x[R];
     auto rowsin = [&](auto r0c, auto r1c) {
@@ -283,7 +318,7 @@ __global__ void __launch_bounds__(WT, 4) k_wcol_fwd(const __grid_constant__ WArg
 #pragma unroll
         for (int r = r0; r < r1; r++) v[r - r0] = c + (r << lm) < n ? __ldg(src + ((size_t)r << lm)) : 0ull;
 #pragma unroll
-        for (int r = r0; r < r1; r++) x[r] = r < rows ? wpack<(ODD > 1)>(v[r - r0], pi, p) : 0u;
+        for (int r = r0; r < r1; r++) x[r] = r < rows ? wpack<(ODD > 1), SET>(v[r - r0], pi, p) : 0u;
     };
     constexpr int H = R / 2;
     if (ODD == 1 && LJ > 0 && rows <= H) {
@@ -298,7 +333,7 @@ __global__ void __launch_bounds__(WT, 4) k_wcol_fwd(const __grid_constant__ WArg
         } else {
             rowsin(std::integral_constant<int, 0>{}, std::integral_constant<int, R>{});
         }
-        dft_odd<ODD, LJ>(x, pi, p);
+        dft_odd<ODD, LJ, SET>(x, pi, p);
 #pragma unroll
         for (int j = 0; j < ODD; j++) wd::tree_fwd<LJ, 1>(x + (j << LJ), tab + ((size_t)j << P.wL), 1u, p);
     }
@@ -306,25 +341,25 @@ __global__ void __launch_bounds__(WT, 4) k_wcol_fwd(const __grid_constant__ WArg
     for (int r = 0; r < R; r++) dst[(size_t)r << lm] = x[r];
 }
 
-template <int ODD, int LJ, int LM>
+template <int ODD, int LJ, int LM, int SET>
 __global__ void __launch_bounds__(WT, LM ? 4 : 3) k_wcol_rev(const __grid_constant__ WArgs A) {
-    constexpr int R = ODD << LJ;
+    constexpr int R = ODD << LJ, NP = word_np(SET);
     int local;
     const DProd& P = wjob(A, local);
     const int lm = LM ? LM : P.wlm + P.wj2;
     const int id = local * WT + (int)threadIdx.x;
     const int c = id & ((1 << lm) - 1);
     const int pi = id >> lm;
-    if (pi >= WPR) return;
+    if (pi >= NP) return;
     uint32_t* __restrict__ dst = P.wa + (size_t)pi * (size_t)P.wN + c;
-    const uint32_t p = c_w.p[pi];
+    const uint32_t p = c_w[SET].p[pi];
     uint32_t x[R];
 #pragma unroll
     for (int r = 0; r < R; r++) x[r] = dst[(size_t)r << lm];
     const Tw* tab = (const Tw*)P.wti + (((size_t)pi * ODD) << P.wL);
 #pragma unroll
     for (int j = 0; j < ODD; j++) wd::tree_rev<LJ, 1>(x + (j << LJ), tab + ((size_t)j << P.wL), 1u, p);
-    dft_odd<ODD, LJ>(x, pi, p);
+    dft_odd<ODD, LJ, SET>(x, pi, p);
     // the inverse step is the forward one with output i at -i mod odd
 #pragma unroll
     for (int r = 0; r < R; r++) {
@@ -336,36 +371,128 @@ __global__ void __launch_bounds__(WT, LM ? 4 : 3) k_wcol_rev(const __grid_consta
 // Middle passes: the 2^J rows (2^lm apart) of one column of a segment, the
 // subtree of the segment's node, above blocks of 4096.  In place; all columns of a segment share
 // their constants.
-template <int J, bool FWD>
+// Column pass `id` of 16-value threads: its values' first word, constants and node.
+struct MidJob {
+    uint32_t* x;
+    const Tw* tab;
+    uint32_t node, p;
+    bool live;
+};
+// item: (operand, prime, segment) in that order; j levels, R1 segments per prime
+template <bool FWD, int SET>
+__device__ __forceinline__ MidJob mid_job(const DProd& P, int item, int j) {
+    constexpr int NP = word_np(SET);
+    const int j1 = P.wlj - j, R1 = P.wodd << j1;
+    const int op = item / R1, seg = item - op * R1;
+    const bool isb = op >= NP;
+    const int pi = isb ? op - NP : op;
+    MidJob J;
+    J.live = pi < NP && !(isb && (!FWD || P.sqr));
+    if (!J.live) return J;
+    J.x = (isb ? P.wb : P.wa) + (size_t)pi * (size_t)P.wN + ((size_t)seg << (12 + j));
+    J.tab = (const Tw*)(FWD ? P.wtf : P.wti) + (((size_t)pi * P.wodd + (seg >> j1)) << P.wL);
+    J.node = (1u << j1) + (uint32_t)(seg & ((1 << j1) - 1));
+    J.p = c_w[SET].p[pi];
+    return J;
+}
+
+template <int J, bool FWD, int SET>
 __global__ void __launch_bounds__(WT) k_wmid(const __grid_constant__ WArgs A) {
+    constexpr int lm = 12;  // more than 32 rows only stand above 4096-value blocks
     int local;
     const DProd& P = wjob(A, local);
-    constexpr int lm = 12;  // more than 32 rows only stand above 4096-value blocks
-    const int j1 = P.wlj - J, R1 = P.wodd << j1;
     const int id = local * WT + (int)threadIdx.x;
-    const int c = id & ((1 << lm) - 1);
-    int op = (id >> lm) / R1;  // operand-major, then prime
-    const int seg = (id >> lm) - op * R1;
-    const bool isb = op >= WPR;
-    const int pi = isb ? op - WPR : op;
-    if (pi >= WPR || (isb && (!FWD || P.sqr))) return;
-    uint32_t* __restrict__ x0 = (isb ? P.wb : P.wa) + (size_t)pi * (size_t)P.wN + ((size_t)seg << (lm + J)) + c;
-    const uint32_t p = c_w.p[pi];
-    const Tw* tab = (const Tw*)(FWD ? P.wtf : P.wti) + (((size_t)pi * P.wodd + (seg >> j1)) << P.wL);
-    const uint32_t node = (1u << j1) + (uint32_t)(seg & ((1 << j1) - 1));
+    const MidJob M = mid_job<FWD, SET>(P, id >> lm, J);
+    if (!M.live) return;
+    uint32_t* __restrict__ x0 = M.x + (id & ((1 << lm) - 1));
     uint32_t x[1 << J];
 #pragma unroll
     for (int r = 0; r < (1 << J); r++) x[r] = x0[(size_t)r << lm];
-    if (FWD) wd::tree_fwd<J, 1>(x, tab, node, p);
-    else wd::tree_rev<J, 1>(x, tab, node, p);
+    if (FWD) wd::tree_fwd<J, 1>(x, M.tab, M.node, M.p);
+    else wd::tree_rev<J, 1>(x, M.tab, M.node, M.p);
 #pragma unroll
     for (int r = 0; r < (1 << J); r++) x0[(size_t)r << lm] = x[r];
+}
+
+// 64 to 256 rows: tiles of 2^J rows by 2^(12-J) columns (64 to 256 bytes per
+// row), four levels in registers, a turn through shared memory, the other J - 4
+// levels.  One pass over memory instead of two: at these lengths the register
+// passes run at the memory's rate (2^24-limb square, per pass 1.6 GB).
+template <int J, bool FWD, int SET>
+__global__ void __launch_bounds__(WT, 4) k_wmid_sm(const __grid_constant__ WArgs A) {
+    constexpr int lm = 12, CW = 1 << (12 - J), K = J - 4, NG = 1 << (4 - K);  // NG groups of 2^K values per thread
+    __shared__ uint32_t s[4096 + 16 * 16];
+    auto at = [](int i) { return i + ((i >> 8) << 4); };  // rows of 16 words: the two half-warps in distinct banks
+    int local;
+    const DProd& P = wjob(A, local);
+    const MidJob M = mid_job<FWD, SET>(P, local >> J, J);  // 2^J tiles per segment
+    if (!M.live) return;                                    // the whole CTA
+    const int tid = (int)threadIdx.x, c = tid & (CW - 1), g = tid >> (12 - J);
+    uint32_t* __restrict__ x0 = M.x + (local & ((1 << J) - 1)) * CW + c;
+    uint32_t x[16];
+    auto outer_io = [&](bool st) {  // rows g + e * 2^K
+#pragma unroll
+        for (int e = 0; e < 16; e++) {
+            uint32_t* w = x0 + ((size_t)(g + (e << K)) << lm);
+            if (st) *w = x[e];
+            else x[e] = *w;
+        }
+    };
+    auto inner_io = [&](bool st) {  // group q: sub-block b = g + q * (16 / NG), rows b * 2^K + e
+#pragma unroll
+        for (int q = 0; q < NG; q++)
+#pragma unroll
+            for (int e = 0; e < (1 << K); e++) {
+                uint32_t* w = x0 + ((size_t)(((g + q * (16 / NG)) << K) + e) << lm);
+                if (st) *w = x[(q << K) + e];
+                else x[(q << K) + e] = *w;
+            }
+    };
+    auto outer_sm = [&](bool st) {
+#pragma unroll
+        for (int e = 0; e < 16; e++) {
+            uint32_t& w = s[at((g + (e << K)) * CW + c)];
+            if (st) w = x[e];
+            else x[e] = w;
+        }
+    };
+    auto inner_sm = [&](bool st) {
+#pragma unroll
+        for (int q = 0; q < NG; q++)
+#pragma unroll
+            for (int e = 0; e < (1 << K); e++) {
+                uint32_t& w = s[at((((g + q * (16 / NG)) << K) + e) * CW + c)];
+                if (st) w = x[(q << K) + e];
+                else x[(q << K) + e] = w;
+            }
+    };
+    if (FWD) {
+        outer_io(false);
+        wd::tree_fwd<4, 1>(x, M.tab, M.node, M.p);
+        outer_sm(true);
+        __syncthreads();
+        inner_sm(false);
+#pragma unroll
+        for (int q = 0; q < NG; q++)
+            wd::tree_fwd<K, 1>(x + (q << K), M.tab, (M.node << 4) + (uint32_t)(g + q * (16 / NG)), M.p);
+        inner_io(true);
+    } else {
+        inner_io(false);
+#pragma unroll
+        for (int q = 0; q < NG; q++)
+            wd::tree_rev<K, 1>(x + (q << K), M.tab, (M.node << 4) + (uint32_t)(g + q * (16 / NG)), M.p);
+        inner_sm(true);
+        __syncthreads();
+        outer_sm(false);
+        wd::tree_rev<4, 1>(x, M.tab, M.node, M.p);
+        outer_io(true);
+    }
 }
 
 // ---------------------------------------------------------------------------
 // blocks
 
-template <int LM>
+template <int LM, int SET>
 __global__ void __launch_bounds__(WT, 3) k_wblock(const __grid_constant__ WArgs A) {
     constexpr int T = 1 << (LM - 4), PER = WT / T;  // threads per block, blocks per CTA
     constexpr int SM = wwords(1 << LM);
@@ -376,11 +503,11 @@ __global__ void __launch_bounds__(WT, 3) k_wblock(const __grid_constant__ WArgs 
     const int g = (int)threadIdx.x / T, t = (int)threadIdx.x & (T - 1);
     const int R = P.wodd << P.wlj;
     const int blk = local * PER + g;  // prime-major, then block
-    const bool live = blk < WPR * R;
+    const bool live = blk < word_np(SET) * R;
     const int pi = live ? blk / R : 0, row = live ? blk - pi * R : 0;
     const int j = row >> P.wlj;
     const uint32_t h0 = (1u << P.wlj) + (uint32_t)(row & ((1 << P.wlj) - 1));
-    const uint32_t p = c_w.p[pi], pinv = c_w.pinv[pi];
+    const uint32_t p = c_w[SET].p[pi], pinv = c_w[SET].pinv[pi];
     const size_t toff = ((size_t)pi * P.wodd + j) << P.wL, xoff = (size_t)pi * (size_t)P.wN + ((size_t)row << LM);
     const Tw* tf = (const Tw*)P.wtf + toff;
     uint32_t* xa = P.wa + xoff;
@@ -410,7 +537,9 @@ __global__ void __launch_bounds__(WT, 3) k_wblock(const __grid_constant__ WArgs 
 // ---------------------------------------------------------------------------
 // unpack: coefficients and carried limbs, tiles of UNPACK_TL limbs
 
+template <int SET>
 __global__ void __launch_bounds__(WT) k_wunpack(const __grid_constant__ WArgs A) {
+    constexpr int NP = word_np(SET);
     __shared__ LimbShared<WT> S;
     __shared__ uint64_t h_lo, h_mid2;  // the limb sum below the tile
     __shared__ uint32_t h_hi3;
@@ -420,19 +549,19 @@ __global__ void __launch_bounds__(WT) k_wunpack(const __grid_constant__ WArgs A)
     const int N = P.wN;
     const uint32_t* __restrict__ x = P.wa;
     const int64_t w0 = (int64_t)tile * UNPACK_TL, w1 = min(w0 + (int64_t)UNPACK_TL, P.rn);
-    uint32_t sc[WPR];
+    uint32_t sc[NP];
 #pragma unroll
-    for (int i = 0; i < WPR; i++) sc[i] = P.wsc[i];
+    for (int i = 0; i < NP; i++) sc[i] = P.wsc[i];
     // the three coefficients before the tile
     if (t < 3) {
         const int64_t i = w0 - 1 - t;
         uint64_t lo = 0, mid = 0;
         uint32_t hi = 0;
         if (i >= 0 && i < N) {
-            uint32_t r[WPR];
+            uint32_t r[NP];
 #pragma unroll
-            for (int k = 0; k < WPR; k++) r[k] = x[(size_t)k * N + i];
-            coef_words(r, sc, lo, mid, hi);
+            for (int k = 0; k < NP; k++) r[k] = x[(size_t)k * N + i];
+            coef_words<SET>(r, sc, lo, mid, hi);
         }
         if (t == 0) {
             h_lo = lo;
@@ -457,7 +586,7 @@ __global__ void __launch_bounds__(WT) k_wunpack(const __grid_constant__ WArgs A)
     uint64_t lo[4] = {0, 0, 0, 0}, mid[4] = {0, 0, 0, 0}, own[4];
     uint32_t hi[4] = {0, 0, 0, 0};
     if (wt < N) {  // N is a multiple of 4: all four or none
-        coef4(reinterpret_cast<const uint4*>(x + wt), N / 4, sc, lo, mid, hi);
+        coef4<SET>(reinterpret_cast<const uint4*>(x + wt), N / 4, sc, lo, mid, hi);
     }
     const uint32_t tot = limb_sums<WT>(S, t, WT, lo, mid, hi, (int)(w1 - w0), own);
     store_limbs(P.r, wt, w1, own);
@@ -562,14 +691,14 @@ __global__ void __launch_bounds__(WSmall<ODD, LM>::NT, WSmall<ODD, LM>::NT > 320
 
 int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t rn) {
     const int64_t M = int64_t(1) << s.lm, R = (int64_t)s.odd << s.lj;
-    const int64_t cols = M << s.j2, mcols = (int64_t)s.N >> s.j2;
+    const int64_t cols = M << s.j2, mthreads = (int64_t)s.N >> (s.j2 > 5 ? 4 : s.j2), np = word_np(s.set);
     const int64_t tiles = (rn + UNPACK_TL - 1) / UNPACK_TL;
     switch (kind) {
-        case JK_WCOL_FWD: return ((sqr ? 1 : 2) * WPR * cols + WT - 1) / WT;
-        case JK_WCOL_REV: return (WPR * cols + WT - 1) / WT;
-        case JK_WMID_FWD: return ((sqr ? 1 : 2) * WPR * mcols + WT - 1) / WT;
-        case JK_WMID_REV: return (WPR * mcols + WT - 1) / WT;
-        case JK_WBLOCK: return (WPR * R * (M / 16) + WT - 1) / WT;
+        case JK_WCOL_FWD: return ((sqr ? 1 : 2) * np * cols + WT - 1) / WT;
+        case JK_WCOL_REV: return (np * cols + WT - 1) / WT;
+        case JK_WMID_FWD: return ((sqr ? 1 : 2) * np * mthreads + WT - 1) / WT;
+        case JK_WMID_REV: return (np * mthreads + WT - 1) / WT;
+        case JK_WBLOCK: return (np * R * (M / 16) + WT - 1) / WT;
         case JK_WSMALL: return 1;
         case JK_WCARRY: return (tiles + WT - 1) / WT;  // 8 warps of 32 tiles
         default: return tiles;
@@ -589,24 +718,50 @@ static WLaunch small_kernel() {
 }
 template <int ODD, int LJ>
 static WLaunch col_kernel(int kind, bool lm12) {
-    if (kind == JK_WCOL_FWD) return WLaunch{lm12 ? k_wcol_fwd<ODD, LJ, 12> : k_wcol_fwd<ODD, LJ, 0>, WT, 0};
-    return WLaunch{lm12 ? k_wcol_rev<ODD, LJ, 12> : k_wcol_rev<ODD, LJ, 0>, WT, 0};
+    if (kind == JK_WCOL_FWD) return WLaunch{lm12 ? k_wcol_fwd<ODD, LJ, 12, 0> : k_wcol_fwd<ODD, LJ, 0, 0>, WT, 0};
+    return WLaunch{lm12 ? k_wcol_rev<ODD, LJ, 12, 0> : k_wcol_rev<ODD, LJ, 0, 0>, WT, 0};
 }
 template <int J>
 static WLaunch mid_kernel(int kind) {
-    return WLaunch{kind == JK_WMID_FWD ? k_wmid<J, true> : k_wmid<J, false>, WT, 0};
+    return WLaunch{kind == JK_WMID_FWD ? k_wmid<J, true, 0> : k_wmid<J, false, 0>, WT, 0};
+}
+template <int J, int SET>
+static WLaunch mid_sm_kernel(int kind) {
+    return WLaunch{kind == JK_WMID_FWD ? k_wmid_sm<J, true, SET> : k_wmid_sm<J, false, SET>, WT, 0};
+}
+
+// Kernels of the six-prime sets.
+template <int SET, int ODD, int LJ>
+static WLaunch big_kernel(int kind, int variant) {
+    switch (kind) {
+        case JK_WCOL_FWD: return WLaunch{k_wcol_fwd<ODD, LJ, 0, SET>, WT, 0};
+        case JK_WCOL_REV: return WLaunch{k_wcol_rev<ODD, LJ, 0, SET>, WT, 0};
+        case JK_WBLOCK: return WLaunch{k_wblock<12, SET>, WT, 0};
+        case JK_WUNPACK: return WLaunch{k_wunpack<SET>, WT, 0};
+        case JK_WMID_FWD:
+        case JK_WMID_REV:
+            switch (variant) {
+                case 5: return WLaunch{kind == JK_WMID_FWD ? k_wmid<5, true, SET> : k_wmid<5, false, SET>, WT, 0};
+                case 6: return mid_sm_kernel<6, SET>(kind);
+                case 7: return mid_sm_kernel<7, SET>(kind);
+                case 8: return mid_sm_kernel<8, SET>(kind);
+            }
+    }
+    return WLaunch{nullptr, 0, 0};
 }
 
 static WLaunch word_kernel(int kind, int variant) {
+    if (kind == JK_WCARRY) return WLaunch{k_wcarry, WT, 0};
+    if (variant >> 20 == 1) return big_kernel<1, 3, 3>(kind, variant & 0xfffff);
+    if (variant >> 20 == 2) return big_kernel<2, 1, 5>(kind, variant & 0xfffff);
     switch (kind) {
-        case JK_WUNPACK: return WLaunch{k_wunpack, WT, 0};
-        case JK_WCARRY: return WLaunch{k_wcarry, WT, 0};
+        case JK_WUNPACK: return WLaunch{k_wunpack<0>, WT, 0};
         case JK_WBLOCK:
             switch (variant) {
-                case 12: return WLaunch{k_wblock<12>, WT, 0};
-                case 10: return WLaunch{k_wblock<10>, WT, 0};
-                case 8: return WLaunch{k_wblock<8>, WT, 0};
-                        }
+                case 12: return WLaunch{k_wblock<12, 0>, WT, 0};
+                case 10: return WLaunch{k_wblock<10, 0>, WT, 0};
+                case 8: return WLaunch{k_wblock<8, 0>, WT, 0};
+            }
             break;
         case JK_WMID_FWD:
         case JK_WMID_REV:

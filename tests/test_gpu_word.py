@@ -119,3 +119,17 @@ def test_power_chains_at_transform_edges(gpu_lib, k):
         exps.append(rand_limbs(rng, 1))
     for r, b, e, m in zip(gpu_lib.powermod_batch(bases, exps, mods), bases, exps, mods):
         assert num(r) == pow(num(b), num(e), num(m))
+
+
+@pytest.mark.parametrize("odd,k", [(1, 22), (3, 21), (1, 23), (3, 22), (1, 24), (3, 23)])
+def test_six_prime_shapes(gpu_lib, odd, k):
+    # each middle pass (32 to 256 rows) at its exact length; the largest coefficients
+    N = odd << k
+    rng = np.random.default_rng(N)
+    a = rand_limbs(rng, (N + 1) // 2)
+    if k == 22:
+        a[:] = 2**64 - 1
+    assert np.array_equal(gpu_lib.sqr(a), _want(a, None))
+    b = rand_limbs(rng, 70001)
+    c = rand_limbs(rng, N + 1 - b.size)
+    assert np.array_equal(gpu_lib.mul(c, b), _want(c, b))
