@@ -345,6 +345,8 @@ int Engine::init(int device) {
     CUDA_TRY(cudaStreamCreateWithFlags(&copy_in, cudaStreamNonBlocking));
     CUDA_TRY(cudaStreamCreateWithFlags(&copy_out, cudaStreamNonBlocking));
     for (cudaStream_t& s : side) CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    CUDA_TRY(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
+    for (cudaEvent_t& e : join_ev) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (auto& row : hb_ev)
         for (cudaEvent_t& e : row) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CUDA_TRY(kernels_init((double)PR[0], (double)PR[1]));
@@ -844,25 +846,37 @@ static std::vector<std::pair<int, int>> word_steps(const WordShape& s) {
     const int col = set | (s.lm + s.j2 == 12 ? 1 << 16 : 0) | (s.odd << 8) | (s.lj - s.j2);
     std::vector<std::pair<int, int>> v{{JK_WCOL_FWD, col}};
     if (s.j2) v.push_back({JK_WMID_FWD, set | s.j2});
-    v.push_back({JK_WBLOCK, set | s.lm});
+    v.push_back({JK_WBLOCK, set});
     if (s.j2) v.push_back({JK_WMID_REV, set | s.j2});
     v.push_back({JK_WCOL_REV, col});
     v.push_back({JK_WUNPACK, set});
     return v;
 }
 
-int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, cudaStream_t st) {
+static size_t word_op_bytes(const WordShape& s) {
+    return align_up(sizeof(uint32_t) * (size_t)word_np(s.set) * (size_t)s.N, 256);
+}
+
+size_t word_work_bytes(const ProdIn& q, const WordShape& s) {
+    if (s.small) return 0;
+    const int64_t rn = q.m + (q.sqr ? q.m : q.n);
+    return word_op_bytes(s) * (q.sqr ? 1 : 2) + sizeof(uint32_t) * (size_t)((rn + UNPACK_TL - 1) / UNPACK_TL);
+}
+
+int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, char* work, cudaStream_t st) {
     DProd P;
     int rc = word_setup(E, q, s, P);
     if (rc) return rc;
+    const bool pool = !s.small && !work;
     if (!s.small) {
-        const size_t op = align_up(sizeof(uint32_t) * (size_t)word_np(s.set) * (size_t)s.N, 256);
-        const size_t res = op * (q.sqr ? 1 : 2);
-        if ((rc = E.ensure_pool(res + sizeof(uint32_t) * (size_t)P.ntl, st))) return rc;
-        char* d = (char*)E.pool;
-        P.wa = (uint32_t*)d;
-        P.wb = q.sqr ? nullptr : (uint32_t*)(d + op);
-        P.agg = (uint32_t*)(d + res);
+        if (pool) {
+            if ((rc = E.ensure_pool(word_work_bytes(q, s), st))) return rc;
+            work = (char*)E.pool;
+        }
+        const size_t op = word_op_bytes(s);
+        P.wa = (uint32_t*)work;
+        P.wb = q.sqr ? nullptr : (uint32_t*)(work + op);
+        P.agg = (uint32_t*)(work + op * (q.sqr ? 1 : 2));
     }
     auto steps = word_steps(s);
     if (P.ntl > 1) steps.push_back({JK_WCARRY, 0});
@@ -870,7 +884,7 @@ int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, cudaStream_t st
         CUDA_TRY(launch_word_one(kv.first, kv.second, P, word_ctas(kv.first, s, P.sqr, P.rn), st));
         g_launches++;
     }
-    return s.small ? NBG_OK : E.pool_release(st);
+    return pool ? E.pool_release(st) : NBG_OK;
 }
 
 int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
@@ -1406,36 +1420,25 @@ int run_launches_branched(Engine& E, const BatchBuild& bb, char* dbase, cudaStre
     while (i < bb.launches.size()) {
         size_t j = i;
         while (j < bb.launches.size() && bb.launches[j].step == bb.launches[i].step) j++;
-        // launches [i, j) share a step: the first on st, the rest forked
-        std::vector<cudaEvent_t> joins;
-        cudaEvent_t fork = nullptr;
-        if (j - i > 1) {
-            CUDA_TRY(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-            CUDA_TRY(cudaEventRecord(fork, st));
+        // launches [i, j) share a step: the first on st, the rest dealt to the
+        // side streams, each forked from st and joined to it once
+        const int ns = (int)std::min<size_t>((size_t)std::max(nside, 0), j - i - 1);
+        if (ns) {
+            CUDA_TRY(cudaEventRecord(E.fork_ev, st));
+            for (int q = 0; q < ns; q++) CUDA_TRY(cudaStreamWaitEvent(side[q], E.fork_ev, 0));
         }
         for (size_t k = i; k < j; k++) {
             const Launch& L = bb.launches[k];
-            cudaStream_t s = st;
-            if (k > i && nside > 0) {
-                s = side[(k - i - 1) % (size_t)nside];
-                CUDA_TRY(cudaStreamWaitEvent(s, fork, 0));
-            }
+            cudaStream_t s = k > i && ns ? side[(k - i - 1) % (size_t)ns] : st;
             cudaError_t e = launch_one(E, bb, L, dbase, s);
             if (e != cudaSuccess)
                 return fail(NBG_ECUDA, "launch (kind %d, %lld jobs): %s", L.kind, (long long)L.n, cudaGetErrorString(e));
             g_launches++;
-            if (s != st) {
-                cudaEvent_t jv;
-                CUDA_TRY(cudaEventCreateWithFlags(&jv, cudaEventDisableTiming));
-                CUDA_TRY(cudaEventRecord(jv, s));
-                joins.push_back(jv);
-            }
         }
-        for (cudaEvent_t jv : joins) {
-            CUDA_TRY(cudaStreamWaitEvent(st, jv, 0));
-            cudaEventDestroy(jv);
+        for (int q = 0; q < ns; q++) {
+            CUDA_TRY(cudaEventRecord(E.join_ev[q], side[q]));
+            CUDA_TRY(cudaStreamWaitEvent(st, E.join_ev[q], 0));
         }
-        if (fork) cudaEventDestroy(fork);
         i = j;
     }
     return NBG_OK;

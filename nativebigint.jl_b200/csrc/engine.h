@@ -76,6 +76,7 @@ struct Engine {
     cudaStream_t copy_in = nullptr;  // host-to-device copies of the pipelined host calls
     cudaStream_t copy_out = nullptr; // device-to-host copies
     cudaStream_t side[4] = {};       // parallel branches of one pipeline step (host-buffer batches)
+    cudaEvent_t fork_ev = nullptr, join_ev[4] = {};  // branches of a step (under the lock; waits bind at the call)
     cudaEvent_t hb_ev[3][4] = {};    // host-buffer batches: per slot, operands in / computed / results out
     std::recursive_mutex mu;
     Tuning tun;
@@ -138,8 +139,10 @@ bool word_product(const Engine& E, const ProdIn& q, WordShape* s);
 // Fills P for a word product (device pointers as in q; workspace pointers left null).
 int word_setup(Engine& E, const ProdIn& q, const WordShape& s, DProd& P);
 // One word product on `st` with its descriptor passed by value: no copies and
-// no host wait; the shared workspace holds its transforms.
-int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, cudaStream_t st);
+// no host wait.  Its transforms are in `work` (word_work_bytes), or in the
+// shared workspace when that is null.
+int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, char* work, cudaStream_t st);
+size_t word_work_bytes(const ProdIn& q, const WordShape& s);
 // Transform buffers of the product on the multi-pass FP64 engine (SIZE_MAX: no such transform).
 size_t fp64_work_bytes(const ProdIn& q);
 

@@ -57,8 +57,9 @@ struct WSeg {
     int32_t pad_;
 };
 
-// variant of a word launch: bits 20 on the prime set, then (odd << 8) | (lj - j2) for column passes (bit 16: of 4096 columns), j2 for middle ones, lm for
-// blocks, (odd << 8) | lm for one-CTA products
+// Variant of a word launch: bits 20 on the prime set, below them
+// (odd << 8) | (lj - j2) for column passes (bit 16: of 4096 columns), j2 for
+// middle passes, (odd << 8) | lm for one-CTA products, 0 for the rest.
 cudaError_t word_init();  // constant memory of the current device
 cudaError_t launch_word(int kind, int variant, const DProd* prods, const WSeg* segs, int nseg, const int32_t* plist,
                         int64_t nctas, cudaStream_t st);

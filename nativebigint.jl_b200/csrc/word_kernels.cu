@@ -148,7 +148,7 @@ static bool row_split(int odd, int lj, int& j2) {
     const int64_t R = (int64_t)odd << lj;
     if (R <= 32) return R >= 2;
     int64_t best = INT64_MAX;
-    for (int j = 2; j <= 5 && j <= lj; j++) {
+    for (int j = 3; j <= 5 && j <= lj; j++) {
         const int64_t r1 = (int64_t)odd << (lj - j), r2 = int64_t(1) << j;
         if (r1 < 2 || r1 > 32 || std::max(r1, r2) >= best) continue;
         best = std::max(r1, r2);
@@ -492,14 +492,16 @@ __global__ void __launch_bounds__(WT, 4) k_wmid_sm(const __grid_constant__ WArgs
 // ---------------------------------------------------------------------------
 // blocks
 
+template <int LM>
+struct WBlockSmem {
+    static constexpr int PER = WT >> (LM - 4), SM = wwords(1 << LM);  // blocks per CTA, words of one
+    static constexpr int words = PER * 2 * SM;
+};
 template <int LM, int SET>
-__global__ void __launch_bounds__(WT, 3) k_wblock(const __grid_constant__ WArgs A) {
-    constexpr int T = 1 << (LM - 4), PER = WT / T;  // threads per block, blocks per CTA
-    constexpr int SM = wwords(1 << LM);
+__device__ __forceinline__ void wblock(const DProd& P, int local, uint32_t* smw) {
+    constexpr int T = 1 << (LM - 4), PER = WBlockSmem<LM>::PER, SM = WBlockSmem<LM>::SM;
     constexpr int J1 = WSplit<LM>::J1;
-    __shared__ __align__(16) uint32_t sm[PER][2][SM];
-    int local;
-    const DProd& P = wjob(A, local);
+    uint32_t(*sm)[2][SM] = reinterpret_cast<uint32_t(*)[2][SM]>(smw);
     const int g = (int)threadIdx.x / T, t = (int)threadIdx.x & (T - 1);
     const int R = P.wodd << P.wlj;
     const int blk = local * PER + g;  // prime-major, then block
@@ -531,6 +533,21 @@ __global__ void __launch_bounds__(WT, 3) k_wblock(const __grid_constant__ WArgs 
 #pragma unroll
         for (int k = 0; k < 16; k++)
             xa[wpos<LM, LM, J1>(t, k >> J1) + ((k & ((1 << J1) - 1)) << (LM - J1))] = a[k];
+    }
+}
+
+// One launch serves every block size of set 0.
+template <int SET>
+__global__ void __launch_bounds__(WT, 3) k_wblock(const __grid_constant__ WArgs A) {
+    __shared__ __align__(16) uint32_t sm[WBlockSmem<12>::words];
+    static_assert(WBlockSmem<10>::words <= WBlockSmem<12>::words && WBlockSmem<8>::words <= WBlockSmem<12>::words, "");
+    int local;
+    const DProd& P = wjob(A, local);
+    if (SET || P.wlm == 12) {
+        wblock<12, SET>(P, local, sm);
+    } else if constexpr (SET == 0) {
+        if (P.wlm == 10) wblock<10, SET>(P, local, sm);
+        else wblock<8, SET>(P, local, sm);
     }
 }
 
@@ -718,8 +735,10 @@ static WLaunch small_kernel() {
 }
 template <int ODD, int LJ>
 static WLaunch col_kernel(int kind, bool lm12) {
-    if (kind == JK_WCOL_FWD) return WLaunch{lm12 ? k_wcol_fwd<ODD, LJ, 12, 0> : k_wcol_fwd<ODD, LJ, 0, 0>, WT, 0};
-    return WLaunch{lm12 ? k_wcol_rev<ODD, LJ, 12, 0> : k_wcol_rev<ODD, LJ, 0, 0>, WT, 0};
+    if (lm12) return WLaunch{kind == JK_WCOL_FWD ? k_wcol_fwd<ODD, LJ, 12, 0> : k_wcol_rev<ODD, LJ, 12, 0>, WT, 0};
+    // no supported length has these rows above other column counts
+    if constexpr ((ODD == 1 && (LJ == 1 || LJ == 5)) || (ODD == 3 && LJ == 0)) return WLaunch{nullptr, 0, 0};
+    else return WLaunch{kind == JK_WCOL_FWD ? k_wcol_fwd<ODD, LJ, 0, 0> : k_wcol_rev<ODD, LJ, 0, 0>, WT, 0};
 }
 template <int J>
 static WLaunch mid_kernel(int kind) {
@@ -736,7 +755,7 @@ static WLaunch big_kernel(int kind, int variant) {
     switch (kind) {
         case JK_WCOL_FWD: return WLaunch{k_wcol_fwd<ODD, LJ, 0, SET>, WT, 0};
         case JK_WCOL_REV: return WLaunch{k_wcol_rev<ODD, LJ, 0, SET>, WT, 0};
-        case JK_WBLOCK: return WLaunch{k_wblock<12, SET>, WT, 0};
+        case JK_WBLOCK: return WLaunch{k_wblock<SET>, WT, 0};
         case JK_WUNPACK: return WLaunch{k_wunpack<SET>, WT, 0};
         case JK_WMID_FWD:
         case JK_WMID_REV:
@@ -756,24 +775,9 @@ static WLaunch word_kernel(int kind, int variant) {
     if (variant >> 20 == 2) return big_kernel<2, 1, 5>(kind, variant & 0xfffff);
     switch (kind) {
         case JK_WUNPACK: return WLaunch{k_wunpack<0>, WT, 0};
-        case JK_WBLOCK:
-            switch (variant) {
-                case 12: return WLaunch{k_wblock<12, 0>, WT, 0};
-                case 10: return WLaunch{k_wblock<10, 0>, WT, 0};
-                case 8: return WLaunch{k_wblock<8, 0>, WT, 0};
-            }
-            break;
-        case JK_WMID_FWD:
-        case JK_WMID_REV:
-            switch (variant) {
-                case 2: return mid_kernel<2>(kind);
-                case 3: return mid_kernel<3>(kind);
-                case 4: return mid_kernel<4>(kind);
-                case 5: return mid_kernel<5>(kind);
-            }
-            break;
+        case JK_WBLOCK: return WLaunch{k_wblock<0>, WT, 0};
         case JK_WCOL_FWD:
-        case JK_WCOL_REV:
+        case JK_WCOL_REV:  // one kernel per row count: a switch inside one kernel took 25% longer (registers)
             switch (variant & 0xffff) {
 #define NBG_COL(O, J) \
     case (O << 8) | J: return col_kernel<O, J>(kind, variant >> 16);
@@ -782,6 +786,14 @@ static WLaunch word_kernel(int kind, int variant) {
                 NBG_COL(5, 0) NBG_COL(5, 1) NBG_COL(5, 2)
                 NBG_COL(7, 0) NBG_COL(7, 1) NBG_COL(7, 2)
 #undef NBG_COL
+            }
+            break;
+        case JK_WMID_FWD:
+        case JK_WMID_REV:
+            switch (variant) {
+                case 3: return mid_kernel<3>(kind);
+                case 4: return mid_kernel<4>(kind);
+                case 5: return mid_kernel<5>(kind);
             }
             break;
         case JK_WSMALL:

@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sys
 
 import numpy as np
 
@@ -174,6 +175,18 @@ def _stream(s) -> int | None:
     return getattr(s, "cuda_stream", None) or int(s)
 
 
+def _in_flight(stream, *buffers) -> None:
+    """Tensors given to a call on an explicit stream stay allocated until that
+    stream is done with them (the call itself may return earlier)."""
+    if stream is None:
+        return
+    torch = sys.modules.get("torch")
+    for x in buffers:
+        if torch is not None and isinstance(x, torch.Tensor) and x.is_cuda:
+            st = stream if hasattr(stream, "cuda_stream") else torch.cuda.ExternalStream(_stream(stream))
+            x.record_stream(st)
+
+
 # ---------------------------------------------------------------------------
 # mpn-level drop-ins (host buffers)
 
@@ -264,12 +277,16 @@ def radix_powtab(bb: int, x) -> list[np.ndarray]:
 def mul_batch(pairs) -> list[np.ndarray]:
     """Products of a list of (a, b) pairs (b None for a square), one batched
     call; returns the m+n-limb results."""
-    ops = []
+    pairs = [(_u64(a), None if b is None else _u64(b)) for a, b in pairs]
+    sizes = [a.size + (a.size if b is None else b.size) for a, b in pairs]
+    # one allocation for all results (views of it are returned): fresh pages of
+    # many small ones cost more than the products
+    flat = np.empty(sum(sizes), dtype=np.uint64)
+    ops, off = [], 0
     descs = (NbgDesc * len(pairs))()
     for k, (a, b) in enumerate(pairs):
-        a = _u64(a)
-        b = None if b is None else _u64(b)
-        r = np.empty(a.size + (a.size if b is None else b.size), dtype=np.uint64)
+        r = flat[off: off + sizes[k]]
+        off += sizes[k]
         ops.append((a, b, r))
         descs[k] = NbgDesc(_ptr(r), _ptr(a), None if b is None else _ptr(b), a.size,
                            a.size if b is None else b.size, 0, 0)
@@ -294,10 +311,12 @@ def uses_fpntt_sqr(n: int) -> bool:
 
 def mul_dev(r, a, m: int, b, n: int, stream=None) -> None:
     _check(lib().nbg_mul_dev(_dptr(r), _dptr(a), m, _dptr(b), n, _stream(stream)))
+    _in_flight(stream, r, a, b)
 
 
 def sqr_dev(r, a, n: int, stream=None) -> None:
     _check(lib().nbg_sqr_dev(_dptr(r), _dptr(a), n, _stream(stream)))
+    _in_flight(stream, r, a)
 
 
 def mul_dev_noalloc(r, a, m: int, b, n: int, stream=None) -> None:

@@ -133,3 +133,42 @@ def test_six_prime_shapes(gpu_lib, odd, k):
     b = rand_limbs(rng, 70001)
     c = rand_limbs(rng, N + 1 - b.size)
     assert np.array_equal(gpu_lib.mul(c, b), _want(c, b))
+
+
+@pytest.mark.parametrize("m,n", [(200, 150), (1600, 1473), (4864, 4321), (70000, 61000), (250000, 240000)])
+def test_host_buffers_pinned_and_pageable(gpu_lib, m, n):
+    # one-CTA, direct and staged host products, each operand and the result in
+    # pinned or pageable memory
+    rng = np.random.default_rng(m)
+    a, b = rand_limbs(rng, m), rand_limbs(rng, n)
+    want = _want(a, b)
+
+    def buf(x, pinned):
+        t = torch.empty(x.size, dtype=torch.int64, pin_memory=pinned)
+        v = t.numpy().view(np.uint64)
+        v[:] = x
+        return t, v
+
+    for mask in range(8):
+        (ka, va), (kb, vb), (kr, vr) = (buf(x, bool(mask >> i & 1)) for i, x in enumerate((a, b, np.zeros(m + n, np.uint64))))
+        gpu_lib.mul_(vr, 0, va, 0, m, vb, 0, n)
+        assert np.array_equal(vr, want)
+
+
+def test_calls_on_several_streams_share_the_workspace(gpu_lib):
+    rng = np.random.default_rng(91)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    jobs = []
+    torch.cuda.synchronize()
+    for k in range(24):
+        m, n = int(rng.integers(2000, 60000)), int(rng.integers(500, 30000))
+        a, b = rand_limbs(rng, m), rand_limbs(rng, n)
+        with torch.cuda.stream(streams[k % 3]):
+            da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+            r = torch.zeros(m + n, dtype=torch.uint64, device="cuda")
+            gpu_lib.mul_dev(r, da, m, db, n, streams[k % 3])
+        jobs.append((a, b, r))
+        del da, db  # in flight on the stream
+    torch.cuda.synchronize()
+    for a, b, r in jobs:
+        assert np.array_equal(r.cpu().numpy(), _want(a, b))
