@@ -826,7 +826,8 @@ int word_setup(Engine& E, const ProdIn& q, const WordShape& s, DProd& P) {
     P.nca = eff_limbs(P.m, q.bits_a);
     P.ncb = q.sqr ? P.nca : eff_limbs(P.n, q.bits_b);
     P.nconv = P.nca + P.ncb - 1;
-    P.ntl = s.small ? 0 : (P.rn + UNPACK_TL - 1) / UNPACK_TL;
+    P.tl = word_run(s.odd << (s.lj - s.j2));
+    P.ntl = s.small ? 0 : (std::min<int64_t>(P.rn, (int64_t)s.N + 1) + P.tl - 1) / P.tl;
     P.wN = s.N;
     P.wodd = s.odd;
     P.wlj = s.lj;
@@ -848,8 +849,7 @@ static std::vector<std::pair<int, int>> word_steps(const WordShape& s) {
     if (s.j2) v.push_back({JK_WMID_FWD, set | s.j2});
     v.push_back({JK_WBLOCK, set});
     if (s.j2) v.push_back({JK_WMID_REV, set | s.j2});
-    v.push_back({JK_WCOL_REV, col});
-    v.push_back({JK_WUNPACK, set});
+    v.push_back({JK_WTAIL, col});
     return v;
 }
 
@@ -859,8 +859,7 @@ static size_t word_op_bytes(const WordShape& s) {
 
 size_t word_work_bytes(const ProdIn& q, const WordShape& s) {
     if (s.small) return 0;
-    const int64_t rn = q.m + (q.sqr ? q.m : q.n);
-    return word_op_bytes(s) * (q.sqr ? 1 : 2) + sizeof(uint32_t) * (size_t)((rn + UNPACK_TL - 1) / UNPACK_TL);
+    return word_op_bytes(s) * (q.sqr ? 1 : 2) + sizeof(uint32_t) * (size_t)(s.N / 64 + 3);  // runs of 64 limbs or more, two counts
 }
 
 int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, char* work, cudaStream_t st) {
@@ -879,9 +878,9 @@ int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, char* work, cud
         P.agg = (uint32_t*)(work + op * (q.sqr ? 1 : 2));
     }
     auto steps = word_steps(s);
-    if (P.ntl > 1) steps.push_back({JK_WCARRY, 0});
+    if (P.ntl > WORD_FUSED_TILES) steps.push_back({JK_WCARRY, 0});
     for (const auto& kv : steps) {
-        CUDA_TRY(launch_word_one(kv.first, kv.second, P, word_ctas(kv.first, s, P.sqr, P.rn), st));
+        CUDA_TRY(launch_word_one(kv.first, kv.second, P, word_ctas(kv.first, s, P.sqr, P.ntl), st));
         g_launches++;
     }
     return pool ? E.pool_release(st) : NBG_OK;
@@ -947,6 +946,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         P.npass = pr->d.npass;
         P.flags = 0;
         P.ntl = (P.rn + UNPACK_TL - 1) / UNPACK_TL;
+        P.tl = UNPACK_TL;
         npass[(size_t)k] = P.npass;
         pmax = std::max(pmax, P.npass);
         bmin = std::min(bmin, bch);
@@ -1177,7 +1177,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     auto put = [&](int step, int kind, int variant, int32_t k, const WordShape& ws, double bytes) {
         WGroup& g = wgroups[std::make_tuple(step, kind, variant)];
         const DProd& P = bb.prods[(size_t)k];
-        const int64_t cpp = word_ctas(kind, ws, P.sqr, P.rn);
+        const int64_t cpp = word_ctas(kind, ws, P.sqr, P.ntl);
         if (g.segs.empty() || g.segs.back().cpp != cpp)
             g.segs.push_back(WSeg{(int32_t)g.nctas, (int32_t)g.plist.size(), (int32_t)cpp, 0});
         g.plist.push_back(k);
@@ -1199,9 +1199,8 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
                 case JK_WMID_FWD: put(pmax - 2, kv.first, kv.second, w.k, w.s, 2 * nop * res); break;
                 case JK_WBLOCK: put(pmax - 1, kv.first, kv.second, w.k, w.s, (nop + 1) * res); break;
                 case JK_WMID_REV: put(pmax, kv.first, kv.second, w.k, w.s, 2 * res); break;
-                case JK_WCOL_REV: put(pmax - 1 + far, kv.first, kv.second, w.k, w.s, 2 * res); break;
                 case JK_WSMALL: put(pmax - 1, kv.first, kv.second, w.k, w.s, in_b + out_b); break;
-                default: put(2 * pmax - 1, kv.first, kv.second, w.k, w.s, res + out_b); break;
+                default: put(pmax - 1 + far, kv.first, kv.second, w.k, w.s, res + out_b); break;  // JK_WTAIL
             }
         }
     }

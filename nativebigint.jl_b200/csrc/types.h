@@ -81,6 +81,7 @@ struct DProd {
     double* xb[2];       // per-prime buffers of operand b (multi-pass products only)
     uint32_t* agg;       // per limb-tile carry aggregates (bit0 generate, bit1 propagate)
     int64_t ntl;         // number of limb tiles
+    int64_t tl;          // limbs per tile
     // word products (word.h; `wN` nonzero): residues of operand a (and the
     // result) and b as one array of wN words per prime, constant tables, shape
     uint32_t* wa;
@@ -216,12 +217,11 @@ enum JobKind : int32_t {
     JK_REV_TMA = 9,  // JK_REV with tiles staged by TMA
     JK_WCOL_FWD = 10,// word products (word.h): limbs to residues and the first levels
     JK_WBLOCK = 11,  // word products: blocks of the remaining levels, leaf products, and back
-    JK_WCOL_REV = 12,// word products: the first levels backwards
-    JK_WUNPACK = 13, // word products: coefficients and carried limbs
+    JK_WTAIL = 12,   // word products: the first levels backwards, coefficients and carried limbs
     JK_WMID_FWD = 14,// word products: a middle column pass
     JK_WMID_REV = 15,// word products: a middle column pass backwards
     JK_WSMALL = 16,  // word products: a whole small product per CTA
-    JK_WCARRY = 17,  // carries between unpack tiles (any product)
+    JK_WCARRY = 17,  // carries between limb tiles (any product)
 };
 
 constexpr int UNPACK_TL = 1024;  // output limbs per unpack tile

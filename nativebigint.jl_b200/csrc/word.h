@@ -46,6 +46,12 @@ struct WordShape {
     bool small = false;  // one CTA per product (at most 3072 values; lj = 0, no column pass)
     int32_t set = 0;     // prime set
 };
+// Limbs of a run of the last pass for R rows in the first one: fewer where R rows
+// of every prime fill the shared memory sooner.
+constexpr int word_run(int R) { return R > 16 ? 64 : 128; }
+// Up to this many tiles a word product's last pass adds the carries between them
+// itself: its limb tiles are followed by two count words.
+constexpr int64_t WORD_FUSED_TILES = 2048;
 // The smallest supported length >= nconv; false when there is none.
 bool word_shape(int64_t nconv, WordShape& s);
 
@@ -65,8 +71,8 @@ cudaError_t launch_word(int kind, int variant, const DProd* prods, const WSeg* s
                         int64_t nctas, cudaStream_t st);
 // The same for one product passed by value (no device tables).
 cudaError_t launch_word_one(int kind, int variant, const DProd& P, int64_t nctas, cudaStream_t st);
-// CTAs one product needs in a word launch.
-int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t rn);
+// CTAs one product needs in a word launch (ntl: its limb tiles).
+int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t ntl);
 
 // Tables of one `odd` for heap sizes up to 2^L: per prime and block, fwd then inverse.
 size_t word_table_bytes(int set, int odd, int L);

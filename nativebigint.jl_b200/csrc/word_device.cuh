@@ -380,6 +380,14 @@ __device__ __forceinline__ uint32_t cta_scan(uint32_t agg, uint32_t* wagg, uint3
     return gp_join(wid ? below : 2u, excl) & 1u;
 }
 
+__device__ __forceinline__ void add_carry(uint64_t* own, uint64_t cin) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        own[q] += cin;
+        cin = cin && own[q] == 0;
+    }
+}
+
 // Limb sums of up to 4 * NT limbs, four per thread, from their coefficients'
 // words lo + mid 2^64 + hi 2^128.  s_mid/s_hi entry 0 and s_c[0]: what reaches
 // the first limb from below (s_c[0] may be written until the first barrier).
@@ -432,14 +440,8 @@ __device__ __forceinline__ uint32_t limb_sums(LimbShared<NT>& S, int t, int nt, 
         agg = g | (prop << 1);
     }
     uint32_t total;
-    uint64_t cin = cta_scan(agg, S.wagg, total);  // carry into the run taken as 0
-    if (in) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            own[q] += cin;
-            cin = cin && own[q] == 0;
-        }
-    }
+    const uint64_t cin = cta_scan(agg, S.wagg, total);  // carry into the run taken as 0
+    if (in) add_carry(own, cin);
     return total;
 }
 

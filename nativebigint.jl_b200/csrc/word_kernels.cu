@@ -7,9 +7,9 @@
 //               the blocks, in registers
 //   k_wblock    per block of M values: the other levels of a and b, the leaf
 //               products, the levels back
-//   k_wcol_rev  the first lj levels and the radix-`odd` step backwards
-//   k_wunpack   five residues -> coefficient (mixed radix), carried limb sums
-//   k_wcarry    carries between unpack tiles
+//   k_wtail     the first lj levels and the radix-`odd` step backwards, residues
+//               -> coefficient (mixed radix), carried limb sums
+//   k_wcarry    carries between the runs of limbs
 //   k_wsmall    a whole product of at most 3072 coefficients in one CTA
 #include <cuda_runtime.h>
 
@@ -268,6 +268,15 @@ struct WArgs {
     DProd one;
 };
 
+// A kernel of a single product may be on the GPU before the one it follows has
+// finished (programmatic launch): nothing that one wrote, and nothing it may
+// still read, is touched before this.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel's CTAs may come once every CTA is here: near the end, so that
+// they spread over the SMs as those empty (from the start of the kernel, the
+// blocks of a 65536 x 65521-limb product piled up: 31 -> 38 us per call).
+__device__ __forceinline__ void let_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+
 __device__ __forceinline__ const DProd& wjob(const WArgs& A, int& local) {
     local = (int)blockIdx.x;
     if (A.nseg == 0) return A.one;
@@ -298,12 +307,14 @@ __global__ void __launch_bounds__(WT, 4) k_wcol_fwd(const __grid_constant__ WArg
     constexpr int R = ODD << LJ, NP = word_np(SET);
     int local;
     const DProd& P = wjob(A, local);
+    wait_previous();
     const int lm = LM ? LM : P.wlm + P.wj2;
     const int id = local * WT + (int)threadIdx.x;
     const int c = id & ((1 << lm) - 1);
     int pi = id >> lm;  // operand-major: a's primes, then b's
     const bool isb = pi >= NP;
     if (isb) pi -= NP;
+    if (A.nseg == 0 && id < 2 && P.ntl <= WORD_FUSED_TILES) P.agg[P.ntl + id] = 0;  // k_wtail's counts of CTAs and of carries
     if (pi >= NP || (isb && P.sqr)) return;
     const int n = (int)(isb ? P.ncb : P.nca);
     const int rows = (n + (1 << lm) - 1) >> lm;
@@ -338,34 +349,7 @@ __global__ void __launch_bounds__(WT, 4) k_wcol_fwd(const __grid_constant__ WArg
         for (int j = 0; j < ODD; j++) wd::tree_fwd<LJ, 1>(x + (j << LJ), tab + ((size_t)j << P.wL), 1u, p);
     }
 #pragma unroll
-    for (int r = 0; r < R; r++) dst[(size_t)r << lm] = x[r];
-}
-
-template <int ODD, int LJ, int LM, int SET>
-__global__ void __launch_bounds__(WT, LM ? 4 : 3) k_wcol_rev(const __grid_constant__ WArgs A) {
-    constexpr int R = ODD << LJ, NP = word_np(SET);
-    int local;
-    const DProd& P = wjob(A, local);
-    const int lm = LM ? LM : P.wlm + P.wj2;
-    const int id = local * WT + (int)threadIdx.x;
-    const int c = id & ((1 << lm) - 1);
-    const int pi = id >> lm;
-    if (pi >= NP) return;
-    uint32_t* __restrict__ dst = P.wa + (size_t)pi * (size_t)P.wN + c;
-    const uint32_t p = c_w[SET].p[pi];
-    uint32_t x[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) x[r] = dst[(size_t)r << lm];
-    const Tw* tab = (const Tw*)P.wti + (((size_t)pi * ODD) << P.wL);
-#pragma unroll
-    for (int j = 0; j < ODD; j++) wd::tree_rev<LJ, 1>(x + (j << LJ), tab + ((size_t)j << P.wL), 1u, p);
-    dft_odd<ODD, LJ, SET>(x, pi, p);
-    // the inverse step is the forward one with output i at -i mod odd
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        const int i = r >> LJ, ri = (ODD - i) % ODD;
-        dst[(size_t)((ri << LJ) + (r & ((1 << LJ) - 1))) << lm] = x[r];
-    }
+    for (int r = 0; r < R; r++) dst[(size_t)r << lm] = x[r];  // no let_next: it cost the batches' passes 4%
 }
 
 // Middle passes: the 2^J rows (2^lm apart) of one column of a segment, the
@@ -401,6 +385,7 @@ __global__ void __launch_bounds__(WT) k_wmid(const __grid_constant__ WArgs A) {
     constexpr int lm = 12;  // more than 32 rows only stand above 4096-value blocks
     int local;
     const DProd& P = wjob(A, local);
+    wait_previous();
     const int id = local * WT + (int)threadIdx.x;
     const MidJob M = mid_job<FWD, SET>(P, id >> lm, J);
     if (!M.live) return;
@@ -410,6 +395,7 @@ __global__ void __launch_bounds__(WT) k_wmid(const __grid_constant__ WArgs A) {
     for (int r = 0; r < (1 << J); r++) x[r] = x0[(size_t)r << lm];
     if (FWD) wd::tree_fwd<J, 1>(x, M.tab, M.node, M.p);
     else wd::tree_rev<J, 1>(x, M.tab, M.node, M.p);
+    let_next();
 #pragma unroll
     for (int r = 0; r < (1 << J); r++) x0[(size_t)r << lm] = x[r];
 }
@@ -425,6 +411,7 @@ __global__ void __launch_bounds__(WT, 4) k_wmid_sm(const __grid_constant__ WArgs
     auto at = [](int i) { return i + ((i >> 8) << 4); };  // rows of 16 words: the two half-warps in distinct banks
     int local;
     const DProd& P = wjob(A, local);
+    wait_previous();
     const MidJob M = mid_job<FWD, SET>(P, local >> J, J);  // 2^J tiles per segment
     if (!M.live) return;                                    // the whole CTA
     const int tid = (int)threadIdx.x, c = tid & (CW - 1), g = tid >> (12 - J);
@@ -475,6 +462,7 @@ __global__ void __launch_bounds__(WT, 4) k_wmid_sm(const __grid_constant__ WArgs
 #pragma unroll
         for (int q = 0; q < NG; q++)
             wd::tree_fwd<K, 1>(x + (q << K), M.tab, (M.node << 4) + (uint32_t)(g + q * (16 / NG)), M.p);
+        let_next();
         inner_io(true);
     } else {
         inner_io(false);
@@ -485,6 +473,7 @@ __global__ void __launch_bounds__(WT, 4) k_wmid_sm(const __grid_constant__ WArgs
         __syncthreads();
         outer_sm(false);
         wd::tree_rev<4, 1>(x, M.tab, M.node, M.p);
+        let_next();
         outer_io(true);
     }
 }
@@ -529,6 +518,7 @@ __device__ __forceinline__ void wblock(const DProd& P, int local, uint32_t* smw)
     }
     if (live) wpoint<LM>(x, x + 16, P.sqr, t, tf, h0, p, pinv);
     wblock_up<LM>(x, sm[g][0], t, (const Tw*)P.wti + toff, h0, p, live);
+    let_next();
     if (live) {
 #pragma unroll
         for (int k = 0; k < 16; k++)
@@ -543,6 +533,7 @@ __global__ void __launch_bounds__(WT, 3) k_wblock(const __grid_constant__ WArgs 
     static_assert(WBlockSmem<10>::words <= WBlockSmem<12>::words && WBlockSmem<8>::words <= WBlockSmem<12>::words, "");
     int local;
     const DProd& P = wjob(A, local);
+    wait_previous();
     if (SET || P.wlm == 12) {
         wblock<12, SET>(P, local, sm);
     } else if constexpr (SET == 0) {
@@ -552,78 +543,20 @@ __global__ void __launch_bounds__(WT, 3) k_wblock(const __grid_constant__ WArgs 
 }
 
 // ---------------------------------------------------------------------------
-// unpack: coefficients and carried limbs, tiles of UNPACK_TL limbs
+// carries between a product's tiles (runs of k_wtail, tiles of the FP64 unpack;
+// P.tl limbs each)
 
-template <int SET>
-__global__ void __launch_bounds__(WT) k_wunpack(const __grid_constant__ WArgs A) {
-    constexpr int NP = word_np(SET);
-    __shared__ LimbShared<WT> S;
-    __shared__ uint64_t h_lo, h_mid2;  // the limb sum below the tile
-    __shared__ uint32_t h_hi3;
-    int tile;
-    const DProd& P = wjob(A, tile);
-    const int t = (int)threadIdx.x;
-    const int N = P.wN;
-    const uint32_t* __restrict__ x = P.wa;
-    const int64_t w0 = (int64_t)tile * UNPACK_TL, w1 = min(w0 + (int64_t)UNPACK_TL, P.rn);
-    uint32_t sc[NP];
-#pragma unroll
-    for (int i = 0; i < NP; i++) sc[i] = P.wsc[i];
-    // the three coefficients before the tile
-    if (t < 3) {
-        const int64_t i = w0 - 1 - t;
-        uint64_t lo = 0, mid = 0;
-        uint32_t hi = 0;
-        if (i >= 0 && i < N) {
-            uint32_t r[NP];
-#pragma unroll
-            for (int k = 0; k < NP; k++) r[k] = x[(size_t)k * N + i];
-            coef_words<SET>(r, sc, lo, mid, hi);
-        }
-        if (t == 0) {
-            h_lo = lo;
-            S.mid[0] = mid;
-            S.hi[0][1] = hi;
-        } else if (t == 1) {
-            h_mid2 = mid;
-            S.hi[0][0] = hi;
-        } else {
-            h_hi3 = hi;
-        }
-        __syncwarp(7u);
-        if (t == 0) {
-            uint64_t s = h_lo + h_mid2;
-            uint32_t c = s < h_mid2;
-            s += h_hi3;
-            c += s < h_hi3;
-            S.c[0] = c;
-        }
-    }
-    const int64_t wt = w0 + 4 * t;
-    uint64_t lo[4] = {0, 0, 0, 0}, mid[4] = {0, 0, 0, 0}, own[4];
-    uint32_t hi[4] = {0, 0, 0, 0};
-    if (wt < N) {  // N is a multiple of 4: all four or none
-        coef4<SET>(reinterpret_cast<const uint4*>(x + wt), N / 4, sc, lo, mid, hi);
-    }
-    const uint32_t tot = limb_sums<WT>(S, t, WT, lo, mid, hi, (int)(w1 - w0), own);
-    store_limbs(P.r, wt, w1, own);
-    if (t == WT - 1) P.agg[tile] = tot;
-}
-
-// Carries between a product's unpack tiles: one warp per 32 tiles.  The carry
-// into its first tile comes from the last lower tile that does not propagate
-// (almost always the one before); a tile's carry stops at its first limb
-// unless that limb is all ones, and then the warp walks the run.  Only r is
-// written, each tile by one warp.
-__global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) {
-    int local;
-    const DProd& P = wjob(A, local);
+// Tiles [k0, k0 + 32) by one warp.  The carry into the first comes from the last
+// lower tile that does not propagate (almost always the one before); a tile's
+// carry stops at its first limb unless that limb is all ones, and then the warp
+// walks the run.  Only r is written, each tile by one warp.  (Reads go to L2:
+// other CTAs of a running kernel may have written what is read.)
+__device__ __forceinline__ void carry_tiles(const DProd& P, int64_t k0) {
     const int lane = (int)threadIdx.x & 31;
-    const int64_t k0 = ((int64_t)local * (WT / 32) + (threadIdx.x >> 5)) * 32, nt = P.ntl;
-    if (k0 >= nt) return;
+    const int64_t nt = P.ntl;
     uint32_t cin = 0;
     for (int64_t k = k0 - 32; k >= 0; k -= 32) {
-        const uint32_t a = P.agg[k + lane];
+        const uint32_t a = __ldcg(P.agg + k + lane);
         const unsigned stop = __ballot_sync(0xffffffffu, !(a & 2u));
         if (stop) {
             cin = __shfl_sync(0xffffffffu, a, 31 - __clz(stop)) & 1u;
@@ -631,7 +564,7 @@ __global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) 
         }
     }
     const int64_t k = k0 + lane;
-    uint32_t incl = k < nt ? P.agg[k] : 0u;
+    uint32_t incl = k < nt ? __ldcg(P.agg + k) : 0u;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
         const uint32_t o = __shfl_up_sync(0xffffffffu, incl, off);
@@ -641,15 +574,16 @@ __global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) 
     if (lane == 0) excl = 2u;
     bool walk = false;
     if (k < nt && (gp_join(cin, excl) & 1u)) {
-        uint64_t* w = P.r + k * UNPACK_TL;
-        if (*w != ~0ULL) *w += 1;
+        uint64_t* w = P.r + k * P.tl;
+        const uint64_t v = __ldcg(w);
+        if (v != ~0ULL) *w = v + 1;
         else walk = true;
     }
     for (unsigned m = __ballot_sync(0xffffffffu, walk); m; m &= m - 1) {
-        const int64_t b0 = (k0 + __ffs(m) - 1) * UNPACK_TL, b1 = min(b0 + (int64_t)UNPACK_TL, P.rn);
+        const int64_t b0 = (k0 + __ffs(m) - 1) * P.tl, b1 = min(b0 + (int64_t)P.tl, P.rn);
         for (int64_t w = b0; w < b1; w += 32) {
             const int64_t wl = w + lane;
-            const uint64_t v = wl < b1 ? P.r[wl] : 0ULL;  // past the tile: stops the run
+            const uint64_t v = wl < b1 ? __ldcg(P.r + wl) : 0ULL;  // past the tile: stops the run
             const unsigned stop = __ballot_sync(0xffffffffu, v != ~0ULL);
             const int e = stop ? __ffs(stop) - 1 : 32;
             if (lane < e) P.r[wl] = 0;
@@ -657,6 +591,181 @@ __global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) 
             if (stop) break;
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// tail: the first levels backwards, coefficients, carried limbs
+
+// A CTA has CW adjacent columns of all R rows and every prime.  Its threads run
+// the columns backwards into shared memory, then a warp (or half of one) takes
+// a row's run of CW consecutive coefficients, four per lane, to limbs.  As two
+// kernels the residues made one more trip through memory (40 of about 70 bytes
+// per coefficient); the arithmetic of the second half hides the loads of
+// another CTA's first half.  The three columns left of the tile are run too:
+// their coefficients reach into its first limbs (in column 0, from the row above).
+template <int ODD, int LJ, int SET>
+struct WTail {
+    static constexpr int R = ODD << LJ, NP = word_np(SET);
+    static constexpr int RUN = word_run(R);               // limbs of a run: a lane has four
+    static constexpr int CW = RUN, W = CW + 4;            // columns: one run; words of a row (4 left of the tile)
+    // a warp per run up to 8 rows, then two runs each; 12 half-warps for the short runs
+    static constexpr int NT = RUN == 64 ? 192 : R <= 8 ? 32 * R : 32 * ((R + 1) / 2);
+    static constexpr int LANES = RUN / 4;                 // lanes of a run
+    static constexpr size_t halo_bytes = ((size_t)R * 3 * 24 + 15) / 16 * 16;  // lo, mid, hi of three coefficients per row
+    static constexpr size_t bytes = halo_bytes + sizeof(uint32_t) * NP * R * W;
+};
+
+// LM as in k_wcol_fwd.
+template <int ODD, int LJ, int LM, int SET>
+__global__ void __launch_bounds__(WTail<ODD, LJ, SET>::NT, 1024 / WTail<ODD, LJ, SET>::NT)
+    k_wtail(const __grid_constant__ WArgs A) {
+    using T = WTail<ODD, LJ, SET>;
+    constexpr int R = T::R, NP = T::NP, W = T::W, LANES = T::LANES;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    struct Halo {
+        uint64_t lo, mid, hi;
+    };
+    Halo* const halo = reinterpret_cast<Halo*>(dyn);
+    uint32_t* const sm = reinterpret_cast<uint32_t*>(dyn + T::halo_bytes);
+    int local;
+    const DProd& P = wjob(A, local);
+    wait_previous();
+    const int tid = (int)threadIdx.x;
+    const int lm = LM ? LM : P.wlm + P.wj2, cols = 1 << lm;
+    const int N = P.wN, c0 = local * T::CW;
+    // columns c0 - 3 .. c0 + CW - 1 of every prime
+    for (int q = tid; q < NP * (T::CW + 3); q += T::NT) {
+        const int pi = q / (T::CW + 3), cc = q - pi * (T::CW + 3) - 3;
+        const bool up = c0 + cc < 0;  // left of column 0: the ends of the rows above
+        const uint32_t* __restrict__ src = P.wa + (size_t)pi * (size_t)N + (c0 + cc + (up ? cols : 0));
+        const uint32_t p = c_w[SET].p[pi];
+        uint32_t x[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) x[r] = src[(size_t)r << lm];
+        const Tw* tab = (const Tw*)P.wti + (((size_t)pi * ODD) << P.wL);
+#pragma unroll
+        for (int j = 0; j < ODD; j++) wd::tree_rev<LJ, 1>(x + (j << LJ), tab + ((size_t)j << P.wL), 1u, p);
+        dft_odd<ODD, LJ, SET>(x, pi, p);
+        // the inverse step is the forward one with output i at -i mod odd
+        uint32_t* d = sm + pi * R * W + 4 + cc;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int row = (((ODD - (r >> LJ)) % ODD) << LJ) + (r & ((1 << LJ) - 1));
+            if (!up) d[row * W] = x[r];
+            else if (row + 1 < R) d[(row + 1) * W] = x[r];
+            else d[0] = 0;  // row 0 has nothing below it
+        }
+    }
+    __syncthreads();
+    uint32_t sc[NP];
+#pragma unroll
+    for (int k = 0; k < NP; k++) sc[k] = P.wsc[k];
+    if (tid < 3 * R) {  // coefficients -1, -2, -3 of each row
+        const int row = tid / 3, j = tid - 3 * row;
+        uint32_t r[NP], hi;
+#pragma unroll
+        for (int k = 0; k < NP; k++) r[k] = sm[(k * R + row) * W + 3 - j];
+        uint64_t lo, mid;
+        coef_words<SET>(r, sc, lo, mid, hi);
+        halo[tid] = Halo{lo, mid, hi};
+    }
+    __syncthreads();
+    const int lane = tid & (LANES - 1);
+    const int64_t rn = P.rn;
+    const bool fused = A.nseg == 0 && P.ntl <= WORD_FUSED_TILES;
+    for (int row = tid / LANES; row < R; row += T::NT / LANES) {
+        // what reaches lane 0's first limbs: mid and hi words of the quad below and its last carry
+        uint64_t in_mid = halo[3 * row].mid;
+        uint32_t in_hi3 = (uint32_t)halo[3 * row].hi, in_hi2 = (uint32_t)halo[3 * row + 1].hi, in_c;
+        {
+            const uint64_t m = halo[3 * row + 1].mid, h = halo[3 * row + 2].hi;
+            uint64_t s = halo[3 * row].lo + m;
+            in_c = s < m;
+            s += h;
+            in_c += s < h;
+        }
+        uint64_t lo[4], mid[4], own[4];
+        uint32_t hi[4], cy[4];
+        coef4<SET>(reinterpret_cast<const uint4*>(sm + row * W + 4 + 4 * lane), R * W / 4, sc, lo, mid,
+                   hi);
+        auto sum = [&](int q, uint64_t m, uint32_t h) {
+            uint64_t s = lo[q] + m;
+            uint32_t c = s < m;
+            s += h;
+            c += s < h;
+            own[q] = s;
+            cy[q] = c;
+        };
+        sum(2, mid[1], hi[0]);
+        sum(3, mid[2], hi[1]);
+        uint64_t pm = __shfl_up_sync(0xffffffffu, mid[3], 1, LANES);
+        uint32_t ph2 = __shfl_up_sync(0xffffffffu, hi[2], 1, LANES), ph3 = __shfl_up_sync(0xffffffffu, hi[3], 1, LANES);
+        uint32_t pc = __shfl_up_sync(0xffffffffu, cy[3], 1, LANES);
+        if (lane == 0) {
+            pm = in_mid;
+            ph2 = in_hi2;
+            ph3 = in_hi3;
+            pc = in_c;
+        }
+        in_mid = __shfl_sync(0xffffffffu, mid[3], LANES - 1, LANES);
+        in_hi2 = __shfl_sync(0xffffffffu, hi[2], LANES - 1, LANES);
+        in_hi3 = __shfl_sync(0xffffffffu, hi[3], LANES - 1, LANES);
+        in_c = __shfl_sync(0xffffffffu, cy[3], LANES - 1, LANES);
+        sum(0, pm, ph2);
+        sum(1, mid[0], ph3);
+        const int64_t wr = (int64_t)row * cols + c0, wt = wr + 4 * lane;
+        uint32_t k = pc, gen = 0, prop = 1;  // carry of the sum below; carry of adding it
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint64_t s = own[q] + k + gen;  // k + gen <= 3
+            gen = s < (uint64_t)(k + gen);
+            own[q] = s;
+            k = cy[q];
+            prop &= (wt + q < rn && s == ~0ULL) ? 1u : 0u;
+        }
+        uint32_t incl = gen | (prop << 1);
+#pragma unroll
+        for (int off = 1; off < LANES; off <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, incl, off, LANES);
+            if (lane >= off) incl = gp_join(o, incl);
+        }
+        const uint32_t below = __shfl_up_sync(0xffffffffu, incl, 1, LANES);
+        add_carry(own, lane ? below & 1u : 0u);  // carry into the run taken as 0, added later
+        store_limbs(P.r, wt, rn, own);
+        if (lane == LANES - 1 && wr < rn) {
+            P.agg[wr / T::RUN] = incl;
+            if (fused && (incl & 1u)) atomicAdd(P.agg + P.ntl + 1, 1u);
+            if (wr + T::RUN == N && rn > N) {  // limb N: the last coefficients' upper words
+                P.r[N] = in_mid + in_hi2 + in_c;
+                P.agg[N / T::RUN] = 0;
+            }
+        }
+    }
+    let_next();
+    // limbs above the operands' magnitudes
+    for (int64_t i = (int64_t)N + 1 + (int64_t)local * T::NT + tid; i < rn; i += (int64_t)(cols / T::CW) * T::NT) P.r[i] = 0;
+    if (!fused) return;
+    // few runs: the product's last CTA carries between them instead of another
+    // launch, and only if some run carries out at all (a limb sum within 3 of
+    // 2^64, so hardly ever but for operands made of ones or zeros)
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+        last = atomicAdd(P.agg + P.ntl, 1u) == (uint32_t)(cols / T::CW - 1);
+        __threadfence();
+    }
+    __syncthreads();
+    if (last && __ldcg(P.agg + P.ntl + 1) != 0)
+        for (int64_t k0 = 32 * (tid >> 5); k0 < P.ntl; k0 += 32 * (T::NT / 32)) carry_tiles(P, k0);
+}
+
+__global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) {
+    int local;
+    const DProd& P = wjob(A, local);
+    wait_previous();
+    const int64_t k0 = ((int64_t)local * (WT / 32) + (threadIdx.x >> 5)) * 32;
+    if (k0 < P.ntl) carry_tiles(P, k0);
 }
 
 // ---------------------------------------------------------------------------
@@ -675,6 +784,7 @@ __global__ void __launch_bounds__(WSmall<ODD, LM>::NT, WSmall<ODD, LM>::NT > 320
     const DProd& P = wjob(A, local);
     const int tid = (int)threadIdx.x;
     const SmallThread<ODD, LM> th(sm, P.wtf, P.wti, P.wL);
+    wait_previous();
     uint32_t x[32];  // a's 16 values, then b's
     const uint64_t *__restrict__ pa = P.a, *__restrict__ pb = P.b;
     th.load(x, th.sp, (int)P.nca, [&](int i) { return __ldg(pa + i); });
@@ -699,6 +809,7 @@ __global__ void __launch_bounds__(WSmall<ODD, LM>::NT, WSmall<ODD, LM>::NT > 320
     SmallThread<ODD, LM>::coefs(sm, P.wsc, lo, mid, hi);
     const int rn = (int)P.rn, top = min(rn, 4 * W::LT);
     limb_sums<W::LT>(S, tid, W::LT, lo, mid, hi, top, own);
+    let_next();
     if (tid < W::LT) store_limbs(P.r, 4 * tid, top, own);
     for (int i = top + tid; i < rn; i += W::NT) P.r[i] = 0;  // limbs above the operands' magnitudes
 }
@@ -706,19 +817,18 @@ __global__ void __launch_bounds__(WSmall<ODD, LM>::NT, WSmall<ODD, LM>::NT > 320
 // ---------------------------------------------------------------------------
 // launches
 
-int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t rn) {
+int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t ntl) {
     const int64_t M = int64_t(1) << s.lm, R = (int64_t)s.odd << s.lj;
     const int64_t cols = M << s.j2, mthreads = (int64_t)s.N >> (s.j2 > 5 ? 4 : s.j2), np = word_np(s.set);
-    const int64_t tiles = (rn + UNPACK_TL - 1) / UNPACK_TL;
+    const int R1 = s.odd << (s.lj - s.j2);
     switch (kind) {
         case JK_WCOL_FWD: return ((sqr ? 1 : 2) * np * cols + WT - 1) / WT;
-        case JK_WCOL_REV: return (np * cols + WT - 1) / WT;
         case JK_WMID_FWD: return ((sqr ? 1 : 2) * np * mthreads + WT - 1) / WT;
         case JK_WMID_REV: return (np * mthreads + WT - 1) / WT;
         case JK_WBLOCK: return (np * R * (M / 16) + WT - 1) / WT;
         case JK_WSMALL: return 1;
-        case JK_WCARRY: return (tiles + WT - 1) / WT;  // 8 warps of 32 tiles
-        default: return tiles;
+        case JK_WCARRY: return (ntl + WT - 1) / WT;  // 8 warps of 32 tiles
+        default: return cols / word_run(R1);  // JK_WTAIL
     }
 }
 
@@ -733,12 +843,17 @@ template <int ODD, int LM>
 static WLaunch small_kernel() {
     return WLaunch{k_wsmall<ODD, LM>, WSmall<ODD, LM>::NT, WSmall<ODD, LM>::bytes};
 }
+template <int ODD, int LJ, int LM, int SET>
+static WLaunch tail_kernel() {
+    using T = WTail<ODD, LJ, SET>;
+    return WLaunch{k_wtail<ODD, LJ, LM, SET>, T::NT, T::bytes};
+}
 template <int ODD, int LJ>
 static WLaunch col_kernel(int kind, bool lm12) {
-    if (lm12) return WLaunch{kind == JK_WCOL_FWD ? k_wcol_fwd<ODD, LJ, 12, 0> : k_wcol_rev<ODD, LJ, 12, 0>, WT, 0};
+    if (lm12) return kind == JK_WCOL_FWD ? WLaunch{k_wcol_fwd<ODD, LJ, 12, 0>, WT, 0} : tail_kernel<ODD, LJ, 12, 0>();
     // no supported length has these rows above other column counts
     if constexpr ((ODD == 1 && (LJ == 1 || LJ == 5)) || (ODD == 3 && LJ == 0)) return WLaunch{nullptr, 0, 0};
-    else return WLaunch{kind == JK_WCOL_FWD ? k_wcol_fwd<ODD, LJ, 0, 0> : k_wcol_rev<ODD, LJ, 0, 0>, WT, 0};
+    else return kind == JK_WCOL_FWD ? WLaunch{k_wcol_fwd<ODD, LJ, 0, 0>, WT, 0} : tail_kernel<ODD, LJ, 0, 0>();
 }
 template <int J>
 static WLaunch mid_kernel(int kind) {
@@ -754,9 +869,8 @@ template <int SET, int ODD, int LJ>
 static WLaunch big_kernel(int kind, int variant) {
     switch (kind) {
         case JK_WCOL_FWD: return WLaunch{k_wcol_fwd<ODD, LJ, 0, SET>, WT, 0};
-        case JK_WCOL_REV: return WLaunch{k_wcol_rev<ODD, LJ, 0, SET>, WT, 0};
+        case JK_WTAIL: return tail_kernel<ODD, LJ, 0, SET>();
         case JK_WBLOCK: return WLaunch{k_wblock<SET>, WT, 0};
-        case JK_WUNPACK: return WLaunch{k_wunpack<SET>, WT, 0};
         case JK_WMID_FWD:
         case JK_WMID_REV:
             switch (variant) {
@@ -774,10 +888,9 @@ static WLaunch word_kernel(int kind, int variant) {
     if (variant >> 20 == 1) return big_kernel<1, 3, 3>(kind, variant & 0xfffff);
     if (variant >> 20 == 2) return big_kernel<2, 1, 5>(kind, variant & 0xfffff);
     switch (kind) {
-        case JK_WUNPACK: return WLaunch{k_wunpack<0>, WT, 0};
         case JK_WBLOCK: return WLaunch{k_wblock<0>, WT, 0};
         case JK_WCOL_FWD:
-        case JK_WCOL_REV:  // one kernel per row count: a switch inside one kernel took 25% longer (registers)
+        case JK_WTAIL:  // one kernel per row count: a switch inside one kernel took 25% longer (registers)
             switch (variant & 0xffff) {
 #define NBG_COL(O, J) \
     case (O << 8) | J: return col_kernel<O, J>(kind, variant >> 16);
@@ -812,14 +925,21 @@ static WLaunch word_kernel(int kind, int variant) {
     return WLaunch{nullptr, 0, 0};
 }
 
+// Raises the dynamic shared-memory limit of every kernel above the default.
 static cudaError_t small_attributes() {
     cudaError_t e = cudaSuccess;
-#define NBG_SMALL(O, M)                                                                                     \
-    if (e == cudaSuccess)                                                                                   \
-        e = cudaFuncSetAttribute(k_wsmall<O, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,               \
-                                 (int)WSmall<O, M>::bytes);
+    auto raise = [&](const WLaunch& l) {
+        if (e == cudaSuccess && l.fn && l.smem > 0)
+            e = cudaFuncSetAttribute(l.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem);
+    };
+#define NBG_SMALL(O, M) raise(small_kernel<O, M>());
     NBG_SMALLS
 #undef NBG_SMALL
+    for (int odd : {1, 3, 5, 7})
+        for (int lj = 0; lj <= 5; lj++)
+            for (int l12 = 0; l12 < 2; l12++) raise(word_kernel(JK_WTAIL, l12 << 16 | odd << 8 | lj));
+    raise(word_kernel(JK_WTAIL, 1 << 20));
+    raise(word_kernel(JK_WTAIL, 2 << 20));
     return e;
 }
 
@@ -827,6 +947,19 @@ static cudaError_t launch(int kind, int variant, const WArgs& a, int64_t nctas, 
     if (nctas <= 0) return cudaSuccess;
     const WLaunch k = word_kernel(kind, variant);
     if (!k.fn || nctas > 0x7fffffff) return cudaErrorInvalidValue;
+    if (a.nseg == 0) {  // one product: its short kernels start while the one before drains
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)nctas);
+        cfg.blockDim = dim3((unsigned)k.threads);
+        cfg.dynamicSmemBytes = k.smem;
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, k.fn, a);
+    }
     k.fn<<<(unsigned)nctas, k.threads, k.smem, st>>>(a);
     return cudaGetLastError();
 }

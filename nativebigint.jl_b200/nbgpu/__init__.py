@@ -356,8 +356,8 @@ class Batch:
         byt = (ctypes.c_double * n)()
         _check(lib().nbg_batch_stats(self._h, kinds, njobs, ops, byt, n))
         names = {0: "k_fwd", 1: "k_pwr", 2: "k_rev", 3: "k_unpack", 4: "k_carry", 5: "k_carry_fix", 6: "k_pwr",
-                 7: "k_pwr", 8: "k_col_tma_fwd", 9: "k_col_tma_rev", 10: "k_wcol_fwd", 11: "k_wblock", 12: "k_wcol_rev",
-                 13: "k_wunpack", 14: "k_wmid_fwd", 15: "k_wmid_rev", 16: "k_wsmall", 17: "k_wcarry"}
+                 7: "k_pwr", 8: "k_col_tma_fwd", 9: "k_col_tma_rev", 10: "k_wcol_fwd", 11: "k_wblock", 12: "k_wtail",
+                 14: "k_wmid_fwd", 15: "k_wmid_rev", 16: "k_wsmall", 17: "k_wcarry"}
         return [dict(kind=names[kinds[i]], code=kinds[i], jobs=njobs[i], alg_ops=ops[i], alg_bytes=byt[i])
                 for i in range(n)]
 

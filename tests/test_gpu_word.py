@@ -58,7 +58,7 @@ def test_word_kernels_run_and_edge_operands(gpu_lib):
     rng = np.random.default_rng(77)
     a, b = rand_limbs(rng, 3000), rand_limbs(rng, 2500)
     assert "k_wsmall" in _kinds(gpu_lib, a[:200].copy(), b[:100].copy())
-    assert "k_wunpack" in _kinds(gpu_lib, a, b) and "k_wunpack" in _kinds(gpu_lib, a, None)
+    assert "k_wtail" in _kinds(gpu_lib, a, b) and "k_wtail" in _kinds(gpu_lib, a, None)
     for m, n in ((1, 1), (2, 1), (700, 1), (513, 512), (65536, 65537), (130000, 3)):
         x, y = adversarial(rng, m), adversarial(rng, n)
         assert np.array_equal(gpu_lib.mul(x, y), _want(x, y))
@@ -81,7 +81,7 @@ def test_word_batch_equals_fp64_passes(gpu_lib):
         t = json.loads(old)
         t["cmax"] = 64  # pass knobs other than the loaded ones: the FP64 passes
         gpu_lib.set_tuning(json.dumps(t))
-        assert "k_wunpack" not in _kinds(gpu_lib, *pairs[1])
+        assert "k_wtail" not in _kinds(gpu_lib, *pairs[1])
         ref = gpu_lib.mul_batch(pairs)
     finally:
         gpu_lib.set_tuning(old)
@@ -172,3 +172,24 @@ def test_calls_on_several_streams_share_the_workspace(gpu_lib):
     torch.cuda.synchronize()
     for a, b, r in jobs:
         assert np.array_equal(r.cpu().numpy(), _want(a, b))
+
+
+@pytest.mark.parametrize("n", [1700, 4096, 9000, 33000, 65536, 66000, 300000])
+def test_carries_between_runs(gpu_lib, n):
+    # limb sums that overflow and runs of all-ones limbs across many runs, alone
+    # (the last pass carries up to 2048 runs itself) and in a batch (a launch does)
+    rng = np.random.default_rng(n)
+    ones = np.full(n, 2**64 - 1, dtype=np.uint64)
+    two = np.zeros(n, dtype=np.uint64)
+    two[0] = two[n // 2] = 1
+    ends = np.zeros(n, dtype=np.uint64)
+    ends[0], ends[-1] = 2**64 - 1, 1 << 63
+    third = np.zeros(n // 3 + 1, dtype=np.uint64)
+    third[0] = third[-1] = 1
+    pairs = [(ones, None), (two, ones), (ends, ones), (ends, None), (ones, third),
+             (adversarial(rng, n), adversarial(rng, 2 * n // 3))]
+    batch = gpu_lib.mul_batch(pairs)
+    for (a, b), g in zip(pairs, batch):
+        want = _want(a, b)
+        assert np.array_equal(gpu_lib.sqr(a) if b is None else gpu_lib.mul(a, b), want)
+        assert np.array_equal(g, want)
