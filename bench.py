@@ -12,8 +12,9 @@ Printed JSON line (rank 0):
   value     output limbs/s, batch replay with operands resident in HBM
   e2e       same metric through nbg_mul_batch (host buffers; H2D + D2H inside)
   unbatched the same products issued one per call (nbg_mul_batch_dev, count 1)
-  roofline  dominant kernel's algorithmic FP64 instructions / its measured
-            duration, against the FP64 issue rate measured in this run
+  roofline  dominant kernel's algorithmic instructions (32-bit multiply slots
+            of the 30-bit-prime kernels, FP64 instructions of the others) / its
+            measured duration, against the issue rate measured in this run
   cpu_baseline  the CPU oracle (restatement of the reference) on the host cores
 
 --impl reference times the reference's CPU algorithm (the oracle port; Julia
@@ -224,7 +225,20 @@ def fp64_peak() -> dict:
     rc = L.nbgpeak_fp64(torch.cuda.current_device(), ctypes.byref(fma), ctypes.byref(add))
     if rc:
         raise RuntimeError("fp64 peak probe failed")
-    return {"dfma_per_s": fma.value, "dadd_per_s": add.value}
+    imad = ctypes.c_double()
+    L.nbgpeak_imad.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_double)]
+    if L.nbgpeak_imad(torch.cuda.current_device(), ctypes.byref(imad)):
+        raise RuntimeError("integer multiply peak probe failed")
+    return {"dfma_per_s": fma.value, "dadd_per_s": add.value, "imad_per_s": imad.value}
+
+
+def kernel_peak(kernel: str, peak: dict) -> tuple[float, str, str]:
+    """(instructions/s, bound, unit) that a kernel's algorithmic operations are
+    held against: the 30-bit-prime kernels (k_w...) run on the 32-bit multiply
+    pipe, the others on the FP64 cores."""
+    if kernel.startswith("k_w"):
+        return peak["imad_per_s"], "int32 multiply", "T multiply slots/s"
+    return peak["dfma_per_s"], "fp64", "T FP64 instr/s"
 
 
 def rank_share(W: dict, rank: int, world: int, scaling: str, params) -> list[int]:
@@ -263,14 +277,18 @@ def hbm_peak() -> tuple[float, str]:
     return 6650.0, "fallback: 6.65 TB/s (MEASURED_PEAKS.json absent)"
 
 
-def traffic_from_profiles(kernel: str, point_primes: float):
-    """DRAM bytes of `kernel` for one batch: the committed ncu measurement of
-    bytes per transform point per prime (profiles/ncu_traffic.json, taken on
-    the 105*2^11-point class) times this batch's points x primes."""
+def traffic_from_profiles(kernel: str, point_primes: float, out_limbs: float = 0.0):
+    """DRAM bytes of `kernel` for one batch: the committed ncu measurement
+    (profiles/ncu_traffic.json) of bytes per transform point per prime times
+    this batch's points x primes, or, for the 30-bit-prime kernels, of bytes per
+    output limb times its output limbs."""
     path = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     try:
         with open(path) as f:
             d = json.load(f)
+        bpl = d.get("per_output_limb", {}).get("kernels", {}).get(kernel)
+        if bpl is not None:
+            return float(bpl) * out_limbs
         bpp = d.get("kernels", {}).get(kernel)
         return None if bpp is None else float(bpp) * point_primes
     except (OSError, ValueError):
@@ -376,15 +394,16 @@ def run_ours(args, rank: int, world: int) -> None:
         peak = fp64_peak()
         hbm_gbs, hbm_src = hbm_peak()
         achieved = D["ops"] / (D["ms"] / 1e3) / 1e12
-        pk = peak["dfma_per_s"] / 1e12
+        pk, bound, unit = kernel_peak(dom, peak)
+        pk /= 1e12
         tot_ops = sum(st_["alg_ops"] for st_ in stats)
         roof = {
-            "bound": "fp64", "kernel": dom, "achieved": achieved, "peak": pk, "unit": "T FP64 instr/s",
-            "frac": achieved / pk, "traffic": traffic_from_profiles(dom, point_primes),
+            "bound": bound, "kernel": dom, "achieved": achieved, "peak": pk, "unit": unit,
+            "frac": achieved / pk, "traffic": traffic_from_profiles(dom, point_primes, out_limbs),
             "per": "one batch: all launches of the kernel in one step (launches are grouped by shared-memory size)",
-            "peak_source": "measured: DFMA issue rate of libnbgpu_peak.so in this run (MEASURED_PEAKS.json has no FP64 figure)",
+            "peak_source": "measured: issue rate of libnbgpu_peak.so in this run (MEASURED_PEAKS.json has no such figure)",
             "alg_ops": D["ops"], "ms": D["ms"], "launches": D["launches"],
-            "traffic_source": "profiles/ncu_traffic.json bytes per point per prime x this batch's points",
+            "traffic_source": "profiles/ncu_traffic.json bytes per output limb (or point per prime) x this batch's",
             "hbm": {"alg_bytes": D["bytes"],
                     "achieved_gbs": D["bytes"] / (D["ms"] / 1e3) / 1e9, "peak_gbs": hbm_gbs,
                     "peak_source": hbm_src},
@@ -473,7 +492,7 @@ def run_ours(args, rank: int, world: int) -> None:
 
         single_2p24 = None
         if args.single_2p24:
-            single_2p24 = single_case(24, True, "uniform", max(20, args.steps), peak["dfma_per_s"], stream,
+            single_2p24 = single_case(24, True, "uniform", max(20, args.steps), peak, stream,
                                       check="residues")
         clocks = clk.summary()
         med = statistics.median(step_ms)
@@ -804,15 +823,15 @@ def residues_agree(a: np.ndarray, b: np.ndarray | None, r: np.ndarray) -> bool:
     return all((A % q) * (B % q) % q == R % q for q in RESIDUE_MODULI)
 
 
-def single_case(lg: int, sq: bool, kind: str, reps: int, peak: float, s, check: str = "gmp",
+def single_case(lg: int, sq: bool, kind: str, reps: int, peak: dict, s, check: str = "gmp",
                 gmp_time: bool = False) -> dict:
     """One balanced 2^lg-limb product or square on the plain one-per-call
     device path (nbg_mul_dev / nbg_sqr_dev: plan lookup, job build, launches)
     and as a captured one-product batch (graph replay).  3 warm-up calls, then
     `reps` timed ones, each by CUDA events on stream `s`; SM clocks sampled
-    during the graph replays.  Roofline: the reference schedule's FP64
-    instructions / p50 time, against `peak` (the DFMA issue rate measured in
-    this run) and against 148 SMs x 64 DFMA per clock x the sampled clock.
+    during the graph replays.  Roofline: the algorithm's multiply slots (or
+    FP64 instructions) / p50 time, against the issue rate measured in this run
+    (`peak`) and against 148 SMs x 64 per clock x the sampled clock.
     check: "gmp" compares with mpn_mul / mpn_sqr, "residues" with four
     residues (see residues_agree)."""
     import torch
@@ -861,8 +880,9 @@ def single_case(lg: int, sq: bool, kind: str, reps: int, peak: float, s, check: 
         d["ms"] += ms
         d["alg_ops"] += st_["alg_ops"]
         d["launches"] += 1
-    for d in per_kernel.values():
-        d["frac"] = d["alg_ops"] / (d["ms"] / 1e3) / peak if d["ms"] else 0.0
+    for k, d in per_kernel.items():
+        d["frac"] = d["alg_ops"] / (d["ms"] / 1e3) / kernel_peak(k, peak)[0] if d["ms"] else 0.0
+    peak, bound, unit = kernel_peak(max(per_kernel, key=lambda k: per_kernel[k]["ms"]), peak)
     bt.close()
     got = r.cpu().numpy()
     if check == "gmp":
@@ -891,11 +911,11 @@ def single_case(lg: int, sq: bool, kind: str, reps: int, peak: float, s, check: 
         "per_call_p50_ms": float(np.percentile(t_call, 50)), "per_call_p99_ms": float(np.percentile(t_call, 99)),
         "graph_p50_ms": p50g, "graph_p99_ms": float(np.percentile(t_graph, 99)),
         "output_limbs_per_s": 2 * n / (p50g / 1e3),
-        "roofline": {"bound": "fp64", "alg_ops": alg, "achieved": alg / (p50g / 1e3) / 1e12,
-                     "peak": peak / 1e12, "unit": "T FP64 instr/s", "frac": alg / (p50g / 1e3) / peak,
-                     "peak_source": "measured: DFMA issue rate of libnbgpu_peak.so in this run",
+        "roofline": {"bound": bound, "alg_ops": alg, "achieved": alg / (p50g / 1e3) / 1e12,
+                     "peak": peak / 1e12, "unit": unit, "frac": alg / (p50g / 1e3) / peak,
+                     "peak_source": "measured: issue rate of libnbgpu_peak.so in this run",
                      "frac_of_nominal": alg / (p50g / 1e3) / nominal if nominal else None,
-                     "nominal_source": "148 SMs x 64 DFMA/clock x median sampled SM clock",
+                     "nominal_source": "148 SMs x 64 instructions/clock x median sampled SM clock",
                      "kernels": per_kernel},
         "check": {"kind": check, "ok": ok},
         "clocks": clocks,
@@ -916,7 +936,7 @@ def run_single(args) -> None:
 
     torch.cuda.set_device(0)
     nbgpu._check(nbgpu.lib().nbg_init(0))
-    peak = fp64_peak()["dfma_per_s"]
+    peak = fp64_peak()
     s = torch.cuda.Stream()
     reps = max(20, args.steps)
     lgs = [int(x) for x in args.single_sizes.split(",")]

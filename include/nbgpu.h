@@ -119,7 +119,8 @@ int nbg_batch_destroy(nbg_batch *bt);
  * primes, see nbg_set_tuning: 10 forward column passes, 11 blocks, 12 reverse
  * column passes with the limbs, 14 and 15 middle column passes, 16 whole small
  * products, 17 carries), jobs, and the
- * algorithmic FP64 instruction count (zero for kinds above 9) and compulsory
+ * algorithmic FP64 instruction count (kinds above 9: 32-bit multiply-pipe
+ * slots, a high or wide multiply counting two) and compulsory
  * bytes of the reference schedule for that launch.  Any output pointer may be
  * NULL. */
 int nbg_batch_stats(const nbg_batch *bt, int32_t *kinds, int64_t *njobs, double *alg_ops, double *alg_bytes,

@@ -862,6 +862,26 @@ size_t word_work_bytes(const ProdIn& q, const WordShape& s) {
     return word_op_bytes(s) * (q.sqr ? 1 : 2) + sizeof(uint32_t) * (size_t)(s.N / 64 + 3);  // runs of 64 limbs or more, two counts
 }
 
+// Multiply-pipe slots of one product's launch that the algorithm needs: a low
+// 32-bit multiply is one, a high or wide one two (it issues at half the rate).
+// A butterfly or a product with a constant takes 4, a Montgomery reduction 3.
+static double word_ops(int kind, const WordShape& s, const DProd& P) {
+    const double N = s.N, np = word_np(s.set), nop = P.sqr ? 1 : 2;
+    const double odd = s.odd == 3 ? 4 / 3.0 : s.odd == 5 ? 24 / 5.0 : s.odd == 7 ? (18 * 2 + 6 * 3) / 7.0 : 0;
+    const double rows = 2.0 * (s.lj - s.j2) + odd, pack = 8.0 * np * (double)(P.nca + (P.sqr ? 0 : P.ncb));
+    const double leaf = (19 * 2 + 7 * 3) / 4.0, inner = 2.0 * (s.lm - 2);  // per value
+    const double coef = 2.0 * (np * (np + 1) / 2 + np * (np - 1) / 2) + 3 * np;
+    switch (kind) {
+        case JK_WCOL_FWD: return pack + nop * np * N * rows;
+        case JK_WMID_FWD: return nop * np * N * 2.0 * s.j2;
+        case JK_WMID_REV: return np * N * 2.0 * s.j2;
+        case JK_WBLOCK: return np * N * ((nop + 1) * inner + leaf);
+        case JK_WSMALL: return pack + np * N * ((nop + 1) * (rows + inner) + leaf) + N * coef;
+        case JK_WTAIL: return np * N * rows + N * coef;
+        default: return 0;
+    }
+}
+
 int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, char* work, cudaStream_t st) {
     DProd P;
     int rc = word_setup(E, q, s, P);
@@ -1171,7 +1191,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         std::vector<WSeg> segs;
         std::vector<int32_t> plist;
         int64_t nctas = 0;
-        double bytes = 0;
+        double bytes = 0, ops = 0;
     };
     std::map<std::tuple<int, int, int>, WGroup> wgroups;  // step, kind, variant
     auto put = [&](int step, int kind, int variant, int32_t k, const WordShape& ws, double bytes) {
@@ -1183,6 +1203,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         g.plist.push_back(k);
         g.nctas += cpp;
         g.bytes += bytes;
+        g.ops += word_ops(kind, ws, P);
     };
     std::stable_sort(words.begin(), words.end(), [&](const WordProd& x, const WordProd& y) {
         return x.s.N != y.s.N ? x.s.N > y.s.N : bb.prods[(size_t)x.k].sqr < bb.prods[(size_t)y.k].sqr;
@@ -1238,6 +1259,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         L.odd = false;
         L.step = std::get<0>(kv.first);
         L.variant = std::get<2>(kv.first);
+        L.alg_ops = g.ops;
         L.alg_bytes = g.bytes;
         L.mode = JM_WORD;
         L.nseg = (int)g.segs.size();

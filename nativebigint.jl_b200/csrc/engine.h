@@ -158,7 +158,7 @@ struct Launch {
     int variant = 0;       // word launches (JM_WORD): kernel variant; n counts CTAs
     int step = 0;          // pipeline step: launches of one step are independent
     bool odd = true;       // some pass of the launch holds a radix-3/5/7 stage
-    double alg_ops = 0;    // FP64 instructions of the reference schedule done by this launch
+    double alg_ops = 0;    // FP64 instructions of the reference schedule (word launches: multiply slots) done by this launch
     double alg_bytes = 0;  // compulsory global bytes (operand/limb reads, tile loads and stores)
 };
 
