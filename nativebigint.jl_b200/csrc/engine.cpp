@@ -805,10 +805,10 @@ size_t fp64_work_bytes(const ProdIn& q) {
     return sizeof(double) * 2 * (size_t)N * (q.sqr ? 1 : 2);
 }
 
-bool word_product(const Engine& E, const ProdIn& q, WordShape* s) {
+bool word_product(const Engine& E, const ProdIn& q, WordShape* s, bool coarse) {
     if (!E.word_ok || q.fp64 || q.keep_b) return false;
     const int64_t la = eff_limbs(q.m, q.bits_a), lb = q.sqr ? la : eff_limbs(q.n, q.bits_b);
-    return word_shape(la + lb - 1, *s) && (s->set || std::min(la, lb) <= WORD_MIN_OPERAND_MAX);
+    return word_shape(la + lb - 1, *s, coarse) && (s->set || std::min(la, lb) <= WORD_MIN_OPERAND_MAX);
 }
 
 int word_setup(Engine& E, const ProdIn& q, const WordShape& s, DProd& P) {
@@ -919,6 +919,14 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         WordShape s;
     };
     std::vector<WordProd> words;  // products of the word engine
+    // Small batches of some dozens of products take few transform lengths: their
+    // launches are short, and a launch costs the host about 5 us (256 products,
+    // 4.7M limbs: 59 launches, 599 us, against 32 launches, 536 us).  Large ones
+    // take every length (10,000 products, 185M limbs: 12.2 ms against 12.9).
+    constexpr int64_t COARSE_LIMBS = int64_t(1) << 24;
+    int64_t out_limbs = 0;
+    for (int64_t k = 0; k < count && out_limbs < COARSE_LIMBS; k++) out_limbs += in[k].m + (in[k].sqr ? in[k].m : in[k].n);
+    const bool coarse = count >= 24 && out_limbs < COARSE_LIMBS;
     std::vector<size_t> xa_off((size_t)count), xb_off((size_t)count), agg_off((size_t)count);
     for (int64_t k = 0; k < count; k++) {
         const ProdIn& q = in[k];
@@ -930,7 +938,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         if (q.bits_a < 1 || q.bits_a > 64 * q.m || (!q.sqr && (q.bits_b < 1 || q.bits_b > 64 * q.n)))
             return fail(NBG_EINVAL, "product %lld: magnitude bits out of range (zero operand?)", (long long)k);
         WordShape ws;
-        if (word_product(E, q, &ws)) {
+        if (word_product(E, q, &ws, coarse)) {
             int rc = word_setup(E, q, ws, P);
             if (rc) return rc;
             agg_off[(size_t)k] = aggw;
@@ -1194,8 +1202,7 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         double bytes = 0, ops = 0;
     };
     std::map<std::tuple<int, int, int>, WGroup> wgroups;  // step, kind, variant
-    auto put = [&](int step, int kind, int variant, int32_t k, const WordShape& ws, double bytes) {
-        WGroup& g = wgroups[std::make_tuple(step, kind, variant)];
+    auto add = [&](WGroup& g, int kind, int32_t k, const WordShape& ws, double bytes) {
         const DProd& P = bb.prods[(size_t)k];
         const int64_t cpp = word_ctas(kind, ws, P.sqr, P.ntl);
         if (g.segs.empty() || g.segs.back().cpp != cpp)
@@ -1208,26 +1215,44 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
     std::stable_sort(words.begin(), words.end(), [&](const WordProd& x, const WordProd& y) {
         return x.s.N != y.s.N ? x.s.N > y.s.N : bb.prods[(size_t)x.k].sqr < bb.prods[(size_t)y.k].sqr;
     });
-    for (const WordProd& w : words) {
+    std::vector<std::pair<WGroup*, int>> steps;  // of the run of equal shapes: launch and kind
+    WGroup* carry = nullptr;
+    for (size_t i = 0; i < words.size(); i++) {
+        const WordProd& w = words[i];
         const DProd& P = bb.prods[(size_t)w.k];
-        const double res = 4.0 * word_np(w.s.set) * P.wN, nop = P.sqr ? 1 : 2;
-        const double in_b = 8.0 * (double)(P.nca + (P.sqr ? 0 : P.ncb)), out_b = 8.0 * (double)P.rn;
-        for (const auto& kv : word_steps(w.s)) {
-            // the block step is pmax - 1, a middle column pass takes the steps next to it
-            const int far = w.s.j2 ? 2 : 1;
-            switch (kv.first) {
-                case JK_WCOL_FWD: put(pmax - 1 - far, kv.first, kv.second, w.k, w.s, in_b + nop * res); break;
-                case JK_WMID_FWD: put(pmax - 2, kv.first, kv.second, w.k, w.s, 2 * nop * res); break;
-                case JK_WBLOCK: put(pmax - 1, kv.first, kv.second, w.k, w.s, (nop + 1) * res); break;
-                case JK_WMID_REV: put(pmax, kv.first, kv.second, w.k, w.s, 2 * res); break;
-                case JK_WSMALL: put(pmax - 1, kv.first, kv.second, w.k, w.s, in_b + out_b); break;
-                default: put(pmax - 1 + far, kv.first, kv.second, w.k, w.s, res + out_b); break;  // JK_WTAIL
+        if (i == 0 || words[i - 1].s.N != w.s.N) {
+            steps.clear();
+            const int far = w.s.j2 ? 2 : 1;  // the block step is pmax - 1, a middle column pass takes the steps next to it
+            for (const auto& kv : word_steps(w.s)) {
+                const int step = kv.first == JK_WCOL_FWD    ? pmax - 1 - far
+                                 : kv.first == JK_WMID_FWD  ? pmax - 2
+                                 : kv.first == JK_WMID_REV  ? pmax
+                                 : kv.first == JK_WTAIL     ? pmax - 1 + far
+                                                            : pmax - 1;
+                steps.push_back({&wgroups[std::make_tuple(step, kv.first, kv.second)], kv.first});
             }
         }
+        const double res = 4.0 * word_np(w.s.set) * P.wN, nop = P.sqr ? 1 : 2;
+        const double in_b = 8.0 * (double)(P.nca + (P.sqr ? 0 : P.ncb)), out_b = 8.0 * (double)P.rn;
+        for (const auto& st : steps) {
+            const double bytes = st.second == JK_WCOL_FWD   ? in_b + nop * res
+                                 : st.second == JK_WMID_FWD ? 2 * nop * res
+                                 : st.second == JK_WBLOCK   ? (nop + 1) * res
+                                 : st.second == JK_WMID_REV ? 2 * res
+                                 : st.second == JK_WSMALL   ? in_b + out_b
+                                                            : res + out_b;
+            add(*st.first, st.second, w.k, w.s, bytes);
+        }
+        if (P.ntl > 1) {
+            if (!carry) carry = &wgroups[std::make_tuple(2 * pmax, (int)JK_WCARRY, 0)];
+            add(*carry, JK_WCARRY, w.k, w.s, 4.0 * (double)P.ntl);
+        }
     }
-    for (int64_t k = 0; k < count && !tun.queue; k++)
-        if (bb.prods[(size_t)k].ntl > 1)
-            put(2 * pmax, JK_WCARRY, 0, (int32_t)k, WordShape(), 4.0 * (double)bb.prods[(size_t)k].ntl);
+    for (int32_t k : byclass)
+        if (bb.prods[(size_t)k].ntl > 1 && !tun.queue) {
+            if (!carry) carry = &wgroups[std::make_tuple(2 * pmax, (int)JK_WCARRY, 0)];
+            add(*carry, JK_WCARRY, k, WordShape(), 4.0 * (double)bb.prods[(size_t)k].ntl);
+        }
     for (auto& kv : wgroups)
         if (kv.second.nctas > 0x7fffffff) return fail(NBG_EINVAL, "batch too large");
     // job table: [segments | product list] per launch, then the unpack tile starts

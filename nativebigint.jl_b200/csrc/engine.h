@@ -135,7 +135,7 @@ struct ProdIn {
 };
 
 // Whether the product runs on the word engine (shape in *s), from its sizes alone.
-bool word_product(const Engine& E, const ProdIn& q, WordShape* s);
+bool word_product(const Engine& E, const ProdIn& q, WordShape* s, bool coarse = false);
 // Fills P for a word product (device pointers as in q; workspace pointers left null).
 int word_setup(Engine& E, const ProdIn& q, const WordShape& s, DProd& P);
 // One word product on `st` with its descriptor passed by value: no copies and

@@ -53,7 +53,9 @@ constexpr int word_run(int R) { return R > 16 ? 64 : 128; }
 // itself: its limb tiles are followed by two count words.
 constexpr int64_t WORD_FUSED_TILES = 2048;
 // The smallest supported length >= nconv; false when there is none.
-bool word_shape(int64_t nconv, WordShape& s);
+// coarse: up to 2^17 values only odd = 1 and 3, so that a batch of many lengths
+// needs half the kernels at up to a fifth more work.
+bool word_shape(int64_t nconv, WordShape& s, bool coarse = false);
 
 // One launch's CTAs: products of one shape are consecutive, `cpp` CTAs each.
 struct WSeg {

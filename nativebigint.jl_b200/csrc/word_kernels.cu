@@ -184,8 +184,14 @@ static const std::vector<WordShape>& shape_list() {
     return list;
 }
 
-bool word_shape(int64_t nconv, WordShape& s) {
-    const std::vector<WordShape>& v = shape_list();
+bool word_shape(int64_t nconv, WordShape& s, bool coarse) {
+    static const std::vector<WordShape> few = [] {
+        std::vector<WordShape> v;
+        for (const WordShape& x : shape_list())
+            if (x.odd <= 3 || x.N > 131072) v.push_back(x);
+        return v;
+    }();
+    const std::vector<WordShape>& v = coarse ? few : shape_list();
     const auto it = std::lower_bound(v.begin(), v.end(), nconv,
                                      [](const WordShape& x, int64_t n) { return x.N < n; });
     if (it == v.end()) return false;
