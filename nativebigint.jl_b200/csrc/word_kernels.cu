@@ -534,7 +534,7 @@ __device__ __forceinline__ void wblock(const DProd& P, int local, uint32_t* smw)
 
 // One launch serves every block size of set 0.
 template <int SET>
-__global__ void __launch_bounds__(WT, 3) k_wblock(const __grid_constant__ WArgs A) {
+__global__ void __launch_bounds__(WT, 4) k_wblock(const __grid_constant__ WArgs A) {
     __shared__ __align__(16) uint32_t sm[WBlockSmem<12>::words];
     static_assert(WBlockSmem<10>::words <= WBlockSmem<12>::words && WBlockSmem<8>::words <= WBlockSmem<12>::words, "");
     int local;
