@@ -565,14 +565,15 @@ int dev_batch(const nbg_desc* descs, int64_t count, cudaStream_t st) {
     }
     int rc = E.ensure();
     if (rc) return rc;
+    // sizing, plans and the shared workspace are the host's: no capture
+    cudaStreamCaptureStatus cap;
+    CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return fail(NBG_ECUDA, "products cannot be captured into a CUDA graph");
     rc = fill_bits_dev(in, st);
     if (rc) return rc;
     WordShape ws;
     if (count == 1 && in[0].bits_a > 0 && in[0].bits_a <= 64 * in[0].m && in[0].bits_b > 0 &&
         in[0].bits_b <= 64 * in[0].n && word_product(E, in[0], &ws)) {
-        cudaStreamCaptureStatus cap;
-        CUDA_TRY(cudaStreamIsCapturing(st, &cap));
-        if (cap != cudaStreamCaptureStatusNone) return fail(NBG_ECUDA, "products cannot be captured into a CUDA graph");
         return run_word_one(E, in[0], ws, nullptr, st);
     }
     BatchBuild bb;
