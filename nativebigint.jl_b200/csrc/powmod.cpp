@@ -254,10 +254,15 @@ static int powmod_run(Engine& E, const nbg_powmod_desc* d, int64_t count, int64_
     std::vector<uint64_t> hmu((size_t)(count * lmu_max), 0);
     std::vector<int64_t> lmu((size_t)count), bits_mu((size_t)count), bits_m((size_t)count);
     for_each_chain(count, k, [&](int64_t c) {
-        lmu[(size_t)c] = nbg_barrett_mu(hm[(size_t)c].data(), k, hmu.data() + c * lmu_max);
+        try {
+            lmu[(size_t)c] = nbg_barrett_mu(hm[(size_t)c].data(), k, hmu.data() + c * lmu_max);
+        } catch (...) {  // on whatever thread: out of host memory
+            lmu[(size_t)c] = -(int64_t)NBG_ENOMEM;
+        }
     });
     bool chainable = true;  // every μ has k + 1 limbs (k + 2 only for m = β^(k-1))
     for (int64_t c = 0; c < count; c++) {
+        if (lmu[(size_t)c] == -(int64_t)NBG_ENOMEM) return fail(NBG_ENOMEM, "host memory for the reciprocals");
         if (lmu[(size_t)c] < 0) return fail(NBG_EINVAL, "chain %lld: modulus top limb is zero", (long long)c);
         bits_mu[(size_t)c] = magnitude_bits(hmu.data() + c * lmu_max, lmu[(size_t)c]);
         bits_m[(size_t)c] = magnitude_bits(hm[(size_t)c].data(), k);
