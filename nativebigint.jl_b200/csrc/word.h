@@ -33,6 +33,15 @@ constexpr uint32_t WPRIMES[WSETS][WPR_MAX] = {
     {1073479681u, 1018429441u, 908328961u, 880803841u, 825753601u, 0},
     {943718401u, 918552577u, 880803841u, 754974721u, 666894337u, 415236097u},
     {998244353u, 897581057u, 880803841u, 754974721u, 645922817u, 595591169u}};
+// every residue of 32 bits reaches [0, 3p): by one subtraction of 3p in set 0,
+// else by the multiple of p nearest to 2^31 and then 3p
+constexpr bool word_pack_ok(int set) {
+    for (int i = 0; i < word_np(set); i++) {
+        const uint64_t p = WPRIMES[set][i];
+        if (set ? (uint64_t(1) << 31) + p / 2 > 6 * p : (uint64_t(1) << 32) > 6 * p) return false;
+    }
+    return true;
+}
 constexpr int WORD_MAX_LOG2 = 20;               // set 0: k <= 20 (leaves at level k - 2 <= 18)
 constexpr int64_t WORD_MIN_OPERAND_MAX = int64_t(1) << 21;  // set 0
 
@@ -79,7 +88,7 @@ int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t ntl);
 // Tables of one `odd` for heap sizes up to 2^L: per prime and block, fwd then inverse.
 size_t word_table_bytes(int set, int odd, int L);
 cudaError_t word_build_tables(int set, int odd, int L, void* fwd, void* inv, cudaStream_t st);
-// Per-product scale constants of the unpack (the inverse transform's 1/(odd * 2^(k-2)) and the pointwise 2^-32).
+// Per-product scale constants of the unpack (the inverse transform's 1/(odd * 2^(k-2)) and the 2^-96 of packing and pointwise products).
 void word_scales(const WordShape& s, uint32_t* out);
 
 }  // namespace nbg

@@ -15,7 +15,7 @@ using wd::Tw;
 
 struct WConst {
     uint32_t p[WPR_MAX], pinv[WPR_MAX];
-    Tw c32[WPR_MAX], one[WPR_MAX];       // 2^32 mod p, 1
+    uint32_t half[WPR_MAX];          // the multiple of p nearest to 2^31
     Tw r3[WPR_MAX];                  // e(1/3)
     Tw r5[WPR_MAX][5];               // -1/4, (c1-c2)/2, f1, f2 of e(1/5) (see dft5); [4] unused
     uint32_t c7[WPR_MAX][3], f7[WPR_MAX][3];  // cosine and sine halves of e(j/7) in 2^32 form
@@ -105,10 +105,18 @@ __device__ __forceinline__ void dft_odd(uint32_t* x, int i, uint32_t p) {
 // ---------------------------------------------------------------------------
 // packing
 
-// A limb modulo p, in [0, 4p) (RED: [0, 2p)).
+// A limb times 2^-32 modulo p, in (0, 4p) (RED: [0, 2p)): one Montgomery
+// reduction, whose factor the unpack's scale constants take back.  The upper
+// word goes below 3p first: with p > 2^32/6 (set 0) one subtraction does it, with
+// p > 2^32/11 two (below 2^31 + p/2 after the first).  Two products with constants,
+// 2^32 and 1, took 16 multiply slots instead of 6, a third of
+// k_wcol_fwd's (10,000 mixed products: that pass 3.10 -> 2.89 ms).
 template <bool RED, int SET = 0>
 __device__ __forceinline__ uint32_t wpack(uint64_t v, int pi, uint32_t p) {
-    const uint32_t y = wd::mulw((uint32_t)(v >> 32), c_w[SET].c32[pi], p) + wd::mulw((uint32_t)v, c_w[SET].one[pi], p);
+    static_assert(word_pack_ok(SET), "primes too small for the upper word's reduction");
+    uint32_t hi = (uint32_t)(v >> 32);
+    if (SET) hi = wd::sub_if(hi, c_w[SET].half[pi]);
+    const uint32_t y = wd::redc((uint64_t)wd::sub_if(hi, 3 * p) << 32 | (uint32_t)v, p, c_w[SET].pinv[pi]);
     return RED ? wd::sub_if(y, 2 * p) : y;
 }
 

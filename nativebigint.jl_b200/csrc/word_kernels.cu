@@ -69,8 +69,7 @@ static void fill_set(int set, WConst& h) {
         uint32_t x = 1;
         for (int k = 0; k < 5; k++) x *= 2 - (uint32_t)p * x;  // Newton: p^-1 mod 2^32
         h.pinv[i] = x;
-        h.c32[i] = mk((uint64_t(1) << 32) % p, p);
-        h.one[i] = mk(1, p);
+        h.half[i] = (uint32_t)(((uint64_t(1) << 31) + p / 2) / p * p);
         if ((p - 1) % 3 == 0) h.r3[i] = mk(pw(g, (p - 1) / 3, p), p);
         if (set == 0) {
         const uint64_t h2 = inv(2, p), w5 = pw(g, (p - 1) / 5, p), w7 = pw(g, (p - 1) / 7, p);
@@ -121,19 +120,19 @@ cudaError_t word_init() {
 }
 
 void word_scales(const WordShape& s, uint32_t* out) {
-    // 2^32 (pointwise) * 2^32 (unpack's reduction) / (odd * 2^levels * W_i)
+    // 2^64 (the operands' packing) * 2^32 (pointwise) * 2^32 (unpack's reduction) / (odd * 2^levels * W_i)
     constexpr int LEV = 26;
     static const struct Table {
         uint32_t v[WSETS][8][LEV][WPR_MAX];
         Table() {
             for (int set = 0; set < WSETS; set++)
                 for (int i = 0; i < word_np(set); i++) {
-                    const uint64_t p = WPRIMES[set][i], r = (uint64_t(1) << 32) % p;
+                    const uint64_t p = WPRIMES[set][i], r = (uint64_t(1) << 32) % p, r2 = r * r % p;
                     uint64_t W = 1;
                     for (int j = 0; j < i; j++) W = W * (WPRIMES[set][j] % p) % p;
                     for (int odd = 1; odd < 8; odd += 2)
                         for (int lev = 0; lev < LEV; lev++)
-                            v[set][odd][lev][i] = (uint32_t)(r * r % p * inv(odd * pw(2, (uint64_t)lev, p) % p * W % p, p) % p);
+                            v[set][odd][lev][i] = (uint32_t)(r2 * r2 % p * inv(odd * pw(2, (uint64_t)lev, p) % p * W % p, p) % p);
                 }
         }
     } t;
