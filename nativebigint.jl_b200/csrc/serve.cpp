@@ -255,10 +255,12 @@ bool nbg_server::launch_batch(std::unique_lock<std::mutex>& lk) {
     const size_t dev_in = up256(f.bb.dev_bytes), dev_out = dev_in + host_in;
     const size_t need = up256(head) + host_in + host_out;
     if (pinned_bytes[slot] < need) {
+        // doubled each time it grows, from 1 MB: pinning 8 MB costs milliseconds
+        // that a new server's first requests would wait for
+        const size_t want = std::max({need + need / 4, 2 * pinned_bytes[slot], (size_t)(1 << 20)});
         if (pinned[slot]) cudaFreeHost(pinned[slot]);
         pinned[slot] = nullptr;
         pinned_bytes[slot] = 0;
-        const size_t want = std::max(need + need / 4, (size_t)(8 << 20));
         if (cudaMallocHost(&pinned[slot], want) != cudaSuccess) {
             cudaGetLastError();
             arena.release(off, f.bytes);
