@@ -805,6 +805,10 @@ size_t fp64_work_bytes(const ProdIn& q) {
     return sizeof(double) * 2 * (size_t)N * (q.sqr ? 1 : 2);
 }
 
+// A product takes the 30-bit primes at every length that they support: they were
+// faster than the FP64 passes at each measured one (177 x 152 limbs 56 -> 7 us,
+// 65536 x 65521 105 -> 26, 2^24-limb square 4.5 -> 2.6 ms).  The FP64 passes keep
+// longer ones, kept spectra and callers that set the knobs which describe them.
 bool word_product(const Engine& E, const ProdIn& q, WordShape* s, bool coarse) {
     if (!E.word_ok || q.fp64 || q.keep_b) return false;
     const int64_t la = eff_limbs(q.m, q.bits_a), lb = q.sqr ? la : eff_limbs(q.n, q.bits_b);
@@ -868,8 +872,8 @@ size_t word_work_bytes(const ProdIn& q, const WordShape& s) {
 static double word_ops(int kind, const WordShape& s, const DProd& P) {
     const double N = s.N, np = word_np(s.set), nop = P.sqr ? 1 : 2;
     const double odd = s.odd == 3 ? 4 / 3.0 : s.odd == 5 ? 24 / 5.0 : s.odd == 7 ? (18 * 2 + 6 * 3) / 7.0 : 0;
-    const double rows = 2.0 * (s.lj - s.j2) + odd, pack = 8.0 * np * (double)(P.nca + (P.sqr ? 0 : P.ncb));
-    const double leaf = (19 * 2 + 7 * 3) / 4.0, inner = 2.0 * (s.lm - 2);  // per value
+    const double rows = 2.0 * (s.lj - s.j2) + odd, pack = 3.0 * np * (double)(P.nca + (P.sqr ? 0 : P.ncb));
+    const double leaf = (16 * 2 + 3 * 4 + 4 * 3) / 4.0, inner = 2.0 * (s.lm - 2);  // per value
     const double coef = 2.0 * (np * (np + 1) / 2 + np * (np - 1) / 2) + 3 * np;
     switch (kind) {
         case JK_WCOL_FWD: return pack + nop * np * N * rows;

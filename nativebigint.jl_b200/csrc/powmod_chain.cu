@@ -8,6 +8,8 @@
 // (word_device.cuh) with T and q2 in shared memory, the transforms of mu and m
 // are made once and kept there, a squaring transforms one operand, and the
 // subtraction of r2 reads it from the registers that assembled it.
+// Bound by the latency of a step's serial rounds, about 12 us (64 chains of
+// 256-limb moduli and 1024-bit exponents: 43 -> 15 ms on the device).
 #include <cuda_runtime.h>
 
 #include "powmod_kernels.h"

@@ -306,7 +306,10 @@ constexpr int WT = 256;  // threads per CTA
 // LM: log2 of the column count when the blocks are 4096 values (row strides are
 // then immediate offsets), 0: read from the product.  Rows past the operand are
 // not packed, and when they are its upper half (odd = 1, a half-length operand,
-// which one of two always is) the first level is a copy.
+// which one of two always is) the first level is a copy.  Bound by the multiply
+// pipe (66% busy) and, in long batches, memory: 100 squares of 65536 limbs 0.080 ms,
+// 3.9 TB/s of operands and residues.  64 registers: at 5 CTAs per SM the columns
+// spill (10,000 mixed products 13.05 -> 13.28 ms).
 template <int ODD, int LJ, int LM, int SET>
 __global__ void __launch_bounds__(WT, 4) k_wcol_fwd(const __grid_constant__ WArgs A) {
     constexpr int R = ODD << LJ, NP = word_np(SET);
@@ -408,7 +411,8 @@ __global__ void __launch_bounds__(WT) k_wmid(const __grid_constant__ WArgs A) {
 // 64 to 256 rows: tiles of 2^J rows by 2^(12-J) columns (64 to 256 bytes per
 // row), four levels in registers, a turn through shared memory, the other J - 4
 // levels.  One pass over memory instead of two: at these lengths the register
-// passes run at the memory's rate (2^24-limb square, per pass 1.6 GB).
+// passes run at the memory's rate (2^24-limb square: 1.6 GB and 0.40 ms, 4.0 TB/s).
+// Wider tiles (32 columns, 512 threads) took 0.43 ms.
 template <int J, bool FWD, int SET>
 __global__ void __launch_bounds__(WT, 4) k_wmid_sm(const __grid_constant__ WArgs A) {
     constexpr int lm = 12, CW = 1 << (12 - J), K = J - 4, NG = 1 << (4 - K);  // NG groups of 2^K values per thread
@@ -531,7 +535,10 @@ __device__ __forceinline__ void wblock(const DProd& P, int local, uint32_t* smw)
     }
 }
 
-// One launch serves every block size of set 0.
+// Both operands' 16 values per thread share each level's constants.  Bound by the
+// multiply pipe: 60% of its measured rate over 10,000 mixed products, 6.08 ms.
+// 64 registers for four CTAs per SM: three (80 registers) took 6.38 ms against
+// 6.12 then, two (96) 8% more than three.  One launch serves every block size of set 0.
 template <int SET>
 __global__ void __launch_bounds__(WT, 4) k_wblock(const __grid_constant__ WArgs A) {
     __shared__ __align__(16) uint32_t sm[WBlockSmem<12>::words];
@@ -608,6 +615,8 @@ __device__ __forceinline__ void carry_tiles(const DProd& P, int64_t k0) {
 // per coefficient); the arithmetic of the second half hides the loads of
 // another CTA's first half.  The three columns left of the tile are run too:
 // their coefficients reach into its first limbs (in column 0, from the row above).
+// Bound by the multiply pipe (65% busy; 100 squares of 65536 limbs: 0.178 ms).
+// Several runs per CTA left a 4096-limb square four CTAs, 19 -> 27 us.
 template <int ODD, int LJ, int SET>
 struct WTail {
     static constexpr int R = ODD << LJ, NP = word_np(SET);
@@ -750,8 +759,8 @@ __global__ void __launch_bounds__(WTail<ODD, LJ, SET>::NT, 1024 / WTail<ODD, LJ,
     // limbs above the operands' magnitudes
     for (int64_t i = (int64_t)N + 1 + (int64_t)local * T::NT + tid; i < rn; i += (int64_t)(cols / T::CW) * T::NT) P.r[i] = 0;
     if (!fused) return;
-    // few runs: the product's last CTA carries between them instead of another
-    // launch, and only if some run carries out at all (a limb sum within 3 of
+    // one product of few runs: its last CTA carries between them instead of another
+    // launch (in batches the fences cost 10% of the pass, so k_wcarry does it there), and only if some run carries out at all (a limb sum within 3 of
     // 2^64, so hardly ever but for operands made of ones or zeros)
     __shared__ bool last;
     __threadfence();
@@ -775,7 +784,8 @@ __global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) 
 
 // ---------------------------------------------------------------------------
 // small products: one CTA does all of it; the transforms, the residues and the
-// limbs stay on chip
+// limbs stay on chip.  Bound by the latency of one CTA's rounds (177 x 152 limbs: 7 us
+// per call in sequence, 5 of them the launch itself; FP64 passes 56 us).
 
 template <int ODD, int LM>
 __global__ void __launch_bounds__(WSmall<ODD, LM>::NT, WSmall<ODD, LM>::NT > 320 ? 1 : 640 / WSmall<ODD, LM>::NT)

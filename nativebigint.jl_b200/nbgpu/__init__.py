@@ -276,7 +276,7 @@ def radix_powtab(bb: int, x) -> list[np.ndarray]:
 
 def mul_batch(pairs) -> list[np.ndarray]:
     """Products of a list of (a, b) pairs (b None for a square), one batched
-    call; returns the m+n-limb results."""
+    call; returns the m+n-limb results (views of one allocation)."""
     pairs = [(_u64(a), None if b is None else _u64(b)) for a, b in pairs]
     sizes = [a.size + (a.size if b is None else b.size) for a, b in pairs]
     # one allocation for all results (views of it are returned): fresh pages of
