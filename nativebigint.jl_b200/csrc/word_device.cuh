@@ -108,8 +108,8 @@ __device__ __forceinline__ void dft_odd(uint32_t* x, int i, uint32_t p) {
 // A limb times 2^-32 modulo p, in (0, 4p) (RED: [0, 2p)): one Montgomery
 // reduction, whose factor the unpack's scale constants take back.  The upper
 // word goes below 3p first: with p > 2^32/6 (set 0) one subtraction does it, with
-// p > 2^32/11 two (below 2^31 + p/2 after the first).  Two products with constants,
-// 2^32 and 1, took 16 multiply slots instead of 6, a third of
+// p > 2^32/11 two (below 2^31 + p/2 after the first).  Two products with the constants
+// 2^32 and 1 took 8 multiply slots instead of 3, a third of
 // k_wcol_fwd's (10,000 mixed products: that pass 3.10 -> 2.89 ms).
 template <bool RED, int SET = 0>
 __device__ __forceinline__ uint32_t wpack(uint64_t v, int pi, uint32_t p) {

@@ -193,3 +193,21 @@ def test_carries_between_runs(gpu_lib, n):
         want = _want(a, b)
         assert np.array_equal(gpu_lib.sqr(a) if b is None else gpu_lib.mul(a, b), want)
         assert np.array_equal(g, want)
+
+
+@pytest.mark.parametrize("odd,k", [(1, 8), (3, 8), (1, 13), (5, 13), (7, 13), (1, 18), (1, 22), (3, 22)])
+def test_limbs_at_packing_edges(gpu_lib, odd, k):
+    # upper words at the multiples of p that packing subtracts (p to 3p and the
+    # one nearest 2^31, for 30-bit primes of each set), low words that make the
+    # reduction's quotient its least and greatest
+    n = ((odd << k) + 1) // 2
+    rng = np.random.default_rng(n)
+    ps = np.array([1073479681, 825753601, 943718401, 415236097, 998244353, 595591169], dtype=np.int64)
+    near = np.concatenate([c * ps for c in (1, 2, 3)] + [((1 << 31) + ps // 2) // ps * ps])
+    hi = np.unique(np.concatenate([near + d for d in (-1, 0, 1)] + [[0, 1, 2**32 - 1]]))
+    lo = np.concatenate([ps, (1 << 32) - ps, [0, 1, 2**31, 2**32 - 1]])
+    hi = hi[hi < 2**32].astype(np.uint64)
+    a, b = (rng.choice(hi, n) << np.uint64(32) | rng.choice(lo, n).astype(np.uint64) for _ in range(2))
+    a[-1] = b[-1] = 2**64 - 1
+    assert np.array_equal(gpu_lib.mul(a, b), _want(a, b))
+    assert np.array_equal(gpu_lib.sqr(a), _want(a, None))
