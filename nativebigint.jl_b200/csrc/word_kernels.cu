@@ -275,7 +275,9 @@ struct WArgs {
 
 // A kernel of a single product may be on the GPU before the one it follows has
 // finished (programmatic launch): nothing that one wrote, and nothing it may
-// still read, is touched before this.
+// still read, is touched before this, and what it wrote (operands, which may be
+// the result before, and residues) is read by __ldcg: the read-only path wants
+// data that nothing writes while this kernel is on the GPU.
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The next kernel's CTAs may come once every CTA is here: near the end, so that
 // they spread over the SMs as those empty (from the start of the kernel, the
@@ -326,7 +328,7 @@ __global__ void __launch_bounds__(WT, 4) k_wcol_fwd(const __grid_constant__ WArg
     if (pi >= NP || (isb && P.sqr)) return;
     const int n = (int)(isb ? P.ncb : P.nca);
     const int rows = (n + (1 << lm) - 1) >> lm;
-    const uint64_t* __restrict__ src = (isb ? P.b : P.a) + c;
+    const uint64_t* src = (isb ? P.b : P.a) + c;
     uint32_t* __restrict__ dst = (isb ? P.wb : P.wa) + (size_t)pi * (size_t)P.wN + c;
     const uint32_t p = c_w[SET].p[pi];
     const Tw* tab = (const Tw*)P.wtf + (((size_t)pi * ODD) << P.wL);
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(WT, 4) k_wcol_fwd(const __grid_constant__ WArg
         constexpr int r0 = decltype(r0c)::value, r1 = decltype(r1c)::value;
         uint64_t v[r1 - r0];
 #pragma unroll
-        for (int r = r0; r < r1; r++) v[r - r0] = c + (r << lm) < n ? __ldg(src + ((size_t)r << lm)) : 0ull;
+        for (int r = r0; r < r1; r++) v[r - r0] = c + (r << lm) < n ? __ldcg(src + ((size_t)r << lm)) : 0ull;
 #pragma unroll
         for (int r = r0; r < r1; r++) x[r] = r < rows ? wpack<(ODD > 1), SET>(v[r - r0], pi, p) : 0u;
     };
@@ -651,11 +653,11 @@ __global__ void __launch_bounds__(WTail<ODD, LJ, SET>::NT, 1024 / WTail<ODD, LJ,
     for (int q = tid; q < NP * (T::CW + 3); q += T::NT) {
         const int pi = q / (T::CW + 3), cc = q - pi * (T::CW + 3) - 3;
         const bool up = c0 + cc < 0;  // left of column 0: the ends of the rows above
-        const uint32_t* __restrict__ src = P.wa + (size_t)pi * (size_t)N + (c0 + cc + (up ? cols : 0));
+        const uint32_t* src = P.wa + (size_t)pi * (size_t)N + (c0 + cc + (up ? cols : 0));
         const uint32_t p = c_w[SET].p[pi];
         uint32_t x[R];
 #pragma unroll
-        for (int r = 0; r < R; r++) x[r] = src[(size_t)r << lm];
+        for (int r = 0; r < R; r++) x[r] = __ldcg(src + ((size_t)r << lm));
         const Tw* tab = (const Tw*)P.wti + (((size_t)pi * ODD) << P.wL);
 #pragma unroll
         for (int j = 0; j < ODD; j++) wd::tree_rev<LJ, 1>(x + (j << LJ), tab + ((size_t)j << P.wL), 1u, p);
@@ -801,9 +803,9 @@ __global__ void __launch_bounds__(WSmall<ODD, LM>::NT, WSmall<ODD, LM>::NT > 320
     const SmallThread<ODD, LM> th(sm, P.wtf, P.wti, P.wL);
     wait_previous();
     uint32_t x[32];  // a's 16 values, then b's
-    const uint64_t *__restrict__ pa = P.a, *__restrict__ pb = P.b;
-    th.load(x, th.sp, (int)P.nca, [&](int i) { return __ldg(pa + i); });
-    if (!P.sqr) th.load(x + 16, th.sp + W::OPW, (int)P.ncb, [&](int i) { return __ldg(pb + i); });
+    const uint64_t *pa = P.a, *pb = P.b;
+    th.load(x, th.sp, (int)P.nca, [&](int i) { return __ldcg(pa + i); });
+    if (!P.sqr) th.load(x + 16, th.sp + W::OPW, (int)P.ncb, [&](int i) { return __ldcg(pb + i); });
     if (ODD > 1) {
         __syncthreads();
         th.fetch(x, 0);

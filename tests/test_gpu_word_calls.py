@@ -1,0 +1,38 @@
+"""Device calls that return before their kernels have run: dependent calls on
+one stream, their buffers' lifetimes and their order, against GMP's products."""
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import rand_limbs
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("n", [40, 177, 700, 1500, 2100, 40000])
+@pytest.mark.parametrize("style", ["uniform", "ones"])
+def test_dependent_calls_on_one_stream(gpu_lib, n, style):
+    # each call reads what the one before wrote, and writes an operand of the
+    # calls before it (one-CTA and longer products, before and after one
+    # another); all-ones operands: the last pass carries across its runs
+    rng = np.random.default_rng(n)
+    x = rand_limbs(rng, n) if style == "uniform" else np.full(n, 2**64 - 1, dtype=np.uint64)
+    h = n // 2
+    dev = {k: torch.zeros(s, dtype=torch.uint64, device="cuda") for k, s in (("x", n), ("p", 2 * n), ("q", 4 * n))}
+    dev["x"].copy_(torch.from_numpy(x))
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    rounds = 12
+    for _ in range(rounds):
+        gpu_lib.sqr_dev(dev["p"], dev["x"], n, st)
+        gpu_lib.sqr_dev(dev["q"], dev["p"], 2 * n, st)
+        gpu_lib.mul_dev(dev["x"], dev["p"][n:], h, dev["q"][n:], n - h, st)
+    torch.cuda.synchronize()
+    for _ in range(rounds):
+        p = O.gmp_sqr(x)
+        q = O.gmp_sqr(p)
+        x = O.gmp_mul(p[n: n + h].copy(), q[n: 2 * n - h].copy())
+    for k, want in (("p", p), ("q", q), ("x", x)):
+        assert np.array_equal(dev[k].cpu().numpy(), want), k
