@@ -815,6 +815,15 @@ bool word_product(const Engine& E, const ProdIn& q, WordShape* s, bool coarse) {
     return word_shape(la + lb - 1, *s, coarse) && (s->set || std::min(la, lb) <= WORD_MIN_OPERAND_MAX);
 }
 
+bool word_to_fp64(const Engine& E, std::vector<ProdIn>& in) {
+    bool any = false;
+    for (ProdIn& q : in) {
+        WordShape s;
+        if (word_product(E, q, &s) && !s.small) q.fp64 = any = true;
+    }
+    return any;
+}
+
 int word_setup(Engine& E, const ProdIn& q, const WordShape& s, DProd& P) {
     const WordTab* wt = nullptr;
     int rc = E.word_table(s.set, s.odd, s.lj + s.lm - 2, &wt);

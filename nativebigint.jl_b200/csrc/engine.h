@@ -143,6 +143,9 @@ int word_setup(Engine& E, const ProdIn& q, const WordShape& s, DProd& P);
 // shared workspace when that is null.
 int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, char* work, cudaStream_t st);
 size_t word_work_bytes(const ProdIn& q, const WordShape& s);
+// Sends the products that run as several word kernels to the FP64 passes, for
+// want of memory; false when there are none.
+bool word_to_fp64(const Engine& E, std::vector<ProdIn>& in);
 // Transform buffers of the product on the multi-pass FP64 engine (SIZE_MAX: no such transform).
 size_t fp64_work_bytes(const ProdIn& q);
 

@@ -194,14 +194,19 @@ bool nbg_server::launch_batch(std::unique_lock<std::mutex>& lk) {
     int refuse = 0;
     {
         std::lock_guard<std::recursive_mutex> elk(E.mu);
-        // Admission is by the FP64 engine's workspace, the larger one: the
-        // budget admits the same requests whichever engine runs them.  An
-        // oversized request is refused when it reaches the front.
+        // Admission is by the FP64 engine's workspace: the budget admits the
+        // same requests whichever engine runs them.  Word products take less up
+        // to 1.5M output limbs and up to 1.29 times as much above (six primes,
+        // fewer lengths); one that does not fit the budget runs on the FP64
+        // passes.  An oversized request is refused when it reaches the front.
         for (size_t k = 0; k < in.size(); k++) {
             if (in[k].bits_a < 1 || (!in[k].sqr && in[k].bits_b < 1)) continue;
             size_t need = fp64_work_bytes(in[k]);
             if (need < ((size_t)1 << 20) || need == SIZE_MAX) continue;  // one pass, or refused by build_batch
-            if (host[k]) need += 8 * (size_t)(in[k].sqr ? 3 * in[k].m : 2 * (in[k].m + in[k].n));
+            const size_t copies = host[k] ? 8 * (size_t)(in[k].sqr ? 3 * in[k].m : 2 * (in[k].m + in[k].n)) : 0;
+            need += copies;
+            WordShape ws;
+            if (word_product(E, in[k], &ws) && word_work_bytes(in[k], ws) + copies > arena.size()) in[k].fp64 = 1;
             if (need <= arena.size()) continue;
             if (k) in.resize(k);
             else refuse = fail(NBG_ENOMEM, "request needs %zu bytes, over the server's HBM budget", need);
@@ -212,6 +217,7 @@ bool nbg_server::launch_batch(std::unique_lock<std::mutex>& lk) {
             int rc = build_batch(E, in.data(), (int64_t)in.size(), f.bb);
             if (rc) {  // a request the engine refuses (size): fail it alone
                 if (in.size() == 1) {
+                    if (rc == NBG_ENOMEM && word_to_fp64(E, in)) continue;
                     refuse = rc;
                     break;
                 }
@@ -227,6 +233,7 @@ bool nbg_server::launch_batch(std::unique_lock<std::mutex>& lk) {
             f.bytes = up256(f.bb.dev_bytes) + host_in + host_out;
             if (arena.alloc(f.bytes, off)) break;
             if (in.size() == 1) {
+                if (f.bytes > arena.size() && word_to_fp64(E, in)) continue;
                 if (f.bytes > arena.size())  // can never fit
                     refuse = fail(NBG_ENOMEM, "request needs %zu bytes, over the server's HBM budget", f.bytes);
                 else

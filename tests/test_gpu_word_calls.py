@@ -36,3 +36,20 @@ def test_dependent_calls_on_one_stream(gpu_lib, n, style):
         x = O.gmp_mul(p[n: n + h].copy(), q[n: 2 * n - h].copy())
     for k, want in (("p", p), ("q", q), ("x", x)):
         assert np.array_equal(dev[k].cpu().numpy(), want), k
+
+
+@pytest.mark.parametrize("budget", [320_000_000, 270_000_000])
+def test_server_budget_between_the_two_workspaces(gpu_lib, budget):
+    # 4.3M output limbs: 302 MB of six-prime residues, 235 MB of FP64 transforms
+    n = 2_150_000
+    rng = np.random.default_rng(n)
+    a, b = rand_limbs(rng, n), rand_limbs(rng, n)
+    da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    r = torch.zeros(2 * n, dtype=torch.uint64, device="cuda")
+    torch.cuda.synchronize()
+    s = gpu_lib.Server(hbm_budget_bytes=budget)
+    t = s.submit_dev(r, da, n, db, n, 64 * n, 64 * n)
+    s.wait(t)
+    s.release(t)
+    s.close()
+    assert np.array_equal(r.cpu().numpy(), O.gmp_mul(a, b))
