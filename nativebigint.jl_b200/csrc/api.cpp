@@ -304,22 +304,15 @@ void scatter_out(PendingOut& po, const char* staged) {
     po.any = false;
 }
 
-int host_batch(const nbg_desc* descs, int64_t count) {
-    if (!descs || count <= 0) return fail(NBG_EINVAL, "empty batch");
-    Engine& E = g_eng;
-    std::vector<ProdIn> in((size_t)count);
-    for (int64_t k = 0; k < count; k++) {
-        int rc = check_desc(descs[k], in[(size_t)k], true);
-        if (rc) return rc;
-    }
-    {
-        int rc = E.ensure();
-        if (rc) return rc;
-    }
+int host_chunks(Engine& E, const std::vector<ProdIn>& in) {
+    const int64_t count = (int64_t)in.size();
     WordShape ws;
     if (count == 1 && in[0].bits_a > 0 && in[0].bits_b > 0 && word_product(E, in[0], &ws) &&
-        8 * (size_t)(2 * (in[0].m + in[0].n)) < STAGE_MIN_BYTES)
-        return host_one(in[0], ws);
+        8 * (size_t)(2 * (in[0].m + in[0].n)) < STAGE_MIN_BYTES) {
+        // (the pipeline allocates just what the product needs, and no pinned buffers at this size)
+        const int rc1 = host_one(in[0], ws);
+        if (rc1 != NBG_ENOMEM) return rc1;
+    }
     // chunks of ~CHUNK_BYTES operands, in input order
     std::vector<std::pair<int64_t, int64_t>> bounds;  // (start, count)
     {
@@ -506,6 +499,19 @@ int host_batch(const nbg_desc* descs, int64_t count) {
     return NBG_OK;
 }
 
+int host_batch(const nbg_desc* descs, int64_t count) {
+    if (!descs || count <= 0) return fail(NBG_EINVAL, "empty batch");
+    Engine& E = g_eng;
+    std::vector<ProdIn> in((size_t)count);
+    for (int64_t k = 0; k < count; k++) {
+        int rc = check_desc(descs[k], in[(size_t)k], true);
+        if (rc) return rc;
+    }
+    int rc = E.ensure();
+    if (rc) return rc;
+    return word_or_fp64(E, in, [&] { return host_chunks(E, in); });
+}
+
 // Reads the operands' top limbs on the device (magnitude_bits) for
 // descriptors that leave bits_a / bits_b at 0.
 int fill_bits_dev(std::vector<ProdIn>& in, cudaStream_t st) {
@@ -555,29 +561,16 @@ int fill_bits_dev(std::vector<ProdIn>& in, cudaStream_t st) {
     return NBG_OK;
 }
 
-int dev_batch(const nbg_desc* descs, int64_t count, cudaStream_t st) {
-    if (!descs || count <= 0) return fail(NBG_EINVAL, "empty batch");
-    Engine& E = g_eng;
-    std::vector<ProdIn> in((size_t)count);
-    for (int64_t k = 0; k < count; k++) {
-        int rc = check_desc(descs[k], in[(size_t)k], false);
-        if (rc) return rc;
-    }
-    int rc = E.ensure();
-    if (rc) return rc;
-    // sizing, plans and the shared workspace are the host's: no capture
-    cudaStreamCaptureStatus cap;
-    CUDA_TRY(cudaStreamIsCapturing(st, &cap));
-    if (cap != cudaStreamCaptureStatusNone) return fail(NBG_ECUDA, "products cannot be captured into a CUDA graph");
-    rc = fill_bits_dev(in, st);
+int dev_run(Engine& E, std::vector<ProdIn>& in, cudaStream_t st) {
+    int rc = fill_bits_dev(in, st);
     if (rc) return rc;
     WordShape ws;
-    if (count == 1 && in[0].bits_a > 0 && in[0].bits_a <= 64 * in[0].m && in[0].bits_b > 0 &&
+    if (in.size() == 1 && in[0].bits_a > 0 && in[0].bits_a <= 64 * in[0].m && in[0].bits_b > 0 &&
         in[0].bits_b <= 64 * in[0].n && word_product(E, in[0], &ws)) {
         return run_word_one(E, in[0], ws, nullptr, st);
     }
     BatchBuild bb;
-    rc = build_batch(E, in.data(), count, bb);
+    rc = build_batch(E, in.data(), (int64_t)in.size(), bb);
     if (rc) return rc;
     rc = E.ensure_pool(bb.dev_bytes, st);
     if (rc) return rc;
@@ -592,6 +585,23 @@ int dev_batch(const nbg_desc* descs, int64_t count, cudaStream_t st) {
     // keep them valid until the copies ran.
     CUDA_TRY(cudaStreamSynchronize(st));
     return NBG_OK;
+}
+
+int dev_batch(const nbg_desc* descs, int64_t count, cudaStream_t st) {
+    if (!descs || count <= 0) return fail(NBG_EINVAL, "empty batch");
+    Engine& E = g_eng;
+    std::vector<ProdIn> in((size_t)count);
+    for (int64_t k = 0; k < count; k++) {
+        int rc = check_desc(descs[k], in[(size_t)k], false);
+        if (rc) return rc;
+    }
+    int rc = E.ensure();
+    if (rc) return rc;
+    // sizing, plans and the shared workspace are the host's: no capture
+    cudaStreamCaptureStatus cap;
+    CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return fail(NBG_ECUDA, "products cannot be captured into a CUDA graph");
+    return word_or_fp64(E, in, [&] { return dev_run(E, in, st); });
 }
 
 // NULL is the legacy default stream, as everywhere in CUDA
@@ -867,16 +877,19 @@ int nbg_batch_create(const nbg_desc* descs, int64_t count, nbg_batch** out) {
     rc = fill_bits_dev(in, E.stream);
     if (rc) return rc;
     nbg_batch* bt = new nbg_batch();
-    rc = build_batch(E, in.data(), count, bt->bb);
+    rc = word_or_fp64(E, in, [&] {
+        const int rb = build_batch(E, in.data(), count, bt->bb);
+        if (rb) return rb;
+        if (cudaMalloc(&bt->dmem, bt->bb.dev_bytes) != cudaSuccess) {
+            cudaGetLastError();
+            bt->dmem = nullptr;
+            return fail(NBG_ENOMEM, "batch workspace of %zu bytes unavailable", bt->bb.dev_bytes);
+        }
+        return (int)NBG_OK;
+    });
     if (rc) {
         delete bt;
         return rc;
-    }
-    if (cudaMalloc(&bt->dmem, bt->bb.dev_bytes) != cudaSuccess) {
-        cudaGetLastError();
-        const size_t want = bt->bb.dev_bytes;
-        delete bt;
-        return fail(NBG_ENOMEM, "batch workspace of %zu bytes unavailable", want);
     }
     rc = upload_batch(E, bt->bb, bt->dmem, E.stream);
     const bool queue = E.tun.queue > 0;

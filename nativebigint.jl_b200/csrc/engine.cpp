@@ -574,10 +574,11 @@ int Engine::build_plan(int64_t N, PlanRec& pr, int for_sqr) {
     std::vector<double> hilo((size_t)(nhi + 4096));
     double* dtab = nullptr;
     double* dtmp = nullptr;
-    CUDA_TRY(cudaMalloc(&dtab, sizeof(double) * 2 * per));
-    if (cudaMalloc(&dtmp, sizeof(double) * hilo.size()) != cudaSuccess) {
+    if (cudaMalloc(&dtab, sizeof(double) * 2 * per) != cudaSuccess ||
+        cudaMalloc(&dtmp, sizeof(double) * hilo.size()) != cudaSuccess) {
+        cudaGetLastError();
         cudaFree(dtab);
-        return fail(NBG_ENOMEM, "twiddle staging allocation failed");
+        return fail(NBG_ENOMEM, "twiddle tables of %zu bytes unavailable", sizeof(double) * 2 * per);
     }
     int rc = NBG_OK;
     for (int f = 0; f < 2 && rc == NBG_OK; f++) {
@@ -694,9 +695,11 @@ int Engine::word_table(int set, int odd, int L, const WordTab** out) {
         cudaError_t e = word_build_tables(set, odd, want, n.fwd, n.inv, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) {
+            cudaGetLastError();
             cudaFree(n.fwd);
             cudaFree(n.inv);
-            return fail(NBG_ECUDA, "constant tables: %s", cudaGetErrorString(e));
+            return fail(e == cudaErrorMemoryAllocation ? NBG_ENOMEM : NBG_ECUDA, "constant tables: %s",
+                        cudaGetErrorString(e));
         }
         if (w.fwd) graveyard.push_back((double*)w.fwd);
         if (w.inv) graveyard.push_back((double*)w.inv);
@@ -704,6 +707,22 @@ int Engine::word_table(int set, int odd, int L, const WordTab** out) {
     }
     *out = &w;
     return NBG_OK;
+}
+
+void Engine::word_tables_back(const WordTabs& t) {
+    for (int set = 0; set < WSETS; set++)
+        for (int odd = 0; odd < 8; odd++) {
+            WordTab& w = wtab[(size_t)set][(size_t)odd];
+            const WordTab& b = t[(size_t)set][(size_t)odd];
+            if (w.fwd == b.fwd) continue;
+            cudaFree(w.fwd);
+            cudaFree(w.inv);
+            w = b;
+            for (void* old : {b.fwd, b.inv}) {  // current again
+                auto it = std::find(graveyard.begin(), graveyard.end(), (double*)old);
+                if (old && it != graveyard.end()) graveyard.erase(it);
+            }
+        }
 }
 
 int Engine::ensure_stage(int i, size_t bytes) {

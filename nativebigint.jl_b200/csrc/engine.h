@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <array>
 #include <atomic>
 #include <cstdint>
 #include <map>
@@ -9,6 +10,7 @@
 #include <string>
 #include <vector>
 
+#include "../../include/nbgpu.h"
 #include "types.h"
 #include "word.h"
 
@@ -85,7 +87,8 @@ struct Engine {
     // that sets other pass knobs gets the FP64 passes they describe
     std::string base_tuning = Tuning().to_json();
     bool word_ok = true;
-    WordTab wtab[WSETS][8];  // by prime set and odd
+    using WordTabs = std::array<std::array<WordTab, 8>, WSETS>;
+    WordTabs wtab;  // by prime set and odd
     std::map<int64_t, PlanRec> plans;
     std::vector<double*> graveyard;
     DPlan* d_plans = nullptr;
@@ -110,6 +113,7 @@ struct Engine {
     void drop_plans();
     void tuning_changed(bool loaded);  // after `tun` was set (loaded: it is the new base)
     int word_table(int set, int odd, int L, const WordTab** out);
+    void word_tables_back(const WordTabs& t);  // frees the tables built since `t` was taken (nothing may use them)
     void trim_plans();  // frees every plan's tables: no batch may exist or be running
     // The shared workspace, at least `bytes`, for work on `st`: ordered after the
     // last call that left work using it in flight (pool_release).
@@ -146,6 +150,17 @@ size_t word_work_bytes(const ProdIn& q, const WordShape& s);
 // Sends the products that run as several word kernels to the FP64 passes, for
 // want of memory; false when there are none.
 bool word_to_fp64(const Engine& E, std::vector<ProdIn>& in);
+// run(), and when memory is short, again with those products on the FP64 passes:
+// above 1.5M output limbs these can need less (4.3M: 235 MB against 302 and the
+// constants), and what they fitted stays served.
+template <class F>
+int word_or_fp64(Engine& E, std::vector<ProdIn>& in, F run) {
+    const Engine::WordTabs before = E.wtab;
+    const int rc = run();
+    if (rc != NBG_ENOMEM || !word_to_fp64(E, in)) return rc;
+    E.word_tables_back(before);
+    return run();
+}
 // Transform buffers of the product on the multi-pass FP64 engine (SIZE_MAX: no such transform).
 size_t fp64_work_bytes(const ProdIn& q);
 

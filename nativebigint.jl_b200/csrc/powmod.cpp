@@ -362,10 +362,13 @@ static int powmod_run(Engine& E, const nbg_powmod_desc* d, int64_t count, int64_
     }
     BatchBuild bb[3];
     char* reg[3];
-    const std::vector<ProdIn>* ins[3] = {&in1, &in2, &in3};
+    std::vector<ProdIn>* ins[3] = {&in1, &in2, &in3};
     for (int i = 0; i < 3; i++) {
-        if ((rc = build_batch(E, ins[i]->data(), count, bb[i]))) return rc;
-        if ((rc = mem.get(&reg[i], bb[i].dev_bytes))) return rc;
+        rc = word_or_fp64(E, *ins[i], [&] {
+            const int rb = build_batch(E, ins[i]->data(), count, bb[i]);
+            return rb ? rb : mem.get(&reg[i], bb[i].dev_bytes);
+        });
+        if (rc) return rc;
         if ((rc = upload_batch(E, bb[i], reg[i], st))) return rc;
         PM_TRY(expand_jobs(bb[i], reg[i], st));
     }

@@ -79,3 +79,65 @@ def test_server_serves_what_fits_the_fp64_passes(fake, limbs, budget, word):
     assert (w > 0) == word and (f > 0) == (not word)
     # and one that neither fits is refused
     assert serve(fake, 20_000_000, limbs) == NBG_ENOMEM
+
+
+def descs(*items):
+    d = (NbgDesc * len(items))()
+    for k, x in enumerate(items):
+        d[k] = NbgDesc(*x)
+    return ctypes.cast(d, ctypes.c_void_p), len(items), d
+
+
+# 8.5M output limbs: six-prime residues and constants 604 MB (a square) or 906,
+# FP64 transforms and twiddles 470 or 705
+LIMBS = 4_250_000
+SHORT = {"sqr_dev": 550, "mul_dev": 800, "mul_batch_dev": 1000, "batch_create": 800, "mul_batch": 920}
+
+
+@pytest.mark.parametrize("call", SHORT)
+def test_products_that_only_fit_as_fp64_passes(fake, call):
+    n, L = LIMBS, fake
+    host = [(ctypes.c_uint64 * k)() for k in (2 * n, n, n)] if call == "mul_batch" else []
+    for h in host:
+        h[len(h) - 1] = 1
+    r, a, b = (ctypes.addressof(h) for h in host) if host else (R, A, B)
+
+    def run():
+        if call == "sqr_dev":
+            return L.nbg_sqr_dev(R, A, n, None)
+        if call == "mul_dev":
+            return L.nbg_mul_dev(R, A, n, B, n, None)
+        if call == "batch_create":
+            bt = ctypes.c_void_p()
+            rc = L.nbg_batch_create(*descs((R, A, B, n, n, 0, 0))[:2], ctypes.byref(bt))
+            return rc
+        if call == "mul_batch":
+            return L.nbg_mul_batch(*descs((r, a, b, n, n, 0, 0))[:2])
+        return L.nbg_mul_batch_dev(*descs((R, A, B, n, n, 0, 0), (R + (1 << 40), A, None, n // 2, n // 2, 0, 0))[:2], None)
+
+    L.fake_limit(SHORT[call] * 1_000_000)
+    counts(L)
+    assert run() == NBG_OK
+    w, f = counts(L)
+    assert w == 0 and f > 0
+    # with room for them, word products again
+    L.fake_limit(ctypes.c_size_t(-1).value)
+    assert run() == NBG_OK
+    w, f = counts(L)
+    assert w > 0 and f == 0
+    # nothing fits: refused, and the next call works
+    L.fake_limit(0)
+    big = 3 * n
+    assert L.nbg_sqr_dev(R, A, big, None) == NBG_ENOMEM
+    L.fake_limit(ctypes.c_size_t(-1).value)
+    assert L.nbg_sqr_dev(R, A, big, None) == NBG_OK
+
+
+def test_host_product_with_little_device_memory(fake):
+    # residues, constants and limbs (43 MB) fit 62 MB, the shared workspace (64 MB at least) does not
+    n = 200_000
+    r, a, b = ((ctypes.c_uint64 * k)() for k in (2 * n, n, n))
+    a[n - 1] = b[n - 1] = 1
+    fake.nbg_mul.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64]
+    fake.fake_limit(62_000_000)
+    assert fake.nbg_mul(ctypes.addressof(r), ctypes.addressof(a), n, ctypes.addressof(b), n) == NBG_OK
