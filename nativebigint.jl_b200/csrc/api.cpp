@@ -257,6 +257,7 @@ int host_one(const ProdIn& q, const WordShape& ws) {
     }
     const size_t work = align_up(word_work_bytes(q, ws), 256);
     if ((rc = E.ensure_pool(work + in_bytes + out_bytes, st))) return rc;
+    PoolUse use(st);  // (the pinned buffers' too)
     char* base = (char*)E.pool;
     char *din = base + work, *dout = din + in_bytes;
     std::vector<CopyPool::Piece> pieces;
@@ -276,6 +277,7 @@ int host_one(const ProdIn& q, const WordShape& ws) {
     rc = run_word_one(E, d, ws, base, st);
     cudaError_t e = cudaSuccess;
     if (!rc) e = cudaMemcpyAsync(dr ? (char*)q.r : E.pg_out[0], dout, nr, cudaMemcpyDeviceToHost, st);
+    use.done = true;
     const cudaError_t es = cudaStreamSynchronize(st);  // the pool and the buffers are free again
     if (rc) return rc;
     if (e != cudaSuccess || es != cudaSuccess)
@@ -544,14 +546,16 @@ int fill_bits_dev(std::vector<ProdIn>& in, cudaStream_t st) {
     }
     const size_t pb = align_up(sizeof(DProd) * tmp.size(), 256);
     const size_t bb = sizeof(int64_t) * 2 * tmp.size();
+    std::vector<int64_t> bits(2 * tmp.size());
     int rc = E.ensure_pool(pb + bb, st);
     if (rc) return rc;
+    PoolUse use(st);
     char* d = (char*)E.pool;
     CUDA_TRY(cudaMemcpyAsync(d, tmp.data(), sizeof(DProd) * tmp.size(), cudaMemcpyHostToDevice, st));
     CUDA_TRY(launch_topbits((const DProd*)d, (int64_t)tmp.size(), (int64_t*)(d + pb), st));
     g_launches++;
-    std::vector<int64_t> bits(2 * tmp.size());
     CUDA_TRY(cudaMemcpyAsync(bits.data(), d + pb, bb, cudaMemcpyDeviceToHost, st));
+    use.done = true;
     CUDA_TRY(cudaStreamSynchronize(st));
     for (size_t i = 0; i < need.size(); i++) {
         ProdIn& q = in[(size_t)need[i]];
@@ -574,6 +578,7 @@ int dev_run(Engine& E, std::vector<ProdIn>& in, cudaStream_t st) {
     if (rc) return rc;
     rc = E.ensure_pool(bb.dev_bytes, st);
     if (rc) return rc;
+    PoolUse use(st);
     char* dbase = (char*)E.pool;
     rc = upload_batch(E, bb, dbase, st);
     if (rc) return rc;
@@ -583,6 +588,7 @@ int dev_run(Engine& E, std::vector<ProdIn>& in, cudaStream_t st) {
     if (rc) return rc;
     // descriptors/jobs live in pageable host memory copied asynchronously;
     // keep them valid until the copies ran.
+    use.done = true;
     CUDA_TRY(cudaStreamSynchronize(st));
     return NBG_OK;
 }
@@ -702,6 +708,7 @@ int transform_passes(double* x, int64_t N, int prime, bool fwd, cudaStream_t st)
     const size_t so = align_up(jo + sizeof(Job) * jobs.size(), 256);
     rc = E.ensure_pool(so + sizeof(double) * (size_t)N, st);
     if (rc) return rc;
+    PoolUse use(st);
     char* d = (char*)E.pool;
     P.xa[prime] = x;
     P.xa[1 - prime] = (double*)(d + so);
@@ -711,6 +718,7 @@ int transform_passes(double* x, int64_t N, int prime, bool fwd, cudaStream_t st)
         CUDA_TRY(launch_jobs(L.kind, (const DProd*)d, E.d_plans, job_list((const Job*)(d + jo) + L.off), L.n, L.smem, 0, st));
         g_launches++;
     }
+    use.done = true;
     CUDA_TRY(cudaStreamSynchronize(st));
     return NBG_OK;
 }
@@ -1069,6 +1077,7 @@ int nbg_unpack_dev(uint64_t* r, int64_t rn, const double* x1, const double* x2, 
     const size_t jo = 256, ao = align_up(jo + sizeof(Job) * jobs.size(), 256);
     rc = E.ensure_pool(ao + sizeof(uint32_t) * (size_t)P.ntl, st);
     if (rc) return rc;
+    PoolUse use(st);
     char* d = (char*)E.pool;
     P.agg = (uint32_t*)(d + ao);
     CUDA_TRY(cudaMemcpyAsync(d, &P, sizeof P, cudaMemcpyHostToDevice, st));
@@ -1078,6 +1087,7 @@ int nbg_unpack_dev(uint64_t* r, int64_t rn, const double* x1, const double* x2, 
     CUDA_TRY(launch_jobs(JK_CARRY, (const DProd*)d, E.d_plans, job_list((const Job*)(d + jo) + P.ntl), 1, 0, 0, st));
     CUDA_TRY(launch_jobs(JK_CARRYFIX, (const DProd*)d, E.d_plans, job_list((const Job*)(d + jo)), P.ntl, 0, 0, st));
     g_launches += 3;
+    use.done = true;
     CUDA_TRY(cudaStreamSynchronize(st));
     return NBG_OK;
 }

@@ -919,6 +919,7 @@ int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, char* work, cud
     int rc = word_setup(E, q, s, P);
     if (rc) return rc;
     const bool pool = !s.small && !work;
+    PoolUse use(st);
     if (!s.small) {
         if (pool) {
             if ((rc = E.ensure_pool(word_work_bytes(q, s), st))) return rc;
@@ -935,7 +936,9 @@ int run_word_one(Engine& E, const ProdIn& q, const WordShape& s, char* work, cud
         CUDA_TRY(launch_word_one(kv.first, kv.second, P, word_ctas(kv.first, s, P.sqr, P.ntl), st));
         g_launches++;
     }
-    return pool ? E.pool_release(st) : NBG_OK;
+    rc = pool ? E.pool_release(st) : NBG_OK;
+    use.done = rc == NBG_OK;
+    return rc;
 }
 
 int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
@@ -1505,18 +1508,21 @@ int run_launches_branched(Engine& E, const BatchBuild& bb, char* dbase, cudaStre
             CUDA_TRY(cudaEventRecord(E.fork_ev, st));
             for (int q = 0; q < ns; q++) CUDA_TRY(cudaStreamWaitEvent(side[q], E.fork_ev, 0));
         }
-        for (size_t k = i; k < j; k++) {
+        int rc = NBG_OK;
+        for (size_t k = i; k < j && !rc; k++) {
             const Launch& L = bb.launches[k];
             cudaStream_t s = k > i && ns ? side[(k - i - 1) % (size_t)ns] : st;
             cudaError_t e = launch_one(E, bb, L, dbase, s);
             if (e != cudaSuccess)
-                return fail(NBG_ECUDA, "launch (kind %d, %lld jobs): %s", L.kind, (long long)L.n, cudaGetErrorString(e));
-            g_launches++;
+                rc = fail(NBG_ECUDA, "launch (kind %d, %lld jobs): %s", L.kind, (long long)L.n, cudaGetErrorString(e));
+            else
+                g_launches++;
         }
         for (int q = 0; q < ns; q++) {
             CUDA_TRY(cudaEventRecord(E.join_ev[q], side[q]));
             CUDA_TRY(cudaStreamWaitEvent(st, E.join_ev[q], 0));
         }
+        if (rc) return rc;  // st is behind what was launched
         i = j;
     }
     return NBG_OK;

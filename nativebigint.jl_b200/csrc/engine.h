@@ -125,6 +125,19 @@ struct Engine {
 };
 extern Engine g_eng;
 
+// A call's use of the shared workspace on `st`: ends when the call has waited for
+// the stream (done = true) or left its work in flight (pool_release); a call that
+// returns on an error before waits for what it had launched.
+struct PoolUse {
+    cudaStream_t st;
+    bool done = false;
+    explicit PoolUse(cudaStream_t s) : st(s) {}
+    ~PoolUse() {
+        if (!done) cudaStreamSynchronize(st);
+    }
+    PoolUse(const PoolUse&) = delete;
+};
+
 // One product as the batch builder sees it (device pointers).
 struct ProdIn {
     const uint64_t* a;

@@ -141,3 +141,35 @@ def test_host_product_with_little_device_memory(fake):
     fake.nbg_mul.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64]
     fake.fake_limit(62_000_000)
     assert fake.nbg_mul(ctypes.addressof(r), ctypes.addressof(a), n, ctypes.addressof(b), n) == NBG_OK
+
+
+@pytest.mark.parametrize("call", ["one", "batch", "host", "host_batch"])
+def test_failed_launch_leaves_the_workspace_ordered(fake, call):
+    # a launch fails: what was launched before it may still use the shared
+    # workspace, so the next call's kernels come after it, on whatever stream
+    L, s1, s2 = fake, 0x100, 0x200
+    sizes = (5000, 40_000, 70_000, 90_000, 1000)
+    hosts = [[(ctypes.c_uint64 * k)() for k in (2 * n, n)] for n in sizes]
+    for _, a in hosts:
+        a[len(a) - 1] = 1
+
+    def run():
+        if call == "one":
+            return L.nbg_mul_dev(R, A, 40_000, B, 30_000, s1)
+        if call.startswith("host"):
+            use = hosts if call == "host_batch" else hosts[:1]
+            return L.nbg_mul_batch(*descs(*((ctypes.addressof(r), ctypes.addressof(a), None, len(a), len(a), 0, 0)
+                                            for r, a in use))[:2])
+        return L.nbg_mul_batch_dev(*descs(*((R + (k << 30), A, B, n, n, 0, 0) for k, n in enumerate(sizes)))[:2], s1)
+
+    assert run() == NBG_OK
+    counts(L)
+    assert run() == NBG_OK
+    launches = counts(L)[0]
+    assert launches >= (8 if "batch" in call else 3)
+    for k in range(launches):
+        L.fake_fail_at(k)
+        assert run() == NBG_ECUDA
+        L.fake_mark()
+        assert L.nbg_mul_dev(R, A, 50_000, B, 30_000, s2) == NBG_OK
+        assert L.fake_unordered() == 0, k
