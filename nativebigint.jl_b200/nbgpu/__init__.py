@@ -175,15 +175,26 @@ def _stream(s) -> int | None:
     return getattr(s, "cuda_stream", None) or int(s)
 
 
+_default_streams: dict = {}  # by device: torch's object for the legacy default stream
+
+
 def _in_flight(stream, *buffers) -> None:
-    """Tensors given to a call on an explicit stream stay allocated until that
-    stream is done with them (the call itself may return earlier)."""
-    if stream is None:
-        return
+    """Tensors given to a call stay allocated until the call's stream (None or
+    0: the legacy default stream) is done with them: the call returns earlier,
+    and a tensor allocated under another stream would be reused meanwhile."""
     torch = sys.modules.get("torch")
+    if torch is None:
+        return
+    st = stream if hasattr(stream, "cuda_stream") else None
     for x in buffers:
-        if torch is not None and isinstance(x, torch.Tensor) and x.is_cuda:
-            st = stream if hasattr(stream, "cuda_stream") else torch.cuda.ExternalStream(_stream(stream))
+        if isinstance(x, torch.Tensor) and x.is_cuda:
+            if st is None:
+                if stream:
+                    st = torch.cuda.ExternalStream(_stream(stream))
+                else:
+                    st = _default_streams.get(x.device)
+                    if st is None:
+                        st = _default_streams[x.device] = torch.cuda.default_stream(x.device)
             x.record_stream(st)
 
 
@@ -310,11 +321,15 @@ def uses_fpntt_sqr(n: int) -> bool:
 # device-buffer calls (torch tensors or raw device addresses)
 
 def mul_dev(r, a, m: int, b, n: int, stream=None) -> None:
+    """r = a*b on `stream` (None: the legacy default stream).  May return before
+    the product is there: tensors may be dropped at once, memory behind raw
+    addresses has to stay until the stream is done."""
     _check(lib().nbg_mul_dev(_dptr(r), _dptr(a), m, _dptr(b), n, _stream(stream)))
     _in_flight(stream, r, a, b)
 
 
 def sqr_dev(r, a, n: int, stream=None) -> None:
+    """r = a^2; see mul_dev."""
     _check(lib().nbg_sqr_dev(_dptr(r), _dptr(a), n, _stream(stream)))
     _in_flight(stream, r, a)
 
@@ -326,15 +341,22 @@ def mul_dev_noalloc(r, a, m: int, b, n: int, stream=None) -> None:
 
 
 def make_descs(items) -> ctypes.Array:
-    """items: (r, a, b_or_None, m, n, bits_a, bits_b) with device tensors or addresses."""
+    """items: (r, a, b_or_None, m, n, bits_a, bits_b) with device tensors or
+    addresses; the array keeps the tensors (`tensors`)."""
     descs = (NbgDesc * len(items))()
+    descs.tensors = []
     for k, (r, a, b, m, n, ba, bb) in enumerate(items):
         descs[k] = NbgDesc(_dptr(r), _dptr(a), None if b is None else _dptr(b), m, n, ba, bb)
+        descs.tensors += [x for x in (r, a, b) if x is not None and not isinstance(x, int)]
     return descs
 
 
 def mul_batch_dev(descs: ctypes.Array, stream=None) -> None:
+    """The products of `descs` on `stream`; may return before they are there
+    (see mul_dev; descriptors not made by make_descs count as raw addresses)."""
     _check(lib().nbg_mul_batch_dev(ctypes.cast(descs, ctypes.c_void_p), len(descs), _stream(stream)))
+    if len(descs) == 1:  # several products are waited for
+        _in_flight(stream, *getattr(descs, "tensors", ()))
 
 
 class Batch:

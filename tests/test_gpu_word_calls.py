@@ -53,3 +53,33 @@ def test_server_budget_between_the_two_workspaces(gpu_lib, budget):
     s.release(t)
     s.close()
     assert np.array_equal(r.cpu().numpy(), O.gmp_mul(a, b))
+
+
+@pytest.mark.parametrize("how", ["mul_dev", "mul_batch_dev"])
+@pytest.mark.parametrize("n", [500, 500_000])
+def test_temporaries_dropped_after_the_call(gpu_lib, how, n):
+    # operands allocated under another stream than the call's (the legacy
+    # default one), dropped at once, and that stream's next tensors written
+    rng = np.random.default_rng(n)
+    side = torch.cuda.Stream()
+    a, b = rand_limbs(rng, n), rand_limbs(rng, n)
+    pa, pb = (torch.from_numpy(x.view(np.int64)).pin_memory() for x in (a, b))
+    rs = []
+    for _ in range(4):
+        with torch.cuda.stream(side):
+            da, db = pa.cuda(non_blocking=True), pb.cuda(non_blocking=True)
+            r = torch.zeros(2 * n, dtype=torch.int64, device="cuda")
+        side.synchronize()
+        if how == "mul_dev":
+            gpu_lib.mul_dev(r, da, n, db, n)
+        else:
+            gpu_lib.mul_batch_dev(gpu_lib.make_descs([(r, da, db, n, n, 0, 0)]))
+        del da, db
+        with torch.cuda.stream(side):
+            over = [torch.full((n,), -1, dtype=torch.int64, device="cuda") for _ in range(4)]
+        del over
+        rs.append(r)
+    torch.cuda.synchronize()
+    want = O.gmp_mul(a, b)
+    for r in rs:
+        assert np.array_equal(r.cpu().numpy().view(np.uint64), want)
