@@ -67,6 +67,8 @@ constexpr size_t CHUNK_BYTES = size_t(128) << 20;
 constexpr int NBUF = 3;
 // chunks with fewer operand and result bytes copy pageable spans directly
 constexpr size_t STAGE_MIN_BYTES = size_t(8) << 20;
+// operand bytes from which a single product's copies are left to the driver
+constexpr size_t ONE_STAGE_BYTES = size_t(256) << 10;
 
 struct Span {
     const char* h;  // host start
@@ -228,21 +230,25 @@ bool all_set(const std::vector<char>& v) {
     return !v.empty() && std::find(v.begin(), v.end(), 0) == v.end();
 }
 
-// One word product between host buffers: operands through a pinned buffer in
-// one copy, the kernels, the result back through a pinned buffer, on the engine
-// stream.  A one-CTA product reads and writes the pinned buffers itself (a few
-// KB over the bus cost less than a copy's start).  Buffers the GPU can reach
-// are copied without staging.  Against the chunk pipeline (three streams, five
-// events, stream-ordered allocations, the driver's pageable copies), 4864 x
-// 4321 limbs: 86 -> 60 us per call.
+// One word product between host buffers on the engine stream.  Operands of less
+// than ONE_STAGE_BYTES go through a pinned buffer in one copy and the result back
+// through another; longer ones, and buffers the GPU can reach, are copied as they
+// are (pageable ones by the driver).  A one-CTA product reads and writes the
+// pinned buffers itself (a few KB over the bus cost less than a copy's start).
+// us per call, m x 0.9m limbs, staged / copied by the driver / chunk pipeline
+// (three streams, five events, stream-ordered allocations): m = 2000 47/65/122,
+// 4864 54/55/108, 16000 75/75/135, 32000 113/112/160, 64000 210/182/240, 100000
+// 300/250/342, 262000 695/540/670 (staged by the copy threads: 100000 550, as
+// waking them takes 200).
 int host_one(const ProdIn& q, const WordShape& ws) {
     Engine& E = g_eng;
     cudaStream_t st = E.stream;
     const size_t na = 8 * (size_t)q.m, nb = q.sqr ? 0 : 8 * (size_t)q.n, nr = 8 * (size_t)(q.m + q.n);
     const size_t ob = align_up(na, 256), in_bytes = align_up(ob + nb, 256), out_bytes = align_up(nr, 256);
+    const bool staged = na + nb < ONE_STAGE_BYTES;
     int rc;
-    if ((rc = ensure_pinned(E.pg_in[0], E.pg_in_bytes[0], in_bytes))) return rc;
-    if ((rc = ensure_pinned(E.pg_out[0], E.pg_out_bytes[0], out_bytes))) return rc;
+    if (staged && (rc = ensure_pinned(E.pg_in[0], E.pg_in_bytes[0], in_bytes))) return rc;
+    if (staged && (rc = ensure_pinned(E.pg_out[0], E.pg_out_bytes[0], out_bytes))) return rc;
     ProdIn d = q;
     if (ws.small) {
         memcpy(E.pg_in[0], q.a, na);
@@ -261,7 +267,8 @@ int host_one(const ProdIn& q, const WordShape& ws) {
     char* base = (char*)E.pool;
     char *din = base + work, *dout = din + in_bytes;
     std::vector<CopyPool::Piece> pieces;
-    const bool da = dma_ok(q.a, na), db = q.sqr || dma_ok(q.b, nb), dr = dma_ok(q.r, nr);
+    const bool da = !staged || dma_ok(q.a, na), db = !staged || q.sqr || dma_ok(q.b, nb);
+    const bool dr = !staged || dma_ok(q.r, nr);
     if (!da) pieces.push_back({E.pg_in[0], (const char*)q.a, na});
     if (!db) pieces.push_back({E.pg_in[0] + ob, (const char*)q.b, nb});
     CopyPool::get().run(pieces);

@@ -29,6 +29,7 @@ struct State {
     bool marked = false;
     int unordered = 0;       // launches after the mark not ordered after all before it
     long word = 0, fp64 = 0;
+    std::vector<const void*> copied;  // both ends of every copy since the last question
     cudaError_t last = cudaSuccess;
 };
 State& S() {
@@ -102,6 +103,13 @@ void fake_counts(long* word, long* fp64) {
     *fp64 = S().fp64;
     S().word = S().fp64 = 0;
 }
+// how many of the pointers a copy started at, since the last call
+int fake_copied(const void* const* p, int n) {
+    int k = 0;
+    for (int i = 0; i < n; i++) k += std::count(S().copied.begin(), S().copied.end(), p[i]) > 0;
+    S().copied.clear();
+    return k;
+}
 
 // ---- runtime
 cudaError_t cudaMalloc(void** p, size_t n) { return take(p, n); }
@@ -118,6 +126,10 @@ cudaError_t cudaFreeHost(void* p) {
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
+    {
+        std::lock_guard<std::mutex> lk(S().mu);
+        S().copied.insert(S().copied.end(), {d, s});
+    }
     std::memcpy(d, s, n);
     return cudaSuccess;
 }
