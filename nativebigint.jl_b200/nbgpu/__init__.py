@@ -285,24 +285,46 @@ def radix_powtab(bb: int, x) -> list[np.ndarray]:
     return [out[offs[i]: offs[i + 1]].copy() for i in range(ne.value)]
 
 
+def _result_arrays(sizes: list[int]) -> list[np.ndarray]:
+    """Uninitialised arrays of `sizes` limbs: short ones are views of shared
+    allocations of up to 4 MB, the others have their own.  Neighbours come back in
+    one copy (60 products of up to 1500 limbs: 0.61 ms, 1.30 with an allocation
+    each), and a result that is kept does not keep a large batch (one allocation
+    for everything was no faster: 2000 products of up to 3000 limbs 12.4 ms
+    against 12.5, 300 of up to 65536 7.6 against 6.7 to 8.0)."""
+    shared, own = 1 << 19, 1 << 17  # limbs
+    out: list[np.ndarray] = []
+    i = 0
+    while i < len(sizes):
+        j, total = i, 0
+        while j < len(sizes) and sizes[j] < own and total + sizes[j] <= shared:
+            total += sizes[j]
+            j += 1
+        if j == i:
+            out.append(np.empty(sizes[i], dtype=np.uint64))
+            i += 1
+            continue
+        flat = np.empty(total, dtype=np.uint64)
+        off = 0
+        for n in sizes[i:j]:
+            out.append(flat[off: off + n])
+            off += n
+        i = j
+    return out
+
+
 def mul_batch(pairs) -> list[np.ndarray]:
     """Products of a list of (a, b) pairs (b None for a square), one batched
-    call; returns the m+n-limb results (views of one allocation)."""
+    call; returns the m+n-limb results (short ones may share an allocation of up
+    to 4 MB)."""
     pairs = [(_u64(a), None if b is None else _u64(b)) for a, b in pairs]
-    sizes = [a.size + (a.size if b is None else b.size) for a, b in pairs]
-    # one allocation for all results (views of it are returned): fresh pages of
-    # many small ones cost more than the products
-    flat = np.empty(sum(sizes), dtype=np.uint64)
-    ops, off = [], 0
+    res = _result_arrays([a.size + (a.size if b is None else b.size) for a, b in pairs])
     descs = (NbgDesc * len(pairs))()
-    for k, (a, b) in enumerate(pairs):
-        r = flat[off: off + sizes[k]]
-        off += sizes[k]
-        ops.append((a, b, r))
+    for k, ((a, b), r) in enumerate(zip(pairs, res)):
         descs[k] = NbgDesc(_ptr(r), _ptr(a), None if b is None else _ptr(b), a.size,
                            a.size if b is None else b.size, 0, 0)
     _check(lib().nbg_mul_batch(ctypes.cast(descs, ctypes.c_void_p), len(pairs)))
-    return [r for (_, _, r) in ops]
+    return res
 
 
 def uses_fpntt_mul(m: int, n: int) -> bool:

@@ -2,6 +2,7 @@
 library and the tensors' device side are stand-ins)."""
 import types
 
+import numpy as np
 import pytest
 
 import nbgpu
@@ -60,3 +61,23 @@ def test_calls_record_their_tensors(calls, stream, where):
     # raw addresses are the caller's
     nbgpu.mul_dev(1 << 20, 2 << 20, 4, 3 << 20, 4, s)
     nbgpu.mul_batch_dev(nbgpu.make_descs([(1 << 20, 2 << 20, None, 4, 4, 0, 0)]), s)
+
+
+def test_results_of_a_batch_do_not_hold_each_other(monkeypatch):
+    # a kept result keeps at most the few MB it was allocated with
+    fake = types.SimpleNamespace(nbg_mul_batch=lambda *a: nbgpu.NBG_OK)
+    monkeypatch.setattr(nbgpu, "lib", lambda: fake)
+    sizes = [1, 100, 200_000, 3000, 131_072, 70_000, 1_000_000] * 5 + [2000] * 1000
+    pairs = [(np.ones(n, np.uint64), None if n % 3 else np.ones(n, np.uint64)) for n in sizes]
+    res = nbgpu.mul_batch(pairs)
+    assert [r.size for r in res] == [2 * n for n in sizes]
+    spans = []
+    for r in res:
+        base = r if r.base is None else r.base
+        assert base.nbytes <= max(4 << 20, r.nbytes)
+        if r.nbytes >= 1 << 20:
+            assert r.base is None
+        spans.append((r.ctypes.data, r.ctypes.data + r.nbytes))
+    spans.sort()
+    assert all(x[1] <= y[0] for x, y in zip(spans, spans[1:]))
+    assert nbgpu.mul_batch(pairs[:1])[0].size == 2
