@@ -241,6 +241,25 @@ def kernel_peak(kernel: str, peak: dict) -> tuple[float, str, str]:
     return peak["dfma_per_s"], "fp64", "T FP64 instr/s"
 
 
+def compute_dtype(kernel: str) -> str:
+    """What the kernel computes in: 32-bit residues modulo 30-bit primes (k_w...)
+    or FP64 residues; the products are exact integers either way."""
+    return "u32" if kernel.startswith("k_w") else "f64"
+
+
+def per_call_latency(call, wait, n: int) -> tuple[list[float], list[float]]:
+    """Milliseconds of call(i) for i < n, each followed by wait(): until the
+    call returned, and until its results were there."""
+    enqueue, done = [], []
+    for i in range(n):
+        t0 = time.perf_counter()
+        call(i)
+        enqueue.append(1e3 * (time.perf_counter() - t0))
+        wait()
+        done.append(1e3 * (time.perf_counter() - t0))
+    return enqueue, done
+
+
 def rank_share(W: dict, rank: int, world: int, scaling: str, params) -> list[int]:
     """Products of workload W that this rank runs.  weak: every rank draws its
     own batch (seed + rank), so it runs all of W.  strong: every rank draws the
@@ -414,27 +433,28 @@ def run_ours(args, rank: int, world: int) -> None:
         }
 
         # unbatched: the same products one call each (device buffers)
-        lat = []
         nb = min(args.unbatched, count)
         unbatched = None
         one = (nbgpu.NbgDesc * 1)()
-        e0 = torch.cuda.Event(enable_timing=True)
-        e1 = torch.cuda.Event(enable_timing=True)
         torch.cuda.synchronize()
         t0 = time.perf_counter()
         ul = 0
         for i in range(nb if nb > 0 else 0):
             one[0] = descs[i]
-            c0 = time.perf_counter()
             nbgpu.mul_batch_dev(one, s)
-            lat.append(1e3 * (time.perf_counter() - c0))
             ul += int(W["m"][mine[i]] + W["n"][mine[i]])
         torch.cuda.synchronize()
         un_s = time.perf_counter() - t0
         if nb > 0:
+            # each call waited for (the calls return before their kernels have run)
+            def one_call(i):
+                one[0] = descs[i]
+                nbgpu.mul_batch_dev(one, s)
+
+            enq, lat = per_call_latency(one_call, torch.cuda.synchronize, min(nb, 2000))
             unbatched = {"value": ul / un_s, "unit": "output limbs/s", "products": nb,
                          "p50_ms": float(np.percentile(lat, 50)), "p99_ms": float(np.percentile(lat, 99)),
-                         "products_per_s": nb / un_s}
+                         "enqueue_p50_ms": float(np.percentile(enq, 50)), "products_per_s": nb / un_s}
 
         # e2e: host buffers through nbg_mul_batch (pinned), copies inside the call
         pin_in = torch.from_numpy(limbs).pin_memory()
@@ -499,10 +519,10 @@ def run_ours(args, rank: int, world: int) -> None:
         line = {
             "metric": METRIC, "value": value, "unit": "output limbs/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": total_ms_max / args.steps, "higher_is_better": True,
-            "scaling": args.scaling, "vs_baseline": None, "dtype": "f64", "data": "synthetic",
+            "scaling": args.scaling, "vs_baseline": None, "dtype": compute_dtype(dom), "data": "synthetic",
             "config": {"workload": WORKLOAD, "products": job_products, "products_per_rank": count,
                        "seed": args.seed,
-                       "output_limbs_per_step": out_limbs, "l2": "inputs larger than L2 (0.7 GB operands, 9 GB workspace)",
+                       "output_limbs_per_step": out_limbs, "l2": "inputs larger than L2 (1.3 GB of operands, 1.5 GB of results, residues between them)",
                        "parallelism": (f"{world} ranks, each its own seeded batch (seed + rank), no collective"
                                        if args.scaling == "weak" else
                                        f"one batch split by LPT cost over {world} ranks, no collective")},
@@ -682,7 +702,7 @@ def run_serve(args) -> None:
             "batches": st["batches"], "mean_batch_requests": st["mean_batch_requests"],
             "pool_as_one_batch": {"value": pool_batch_rate, "unit": "output limbs/s"},
             "bitexact": {"checked_vs_gmp": count, "mismatches": mismatches},
-            "dtype": "f64", "data": "synthetic", "n_gpus": 1,
+            "dtype": "u32", "data": "synthetic", "n_gpus": 1,
             "config": {"workload": SERVE_WORKLOAD, "pool_products": P, "pool_output_limbs": out_total,
                        "hbm_budget_gb": args.serve_budget_gb, "seconds": args.serve_seconds, "seed": args.seed,
                        "max_hold_us": args.serve_hold_us, "ring_copies": RING,
@@ -780,7 +800,7 @@ def run_powmod(args) -> None:
         "metric": "Barrett powermod chains/s (256 chains, 16384-bit moduli, 4096-bit exponents), bit-exact",
         "mode": "powmod", "impl": "ours", "value": n / med, "unit": "chains/s", "n_gpus": 1,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * med, "higher_is_better": True,
-        "dtype": "f64", "data": "synthetic",
+        "dtype": "u32", "data": "synthetic",
         "config": {"workload": POWMOD_WORKLOAD, "chains": n, "k": k, "exponent_bits": 64 * le, "seed": args.seed,
                    "timing": "wall clock around each synchronous call (setup, all steps, result copy)"},
         "e2e": {"value": n / statistics.median(e2e_t), "unit": "chains/s",
@@ -882,7 +902,8 @@ def single_case(lg: int, sq: bool, kind: str, reps: int, peak: dict, s, check: s
         d["launches"] += 1
     for k, d in per_kernel.items():
         d["frac"] = d["alg_ops"] / (d["ms"] / 1e3) / kernel_peak(k, peak)[0] if d["ms"] else 0.0
-    peak, bound, unit = kernel_peak(max(per_kernel, key=lambda k: per_kernel[k]["ms"]), peak)
+    dom = max(per_kernel, key=lambda k: per_kernel[k]["ms"])
+    peak, bound, unit = kernel_peak(dom, peak)
     bt.close()
     got = r.cpu().numpy()
     if check == "gmp":
@@ -907,7 +928,7 @@ def single_case(lg: int, sq: bool, kind: str, reps: int, peak: dict, s, check: s
     del da, db, r
     torch.cuda.empty_cache()
     return {
-        "op": "sqr" if sq else "mul", "limbs": n, "pattern": kind,
+        "op": "sqr" if sq else "mul", "limbs": n, "pattern": kind, "dtype": compute_dtype(dom),
         "per_call_p50_ms": float(np.percentile(t_call, 50)), "per_call_p99_ms": float(np.percentile(t_call, 99)),
         "graph_p50_ms": p50g, "graph_p99_ms": float(np.percentile(t_graph, 99)),
         "output_limbs_per_s": 2 * n / (p50g / 1e3),
@@ -951,7 +972,7 @@ def run_single(args) -> None:
                                   gmp_time=kind == "uniform" and args.single_check == "gmp")
                 line = {"mode": "single", "impl": "ours",
                         "metric": "single large product time, bit-exact", "unit": "ms", "higher_is_better": False,
-                        **rec, "dtype": "f64", "data": "synthetic", "n_gpus": 1}
+                        **rec, "data": "synthetic", "n_gpus": 1}
                 print(json.dumps(line), flush=True)
 
 
