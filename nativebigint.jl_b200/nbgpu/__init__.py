@@ -286,13 +286,13 @@ def radix_powtab(bb: int, x) -> list[np.ndarray]:
 
 
 def _result_arrays(sizes: list[int]) -> list[np.ndarray]:
-    """Uninitialised arrays of `sizes` limbs: short ones are views of shared
-    allocations of up to 4 MB, the others have their own.  Neighbours come back in
-    one copy (60 products of up to 1500 limbs: 0.61 ms, 1.30 with an allocation
-    each), and a result that is kept does not keep a large batch (one allocation
-    for everything was no faster: 2000 products of up to 3000 limbs 12.4 ms
-    against 12.5, 300 of up to 65536 7.6 against 6.7 to 8.0)."""
-    shared, own = 1 << 19, 1 << 17  # limbs
+    """Uninitialised arrays of `sizes` limbs: those of less than 4 MB are views of
+    shared allocations of up to 8 MB, the others have their own.  Neighbours come
+    back in one copy (60 products of up to 1500 limbs: 0.55 ms, 1.20 with an
+    allocation each) into large pages (numpy asks for them from 4 MB on: 60 mixed
+    products into fresh memory 2.6 ms, 3.1 in 4 MB allocations), and a result that
+    is kept does not keep a large batch."""
+    shared, own = 1 << 20, 1 << 19  # limbs
     out: list[np.ndarray] = []
     i = 0
     while i < len(sizes):
@@ -316,7 +316,7 @@ def _result_arrays(sizes: list[int]) -> list[np.ndarray]:
 def mul_batch(pairs) -> list[np.ndarray]:
     """Products of a list of (a, b) pairs (b None for a square), one batched
     call; returns the m+n-limb results (short ones may share an allocation of up
-    to 4 MB)."""
+    to 8 MB)."""
     pairs = [(_u64(a), None if b is None else _u64(b)) for a, b in pairs]
     res = _result_arrays([a.size + (a.size if b is None else b.size) for a, b in pairs])
     descs = (NbgDesc * len(pairs))()

@@ -74,8 +74,8 @@ def test_results_of_a_batch_do_not_hold_each_other(monkeypatch):
     spans = []
     for r in res:
         base = r if r.base is None else r.base
-        assert base.nbytes <= max(4 << 20, r.nbytes)
-        if r.nbytes >= 1 << 20:
+        assert base.nbytes <= max(8 << 20, r.nbytes)
+        if r.nbytes >= 4 << 20:
             assert r.base is None
         spans.append((r.ctypes.data, r.ctypes.data + r.nbytes))
     spans.sort()
