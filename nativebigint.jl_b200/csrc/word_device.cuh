@@ -363,9 +363,9 @@ __device__ __forceinline__ uint32_t gp_join(uint32_t lower, uint32_t upper) {
     return ((upper & 1u) | ((upper >> 1) & lower & 1u)) | (upper & lower & 2u);
 }
 
-// Carry-lookahead over the threads, then over the warps: the carry into this
-// thread's part for a carry of 0 into the CTA's run, and the whole run's state.
-__device__ __forceinline__ uint32_t cta_scan(uint32_t agg, uint32_t* wagg, uint32_t& total) {
+// Carry-lookahead over the threads, then over the warps: the state of the parts
+// below this thread's, and the whole run's.
+__device__ __forceinline__ uint32_t cta_state(uint32_t agg, uint32_t* wagg, uint32_t& total) {
     const int lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
     uint32_t incl = agg;
 #pragma unroll
@@ -385,7 +385,11 @@ __device__ __forceinline__ uint32_t cta_scan(uint32_t agg, uint32_t* wagg, uint3
     const uint32_t below = __shfl_sync(0xffffffffu, w, wid ? wid - 1 : 0);
     uint32_t excl = __shfl_up_sync(0xffffffffu, incl, 1);
     if (lane == 0) excl = 2u;
-    return gp_join(wid ? below : 2u, excl) & 1u;
+    return gp_join(wid ? below : 2u, excl);
+}
+// The carry into this thread's part for a carry of 0 into the CTA's run.
+__device__ __forceinline__ uint32_t cta_scan(uint32_t agg, uint32_t* wagg, uint32_t& total) {
+    return cta_state(agg, wagg, total) & 1u;
 }
 
 __device__ __forceinline__ void add_carry(uint64_t* own, uint64_t cin) {

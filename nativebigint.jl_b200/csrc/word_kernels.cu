@@ -560,51 +560,95 @@ __global__ void __launch_bounds__(WT, 4) k_wblock(const __grid_constant__ WArgs 
 // carries between a product's tiles (runs of k_wtail, tiles of the FP64 unpack;
 // P.tl limbs each)
 
-// Tiles [k0, k0 + 32) by one warp.  The carry into the first comes from the last
-// lower tile that does not propagate (almost always the one before); a tile's
-// carry stops at its first limb unless that limb is all ones, and then the warp
-// walks the run.  Only r is written, each tile by one warp.  (Reads go to L2:
-// other CTAs of a running kernel may have written what is read.)
-__device__ __forceinline__ void carry_tiles(const DProd& P, int64_t k0) {
+// A warp's 32 tiles, one per lane (k: this lane's, a: its state, carry: whether
+// one comes in).  It stops at the first limb unless that is all ones.  A tile that
+// propagates is all ones and becomes zeros, unread, runs of such tiles together;
+// in the others the warp finds the end of the run.  Only r is written, each tile
+// by one warp.  (Reads go to L2: other CTAs of a running kernel may have written
+// what is read.)  Bound by the stores; walking every tile, 32 limbs at a time, and
+// looking down 32 tiles at a time took 4096-limb all-ones squares 58 us per call,
+// 65536 210 and 2^22 1175, now 17, 39 and 673 (uniform limbs 15, 22, 640).
+__device__ __forceinline__ void carry_fix(const DProd& P, int64_t k, uint32_t a, bool carry) {
     const int lane = (int)threadIdx.x & 31;
-    const int64_t nt = P.ntl;
-    uint32_t cin = 0;
-    for (int64_t k = k0 - 32; k >= 0; k -= 32) {
-        const uint32_t a = __ldcg(P.agg + k + lane);
-        const unsigned stop = __ballot_sync(0xffffffffu, !(a & 2u));
-        if (stop) {
-            cin = __shfl_sync(0xffffffffu, a, 31 - __clz(stop)) & 1u;
-            break;
-        }
-    }
-    const int64_t k = k0 + lane;
-    uint32_t incl = k < nt ? __ldcg(P.agg + k) : 0u;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t o = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl = gp_join(o, incl);
-    }
-    uint32_t excl = __shfl_up_sync(0xffffffffu, incl, 1);
-    if (lane == 0) excl = 2u;
+    const int64_t kw = k - lane;
+    const bool ones = carry && (a & 2u);
     bool walk = false;
-    if (k < nt && (gp_join(cin, excl) & 1u)) {
+    if (carry && !ones) {
         uint64_t* w = P.r + k * P.tl;
         const uint64_t v = __ldcg(w);
         if (v != ~0ULL) *w = v + 1;
         else walk = true;
     }
+    for (unsigned m = __ballot_sync(0xffffffffu, ones); m;) {
+        const int s = __ffs(m) - 1, up = __ffs(~(m >> s));
+        const int len = up ? up - 1 : 32;  // tiles s .. s + len - 1
+        const int64_t b1 = (kw + s + len) * P.tl;
+        for (int64_t w = (kw + s) * P.tl + lane; w < b1; w += 32) P.r[w] = 0;
+        m &= len == 32 ? 0u : ~(((1u << len) - 1) << s);
+    }
     for (unsigned m = __ballot_sync(0xffffffffu, walk); m; m &= m - 1) {
-        const int64_t b0 = (k0 + __ffs(m) - 1) * P.tl, b1 = min(b0 + (int64_t)P.tl, P.rn);
-        for (int64_t w = b0; w < b1; w += 32) {
-            const int64_t wl = w + lane;
-            const uint64_t v = wl < b1 ? __ldcg(P.r + wl) : 0ULL;  // past the tile: stops the run
-            const unsigned stop = __ballot_sync(0xffffffffu, v != ~0ULL);
-            const int e = stop ? __ffs(stop) - 1 : 32;
-            if (lane < e) P.r[wl] = 0;
-            else if (lane == e && wl < b1) P.r[wl] = v + 1;
-            if (stop) break;
+        const int64_t b0 = (kw + __ffs(m) - 1) * P.tl, b1 = min(b0 + (int64_t)P.tl, P.rn);
+        bool end = false;
+        for (int64_t w = b0 + lane; !end && w - lane < b1; w += 128) {
+            uint64_t v[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) v[q] = w + 32 * q < b1 ? __ldcg(P.r + w + 32 * q) : 0ULL;  // past the tile: ends the run
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (end) break;
+                const unsigned stop = __ballot_sync(0xffffffffu, v[q] != ~0ULL);
+                const int e = stop ? __ffs(stop) - 1 : 32;
+                if (lane < e) P.r[w + 32 * q] = 0;
+                else if (lane == e && w + 32 * q < b1) P.r[w + 32 * q] = v[q] + 1;
+                end = stop != 0;
+            }
         }
     }
+}
+
+// Every carry of a product of few tiles, by one CTA.
+template <int NT>
+__device__ __forceinline__ void carry_all(const DProd& P, uint32_t* wagg) {
+    uint32_t cin = 0;
+    for (int64_t k0 = 0; k0 < P.ntl; k0 += NT) {
+        const int64_t k = k0 + (int)threadIdx.x;
+        const uint32_t a = k < P.ntl ? __ldcg(P.agg + k) : 0u;
+        __syncthreads();  // wagg's previous readers
+        uint32_t total;
+        const uint32_t st = cta_state(a, wagg, total);
+        carry_fix(P, k, a, k < P.ntl && (gp_join(cin, st) & 1u));
+        cin = gp_join(cin, total) & 1u;
+    }
+}
+
+// The carry into tile k0: of the last lower tile that does not propagate, almost
+// always among the 32 before, which every warp looks at; past those the CTA
+// goes down 16 tiles per thread at a time.
+__device__ __forceinline__ uint32_t carry_below(const DProd& P, int64_t k0, uint32_t* found) {
+    const int lane = (int)threadIdx.x & 31;
+    {
+        const uint32_t a = k0 > lane ? __ldcg(P.agg + (k0 - 1 - lane)) : 0u;
+        const unsigned stop = __ballot_sync(0xffffffffu, !(a & 2u));
+        if (stop) return __shfl_sync(0xffffffffu, a, __ffs(stop) - 1) & 1u;
+    }
+    for (int64_t top = k0 - 33; top >= 0; top -= 16 * WT) {  // the whole CTA: all warps saw the same 32
+        uint32_t best = 0;  // greatest (tile, generates) that does not propagate, plus one
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            const int64_t i = top - (j * WT + (int)threadIdx.x);
+            const uint32_t a = i >= 0 ? __ldcg(P.agg + i) : 2u;
+            if (!(a & 2u)) best = max(best, ((uint32_t)i << 1 | (a & 1u)) + 1u);
+        }
+        best = __reduce_max_sync(0xffffffffu, best);
+        if (threadIdx.x == 0) *found = 0;
+        __syncthreads();
+        if (lane == 0 && best) atomicMax(found, best);
+        __syncthreads();
+        best = *found;
+        __syncthreads();
+        if (best) return (best - 1) & 1u;
+    }
+    return 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -762,7 +806,8 @@ __global__ void __launch_bounds__(WTail<ODD, LJ, SET>::NT, 1024 / WTail<ODD, LJ,
     for (int64_t i = (int64_t)N + 1 + (int64_t)local * T::NT + tid; i < rn; i += (int64_t)(cols / T::CW) * T::NT) P.r[i] = 0;
     if (!fused) return;
     // one product of few runs: its last CTA carries between them instead of another
-    // launch (in batches the fences cost 10% of the pass, so k_wcarry does it there), and only if some run carries out at all (a limb sum within 3 of
+    // launch (in batches the fences cost 10% of the pass, so k_wcarry does it
+    // there), and only if some run carries out at all (a limb sum within 3 of
     // 2^64, so hardly ever but for operands made of ones or zeros)
     __shared__ bool last;
     __threadfence();
@@ -772,16 +817,20 @@ __global__ void __launch_bounds__(WTail<ODD, LJ, SET>::NT, 1024 / WTail<ODD, LJ,
         __threadfence();
     }
     __syncthreads();
-    if (last && __ldcg(P.agg + P.ntl + 1) != 0)
-        for (int64_t k0 = 32 * (tid >> 5); k0 < P.ntl; k0 += 32 * (T::NT / 32)) carry_tiles(P, k0);
+    __shared__ uint32_t wagg[T::NT / 32];
+    if (last && __ldcg(P.agg + P.ntl + 1) != 0) carry_all<T::NT>(P, wagg);
 }
 
 __global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) {
     int local;
     const DProd& P = wjob(A, local);
     wait_previous();
-    const int64_t k0 = ((int64_t)local * (WT / 32) + (threadIdx.x >> 5)) * 32;
-    if (k0 < P.ntl) carry_tiles(P, k0);
+    __shared__ uint32_t wagg[WT / 32], found;
+    const int64_t k0 = (int64_t)local * WT, k = k0 + (int)threadIdx.x;  // a tile per thread
+    const uint32_t a = k < P.ntl ? __ldcg(P.agg + k) : 0u;
+    uint32_t total;
+    const uint32_t cin = carry_below(P, k0, &found), st = cta_state(a, wagg, total);
+    carry_fix(P, k, a, k < P.ntl && (gp_join(cin, st) & 1u));
 }
 
 // ---------------------------------------------------------------------------

@@ -83,3 +83,63 @@ def test_temporaries_dropped_after_the_call(gpu_lib, how, n):
     want = O.gmp_mul(a, b)
     for r in rs:
         assert np.array_equal(r.cpu().numpy().view(np.uint64), want)
+
+
+def _carry_operands(n, rng):
+    ones = np.full(n, 2**64 - 1, dtype=np.uint64)
+    low = np.zeros(n, dtype=np.uint64)  # the carry starts at the bottom, or in the middle
+    low[0] = low[-1] = 1
+    mid = low.copy()
+    mid[n // 2] = 1
+    short = ones[: n // 5 + 1].copy()
+    part = ones.copy()  # runs that end inside a tile, at every distance from its start
+    part[rng.integers(0, n, n // 40)] = 2**64 - 2
+    return [(ones, None), (ones, low), (ones, mid), (ones, short), (part, low), (low, None)]
+
+
+@pytest.mark.parametrize("n", [1537, 2111, 4096, 8200, 40_000, 131_073, 1 << 21])
+def test_long_carries(gpu_lib, n):
+    # carries through thousands of tiles (one CTA's fix up to 2048 of them, a
+    # launch above, which looks 4096 tiles down at a time), alone and in a batch
+    pairs = _carry_operands(n, np.random.default_rng(n))
+    want = [O.gmp_sqr(a) if b is None else O.gmp_mul(a, b) for a, b in pairs]
+    dev = [tuple(None if x is None else torch.from_numpy(x).cuda() for x in p) for p in pairs]
+    for off in (0, 1):  # results at 16 and at 8 bytes
+        rs = [torch.zeros(w.size + 2, dtype=torch.uint64, device="cuda")[off:] for w in want]
+        torch.cuda.synchronize()
+        for r, (a, b) in zip(rs, dev):
+            if b is None:
+                gpu_lib.sqr_dev(r, a, a.numel())
+            else:
+                gpu_lib.mul_dev(r, a, a.numel(), b, b.numel())
+        torch.cuda.synchronize()
+        for k, (r, w) in enumerate(zip(rs, want)):
+            got = r.cpu().numpy()
+            assert np.array_equal(got[: w.size], w), k
+            assert not got[w.size:].any(), k
+    if n < 1 << 20:
+        for k, (g, w) in enumerate(zip(gpu_lib.mul_batch(pairs), want)):
+            assert np.array_equal(g, w), k
+
+
+@pytest.mark.parametrize("n", [4096, 65_536, 131_072])
+def test_carry_runs_are_not_the_products_cost(gpu_lib, n):
+    # all-ones operands (every tile passes a carry on) against uniform ones:
+    # their carries, tile by tile in one warp, once took eight times the product
+    rng = np.random.default_rng(n)
+    r = torch.zeros(2 * n, dtype=torch.uint64, device="cuda")
+    times = []
+    for a in (rand_limbs(rng, n), np.full(n, 2**64 - 1, dtype=np.uint64)):
+        da = torch.from_numpy(a).cuda()
+        e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        best = 1e9
+        for _ in range(6):
+            torch.cuda.synchronize()
+            e0.record()
+            for _ in range(40):
+                gpu_lib.sqr_dev(r, da, n)
+            e1.record()
+            e1.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        times.append(best)
+    assert times[1] < 4 * times[0]
