@@ -831,7 +831,7 @@ size_t fp64_work_bytes(const ProdIn& q) {
 bool word_product(const Engine& E, const ProdIn& q, WordShape* s, bool coarse) {
     if (!E.word_ok || q.fp64 || q.keep_b) return false;
     const int64_t la = eff_limbs(q.m, q.bits_a), lb = q.sqr ? la : eff_limbs(q.n, q.bits_b);
-    return word_shape(la + lb - 1, *s, coarse) && (s->set || std::min(la, lb) <= WORD_MIN_OPERAND_MAX);
+    return word_shape(la + lb - 1, *s, coarse);
 }
 
 bool word_to_fp64(const Engine& E, std::vector<ProdIn>& in) {

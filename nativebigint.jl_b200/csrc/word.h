@@ -21,7 +21,8 @@
 namespace nbg {
 
 // Prime sets.  Set 0 (p = 1 mod 105 * 2^18, product above 2^149) serves
-// lengths odd * 2^k with k <= 20 and any min(m, n) <= 2^21 limbs.  Above 3.6M
+// lengths odd * 2^k up to 7 * 2^19: of m + n - 1 coefficients each is below
+// min(m, n) * 2^128, and min(m, n) below 2^21.  Above 3.6M
 // points the coefficients need a sixth prime and the roots more twos: set 1
 // (p = 1 mod 3 * 2^22) for 3 * 2^k, set 2 (p = 1 mod 2^23) for 2^k, k <= 25;
 // their products exceed 2^176.
@@ -43,7 +44,6 @@ constexpr bool word_pack_ok(int set) {
     return true;
 }
 constexpr int WORD_MAX_LOG2 = 20;               // set 0: k <= 20 (leaves at level k - 2 <= 18)
-constexpr int64_t WORD_MIN_OPERAND_MAX = int64_t(1) << 21;  // set 0
 
 // Shape of a word product's transform: N = odd * 2^lj * M.  Blocks of M = 2^lm
 // consecutive values (each one subtree) are transformed in shared memory;

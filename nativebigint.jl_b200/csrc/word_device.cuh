@@ -17,7 +17,7 @@ struct WConst {
     uint32_t p[WPR_MAX], pinv[WPR_MAX];
     uint32_t half[WPR_MAX];          // the multiple of p nearest to 2^31
     Tw r3[WPR_MAX];                  // e(1/3)
-    Tw r5[WPR_MAX][5];               // -1/4, (c1-c2)/2, f1, f2 of e(1/5) (see dft5); [4] unused
+    Tw r5[WPR_MAX][4];               // -1/4, (c1-c2)/2, f1, f2 of e(1/5) (see dft5)
     uint32_t c7[WPR_MAX][3], f7[WPR_MAX][3];  // cosine and sine halves of e(j/7) in 2^32 form
     uint32_t wt[WPR_MAX][WPR_MAX];       // words of W_i = p_0 ... p_(i-1) (i words)
     uint32_t gar[WPR_MAX][WPR_MAX];      // mixed radix: gar[i][j] = -W_j / W_i mod p_i in 2^32 form (j < i)

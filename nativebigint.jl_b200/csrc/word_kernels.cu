@@ -1,5 +1,5 @@
 // word_kernels.cu — kernels of the word products (word.h): products through
-// transforms modulo five 30-bit primes, one coefficient per 64-bit limb.
+// transforms modulo five or six 30-bit primes, one coefficient per 64-bit limb.
 //
 //   k_wcol_fwd  limbs -> residues, the radix-`odd` step and the first lj levels
 //               of one column's R rows, in registers
@@ -19,7 +19,6 @@
 #include "word_device.cuh"
 
 namespace nbg {
-
 
 // ---------------------------------------------------------------------------
 // host constants
@@ -71,21 +70,21 @@ static void fill_set(int set, WConst& h) {
         h.pinv[i] = x;
         h.half[i] = (uint32_t)(((uint64_t(1) << 31) + p / 2) / p * p);
         if ((p - 1) % 3 == 0) h.r3[i] = mk(pw(g, (p - 1) / 3, p), p);
-        if (set == 0) {
-        const uint64_t h2 = inv(2, p), w5 = pw(g, (p - 1) / 5, p), w7 = pw(g, (p - 1) / 7, p);
-        auto half = [&](uint64_t w, int a, int b, bool minus) {  // (w^a +- w^b) / 2
-            const uint64_t x1 = pw(w, a, p), x2 = pw(w, b, p);
-            return (x1 + (minus ? p - x2 : x2)) % p * h2 % p;
-        };
-        const uint64_t c1 = half(w5, 1, 4, false), c2 = half(w5, 2, 3, false);
-        h.r5[i][0] = mk((p - inv(4, p)) % p, p);
-        h.r5[i][1] = mk((c1 + p - c2) % p * h2 % p, p);
-        h.r5[i][2] = mk(half(w5, 1, 4, true), p);
-        h.r5[i][3] = mk(half(w5, 2, 3, true), p);
-        for (int k = 0; k < 3; k++) {
-            h.c7[i][k] = mont(half(w7, k + 1, 6 - k, false), p);
-            h.f7[i][k] = mont(half(w7, k + 1, 6 - k, true), p);
-        }
+        if (set == 0) {  // radix 5 and 7
+            const uint64_t h2 = inv(2, p), w5 = pw(g, (p - 1) / 5, p), w7 = pw(g, (p - 1) / 7, p);
+            auto half = [&](uint64_t w, int a, int b, bool minus) {  // (w^a +- w^b) / 2
+                const uint64_t x1 = pw(w, a, p), x2 = pw(w, b, p);
+                return (x1 + (minus ? p - x2 : x2)) % p * h2 % p;
+            };
+            const uint64_t c1 = half(w5, 1, 4, false), c2 = half(w5, 2, 3, false);
+            h.r5[i][0] = mk((p - inv(4, p)) % p, p);
+            h.r5[i][1] = mk((c1 + p - c2) % p * h2 % p, p);
+            h.r5[i][2] = mk(half(w5, 1, 4, true), p);
+            h.r5[i][3] = mk(half(w5, 2, 3, true), p);
+            for (int k = 0; k < 3; k++) {
+                h.c7[i][k] = mont(half(w7, k + 1, 6 - k, false), p);
+                h.f7[i][k] = mont(half(w7, k + 1, 6 - k, true), p);
+            }
         }
         uint64_t Wi = 1;
         for (int t = 0; t < i; t++) Wi = Wi * (P[t] % p) % p;
@@ -362,10 +361,9 @@ __global__ void __launch_bounds__(WT, 4) k_wcol_fwd(const __grid_constant__ WArg
     for (int r = 0; r < R; r++) dst[(size_t)r << lm] = x[r];  // no let_next: it cost the batches' passes 4%
 }
 
-// Middle passes: the 2^J rows (2^lm apart) of one column of a segment, the
-// subtree of the segment's node, above blocks of 4096.  In place; all columns of a segment share
-// their constants.
-// Column pass `id` of 16-value threads: its values' first word, constants and node.
+// A middle pass works on segments of 2^j rows (2^12 apart: more than 32 rows only
+// stand above blocks of 4096), each the subtree of a node, in place; all columns of
+// a segment share their constants.  A segment's first word, constants and node:
 struct MidJob {
     uint32_t* x;
     const Tw* tab;
@@ -390,9 +388,10 @@ __device__ __forceinline__ MidJob mid_job(const DProd& P, int item, int j) {
     return J;
 }
 
+// The 2^J rows of one column, in registers.
 template <int J, bool FWD, int SET>
 __global__ void __launch_bounds__(WT) k_wmid(const __grid_constant__ WArgs A) {
-    constexpr int lm = 12;  // more than 32 rows only stand above 4096-value blocks
+    constexpr int lm = 12;
     int local;
     const DProd& P = wjob(A, local);
     wait_previous();
@@ -939,8 +938,9 @@ static WLaunch big_kernel(int kind, int variant) {
         case JK_WBLOCK: return WLaunch{k_wblock<SET>, WT, 0};
         case JK_WMID_FWD:
         case JK_WMID_REV:
+            if constexpr (SET == 2)  // (set 1 has 64 middle rows at least)
+                if (variant == 5) return WLaunch{kind == JK_WMID_FWD ? k_wmid<5, true, SET> : k_wmid<5, false, SET>, WT, 0};
             switch (variant) {
-                case 5: return WLaunch{kind == JK_WMID_FWD ? k_wmid<5, true, SET> : k_wmid<5, false, SET>, WT, 0};
                 case 6: return mid_sm_kernel<6, SET>(kind);
                 case 7: return mid_sm_kernel<7, SET>(kind);
                 case 8: return mid_sm_kernel<8, SET>(kind);
