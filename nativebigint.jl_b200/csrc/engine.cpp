@@ -954,11 +954,15 @@ int build_batch(Engine& E, const ProdIn* in, int64_t count, BatchBuild& bb) {
         WordShape s;
     };
     std::vector<WordProd> words;  // products of the word engine
-    // Small batches of some dozens of products take few transform lengths: their
-    // launches are short, and a launch costs the host about 5 us (256 products,
-    // 4.7M limbs: 59 launches, 599 us, against 32 launches, 536 us).  Large ones
-    // take every length (10,000 products, 185M limbs: 12.2 ms against 12.9).
-    constexpr int64_t COARSE_LIMBS = int64_t(1) << 24;
+    // Batches of some dozens of products take few transform lengths while their
+    // launches are short: a launch costs the host about 5 us, and the GPU a tail.
+    // us of a fresh batch / a replay, all lengths against few (operands log-uniform
+    // in 152-65536 limbs unless said): 16 products 135/72 against 141/82, 24 148/82
+    // against 132/73, 100 331/256 against 267/213, 256 (5.0M output limbs) 545/448
+    // against 500/416, 600 (9.7M) 885/745 against 867/743; 600 of 1000-20000
+    // limbs (6.0M) 588/458 against 603/486; 256 of 5000-65536 (10.3M) 800/733
+    // against 811/761; 1500 of 1000-20000 (15M) 1374/1063 against 1441/1146.
+    constexpr int64_t COARSE_LIMBS = int64_t(5) << 20;
     int64_t out_limbs = 0;
     for (int64_t k = 0; k < count && out_limbs < COARSE_LIMBS; k++) out_limbs += in[k].m + (in[k].sqr ? in[k].m : in[k].n);
     const bool coarse = count >= 24 && out_limbs < COARSE_LIMBS;

@@ -211,6 +211,10 @@ static constexpr ChainKernel chain() {
 static const ChainKernel CHAINS[] = {chain<1, 6>(), chain<1, 7>(), chain<3, 6>(), chain<1, 8>(),  chain<3, 7>(),
                                      chain<1, 9>(), chain<3, 8>(), chain<1, 10>(), chain<3, 9>()};
 
+// Every modulus that fits, at any number of chains: product batches were slower
+// wherever measured (ms per call, batches against chains, 512-bit exponents: 256
+// limbs 1 chain 45/8, 64 60/11, 600 155/56; 400 limbs 8 50/13, 300 141/54; 512
+// limbs 600 372/97; 513 limbs 8 63/19; 768 limbs 1 78/19, 148 247/38, 300 474/89).
 static const ChainKernel* chain_for(int64_t k) {
     for (const ChainKernel& c : CHAINS)
         if (((int64_t)c.odd << c.lm) >= 2 * k) return &c;

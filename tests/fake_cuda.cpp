@@ -29,6 +29,7 @@ struct State {
     bool marked = false;
     int unordered = 0;       // launches after the mark not ordered after all before it
     long word = 0, fp64 = 0;
+    bool coarse = false;  // the lengths the last product was offered
     std::vector<const void*> copied;  // both ends of every copy since the last question
     cudaError_t last = cudaSuccess;
 };
@@ -103,6 +104,7 @@ void fake_counts(long* word, long* fp64) {
     *fp64 = S().fp64;
     S().word = S().fp64 = 0;
 }
+int fake_coarse() { return S().coarse; }
 // how many of the pointers a copy started at, since the last call
 int fake_copied(const void* const* p, int n) {
     int k = 0;
@@ -262,7 +264,8 @@ cudaError_t launch_topbits(const DProd* p, int64_t n, int64_t* bits, cudaStream_
 }
 
 // the real lengths, without their splits into passes
-bool word_shape(int64_t nconv, WordShape& s, bool) {
+bool word_shape(int64_t nconv, WordShape& s, bool coarse) {
+    S().coarse = coarse;
     int64_t best = INT64_MAX;
     auto take = [&](int odd, int k, int set) {
         const int64_t N = (int64_t)odd << k;

@@ -187,3 +187,13 @@ def test_pageable_operands_of_one_product(fake, m, n, direct):
     fake.fake_copied(p, 3)
     assert fake.nbg_mul_batch(*descs((p[0], p[1], p[2], m, n, 0, 0))[:2]) == NBG_OK
     assert fake.fake_copied(p, 3) == direct
+
+
+@pytest.mark.parametrize("count,limbs,coarse", [(23, 1000, 0), (24, 1000, 1), (256, 9000, 1), (100, 25_000, 1),
+                                                (600, 5000, 0), (256, 20_000, 0), (10_000, 9000, 0)])
+def test_batches_take_few_lengths_while_launches_weigh_more(fake, count, limbs, coarse):
+    # from 24 products on, up to 5M output limbs
+    bt = ctypes.c_void_p()
+    d = descs(*((R + (k << 24), A, B, limbs, limbs, 64 * limbs, 64 * limbs) for k in range(count)))
+    assert fake.nbg_batch_create(*d[:2], ctypes.byref(bt)) == NBG_OK
+    assert fake.fake_coarse() == coarse
