@@ -275,9 +275,16 @@ struct WArgs {
 // A kernel of a single product may be on the GPU before the one it follows has
 // finished (programmatic launch): nothing that one wrote, and nothing it may
 // still read, is touched before this, and what it wrote (operands, which may be
-// the result before, and residues) is read by __ldcg: the read-only path wants
+// the result before, and residues) is not read by __ldg: the read-only path wants
 // data that nothing writes while this kernel is on the GPU.
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A pointer whose loads stay below this point (a wait or a barrier before it): the
+// compiler may take the load intrinsics for functions of the address alone.
+template <class T>
+__device__ __forceinline__ T* from_here(T* p) {
+    asm volatile("" : "+l"(p) : : "memory");
+    return p;
+}
 // The next kernel's CTAs may come once every CTA is here: near the end, so that
 // they spread over the SMs as those empty (from the start of the kernel, the
 // blocks of a 65536 x 65521-limb product piled up: 31 -> 38 us per call).
@@ -327,7 +334,7 @@ __global__ void __launch_bounds__(WT, 4) k_wcol_fwd(const __grid_constant__ WArg
     if (pi >= NP || (isb && P.sqr)) return;
     const int n = (int)(isb ? P.ncb : P.nca);
     const int rows = (n + (1 << lm) - 1) >> lm;
-    const uint64_t* src = (isb ? P.b : P.a) + c;
+    const uint64_t* src = from_here(isb ? P.b : P.a) + c;
     uint32_t* __restrict__ dst = (isb ? P.wb : P.wa) + (size_t)pi * (size_t)P.wN + c;
     const uint32_t p = c_w[SET].p[pi];
     const Tw* tab = (const Tw*)P.wtf + (((size_t)pi * ODD) << P.wL);
@@ -567,13 +574,13 @@ __global__ void __launch_bounds__(WT, 4) k_wblock(const __grid_constant__ WArgs 
 // what is read.)  Bound by the stores; walking every tile, 32 limbs at a time, and
 // looking down 32 tiles at a time took 4096-limb all-ones squares 58 us per call,
 // 65536 210 and 2^22 1175, now 17, 39 and 673 (uniform limbs 15, 22, 640).
-__device__ __forceinline__ void carry_fix(const DProd& P, int64_t k, uint32_t a, bool carry) {
+__device__ __forceinline__ void carry_fix(uint64_t* r, int64_t tl, int64_t rn, int64_t k, uint32_t a, bool carry) {
     const int lane = (int)threadIdx.x & 31;
     const int64_t kw = k - lane;
     const bool ones = carry && (a & 2u);
     bool walk = false;
     if (carry && !ones) {
-        uint64_t* w = P.r + k * P.tl;
+        uint64_t* w = r + k * tl;
         const uint64_t v = __ldcg(w);
         if (v != ~0ULL) *w = v + 1;
         else walk = true;
@@ -581,24 +588,24 @@ __device__ __forceinline__ void carry_fix(const DProd& P, int64_t k, uint32_t a,
     for (unsigned m = __ballot_sync(0xffffffffu, ones); m;) {
         const int s = __ffs(m) - 1, up = __ffs(~(m >> s));
         const int len = up ? up - 1 : 32;  // tiles s .. s + len - 1
-        const int64_t b1 = (kw + s + len) * P.tl;
-        for (int64_t w = (kw + s) * P.tl + lane; w < b1; w += 32) P.r[w] = 0;
+        const int64_t b1 = (kw + s + len) * tl;
+        for (int64_t w = (kw + s) * tl + lane; w < b1; w += 32) r[w] = 0;
         m &= len == 32 ? 0u : ~(((1u << len) - 1) << s);
     }
     for (unsigned m = __ballot_sync(0xffffffffu, walk); m; m &= m - 1) {
-        const int64_t b0 = (kw + __ffs(m) - 1) * P.tl, b1 = min(b0 + (int64_t)P.tl, P.rn);
+        const int64_t b0 = (kw + __ffs(m) - 1) * tl, b1 = min(b0 + (int64_t)tl, rn);
         bool end = false;
         for (int64_t w = b0 + lane; !end && w - lane < b1; w += 128) {
             uint64_t v[4];
 #pragma unroll
-            for (int q = 0; q < 4; q++) v[q] = w + 32 * q < b1 ? __ldcg(P.r + w + 32 * q) : 0ULL;  // past the tile: ends the run
+            for (int q = 0; q < 4; q++) v[q] = w + 32 * q < b1 ? __ldcg(r + w + 32 * q) : 0ULL;  // past the tile: ends the run
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 if (end) break;
                 const unsigned stop = __ballot_sync(0xffffffffu, v[q] != ~0ULL);
                 const int e = stop ? __ffs(stop) - 1 : 32;
-                if (lane < e) P.r[w + 32 * q] = 0;
-                else if (lane == e && w + 32 * q < b1) P.r[w + 32 * q] = v[q] + 1;
+                if (lane < e) r[w + 32 * q] = 0;
+                else if (lane == e && w + 32 * q < b1) r[w + 32 * q] = v[q] + 1;
                 end = stop != 0;
             }
         }
@@ -608,14 +615,16 @@ __device__ __forceinline__ void carry_fix(const DProd& P, int64_t k, uint32_t a,
 // Every carry of a product of few tiles, by one CTA.
 template <int NT>
 __device__ __forceinline__ void carry_all(const DProd& P, uint32_t* wagg) {
+    uint64_t* const r = from_here(P.r);
+    const uint32_t* const agg = from_here(P.agg);
     uint32_t cin = 0;
     for (int64_t k0 = 0; k0 < P.ntl; k0 += NT) {
         const int64_t k = k0 + (int)threadIdx.x;
-        const uint32_t a = k < P.ntl ? __ldcg(P.agg + k) : 0u;
+        const uint32_t a = k < P.ntl ? __ldcg(agg + k) : 0u;
         __syncthreads();  // wagg's previous readers
         uint32_t total;
         const uint32_t st = cta_state(a, wagg, total);
-        carry_fix(P, k, a, k < P.ntl && (gp_join(cin, st) & 1u));
+        carry_fix(r, P.tl, P.rn, k, a, k < P.ntl && (gp_join(cin, st) & 1u));
         cin = gp_join(cin, total) & 1u;
     }
 }
@@ -623,10 +632,10 @@ __device__ __forceinline__ void carry_all(const DProd& P, uint32_t* wagg) {
 // The carry into tile k0: of the last lower tile that does not propagate, almost
 // always among the 32 before, which every warp looks at; past those the CTA
 // goes down 16 tiles per thread at a time.
-__device__ __forceinline__ uint32_t carry_below(const DProd& P, int64_t k0, uint32_t* found) {
+__device__ __forceinline__ uint32_t carry_below(const uint32_t* agg, int64_t k0, uint32_t* found) {
     const int lane = (int)threadIdx.x & 31;
     {
-        const uint32_t a = k0 > lane ? __ldcg(P.agg + (k0 - 1 - lane)) : 0u;
+        const uint32_t a = k0 > lane ? __ldcg(agg + (k0 - 1 - lane)) : 0u;
         const unsigned stop = __ballot_sync(0xffffffffu, !(a & 2u));
         if (stop) return __shfl_sync(0xffffffffu, a, __ffs(stop) - 1) & 1u;
     }
@@ -635,7 +644,7 @@ __device__ __forceinline__ uint32_t carry_below(const DProd& P, int64_t k0, uint
 #pragma unroll
         for (int j = 0; j < 16; j++) {
             const int64_t i = top - (j * WT + (int)threadIdx.x);
-            const uint32_t a = i >= 0 ? __ldcg(P.agg + i) : 2u;
+            const uint32_t a = i >= 0 ? __ldcg(agg + i) : 2u;
             if (!(a & 2u)) best = max(best, ((uint32_t)i << 1 | (a & 1u)) + 1u);
         }
         best = __reduce_max_sync(0xffffffffu, best);
@@ -696,7 +705,7 @@ __global__ void __launch_bounds__(WTail<ODD, LJ, SET>::NT, 1024 / WTail<ODD, LJ,
     for (int q = tid; q < NP * (T::CW + 3); q += T::NT) {
         const int pi = q / (T::CW + 3), cc = q - pi * (T::CW + 3) - 3;
         const bool up = c0 + cc < 0;  // left of column 0: the ends of the rows above
-        const uint32_t* src = P.wa + (size_t)pi * (size_t)N + (c0 + cc + (up ? cols : 0));
+        const uint32_t* src = from_here(P.wa) + (size_t)pi * (size_t)N + (c0 + cc + (up ? cols : 0));
         const uint32_t p = c_w[SET].p[pi];
         uint32_t x[R];
 #pragma unroll
@@ -817,7 +826,7 @@ __global__ void __launch_bounds__(WTail<ODD, LJ, SET>::NT, 1024 / WTail<ODD, LJ,
     }
     __syncthreads();
     __shared__ uint32_t wagg[T::NT / 32];
-    if (last && __ldcg(P.agg + P.ntl + 1) != 0) carry_all<T::NT>(P, wagg);
+    if (last && __ldcg(from_here(P.agg) + P.ntl + 1) != 0) carry_all<T::NT>(P, wagg);
 }
 
 __global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) {
@@ -826,10 +835,12 @@ __global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) 
     wait_previous();
     __shared__ uint32_t wagg[WT / 32], found;
     const int64_t k0 = (int64_t)local * WT, k = k0 + (int)threadIdx.x;  // a tile per thread
-    const uint32_t a = k < P.ntl ? __ldcg(P.agg + k) : 0u;
+    uint64_t* const r = from_here(P.r);
+    const uint32_t* const agg = from_here(P.agg);
+    const uint32_t a = k < P.ntl ? __ldcg(agg + k) : 0u;
     uint32_t total;
-    const uint32_t cin = carry_below(P, k0, &found), st = cta_state(a, wagg, total);
-    carry_fix(P, k, a, k < P.ntl && (gp_join(cin, st) & 1u));
+    const uint32_t cin = carry_below(agg, k0, &found), st = cta_state(a, wagg, total);
+    carry_fix(r, P.tl, P.rn, k, a, k < P.ntl && (gp_join(cin, st) & 1u));
 }
 
 // ---------------------------------------------------------------------------
@@ -851,9 +862,11 @@ __global__ void __launch_bounds__(WSmall<ODD, LM>::NT, WSmall<ODD, LM>::NT > 320
     const SmallThread<ODD, LM> th(sm, P.wtf, P.wti, P.wL);
     wait_previous();
     uint32_t x[32];  // a's 16 values, then b's
-    const uint64_t *pa = P.a, *pb = P.b;
-    th.load(x, th.sp, (int)P.nca, [&](int i) { return __ldcg(pa + i); });
-    if (!P.sqr) th.load(x + 16, th.sp + W::OPW, (int)P.ncb, [&](int i) { return __ldcg(pb + i); });
+    // in L1 for the other primes' threads (from pinned host memory, 700 x 630 limbs
+    // 36 us per call, by __ldcg 38; plain loads are not moved up: 43)
+    const uint64_t *pa = from_here(P.a), *pb = from_here(P.b);
+    th.load(x, th.sp, (int)P.nca, [&](int i) { return __ldca(pa + i); });
+    if (!P.sqr) th.load(x + 16, th.sp + W::OPW, (int)P.ncb, [&](int i) { return __ldca(pb + i); });
     if (ODD > 1) {
         __syncthreads();
         th.fetch(x, 0);

@@ -185,16 +185,17 @@ def _in_flight(stream, *buffers) -> None:
     torch = sys.modules.get("torch")
     if torch is None:
         return
-    st = stream if hasattr(stream, "cuda_stream") else None
+    tensor, st = torch.Tensor, None
     for x in buffers:
-        if isinstance(x, torch.Tensor) and x.is_cuda:
+        if isinstance(x, tensor) and x.is_cuda:
             if st is None:
-                if stream:
-                    st = torch.cuda.ExternalStream(_stream(stream))
-                else:
-                    st = _default_streams.get(x.device)
+                if not stream:
+                    dev = x.get_device()
+                    st = _default_streams.get(dev)
                     if st is None:
-                        st = _default_streams[x.device] = torch.cuda.default_stream(x.device)
+                        st = _default_streams[dev] = torch.cuda.default_stream(dev)
+                else:
+                    st = stream if hasattr(stream, "cuda_stream") else torch.cuda.ExternalStream(_stream(stream))
             x.record_stream(st)
 
 

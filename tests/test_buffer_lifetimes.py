@@ -22,7 +22,8 @@ class DeviceTensor(torch.Tensor):
         return x
 
     is_cuda = property(lambda self: True)
-    device = property(lambda self: torch.device("cuda:0"))
+    def get_device(self):
+        return 0
 
     def record_stream(self, s):
         self.recorded.append(s)
