@@ -82,7 +82,7 @@ cudaError_t launch_word(int kind, int variant, const DProd* prods, const WSeg* s
                         int64_t nctas, cudaStream_t st);
 // The same for one product passed by value (no device tables).
 cudaError_t launch_word_one(int kind, int variant, const DProd& P, int64_t nctas, cudaStream_t st);
-// CTAs one product needs in a word launch (ntl: its limb tiles).
+// CTAs one product needs in a word launch (ntl: its limb tiles; of the FP64 passes where s is empty).
 int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t ntl);
 
 // Tables of one `odd` for heap sizes up to 2^L: per prime and block, fwd then inverse.

@@ -829,18 +829,25 @@ __global__ void __launch_bounds__(WTail<ODD, LJ, SET>::NT, 1024 / WTail<ODD, LJ,
     if (last && __ldcg(from_here(P.agg) + P.ntl + 1) != 0) carry_all<T::NT>(P, wagg);
 }
 
+// Tiles of a warp of k_wcarry: one per lane, but 2048 limbs of the FP64 passes' long
+// tiles, so that many warps zero a run of them (600,000-limb all-ones square there,
+// replayed: 130 us with 32 tiles each, 101 so).
+__host__ __device__ constexpr int carry_per_warp(int tl) { return tl > 128 ? 2048 / tl : 32; }
+
 __global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) {
     int local;
     const DProd& P = wjob(A, local);
     wait_previous();
     __shared__ uint32_t wagg[WT / 32], found;
-    const int64_t k0 = (int64_t)local * WT, k = k0 + (int)threadIdx.x;  // a tile per thread
+    const int per = carry_per_warp((int)P.tl), lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5;
+    const int64_t k0 = (int64_t)local * (WT / 32 * per), k = k0 + wid * per + lane;  // a lane's tile
+    const bool in = lane < per && k < P.ntl;
     uint64_t* const r = from_here(P.r);
     const uint32_t* const agg = from_here(P.agg);
-    const uint32_t a = k < P.ntl ? __ldcg(agg + k) : 0u;
+    const uint32_t a = in ? __ldcg(agg + k) : 2u;  // others pass a carry on
     uint32_t total;
     const uint32_t cin = carry_below(agg, k0, &found), st = cta_state(a, wagg, total);
-    carry_fix(r, P.tl, P.rn, k, a, k < P.ntl && (gp_join(cin, st) & 1u));
+    carry_fix(r, P.tl, P.rn, k, a, in && (gp_join(cin, st) & 1u));
 }
 
 // ---------------------------------------------------------------------------
@@ -905,7 +912,10 @@ int64_t word_ctas(int kind, const WordShape& s, int sqr, int64_t ntl) {
         case JK_WMID_REV: return (np * mthreads + WT - 1) / WT;
         case JK_WBLOCK: return (np * R * (M / 16) + WT - 1) / WT;
         case JK_WSMALL: return 1;
-        case JK_WCARRY: return (ntl + WT - 1) / WT;  // 8 warps of 32 tiles
+        case JK_WCARRY: {
+            const int64_t per = WT / 32 * carry_per_warp(s.N ? word_run(R1) : UNPACK_TL);
+            return (ntl + per - 1) / per;
+        }
         default: return cols / word_run(R1);  // JK_WTAIL
     }
 }
