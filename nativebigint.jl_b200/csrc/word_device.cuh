@@ -363,29 +363,32 @@ __device__ __forceinline__ uint32_t gp_join(uint32_t lower, uint32_t upper) {
     return ((upper & 1u) | ((upper >> 1) & lower & 1u)) | (upper & lower & 2u);
 }
 
-// Carry-lookahead over the threads, then over the warps: the state of the parts
-// below this thread's, and the whole run's.
+// Carry-lookahead over a warp: the state of the parts up to this lane's.
+__device__ __forceinline__ uint32_t warp_scan(uint32_t agg) {
+    const int lane = (int)threadIdx.x & 31;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xffffffffu, agg, off);
+        if (lane >= off) agg = gp_join(o, agg);
+    }
+    return agg;
+}
+// The state of the parts below this lane's, from that up to it.
+__device__ __forceinline__ uint32_t warp_below(uint32_t incl) {
+    const uint32_t o = __shfl_up_sync(0xffffffffu, incl, 1);
+    return ((int)threadIdx.x & 31) ? o : 2u;
+}
+// The same over the threads, then over the warps: the state of the parts below this
+// thread's, and the whole run's.
 __device__ __forceinline__ uint32_t cta_state(uint32_t agg, uint32_t* wagg, uint32_t& total) {
     const int lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
-    uint32_t incl = agg;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t o = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl = gp_join(o, incl);
-    }
+    const uint32_t incl = warp_scan(agg);
     if (lane == 31) wagg[wid] = incl;
     __syncthreads();
-    uint32_t w = lane < nw ? wagg[lane] : 2u;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t o = __shfl_up_sync(0xffffffffu, w, off);
-        if (lane >= off) w = gp_join(o, w);
-    }
+    const uint32_t w = warp_scan(lane < nw ? wagg[lane] : 2u);
     total = __shfl_sync(0xffffffffu, w, nw - 1);
     const uint32_t below = __shfl_sync(0xffffffffu, w, wid ? wid - 1 : 0);
-    uint32_t excl = __shfl_up_sync(0xffffffffu, incl, 1);
-    if (lane == 0) excl = 2u;
-    return gp_join(wid ? below : 2u, excl);
+    return gp_join(wid ? below : 2u, warp_below(incl));
 }
 // The carry into this thread's part for a carry of 0 into the CTA's run.
 __device__ __forceinline__ uint32_t cta_scan(uint32_t agg, uint32_t* wagg, uint32_t& total) {

@@ -834,17 +834,25 @@ __global__ void __launch_bounds__(WTail<ODD, LJ, SET>::NT, 1024 / WTail<ODD, LJ,
 // replayed: 130 us with 32 tiles each, 101 so).
 __host__ __device__ constexpr int carry_per_warp(int tl) { return tl > 128 ? 2048 / tl : 32; }
 
-__global__ void __launch_bounds__(WT) k_wcarry(const __grid_constant__ WArgs A) {
+// (Registers for eight CTAs per SM: a batch has a short one per product.)
+__global__ void __launch_bounds__(WT, 8) k_wcarry(const __grid_constant__ WArgs A) {
     int local;
     const DProd& P = wjob(A, local);
     wait_previous();
     __shared__ uint32_t wagg[WT / 32], found;
     const int per = carry_per_warp((int)P.tl), lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5;
+    const bool few = P.ntl <= per;  // most products of a batch: one warp has all tiles
+    if (few && wid) return;
     const int64_t k0 = (int64_t)local * (WT / 32 * per), k = k0 + wid * per + lane;  // a lane's tile
     const bool in = lane < per && k < P.ntl;
     uint64_t* const r = from_here(P.r);
     const uint32_t* const agg = from_here(P.agg);
     const uint32_t a = in ? __ldcg(agg + k) : 2u;  // others pass a carry on
+    if (few) {
+        const uint32_t below = warp_below(warp_scan(a));
+        carry_fix(r, P.tl, P.rn, k, a, in && (below & 1u));
+        return;
+    }
     uint32_t total;
     const uint32_t cin = carry_below(agg, k0, &found), st = cta_state(a, wagg, total);
     carry_fix(r, P.tl, P.rn, k, a, in && (gp_join(cin, st) & 1u));
