@@ -293,7 +293,8 @@ int nbg_plan_layout(int64_t N, int32_t sqr, int64_t *stages, int32_t *nst, int64
  * giving an explicit pass split per transform class).  Changing them drops
  * cached plans.  The knobs describe the FP64 passes.  While they are the ones
  * the library started with or loaded from a tuning file, products within its
- * range run through transforms over 30-bit primes instead, which have no knobs;
+ * range run through transforms over 30-bit primes instead, which have no knobs
+ * (and, when memory is short for those, on the passes);
  * with other knobs every product runs the FP64 passes they describe.  The
  * results are the same integers. */
 int nbg_set_tuning(const char *json);
