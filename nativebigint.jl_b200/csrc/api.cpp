@@ -240,11 +240,12 @@ bool all_set(const std::vector<char>& v) {
 // 4864 54/55/108, 16000 75/75/135, 32000 113/112/160, 64000 210/182/240, 100000
 // 300/250/342, 262000 695/540/670 (staged by the copy threads: 100000 550, as
 // waking them takes 200).
-int host_one(const ProdIn& q, const WordShape& ws) {
+// keep: limbs of the result that the caller takes.
+int host_one(const ProdIn& q, const WordShape& ws, int64_t keep) {
     Engine& E = g_eng;
     cudaStream_t st = E.stream;
-    const size_t na = 8 * (size_t)q.m, nb = q.sqr ? 0 : 8 * (size_t)q.n, nr = 8 * (size_t)(q.m + q.n);
-    const size_t ob = align_up(na, 256), in_bytes = align_up(ob + nb, 256), out_bytes = align_up(nr, 256);
+    const size_t na = 8 * (size_t)q.m, nb = q.sqr ? 0 : 8 * (size_t)q.n, nr = 8 * (size_t)keep;
+    const size_t ob = align_up(na, 256), in_bytes = align_up(ob + nb, 256), out_bytes = align_up(8 * (size_t)(q.m + q.n), 256);
     const bool staged = na + nb < ONE_STAGE_BYTES;
     int rc;
     if (staged && (rc = ensure_pinned(E.pg_in[0], E.pg_in_bytes[0], in_bytes))) return rc;
@@ -313,13 +314,16 @@ void scatter_out(PendingOut& po, const char* staged) {
     po.any = false;
 }
 
+bool takes_host_one(const Engine& E, const ProdIn& q, WordShape& ws) {
+    return q.bits_a > 0 && q.bits_b > 0 && word_product(E, q, &ws) && 8 * (size_t)(2 * (q.m + q.n)) < STAGE_MIN_BYTES;
+}
+
 int host_chunks(Engine& E, const std::vector<ProdIn>& in) {
     const int64_t count = (int64_t)in.size();
     WordShape ws;
-    if (count == 1 && in[0].bits_a > 0 && in[0].bits_b > 0 && word_product(E, in[0], &ws) &&
-        8 * (size_t)(2 * (in[0].m + in[0].n)) < STAGE_MIN_BYTES) {
+    if (count == 1 && takes_host_one(E, in[0], ws)) {
         // (the pipeline allocates just what the product needs, and no pinned buffers at this size)
-        const int rc1 = host_one(in[0], ws);
+        const int rc1 = host_one(in[0], ws, in[0].m + in[0].n);
         if (rc1 != NBG_ENOMEM) return rc1;
     }
     // chunks of ~CHUNK_BYTES operands, in input order
@@ -822,12 +826,22 @@ static int low_product(uint64_t* r, const uint64_t* a, int64_t la, const uint64_
     if (!r || !a || la < 1 || k < 1 || (b && lb < 1)) return fail(NBG_EINVAL, "bad argument");
     la = std::min(la, k);
     lb = b ? std::min(lb, k) : la;
-    std::vector<uint64_t> full((size_t)(la + lb));
-    nbg_desc d{full.data(), a, b, la, lb, 0, 0};
-    int rc = host_batch(&d, 1);
-    if (rc) return rc;
     const int64_t keep = std::min(k, la + lb);
-    memcpy(r, full.data(), sizeof(uint64_t) * (size_t)keep);
+    Engine& E = g_eng;
+    int rc = E.ensure();
+    if (rc) return rc;
+    // a product of one call's size: its low limbs straight to r
+    const bool sqr = !b || (b == a && lb == la);
+    ProdIn q{a, sqr ? a : b, r, la, lb, magnitude_bits(a, la), 0, sqr ? 1 : 0};
+    q.bits_b = sqr ? q.bits_a : magnitude_bits(b, lb);
+    WordShape ws;
+    rc = takes_host_one(E, q, ws) ? host_one(q, ws, keep) : (int)NBG_ENOMEM;
+    if (rc == NBG_ENOMEM) {
+        std::vector<uint64_t> full((size_t)(la + lb));
+        nbg_desc d{full.data(), a, b, la, lb, 0, 0};
+        if ((rc = host_batch(&d, 1)) == NBG_OK) memcpy(r, full.data(), sizeof(uint64_t) * (size_t)keep);
+    }
+    if (rc) return rc;
     if (keep < k) memset(r + keep, 0, sizeof(uint64_t) * (size_t)(k - keep));
     return NBG_OK;
 }

@@ -143,3 +143,20 @@ def test_carry_runs_are_not_the_products_cost(gpu_lib, n):
             best = min(best, e0.elapsed_time(e1))
         times.append(best)
     assert times[1] < 4 * times[0]
+
+
+@pytest.mark.parametrize("la,lb,k", [(100, 80, 60), (100, 80, 300), (900, 900, 900), (5000, 4000, 4500), (20_000, 30_000, 20_000),
+                                     (60_000, 60_000, 60_000), (60_000, 50_000, 200_000), (600_000, 500_000, 550_000)])
+def test_low_products(gpu_lib, la, lb, k):
+    # one-CTA, staged, driver-copied and pipelined products, above and below
+    # the full product's length
+    rng = np.random.default_rng(la + k)
+    a, b = rand_limbs(rng, la), rand_limbs(rng, lb)
+
+    def low(full):
+        out = np.zeros(k, dtype=np.uint64)
+        out[: min(k, full.size)] = full[:k]
+        return out
+
+    assert np.array_equal(gpu_lib.mullo(a, b, k), low(O.gmp_mul(a, b)))
+    assert np.array_equal(gpu_lib.sqrlo(a, k), low(O.gmp_sqr(a)))

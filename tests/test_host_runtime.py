@@ -8,7 +8,7 @@ import subprocess
 import pytest
 
 from conftest import ROOT
-from nbgpu import NBG_ECUDA, NBG_ENOMEM, NBG_OK, NbgDesc, ServerOpts
+from nbgpu import NBG_ECUDA, NBG_EINVAL, NBG_ENOMEM, NBG_OK, NbgDesc, ServerOpts
 
 SRC = os.path.join(ROOT, "nativebigint.jl_b200", "csrc")
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
@@ -197,3 +197,22 @@ def test_batches_take_few_lengths_while_launches_weigh_more(fake, count, limbs, 
     d = descs(*((R + (k << 24), A, B, limbs, limbs, 64 * limbs, 64 * limbs) for k in range(count)))
     assert fake.nbg_batch_create(*d[:2], ctypes.byref(bt)) == NBG_OK
     assert fake.fake_coarse() == coarse
+
+
+@pytest.mark.parametrize("la,lb,k", [(20_000, 20_000, 20_000), (60_000, 3000, 40_000), (100_000, 90_000, 250_000)])
+def test_low_product_copies_what_it_keeps(fake, la, lb, k):
+    # straight to the caller's limbs; through a full product in a fresh buffer
+    # 60,000 limbs took 320 us, 250 before the driver made that copy
+    r, a, b = ((ctypes.c_uint64 * n)(*([7] * n)) for n in (k, la, lb))
+    fake.nbg_mullo.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64,
+                               ctypes.c_int64]
+    fake.fake_copied.argtypes = [ctypes.c_void_p, ctypes.c_int]
+    p = (ctypes.c_void_p * 1)(ctypes.addressof(r))
+    fake.fake_copied(p, 1)
+    assert fake.nbg_mullo(ctypes.addressof(r), ctypes.addressof(a), la, ctypes.addressof(b), lb, k) == NBG_OK
+    assert fake.fake_copied(p, 1) == 1
+    full = min(la, k) + min(lb, k)
+    assert not any(r[full:])  # limbs above the product
+    # a zero operand is refused as before
+    z = (ctypes.c_uint64 * 1)()
+    assert fake.nbg_mullo(ctypes.addressof(r), ctypes.addressof(a), la, ctypes.addressof(z), 1, k) == NBG_EINVAL
